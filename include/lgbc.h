@@ -131,9 +131,10 @@ int lgbc_betweenness_dev(lgbc_graph *g, const int32_t *src, int64_t nsrc,
  * entries starting at 0) and colidx[col_off[i] ..] (local ids).  bc_raw_out
  * receives the graphs' raw vectors concatenated in input order (sum n[i]
  * doubles); the caller rescales each with _rescale!(bc_i, n[i], ...).
- * Graphs are grouped by size into disjoint unions; one 64-lane batch seeds
- * source index b*64 + l of every graph of a group in lane l, so each level
- * launch covers every graph of the group. */
+ * Graphs that fit the per-source kernel (see lgbc_tuning) run one thread
+ * block per source.  The others are grouped by size into disjoint unions; one
+ * batch seeds source index b*L + l of every graph of a group in lane l, so
+ * each level launch covers every graph of the group. */
 int lgbc_betweenness_many(int64_t ngraphs, const int64_t *n, const int64_t *rowptr_off,
                           const int64_t *col_off, const int64_t *rowptr, const int32_t *colidx,
                           int endpoints, double *bc_raw_out);
@@ -160,7 +161,12 @@ typedef struct lgbc_stats {
 } lgbc_stats;
 int lgbc_graph_stats(const lgbc_graph *g, lgbc_stats *out);
 
-/* Tunables (the autotuner writes these; defaults are used otherwise).
+/* Tunables (the autotuner writes these; defaults are used otherwise).  They
+ * shape the bit-lane batches.  With every field at its default, betweenness
+ * of a graph whose vertex state fits one SM's shared memory (about 22,700
+ * vertices, at most 2^20 stored entries) runs one thread block per source
+ * instead, unless a search is deeper than 126 levels or a path count reaches
+ * 2^48; lgbc_stats.batches then counts the blocks' shares of the sources.
  *   alpha, beta   direction switch: go bottom-up when the frontier's edges
  *                 exceed (unvisited edges)/alpha; return top-down when the
  *                 frontier has fewer than n/beta vertices.

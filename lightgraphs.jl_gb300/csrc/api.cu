@@ -967,10 +967,12 @@ int run_stacked(lgbc_graph* g, int64_t copies, double* bc_dev, const std::vector
   return check_launch(g);
 }
 
-// Host-side part shared by the betweenness entry points: validate, filter
-// degree-0 sources (betweenness.jl:58), order and upload the active list.
-int prepare_sources(lgbc_graph* g, const int32_t* src, int64_t nsrc, int64_t* k_act) {
-  std::vector<int32_t> active;
+// Host-side part shared by the source-list entry points: validate and drop
+// degree-0 sources (betweenness.jl:58).
+int filter_sources(lgbc_graph* g, const int32_t* src, int64_t nsrc) {
+  std::vector<int32_t>& active = g->h_active;
+  active.clear();
+  g->h_weights.clear();
   if (!src) {
     active.reserve(static_cast<size_t>(g->n));
     for (int64_t v = 0; v < g->n; ++v)
@@ -981,17 +983,137 @@ int prepare_sources(lgbc_graph* g, const int32_t* src, int64_t nsrc, int64_t* k_
     for (int64_t i = 0; i < nsrc; ++i)
       if (g->has_degree[static_cast<size_t>(src[i])]) active.push_back(src[i]);
   }
-  LGBC_TRY(order_active(g, active, nullptr));
-  *k_act = static_cast<int64_t>(active.size());
-  g->h_active = active;
-  g->h_weights.clear();
-  LGBC_TRY(ensure_src(g, *k_act));
-  if (*k_act > 0)
-    LGBC_CUDA(cudaMemcpyAsync(g->d_src, active.data(), active.size() * sizeof(int32_t),
-                              cudaMemcpyHostToDevice, g->stream));
-  // the pageable source vector must outlive the copy
-  LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  g->stats.active_sources = static_cast<int64_t>(active.size());
   return LGBC_OK;
+}
+
+// g->h_active to g->d_src (a pageable copy: staged before the call returns).
+int upload_sources(lgbc_graph* g) {
+  const int64_t k = static_cast<int64_t>(g->h_active.size());
+  LGBC_TRY(ensure_src(g, k));
+  if (k > 0)
+    LGBC_CUDA(cudaMemcpyAsync(g->d_src, g->h_active.data(), static_cast<size_t>(k) * sizeof(int32_t),
+                              cudaMemcpyHostToDevice, g->stream));
+  return LGBC_OK;
+}
+
+int order_sources(lgbc_graph* g) {
+  LGBC_TRY(order_active(g, g->h_active, g->h_weights.empty() ? nullptr : &g->h_weights));
+  return upload_sources(g);
+}
+
+bool same_tuning(const lgbc_tuning& a, const lgbc_tuning& b) {
+  return a.alpha == b.alpha && a.beta == b.beta && a.hub_degree == b.hub_degree && a.lanes == b.lanes &&
+         a.dense_edges == b.dense_edges && a.segment_degree == b.segment_degree &&
+         a.source_order == b.source_order && a.graph_loop == b.graph_loop &&
+         a.stack_vertices == b.stack_vertices && a.hub_order == b.hub_order &&
+         a.dependency_df32 == b.dependency_df32;
+}
+
+// Whether the per-source kernel takes this handle's betweenness calls.  The
+// vertex state of one source must fit an SM's shared memory and a row's
+// length must not exceed n (the plan's bins).  A handle whose tuning was
+// changed asks for batches of that shape and keeps them.
+bool small_applies(const lgbc_graph* g) {
+  return g->n > 0 && g->n <= g->small_max_n && g->max_out <= g->n && g->nnz <= kSmallMaxNnz && !g->small.refused &&
+         same_tuning(g->tune, kDefaultTuning);
+}
+
+int ensure_small(lgbc_graph* g) {
+  SmallWorkspace& w = g->small;
+  if (w.built) return LGBC_OK;
+  w.release();
+  const size_t n = static_cast<size_t>(g->n);
+  w.view.n = static_cast<int>(g->n);
+  w.view.rowptr = g->d_rowptr;
+  w.view.colidx = g->d_colidx;
+  LGBC_TRY(dev_alloc(&w.view.rank, n));
+  LGBC_TRY(dev_alloc(&w.view.orig, n));
+  LGBC_TRY(dev_alloc(&w.view.row, n + 1));
+  LGBC_TRY(dev_alloc(&w.view.chunk, (n + 31) / 32));
+  LGBC_TRY(dev_alloc(&w.view.col, static_cast<size_t>(small_col_groups(g->n, g->nnz))));
+  LGBC_TRY(dev_alloc(&w.graph, 1));
+  LGBC_TRY(dev_alloc(&w.sum, 1));
+  LGBC_TRY(dev_alloc(&w.counters, 4));
+  w.view.in_rowptr = g->d_in_rowptr;
+  w.view.nwarp = w.counters;
+  w.view.nlive = w.counters + 3;
+  LGBC_CUDA(cudaMemsetAsync(w.counters, 0, 4 * sizeof(int), g->stream));
+  LGBC_CUDA(cudaMemcpyAsync(w.graph, &w.view, sizeof w.view, cudaMemcpyHostToDevice, g->stream));
+  g->launches += small_plan(g->stream, w.graph, 1, g->n);
+  LGBC_TRY(check_launch(g));
+  w.built = true;
+  return LGBC_OK;
+}
+
+// Brandes over g->d_src[0, k) by the per-source kernel; 1 when it refuses.
+int run_small(lgbc_graph* g, int64_t k, double* bc_dev, const double* d_w) {
+  LGBC_TRY(ensure_small(g));
+  SmallWorkspace& w = g->small;
+  const SmallShape sh = small_shape(g->cfg, g->n, k);
+  const int64_t items = std::min<int64_t>(k, sh.grid);
+  if (items * g->n > w.part_cap) {
+    dev_free(w.part);
+    w.part_cap = 0;
+    LGBC_TRY(dev_alloc(&w.part, static_cast<size_t>(items * g->n)));
+    w.part_cap = items * g->n;
+  }
+  if (items != w.items) {
+    const SmallSum sum{0, static_cast<int>(items), -1, 0, 0};
+    LGBC_CUDA(cudaMemcpyAsync(w.sum, &sum, sizeof sum, cudaMemcpyHostToDevice, g->stream));
+    w.items = items;
+  }
+  SmallRun run{};
+  run.graphs = w.graph;
+  run.nitems = static_cast<int>(items);
+  run.nsrc = static_cast<int>(k);
+  run.next = w.counters + 1;
+  run.refused = w.counters + 2;
+  run.src = g->d_src;
+  run.weight = d_w;
+  run.part = w.part;
+  LGBC_CUDA(cudaMemsetAsync(w.counters + 1, 0, 2 * sizeof(int), g->stream));
+  g->launches += small_brandes(g->stream, sh, run, g->n);
+  g->launches += small_sums(g->stream, w.graph, w.sum, 1, g->n, w.part, bc_dev);
+  LGBC_TRY(check_launch(g));
+  int* refused = reinterpret_cast<int*>(g->h_ctl);
+  LGBC_CUDA(cudaMemcpyAsync(refused, w.counters + 2, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+  LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  if (*refused) {
+    w.refused = true;
+    return 1;
+  }
+  g->stats.batches += items;
+  return LGBC_OK;
+}
+
+int accumulate_active(lgbc_graph* g, int endpoints, double* bc_dev) {
+  const int64_t k = static_cast<int64_t>(g->h_active.size());
+  double* d_w = nullptr;
+  std::unique_ptr<double, void (*)(double*)> guard(nullptr, [](double* q) { if (q) cudaFree(q); });
+  auto upload_weights = [&]() -> int {
+    if (g->h_weights.empty()) return LGBC_OK;
+    if (!d_w) {
+      LGBC_TRY(dev_alloc(&d_w, static_cast<size_t>(k)));
+      guard.reset(d_w);
+    }
+    LGBC_CUDA(cudaMemcpyAsync(d_w, g->h_weights.data(), static_cast<size_t>(k) * 8,
+                              cudaMemcpyHostToDevice, g->stream));
+    return LGBC_OK;
+  };
+  if (k > 0 && small_applies(g)) {
+    LGBC_TRY(upload_sources(g));
+    LGBC_TRY(upload_weights());
+    const int rc = run_small(g, k, bc_dev, d_w);
+    if (rc == LGBC_OK) {
+      if (endpoints) g->launches += add_endpoints(g->cfg, g->stream, bc_dev, g->n, g->d_src, k);
+      return check_launch(g);
+    }
+    if (rc != 1) return rc;
+  }
+  LGBC_TRY(order_sources(g));
+  LGBC_TRY(upload_weights());
+  return run_betweenness(g, k, endpoints, bc_dev, d_w);
 }
 
 void reset_stats(lgbc_graph* g) {
@@ -1014,6 +1136,7 @@ int init_handle(lgbc_graph* g, int64_t n, int directed) {
   g->cfg.grid = prop.multiProcessorCount * 8;
   g->max_smem = prop.sharedMemPerBlockOptin;
   bfs_configure(g->max_smem);
+  g->small_max_n = small_configure(g->max_smem);
   LGBC_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
   LGBC_CUDA(cudaEventCreate(&g->ev_start));
   LGBC_CUDA(cudaEventCreate(&g->ev_stop));
@@ -1082,10 +1205,10 @@ void degree_pass(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr)
   const int directed = g->directed;
   g->has_degree.assign(static_cast<size_t>(n), 0);
   uint8_t* has = g->has_degree.data();
-  std::vector<int64_t> max_in(8, 0);
+  std::vector<int64_t> max_in(8, 0), max_out(8, 0);
   std::vector<std::vector<std::pair<int64_t, int32_t>>> tops(8);  // max-heaps of (-degree, id)
   const int parts = parallel_parts(n, [&](int p, int64_t vb, int64_t ve) {
-    int64_t mi = 0;
+    int64_t mi = 0, mo = 0;
     auto& top = tops[static_cast<size_t>(p)];
     for (int64_t v = vb; v < ve; ++v) {
       const int64_t dout = rowptr[v + 1] - rowptr[v];
@@ -1093,6 +1216,7 @@ void degree_pass(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr)
       const int64_t d = directed ? dout + din : dout;
       has[v] = d > 0 ? 1 : 0;
       mi = std::max(mi, din);
+      mo = std::max(mo, dout);
       if (d <= 0) continue;
       if (top.size() < static_cast<size_t>(kLandmarks)) {
         top.emplace_back(-d, static_cast<int32_t>(v));
@@ -1104,8 +1228,10 @@ void degree_pass(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr)
       }
     }
     max_in[static_cast<size_t>(p)] = mi;
+    max_out[static_cast<size_t>(p)] = mo;
   });
   int64_t mi = 0;
+  g->max_out = *std::max_element(max_out.begin(), max_out.end());
   std::vector<std::pair<int64_t, int32_t>> all;
   for (int p = 0; p < parts; ++p) {
     mi = std::max(mi, max_in[static_cast<size_t>(p)]);
@@ -1185,6 +1311,7 @@ int lgbc_graph_destroy(lgbc_graph* g) {
   g->bfs.release();
   g->hubs.release();
   g->learned.release();
+  g->small.release();
   for (auto& lg : g->loops) lg.release();
   g->loops.clear();
   if (g->stack) lgbc_graph_destroy(g->stack);
@@ -1320,10 +1447,8 @@ int lgbc_betweenness_dev(lgbc_graph* g, const int32_t* src, int64_t nsrc, int en
   LGBC_TRY(use_device(g));
   if (!bc_raw_dev && g->n > 0) return fail(LGBC_EINVAL, "null output");
   reset_stats(g);
-  int64_t k_act = 0;
-  LGBC_TRY(prepare_sources(g, src, nsrc, &k_act));
-  g->stats.active_sources = k_act;
-  LGBC_TRY(run_betweenness(g, k_act, endpoints, bc_raw_dev));
+  LGBC_TRY(filter_sources(g, src, nsrc));
+  LGBC_TRY(accumulate_active(g, endpoints, bc_raw_dev));
   finish_stats(g);
   return LGBC_OK;
 }
@@ -1335,12 +1460,10 @@ int lgbc_betweenness(lgbc_graph* g, const int32_t* src, int64_t nsrc, int endpoi
   LGBC_TRY(use_device(g));
   if (!bc_raw_out && g->n > 0) return fail(LGBC_EINVAL, "null output");
   reset_stats(g);
-  int64_t k_act = 0;
-  LGBC_TRY(prepare_sources(g, src, nsrc, &k_act));
-  g->stats.active_sources = k_act;
+  LGBC_TRY(filter_sources(g, src, nsrc));
   if (g->n == 0) return LGBC_OK;
   if (!g->d_bc) LGBC_TRY(dev_alloc(&g->d_bc, static_cast<size_t>(g->n)));
-  LGBC_TRY(run_betweenness(g, k_act, endpoints, g->d_bc));
+  LGBC_TRY(accumulate_active(g, endpoints, g->d_bc));
   LGBC_CUDA(cudaMemcpyAsync(bc_raw_out, g->d_bc, static_cast<size_t>(g->n) * 8,
                             cudaMemcpyDeviceToHost, g->stream));
   LGBC_CUDA(cudaStreamSynchronize(g->stream));

@@ -206,6 +206,33 @@ struct LearnedWorkspace {
   }
 };
 
+// Plan and workspace of the per-source kernel for small graphs (small.cu).
+struct SmallWorkspace {
+  SmallGraph view{};                // host copy of *graph
+  SmallGraph* graph = nullptr;
+  SmallSum* sum = nullptr;
+  int64_t items = 0;                // parts of a call that *sum was written for
+  int* counters = nullptr;          // [0] warp-walked ids, [1] next item, [2] refused, [3] live vertices
+  ulonglong2* part = nullptr;       // partial sums, one n-vector per item
+  int64_t part_cap = 0;
+  bool built = false;
+  bool refused = false;             // too deep or counts too large: the batches take this graph
+  void release() {
+    dev_free(view.rank);
+    dev_free(view.orig);
+    dev_free(view.row);
+    dev_free(view.chunk);
+    dev_free(view.col);
+    dev_free(graph);
+    dev_free(sum);
+    items = 0;
+    dev_free(counters);
+    dev_free(part);
+    part_cap = 0;
+    built = false;
+  }
+};
+
 // A device-driven level loop instantiated for one configuration.
 struct LoopKey {
   int backward;                 // 0 forward sweep, 1 backward (dependency) sweep
@@ -262,6 +289,10 @@ struct PathExport {
 };
 }  // namespace lgbc::api
 
+namespace lgbc::api {
+constexpr lgbc_tuning kDefaultTuning{14.0, 24.0, 256, 128, 32, 0, 1, 1, 1 << 21, 2, 0};
+}
+
 struct lgbc_graph {
   int device = 0;
   int64_t n = 0;
@@ -278,6 +309,9 @@ struct lgbc_graph {
   lgbc::api::BfsWorkspace bfs;
   lgbc::api::HubTable hubs;
   lgbc::api::LearnedWorkspace learned;
+  lgbc::api::SmallWorkspace small;
+  int64_t small_max_n = 0;          // largest graph of the per-source kernel on this device
+  int64_t max_out = 0;              // largest out-list
   int32_t* d_src = nullptr;         // device copy of a call's source list
   int64_t d_src_cap = 0;
   double* d_bc = nullptr;           // device result buffer for host-buffer calls
@@ -291,7 +325,7 @@ struct lgbc_graph {
   size_t max_smem = 0;
   unsigned long long sigma_limit = ~0ull;  // (2^64 - 1) / (max in-degree + 1)
   lgbc_stats stats{};
-  lgbc_tuning tune{14.0, 24.0, 256, 128, 32, 0, 1, 1, 1 << 21, 2, 0};
+  lgbc_tuning tune = lgbc::api::kDefaultTuning;
   lgbc_graph* stack = nullptr;        // R copies of this graph (stacked batches)
   int64_t stack_copies = 0;
   std::vector<int32_t> h_active;      // the last call's ordered active sources
@@ -348,8 +382,13 @@ inline int dep_kind(const lgbc_graph* g) {
 // are scaled by d_w[i].
 int run_betweenness(lgbc_graph* g, int64_t k_act, int endpoints, double* bc_dev,
                     const double* d_w = nullptr);
-int order_active(lgbc_graph* g, std::vector<int32_t>& act, std::vector<double>* w);
-int prepare_sources(lgbc_graph* g, const int32_t* src, int64_t nsrc, int64_t* k_act);
+// Brandes over g->h_active (with g->h_weights unless empty), in the order that
+// suits the path taken, into bc_dev.
+int accumulate_active(lgbc_graph* g, int endpoints, double* bc_dev);
+// Validate and keep the sources of degree > 0 (betweenness.jl:58) in g->h_active.
+int filter_sources(lgbc_graph* g, const int32_t* src, int64_t nsrc);
+// Order g->h_active (and g->h_weights) for batches and copy the sources to g->d_src.
+int order_sources(lgbc_graph* g);
 void reset_stats(lgbc_graph* g);
 void finish_stats(lgbc_graph* g);
 int init_handle(lgbc_graph* g, int64_t n, int directed);

@@ -237,23 +237,11 @@ int lgbc_betweenness_weighted(lgbc_graph* g, const int32_t* src, const double* w
       aw.push_back(e.second);
     }
   }
-  LGBC_TRY(order_active(g, act, &aw));
-  const int64_t k_act = static_cast<int64_t>(act.size());
-  g->stats.active_sources = k_act;
-  g->h_active = act;
-  g->h_weights = aw;
-  LGBC_TRY(ensure_src(g, k_act));
-  double* d_w = nullptr;
-  LGBC_TRY(dev_alloc(&d_w, static_cast<size_t>(std::max<int64_t>(k_act, 1))));
-  std::unique_ptr<double, void (*)(double*)> guard(d_w, [](double* q) { cudaFree(q); });
-  if (k_act > 0) {
-    LGBC_CUDA(cudaMemcpyAsync(g->d_src, act.data(), static_cast<size_t>(k_act) * 4,
-                              cudaMemcpyHostToDevice, g->stream));
-    LGBC_CUDA(cudaMemcpyAsync(d_w, aw.data(), static_cast<size_t>(k_act) * 8, cudaMemcpyHostToDevice,
-                              g->stream));
-  }
+  g->stats.active_sources = static_cast<int64_t>(act.size());
+  g->h_active.swap(act);
+  g->h_weights.swap(aw);
   if (!g->d_bc) LGBC_TRY(dev_alloc(&g->d_bc, static_cast<size_t>(g->n)));
-  LGBC_TRY(run_betweenness(g, k_act, 0, g->d_bc, d_w));
+  LGBC_TRY(accumulate_active(g, 0, g->d_bc));
   LGBC_CUDA(cudaMemcpyAsync(bc_raw_out, g->d_bc, static_cast<size_t>(g->n) * 8,
                             cudaMemcpyDeviceToHost, g->stream));
   LGBC_CUDA(cudaStreamSynchronize(g->stream));

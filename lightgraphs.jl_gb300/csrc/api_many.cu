@@ -278,6 +278,227 @@ int run_groups(const std::vector<std::vector<ManyGraph>>& groups, int endpoints,
   return LGBC_OK;
 }
 
+// The graphs that fit the per-source kernel (small.cu), a chunk at a time: one
+// upload, plans on the device, one launch per size class and one download.
+// A graph whose searches are too deep or whose counts are too large is added
+// to `rest`.
+struct SmallMany {
+  int device = 0;
+  LaunchCfg cfg{};
+  int64_t max_n = 0;
+};
+
+// Size classes: a launch reserves the shared memory of its largest graph, so
+// graphs of one class run with the same number of blocks per SM, within 2.
+constexpr int64_t kSmallClasses[] = {1 << 11, 1 << 12, 1 << 13, 11000, INT64_MAX};
+
+int small_chunk(const SmallMany& dev, const std::vector<ManyGraph>& gs, int endpoints,
+                double* bc_raw_out, std::vector<ManyGraph>& rest) {
+  const int count = static_cast<int>(gs.size());
+  auto up16 = [](size_t x) { return (x + 15) & ~size_t(15); };
+  // packed CSRs on the host; plan arrays behind them on the device
+  std::vector<size_t> o_rp(gs.size()), o_ci(gs.size()), o_rank(gs.size()), o_orig(gs.size()), o_row(gs.size()),
+      o_chunk(gs.size()), o_col(gs.size());
+  size_t bytes = 0;
+  auto take = [&](size_t b) {
+    const size_t o = bytes;
+    bytes = up16(bytes + b);
+    return o;
+  };
+  int64_t total_n = 0, max_n = 0;
+  for (size_t k = 0; k < gs.size(); ++k) {
+    o_rp[k] = take(static_cast<size_t>(gs[k].n + 1) * 8);
+    o_ci[k] = take(static_cast<size_t>(gs[k].nnz) * 4);
+    total_n += gs[k].n;
+    max_n = std::max(max_n, gs[k].n);
+  }
+  const size_t host_bytes = bytes;
+  for (size_t k = 0; k < gs.size(); ++k) {
+    const size_t n = static_cast<size_t>(gs[k].n);
+    o_rank[k] = take(n * 4);
+    o_orig[k] = take(n * 4);
+    o_row[k] = take((n + 1) * 4);
+    o_chunk[k] = take((n + 31) / 32 * 4);
+    o_col[k] = take(static_cast<size_t>(small_col_groups(gs[k].n, gs[k].nnz)) * 8);
+  }
+  const size_t o_graphs = take(gs.size() * sizeof(SmallGraph));
+  const size_t o_ints = take(gs.size() * 4 * 4 + 16 * 4);  // nwarp | refused | bad | nlive | next per class
+  const size_t o_out = take(static_cast<size_t>(total_n) * 8);
+  std::vector<unsigned char> pack(host_bytes);
+  for (size_t k = 0; k < gs.size(); ++k) {
+    std::memcpy(pack.data() + o_rp[k], gs[k].rowptr, static_cast<size_t>(gs[k].n + 1) * 8);
+    if (gs[k].nnz > 0) std::memcpy(pack.data() + o_ci[k], gs[k].colidx, static_cast<size_t>(gs[k].nnz) * 4);
+  }
+  unsigned char* buf = nullptr;
+  LGBC_TRY(dev_alloc(&buf, bytes));
+  std::unique_ptr<unsigned char, cudaError_t (*)(void*)> g1(buf, cudaFree);
+  int* ints = reinterpret_cast<int*>(buf + o_ints);
+  std::vector<SmallGraph> views(gs.size());
+  for (size_t k = 0; k < gs.size(); ++k) {
+    SmallGraph& v = views[k];
+    v.n = static_cast<int>(gs[k].n);
+    v.rowptr = reinterpret_cast<int64_t*>(buf + o_rp[k]);
+    v.colidx = reinterpret_cast<int32_t*>(buf + o_ci[k]);
+    v.rank = reinterpret_cast<int32_t*>(buf + o_rank[k]);
+    v.orig = reinterpret_cast<int32_t*>(buf + o_orig[k]);
+    v.row = reinterpret_cast<uint32_t*>(buf + o_row[k]);
+    v.chunk = reinterpret_cast<uint32_t*>(buf + o_chunk[k]);
+    v.col = reinterpret_cast<uint2*>(buf + o_col[k]);
+    v.in_rowptr = v.rowptr;
+    v.nwarp = ints + k;
+    v.nlive = ints + 3 * count + k;
+  }
+  // one stream per size class, all ordered behind the first until the plans are built
+  constexpr int kClasses = static_cast<int>(sizeof kSmallClasses / sizeof kSmallClasses[0]);
+  cudaStream_t streams[kClasses] = {};
+  struct Streams {
+    cudaStream_t* s;
+    ~Streams() {
+      for (int i = 0; i < kClasses; ++i)
+        if (s[i]) {
+          cudaStreamSynchronize(s[i]);
+          cudaStreamDestroy(s[i]);
+        }
+    }
+  } streams_guard{streams};
+  for (auto& st : streams) LGBC_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  cudaStream_t s = streams[0];
+  const SmallGraph* d_graphs = reinterpret_cast<SmallGraph*>(buf + o_graphs);
+  LGBC_CUDA(cudaMemcpyAsync(buf, pack.data(), host_bytes, cudaMemcpyHostToDevice, s));
+  LGBC_CUDA(cudaMemcpyAsync(buf + o_graphs, views.data(), views.size() * sizeof(SmallGraph),
+                            cudaMemcpyHostToDevice, s));
+  LGBC_CUDA(cudaMemsetAsync(ints, 0, gs.size() * 4 * 4 + 16 * 4, s));
+  small_check(s, d_graphs, count, ints + 2 * count);
+  std::vector<int> flags(gs.size());
+  LGBC_CUDA(cudaMemcpyAsync(flags.data(), ints + 2 * count, flags.size() * 4, cudaMemcpyDeviceToHost, s));
+  LGBC_CUDA(cudaStreamSynchronize(s));
+  for (size_t k = 0; k < gs.size(); ++k) {
+    if (flags[k] & 1) return fail(LGBC_EINVAL, "rowptr must be non-decreasing");
+    if (flags[k] & 2)
+      return fail(LGBC_EINVAL, "graph " + std::to_string(gs[k].idx) + ": column index outside [0, n)");
+    if (flags[k] & 4) {  // repeated entries: the batches walk them as they are
+      for (size_t j = 0; j < gs.size(); ++j) rest.push_back(gs[j]);
+      return LGBC_OK;
+    }
+  }
+  small_plan(s, d_graphs, count, max_n);
+
+  // items of about equal cost, about eight per resident block, the largest
+  // graphs (first in gs) first; a graph's sources are the plan's first ids
+  std::vector<int64_t> active(gs.size());
+  double total = 0.0;
+  auto cost = [&](size_t k) {  // per source: every entry twice, every vertex finished once
+    return static_cast<double>(2 * gs[k].nnz + 8 * gs[k].n);
+  };
+  for (size_t k = 0; k < gs.size(); ++k) {
+    for (int64_t v = 0; v < gs[k].n; ++v) active[k] += gs[k].rowptr[v + 1] > gs[k].rowptr[v] ? 1 : 0;
+    total += cost(k) * static_cast<double>(active[k]);
+  }
+  const double share = total / (8.0 * static_cast<double>(dev.cfg.sms));
+  std::vector<SmallItem> items;
+  std::vector<SmallSum> sums;
+  std::vector<size_t> class_begin(kClasses + 1, 0);
+  std::vector<int64_t> class_n(kClasses, 0);
+  int64_t part = 0, out = 0;
+  std::vector<int64_t> out_at(gs.size());
+  for (int c = kClasses - 1; c >= 0; --c) {
+    const size_t first = items.size();
+    for (size_t k = 0; k < gs.size(); ++k) {
+      const int64_t n = gs[k].n;
+      if (n > kSmallClasses[c] || (c > 0 && n <= kSmallClasses[c - 1])) continue;
+      const double want = share > 0 ? std::ceil(cost(k) * static_cast<double>(active[k]) / share) : 1.0;
+      const int64_t parts = std::min<int64_t>(active[k], std::max<int64_t>(1, static_cast<int64_t>(want)));
+      out_at[k] = out;
+      sums.push_back(SmallSum{static_cast<int>(k), static_cast<int>(parts),
+                              endpoints ? static_cast<int>(active[k]) : -1, part, out});
+      for (int64_t i = 0; i < parts; ++i) {
+        items.push_back(SmallItem{static_cast<int>(k), static_cast<int>(active[k] * i / parts),
+                                  static_cast<int>(active[k] * (i + 1) / parts), part});
+        part += n;
+      }
+      out += n;
+      class_n[static_cast<size_t>(c)] = std::max(class_n[static_cast<size_t>(c)], n);
+    }
+    class_begin[static_cast<size_t>(c)] = first;
+  }
+  SmallItem* d_items = nullptr;
+  LGBC_TRY(dev_alloc(&d_items, items.size()));
+  std::unique_ptr<SmallItem, cudaError_t (*)(void*)> g2(d_items, cudaFree);
+  SmallSum* d_sums = nullptr;
+  LGBC_TRY(dev_alloc(&d_sums, sums.size()));
+  std::unique_ptr<SmallSum, cudaError_t (*)(void*)> g3(d_sums, cudaFree);
+  ulonglong2* d_part = nullptr;
+  LGBC_TRY(dev_alloc(&d_part, static_cast<size_t>(part)));
+  std::unique_ptr<ulonglong2, cudaError_t (*)(void*)> g4(d_part, cudaFree);
+  if (!items.empty())
+    LGBC_CUDA(cudaMemcpyAsync(d_items, items.data(), items.size() * sizeof(SmallItem), cudaMemcpyHostToDevice, s));
+  LGBC_CUDA(cudaMemcpyAsync(d_sums, sums.data(), sums.size() * sizeof(SmallSum), cudaMemcpyHostToDevice, s));
+  LGBC_CUDA(cudaStreamSynchronize(s));
+  // the largest class first: its blocks take whole SMs, the others fill in as they end
+  for (int c = kClasses - 1; c >= 0; --c) {
+    const size_t b = class_begin[static_cast<size_t>(c)];
+    const size_t e = c > 0 ? class_begin[static_cast<size_t>(c - 1)] : items.size();
+    if (e == b) continue;
+    SmallRun run{};
+    run.graphs = d_graphs;
+    run.items = d_items + b;
+    run.nitems = static_cast<int>(e - b);
+    run.next = ints + 4 * count + c;
+    run.refused = ints + count;
+    run.part = d_part;
+    small_brandes(streams[c], small_shape(dev.cfg, class_n[static_cast<size_t>(c)], run.nitems), run,
+                  class_n[static_cast<size_t>(c)]);
+  }
+  for (auto& st : streams) LGBC_CUDA(cudaStreamSynchronize(st));
+  double* d_out = reinterpret_cast<double*>(buf + o_out);
+  small_sums(s, d_graphs, d_sums, count, max_n, d_part, d_out);
+  LGBC_CUDA(cudaGetLastError());
+  std::vector<double> res(static_cast<size_t>(total_n));
+  LGBC_CUDA(cudaMemcpyAsync(res.data(), d_out, res.size() * 8, cudaMemcpyDeviceToHost, s));
+  LGBC_CUDA(cudaMemcpyAsync(flags.data(), ints + count, flags.size() * 4, cudaMemcpyDeviceToHost, s));
+  LGBC_CUDA(cudaStreamSynchronize(s));
+  for (size_t k = 0; k < gs.size(); ++k) {
+    if (flags[k])
+      rest.push_back(gs[k]);
+    else
+      std::memcpy(bc_raw_out + gs[k].out_off, res.data() + out_at[k], static_cast<size_t>(gs[k].n) * 8);
+  }
+  return LGBC_OK;
+}
+
+int run_small_many(const std::vector<ManyGraph>& gs, int endpoints, double* bc_raw_out,
+                   std::vector<ManyGraph>& rest) {
+  SmallMany dev;
+  int smem = 0;
+  LGBC_CUDA(cudaGetDevice(&dev.device));
+  LGBC_CUDA(cudaDeviceGetAttribute(&dev.cfg.sms, cudaDevAttrMultiProcessorCount, dev.device));
+  LGBC_CUDA(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev.device));
+  dev.max_n = small_configure(static_cast<size_t>(smem));
+  constexpr int64_t kChunkVertices = int64_t(1) << 23, kChunkEntries = int64_t(1) << 27;
+  constexpr size_t kChunkGraphs = 32768;  // a grid dimension
+  std::vector<ManyGraph> chunk;
+  int64_t cv = 0, ce = 0;
+  auto flush = [&]() -> int {
+    if (chunk.empty()) return LGBC_OK;
+    const int rc = small_chunk(dev, chunk, endpoints, bc_raw_out, rest);
+    chunk.clear();
+    cv = ce = 0;
+    return rc;
+  };
+  for (const ManyGraph& m : gs) {
+    if (m.n > dev.max_n || m.nnz < 0 || m.nnz > kSmallMaxNnz) {
+      rest.push_back(m);
+      continue;
+    }
+    if (m.n == 0) continue;
+    if (cv + m.n > kChunkVertices || ce + m.nnz > kChunkEntries || chunk.size() == kChunkGraphs) LGBC_TRY(flush());
+    chunk.push_back(m);
+    cv += m.n;
+    ce += m.nnz;
+  }
+  return flush();
+}
+
 }  // namespace lgbc::api
 
 extern "C" int lgbc_betweenness_many(int64_t ngraphs, const int64_t* n, const int64_t* rowptr_off,
@@ -298,16 +519,21 @@ extern "C" int lgbc_betweenness_many(int64_t ngraphs, const int64_t* n, const in
     if (gs[static_cast<size_t>(i)].nnz > 0 && !colidx) return fail(LGBC_EINVAL, "null colidx");
     out += n[i];
   }
+  std::stable_sort(gs.begin(), gs.end(), [](const ManyGraph& a, const ManyGraph& b) { return a.n > b.n; });
+  std::vector<ManyGraph> rest;
+  int rc;
+  try {
+    rc = run_small_many(gs, endpoints, bc_raw_out, rest);
+  } catch (const std::bad_alloc&) {
+    rc = fail(LGBC_ENOMEM, "host allocation failed");
+  }
+  if (rc != LGBC_OK || rest.empty()) return rc;
   // size-sorted groups of at most kGroupVertices vertices (one big graph alone)
-  std::vector<size_t> order(gs.size());
-  for (size_t i = 0; i < order.size(); ++i) order[i] = i;
-  std::stable_sort(order.begin(), order.end(),
-                   [&](size_t a, size_t b) { return gs[a].n > gs[b].n; });
+  std::stable_sort(rest.begin(), rest.end(), [](const ManyGraph& a, const ManyGraph& b) { return a.n > b.n; });
   const int64_t kGroupVertices = int64_t(1) << 21;
   std::vector<std::vector<ManyGraph>> groups(1);
   int64_t gv = 0;
-  for (size_t oi = 0; oi < order.size(); ++oi) {
-    const ManyGraph& m = gs[order[oi]];
+  for (const ManyGraph& m : rest) {
     if (!groups.back().empty() && gv + m.n > kGroupVertices) {
       groups.emplace_back();
       gv = 0;

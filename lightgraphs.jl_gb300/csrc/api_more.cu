@@ -154,9 +154,9 @@ extern "C" int lgbc_stress(lgbc_graph* g, const int32_t* src, int64_t nsrc, int6
   LGBC_TRY(use_device(g));
   if (!stress_out && g->n > 0) return fail(LGBC_EINVAL, "null output");
   reset_stats(g);
-  int64_t k_act = 0;
-  LGBC_TRY(prepare_sources(g, src, nsrc, &k_act));
-  g->stats.active_sources = k_act;
+  LGBC_TRY(filter_sources(g, src, nsrc));
+  LGBC_TRY(order_sources(g));
+  const int64_t k_act = static_cast<int64_t>(g->h_active.size());
   if (g->n == 0) return LGBC_OK;
   unsigned long long* d_st = nullptr;
   LGBC_TRY(dev_alloc(&d_st, static_cast<size_t>(g->n)));

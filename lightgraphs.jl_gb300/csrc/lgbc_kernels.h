@@ -176,6 +176,74 @@ int ms_export(const LaunchCfg& c, cudaStream_t s, const MsBuffers& b, int sigma_
 // Zero visit and both mask buffers outright (after an aborted batch).
 int ms_reset_all(cudaStream_t s, const DevGraph& g, const MsBuffers& b);
 
+// ---- Brandes on graphs that fit one SM's shared memory: small.cu ----------
+constexpr int kSmallMaxN = 32000;        // 16-bit ids with one to spare; the shared memory bounds n further
+constexpr int kSmallMaxThreads = 1024;
+constexpr int kSmallMaxLevels = 128;     // a deeper search is left to the batches
+constexpr int kSmallWarpGroups = 16;    // rows of more than 4 * this entries are walked by a warp
+constexpr int kSmallLenBits = 5;         // holds kSmallWarpGroups
+// One SM walks a source's edges alone: at 1.2M entries (20,000 vertices) a
+// single source took 529 us against 359 us as a batch, at 0.43M 264 against
+// 591 us for 16 sources and 16.3 against 17.0 ms for all 16,384.  (Well below
+// the 2^27 groups that a chunk word can place.)
+constexpr int64_t kSmallMaxNnz = int64_t(1) << 20;
+// A graph and its plan (device pointers): the vertices relabelled by
+// decreasing out-degree, their rows in groups of four 16-bit ids.
+struct SmallGraph {
+  int n;
+  const int64_t* rowptr;   // the graph's own out-CSR
+  const int32_t* colidx;
+  const int64_t* in_rowptr;  // its in-CSR's (rowptr when undirected)
+  int32_t* rank;           // n: new id of a vertex
+  int32_t* orig;           // n: and back
+  uint32_t* row;           // n + 1: first group of a row (warp-walked vertices)
+  uint32_t* chunk;         // (n + 31) / 32: first group << kSmallLenBits | row length, per 32 ids
+  uint2* col;              // small_col_groups(n, nnz) groups, padded with the id n
+  int* nwarp;              // ids below this have rows walked by a warp (zero before the plan)
+  int* nlive;              // vertices that some edge enters (likewise)
+};
+struct SmallItem {
+  int graph;               // index of its graph
+  int begin, end;          // its sources: positions in SmallRun::src, or ids of the plan
+  int64_t part;            // its n partial sums in SmallRun::part (zeroed by the kernel)
+};
+struct SmallRun {
+  const SmallGraph* graphs;
+  const SmallItem* items;  // null: nsrc sources of graph 0 in nitems equal parts
+  int nitems;
+  int nsrc;
+  int* next;               // zero: the next item
+  int* refused;            // per graph, zero: set when a source is too deep or its counts too large
+  const int32_t* src;      // sources as the graph's own ids, or null
+  const double* weight;    // weights of the sources in src, or null
+  ulonglong2* part;        // extended-format sums (xf64.cuh): significand, exponent
+};
+struct SmallShape {
+  int grid, threads;
+};
+// One graph's result: the sum of its items' partial sums, plus the endpoint
+// terms of its `active` sources (add_endpoints) when wanted.
+struct SmallSum {
+  int graph;
+  int items;
+  int active;              // -1: no endpoint terms; else its first ids in the plan are the sources
+  int64_t part;            // items x n
+  int64_t out;
+};
+size_t small_smem(int64_t n);
+int64_t small_col_groups(int64_t n, int64_t nnz);
+// Opt the kernels into the device's shared memory; the largest n they take.
+int small_configure(size_t max_dyn_smem);
+int small_plan(cudaStream_t s, const SmallGraph* graphs, int count, int64_t max_n);
+// Launch shape for `items` items of graphs of up to max_n vertices.
+SmallShape small_shape(const LaunchCfg& c, int64_t max_n, int64_t items);
+int small_brandes(cudaStream_t s, const SmallShape& sh, const SmallRun& run, int64_t max_n);
+// ORs into bad[i] for graph i: 1 = rowptr decreases, 2 = a column outside
+// [0, n), 4 = a row longer than n.
+int small_check(cudaStream_t s, const SmallGraph* graphs, int count, int* bad);
+int small_sums(cudaStream_t s, const SmallGraph* graphs, const SmallSum* sums, int count, int64_t max_n,
+               const ulonglong2* part, double* out);
+
 // ---- single multi-source BFS (gdistances): bfs.cu ------------------------
 struct BfsBuffers {
   int32_t* queue;               // n: every level, concatenated

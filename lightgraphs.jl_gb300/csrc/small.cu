@@ -1,0 +1,676 @@
+// small.cu -- Brandes betweenness of graphs whose vertex state fits in one
+// SM's shared memory: one thread block per source, no launches per level.
+//
+// The bit-lane batches of msbfs.cu keep 16 bytes of state per (vertex, source)
+// in HBM and pay a 1 KB row gather per contributing edge whatever the number
+// of lanes set in it.  Here a block keeps one source's path counts, then its
+// dependencies, in shared memory (8 bytes per vertex) and walks every edge
+// once per sweep, so the random accesses never leave the SM.  What bounds it
+// is instruction issue: 64 % of the issue slots busy with 32 warps per SM
+// (ALU pipe 52 %), the rest barriers and fixed latencies; DRAM is idle.
+// Measured (exact betweenness, batches -> here): G(10,000, 50,000) 11.7 ->
+// 4.24 ms; 24 Barabasi-Albert graphs of up to 20,000 vertices 453 -> 154 ms;
+// a 50-vertex digraph 289 -> 57 us.
+//
+// Replaces, per source, dijkstra_shortest_paths(g, s; allpaths, trackvertices)
+// with unit weights (src/shortestpaths/dijkstra.jl:59-141) and
+// _accumulate_basic! (src/centrality/betweenness.jl:81-107).  Path counts are
+// exact integers and dependencies use the arithmetic of xf64.cuh, as in the
+// batches.
+//
+// Layout.  A plan (built once per graph on the device) relabels the vertices
+// by decreasing out-degree and stores 16-bit neighbour ids in groups of four,
+// padded with the id n, whose state never takes part: a thread reads four
+// neighbours in one 8-byte load, and 32 consecutive vertices of a level have
+// rows of about the same length, so a warp can give each thread a vertex (and
+// each thread finishes its own vertex) without idling on the longest row.
+// The vertices with long rows come first, in plain rows, and are walked by
+// whole warps.  The others are cut into chunks of 32 with one row length;
+// group j of a chunk's rows is contiguous, so neighbouring vertices' loads
+// share sectors, and a row's place follows from one word per chunk, kept in
+// shared memory.  Every load of a row is issued before the previous group (or
+// vertex) is worked on: with one 1,024-thread block per SM nothing else hides
+// the latency of L2.
+//
+// State of vertex v, two words lo / hi (separate arrays: a 4-byte access uses
+// all 32 banks):
+//   0                       not reached
+//   path count, hi bit 31 = 0   being counted (the level after the frontier)
+//   path count | hi bit 31      counted; the forward sweep leaves it alone
+//   binary64 psi | hi bit 31    finished while its level is swept back
+//   binary64 psi, hi > 0        finished, its level complete
+// A vertex of level L has successors only at level L + 1, and every other
+// neighbour carries bit 31 while level L is swept, so the sign of hi decides
+// in both sweeps and no level is stored per vertex.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <type_traits>
+
+#include "lgbc_kernels.h"
+#include "xf64.cuh"
+
+namespace lgbc {
+namespace {
+
+constexpr uint32_t kClosed = 0x80000000u;
+// A count of 2^48 or more ends the attempt: below it no sum over at most
+// kSmallMaxN < 2^15 predecessors can reach bit 31 of hi.
+constexpr uint32_t kCountLimitHi = 1u << 16;
+
+// ---------------------------------------------------------------------------
+// Plan: one block per graph.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(1024) k_small_plan(const SmallGraph* graphs) {
+  extern __shared__ int hist[];  // vertices per row length (in groups), then their first rank
+  const SmallGraph G = graphs[blockIdx.x];
+  const int n = G.n;
+  const int bins = (n + 3) / 4 + 1;
+  int* first = hist;             // [bins] rank of the next vertex of the bin
+  int* start = hist + bins;      // [bins] first rank of the bin
+  int* base = hist + 2 * bins;   // [bins] first group of the bin
+  for (int b = threadIdx.x; b < bins; b += blockDim.x) first[b] = 0;
+  __syncthreads();
+  auto groups_of = [&](int v) { return static_cast<int>((G.rowptr[v + 1] - G.rowptr[v] + 3) >> 2); };
+  for (int v = threadIdx.x; v < n; v += blockDim.x) atomicAdd(&first[groups_of(v)], 1);
+  __syncthreads();
+  // longest rows first: a warp scans the bins downwards
+  if (threadIdx.x < kWarp) {
+    const int ln = lane_id();
+    int rank = 0, grp = 0;
+    for (int top = bins - 1; top >= 0; top -= kWarp) {
+      const int b = top - ln;
+      const int c = b >= 0 ? first[b] : 0;
+      int ic = c, ig = c * b;
+#pragma unroll
+      for (int o = 1; o < kWarp; o <<= 1) {
+        const int yc = __shfl_up_sync(kFull, ic, o), yg = __shfl_up_sync(kFull, ig, o);
+        if (ln >= o) {
+          ic += yc;
+          ig += yg;
+        }
+      }
+      if (b >= 0) {
+        start[b] = rank + ic - c;
+        first[b] = rank + ic - c;
+        base[b] = grp + ig - c * b;
+      }
+      rank += __shfl_sync(kFull, ic, kWarp - 1);
+      grp += __shfl_sync(kFull, ig, kWarp - 1);
+    }
+    if (ln == 0) G.row[n] = static_cast<uint32_t>(grp);
+  }
+  __syncthreads();
+  for (int v = threadIdx.x; v < n; v += blockDim.x) {
+    const int b = groups_of(v);
+    const int r = atomicAdd(&first[b], 1);
+    G.rank[v] = r;
+    G.orig[r] = v;
+    G.row[r] = static_cast<uint32_t>(base[b] + (r - start[b]) * b);
+    if (b > kSmallWarpGroups) atomicMax(G.nwarp, r + 1);
+  }
+  __syncthreads();  // also orders this block's global writes before the reads below
+  {
+    int live = 0;
+    for (int v = threadIdx.x; v < n; v += blockDim.x) live += G.in_rowptr[v + 1] > G.in_rowptr[v] ? 1 : 0;
+    live = static_cast<int>(__reduce_add_sync(kFull, static_cast<unsigned>(live)));
+    if (lane_id() == 0 && live) atomicAdd(G.nlive, live);
+  }
+  // whole chunks (past n when every row is long)
+  const int nw = (*reinterpret_cast<volatile int*>(G.nwarp) + 31) & ~31;
+  const int warps = blockDim.x >> 5, ln = lane_id();
+  // chunks of the thread-walked vertices: first group and row length (that
+  // of the chunk's first vertex, its longest)
+  if (threadIdx.x < kWarp) {
+    uint32_t at = G.row[min(nw, n)];
+    for (int c0 = nw / kWarp; c0 * kWarp < n; c0 += kWarp) {
+      const int c = c0 + ln;
+      const uint32_t len = c * kWarp < n ? G.row[c * kWarp + 1] - G.row[c * kWarp] : 0u;
+      uint32_t incl = len * kWarp;
+#pragma unroll
+      for (int o = 1; o < kWarp; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, incl, o);
+        if (ln >= o) incl += y;
+      }
+      if (c * kWarp < n) G.chunk[c] = ((at + incl - len * kWarp) << kSmallLenBits) | len;
+      at += __shfl_sync(kFull, incl, kWarp - 1);
+    }
+  }
+  __syncthreads();
+  uint16_t* col = reinterpret_cast<uint16_t*>(G.col);
+  for (int v = threadIdx.x >> 5; v < n; v += warps) {
+    const int64_t e0 = G.rowptr[v];
+    const int deg = static_cast<int>(G.rowptr[v + 1] - e0);
+    const int r = G.rank[v];
+    int64_t at = G.row[r];
+    int len = (deg + 3) >> 2, step = 1;
+    if (r >= nw) {
+      const uint32_t w = G.chunk[r >> 5];
+      at = (w >> kSmallLenBits) + (r & 31);
+      len = static_cast<int>(w & ((1u << kSmallLenBits) - 1u));
+      step = kWarp;
+    }
+    for (int i = ln; i < 4 * len; i += kWarp)
+      col[4 * (at + static_cast<int64_t>(i >> 2) * step) + (i & 3)] =
+          static_cast<uint16_t>(i < deg ? G.rank[G.colidx[e0 + i]] : n);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Sweeps
+// ---------------------------------------------------------------------------
+
+// Path count (chi : clo) of a frontier vertex to four neighbours, except those
+// that are closed.  64-bit shared atomics are compare-and-swap loops, so the
+// words are added apart.  With every count of the frontier below 2^16 no sum
+// over fewer than 2^15 predecessors passes 2^31: the adds need no answer and
+// nothing waits for them (NARROW).  Otherwise the low word's old value gives
+// the carry.
+//
+// The shared accesses are written out with predicates: as branches around
+// each of the four they cost more instructions than the adds themselves.
+__device__ __forceinline__ uint32_t lds(uint32_t at) {
+  uint32_t x;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(x) : "r"(at));
+  return x;
+}
+// Byte offsets of a group's four state words.
+__device__ __forceinline__ void offsets(uint2 c, uint32_t (&w)[4]) {
+  w[0] = (c.x << 2) & 0x3FFFCu;
+  w[1] = (c.x >> 14) & 0x3FFFCu;
+  w[2] = (c.y << 2) & 0x3FFFCu;
+  w[3] = (c.y >> 14) & 0x3FFFCu;
+}
+
+template <bool NARROW>
+__device__ __forceinline__ void push4(uint32_t lo, uint32_t hi, uint2 c, uint32_t clo, uint32_t chi) {
+  uint32_t w[4], h[4];
+  offsets(c, w);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) h[k] = lds(hi + w[k]);
+  if (NARROW) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "setp.ge.s32 p, %2, 0;\n\t"
+          "@p red.shared.add.u32 [%0], %1;\n\t}"
+          ::"r"(lo + w[k]), "r"(clo), "r"(h[k]) : "memory");
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    uint32_t old = 0u;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ge.s32 p, %3, 0;\n\t"
+        "@p atom.shared.add.u32 %0, [%1], %2;\n\t}"
+        : "+r"(old) : "r"(lo + w[k]), "r"(clo), "r"(h[k]) : "memory");
+    const uint32_t up = chi + (old > ~clo ? 1u : 0u);
+    if (static_cast<int>(h[k]) >= 0 && up)
+      asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(hi + w[k]), "r"(up) : "memory");
+  }
+}
+
+// psi of the successors among four neighbours into the sum.  Any other
+// neighbour adds a zero of exponent 0, far below every sum's (sum_zero).
+__device__ __forceinline__ void pull4(uint32_t lo, uint32_t hi, uint2 c, xg64& a) {
+  uint32_t w[4], h[4], l[4];
+  offsets(c, w);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) h[k] = lds(hi + w[k]);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    l[k] = 0u;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.gt.s32 p, %2, 0;\n\t"
+        "@p ld.shared.u32 %0, [%1];\n\t}"
+        : "+r"(l[k]) : "r"(lo + w[k]), "r"(h[k]));
+    h[k] = static_cast<uint32_t>(max(static_cast<int>(h[k]), 0));
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) xg_add_bits(a, (static_cast<uint64_t>(h[k]) << 32) | l[k]);
+}
+// An empty sum whose exponent shifts a term of exponent 0 out entirely (psi
+// is at least 2^-48, so its exponent field is above 900).
+__device__ __forceinline__ xg64 sum_zero() { return xg64{0ull, 128}; }
+__device__ __forceinline__ xf64 sum_value(xg64 a) {
+  xg_norm(a);
+  return a.m ? xg_to_xf(a) : xf_zero();
+}
+
+// One block per item (a range of sources of one graph).  Each source: count
+// paths level by level, then sweep the levels back, adding the dependencies
+// to the item's partial sums.
+__global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_brandes(SmallRun run) {
+  extern __shared__ uint32_t sm[];
+  __shared__ int lvl[2][kSmallMaxLevels + 2];  // level starts: [0] warp-walked vertices, [1] the others
+  __shared__ int s_count[kWarp];
+  __shared__ int s_item, s_stop, s_next, s_goal;
+  __shared__ int s_wide[2];                    // [L & 1]: a count of level L is 2^16 or more
+  const int tid = threadIdx.x, T = blockDim.x, ln = lane_id(), wid = tid >> 5, W = T >> 5;
+  for (;;) {
+    __syncthreads();
+    if (tid == 0) {
+      s_item = atomicAdd(run.next, 1);
+      s_stop = 0;
+      if (s_item < run.nitems)  // an earlier source's refusal covers its whole graph
+        s_stop = *reinterpret_cast<volatile int*>(run.refused + (run.items ? run.items[s_item].graph : 0));
+    }
+    __syncthreads();
+    if (s_item >= run.nitems) return;
+    SmallItem I;
+    if (run.items) {
+      I = run.items[s_item];
+    } else {
+      const long long k = run.nsrc;
+      I.graph = 0;
+      I.begin = static_cast<int>(k * s_item / run.nitems);
+      I.end = static_cast<int>(k * (s_item + 1) / run.nitems);
+      I.part = static_cast<int64_t>(s_item) * run.graphs[0].n;
+    }
+    const SmallGraph G = run.graphs[I.graph];
+    const int n = G.n;
+    uint32_t* lo = sm;
+    uint32_t* hi = sm + (n + 1);
+    const uint32_t lo_s = static_cast<uint32_t>(__cvta_generic_to_shared(lo));
+    const uint32_t hi_s = static_cast<uint32_t>(__cvta_generic_to_shared(hi));
+    uint32_t* chunk = sm + 2 * (n + 1);
+    uint16_t* q = reinterpret_cast<uint16_t*>(chunk + (n + 31) / 32);
+    const uint2* const col = G.col;
+    // warp-walked ids [0, nw): whole chunks of 32, so that a chunk's
+    // discoveries go to one list
+    const int nw = (*G.nwarp + 31) & ~31;
+    ulonglong2* part = run.part + I.part;
+    for (int i = tid; i < n; i += T) part[i] = make_ulonglong2(0ull, 0ull);
+    for (int c = nw / kWarp + tid; c * kWarp < n; c += T) chunk[c] = G.chunk[c];
+    // the row of a thread-walked vertex: its first group and their number
+    auto row_of = [&](uint32_t v, uint32_t& e, int& len) {
+      const uint32_t w = chunk[v >> 5];
+      e = (w >> kSmallLenBits) + (v & 31u);
+      len = static_cast<int>(w & ((1u << kSmallLenBits) - 1u));
+    };
+    // A warp's next 32 entries of the level's list: the lists are roughly by
+    // decreasing row length, so taking them as warps come free evens the
+    // warps out.  (i: the lane's entry; its vertex, row and first group.)
+    auto fetch = [&](int end, int& i, uint32_t& v, uint32_t& e, int& len, uint2& c) {
+      int at = 0;
+      if (ln == 0) at = atomicAdd(&s_next, kWarp);
+      i = __shfl_sync(kFull, at, 0) + ln;
+      if (i >= end) return;
+      v = q[nw + i];
+      row_of(v, e, len);
+      if (len > 0) c = col[e];
+    };
+    // Every count of a level to its successors.
+    auto push_level = [&](auto narrow, int a0, int a1, int b1) {
+      constexpr bool N = decltype(narrow)::value;
+      for (int i = a0 + wid; i < a1; i += W) {
+        const int v = q[i];
+        const uint32_t clo = lo[v], chi = hi[v] & ~kClosed, g1 = G.row[v + 1];
+        for (uint32_t e = G.row[v] + ln; e < g1; e += kWarp) push4<N>(lo_s, hi_s, col[e], clo, chi);
+      }
+      int i, len = 0;
+      uint32_t v = 0, e = 0;
+      uint2 c = make_uint2(0u, 0u);
+      fetch(b1, i, v, e, len, c);
+      while (i - ln < b1) {
+        const bool on = i < b1;
+        const uint32_t clo = on ? lo[v] : 0u, chi = on ? hi[v] & ~kClosed : 0u, at = e;
+        const int groups = on ? len : 0;
+        uint2 x = c;
+        fetch(b1, i, v, e, len, c);
+        for (int j = 1; j <= groups; ++j) {
+          uint2 nx = x;
+          if (j < groups) nx = col[at + 32u * j];
+          push4<N>(lo_s, hi_s, x, clo, chi);
+          x = nx;
+        }
+      }
+    };
+    for (int si = I.begin; si < I.end && !s_stop; ++si) {
+      for (int i = tid; i <= 2 * n + 1; i += T) sm[i] = 0u;
+      __syncthreads();
+      if (tid == 0) {
+        const int s = run.src ? G.rank[run.src[si]] : si;
+        hi[n] = kClosed;
+        lo[s] = 1u;
+        hi[s] = kClosed;
+        const int k = s < nw ? 0 : 1;
+        const int own = G.orig[s];
+        s_goal = *G.nlive + (G.in_rowptr[own + 1] == G.in_rowptr[own] ? 1 : 0);
+        q[k ? nw : 0] = static_cast<uint16_t>(s);
+        lvl[0][0] = lvl[1][0] = 0;
+        lvl[0][1] = 1 - k;
+        lvl[1][1] = k;
+        s_next = s_wide[0] = s_wide[1] = 0;
+      }
+      __syncthreads();
+      int L = 0;
+      for (;;) {
+        const int a1 = lvl[0][L + 1], b1 = lvl[1][L + 1];
+        // every vertex that any edge enters is reached: nothing is left to find
+        if (a1 + b1 == s_goal) break;
+        if (tid == 0) s_wide[(L + 1) & 1] = 0;  // last read before the previous barriers
+        if (a1 == lvl[0][L] && b1 - lvl[1][L] <= kWarp && !s_wide[L & 1]) {
+          // A few short rows: a warp each, and whoever adds to an empty count
+          // lists the vertex, which saves the pass over all vertices.
+          if (tid < 2) s_count[tid] = 0;
+          __syncthreads();
+          for (int i = lvl[1][L] + wid; i < b1; i += W) {
+            const uint32_t v = q[nw + i], clo = lo[v];
+            uint32_t e;
+            int len;
+            row_of(v, e, len);
+            if (ln < len) {
+              const uint2 c = col[e + 32u * ln];
+              const uint32_t ids[4] = {c.x & 0xFFFFu, c.x >> 16, c.y & 0xFFFFu, c.y >> 16};
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const uint32_t w = ids[k];
+                if (static_cast<int>(hi[w]) < 0 || atomicAdd(lo + w, clo) != 0u) continue;
+                const int t = w < static_cast<uint32_t>(nw) ? 0 : 1;
+                q[(t ? nw + b1 : a1) + atomicAdd(&s_count[t], 1)] = static_cast<uint16_t>(w);
+              }
+            }
+          }
+          __syncthreads();
+          const int ta = a1 + s_count[0], tb = b1 + s_count[1];
+          if (ta == a1 && tb == b1) break;
+          auto close = [&](int v) {
+            hi[v] = kClosed;
+            if (lo[v] >> 16) s_wide[(L + 1) & 1] = 1;
+          };
+          for (int i = a1 + tid; i < ta; i += T) close(q[i]);
+          for (int i = b1 + tid; i < tb; i += T) close(q[nw + i]);
+          ++L;
+          __syncthreads();  // L is even across the block; s_count is read
+          if (L + 1 > kSmallMaxLevels) {
+            if (tid == 0) {
+              s_stop = 1;
+              run.refused[I.graph] = 1;
+            }
+            L = 0;
+            break;
+          }
+          if (tid == 0) {
+            lvl[0][L + 1] = ta;
+            lvl[1][L + 1] = tb;
+            s_next = lvl[1][L];
+          }
+          __syncthreads();
+          continue;
+        }
+        if (s_wide[L & 1])
+          push_level(std::false_type(), lvl[0][L], a1, b1);
+        else
+          push_level(std::true_type(), lvl[0][L], a1, b1);
+        __syncthreads();
+        // Close the vertices counted in this level and list them in id order:
+        // each warp takes consecutive chunks (32 at most) and keeps chunk j's
+        // fresh ids in lane j, the warps' totals give each its place.
+        const int nc = (n + kWarp - 1) / kWarp, per = (nc + W - 1) / W;
+        const int c0 = wid * per, mine_c = min(per, nc - c0);
+        unsigned bits = 0;
+        for (int j = 0; j < mine_c; ++j) {
+          const int v = (c0 + j) * kWarp + ln;
+          uint32_t h = kClosed, l = 0;
+          if (v < n) {
+            h = hi[v];
+            l = lo[v];
+          }
+          const bool fresh = static_cast<int>(h) >= 0 && (h | l) != 0u;
+          const unsigned bal = __ballot_sync(kFull, fresh);
+          if (ln == j) bits = bal;
+          if (fresh) {
+            hi[v] = h | kClosed;
+            if (h | (l >> 16)) s_wide[(L + 1) & 1] = 1;
+            if (h >= kCountLimitHi) s_stop = 1;
+          }
+        }
+        // counts of both lists in one word: they stay below 2^16
+        const int cnt = __popc(bits) << (c0 + ln < nw / kWarp ? 0 : 16);
+        int incl = cnt;
+#pragma unroll
+        for (int o = 1; o < kWarp; o <<= 1) {
+          const int y = __shfl_up_sync(kFull, incl, o);
+          if (ln >= o) incl += y;
+        }
+        if (ln == kWarp - 1) s_count[wid] = incl;
+        __syncthreads();
+        int before = ln < W ? s_count[ln] : 0;
+        const int all = before;
+        before = ln < wid ? before : 0;
+        const int total = static_cast<int>(__reduce_add_sync(kFull, static_cast<unsigned>(all)));
+        const int place = static_cast<int>(__reduce_add_sync(kFull, static_cast<unsigned>(before))) + incl - cnt;
+        const int ta = a1 + (total & 0xFFFF), tb = b1 + (total >> 16);
+        for (unsigned some = __ballot_sync(kFull, bits != 0u); some; some &= some - 1u) {
+          const int j = __ffs(some) - 1;
+          const unsigned bal = __shfl_sync(kFull, bits, j);
+          const int at = __shfl_sync(kFull, place, j);
+          const int id = (c0 + j) * kWarp;
+          const int pos = id < nw ? a1 + (at & 0xFFFF) : nw + b1 + (at >> 16);
+          if ((bal >> ln) & 1u) q[pos + __popc(bal & ((1u << ln) - 1u))] = static_cast<uint16_t>(id + ln);
+        }
+        if (ta == a1 && tb == b1) break;
+        if (L + 2 > kSmallMaxLevels || s_stop) {
+          // the batches take the graph: leave the item
+          __syncthreads();  // every thread has read s_stop
+          if (tid == 0) {
+            s_stop = 1;
+            run.refused[I.graph] = 1;
+          }
+          L = 0;
+          break;
+        }
+        ++L;
+        if (tid == 0) {
+          lvl[0][L + 1] = ta;
+          lvl[1][L + 1] = tb;
+          s_next = lvl[1][L];
+        }
+        __syncthreads();
+      }
+      const xf64 w = run.weight ? xf_from_bits(__double_as_longlong(run.weight[si])) : xf_zero();
+      // psi = 1 / sigma + acc replaces the count; sigma * acc is the dependency
+      // (sum: v's partial sum, loaded early)
+      auto finish = [&](int v, xf64 acc, ulonglong2 sum) {
+        const uint64_t s = (static_cast<uint64_t>(hi[v] & ~kClosed) << 32) | lo[v];
+        const uint64_t p = xf_to_bits(xf_add(acc, xf_recip_u64(s)));
+        lo[v] = static_cast<uint32_t>(p);
+        hi[v] = static_cast<uint32_t>(p >> 32) | kClosed;
+        if (acc.m == 0) return;
+        xf64 d = xf_mul_u64(acc, s);
+        if (run.weight) d = xf_mul(d, w);
+        const xf64 t = xf_add(d, xf64{sum.x, static_cast<int32_t>(sum.y)});
+        part[v] = make_ulonglong2(t.m, static_cast<unsigned long long>(t.e));
+      };
+      const int deepest = L;
+      if (tid == 0) s_next = lvl[1][max(L - 1, 0)];  // the deepest level is not fetched
+      for (; L > 0; --L) {
+        const int a1 = lvl[0][L + 1], b1 = lvl[1][L + 1];
+        int held = 0, mine_v = 0;
+        xf64 mine = xf_zero();  // lane j keeps the j-th sum of the warp, to finish 32 at once
+        for (int i = lvl[0][L] + wid; i < a1; i += W) {
+          const int v = q[i];
+          xf64 acc = xf_zero();
+          if (L < deepest) {
+            xg64 a = sum_zero();
+            const uint32_t g1 = G.row[v + 1];
+            uint32_t e = G.row[v] + ln;
+            while (e < g1) {
+#pragma unroll 1
+              for (int k = 0; k < 8 && e < g1; ++k, e += kWarp) pull4(lo_s, hi_s, col[e], a);
+              xg_norm(a);
+            }
+            acc = sum_value(a);
+            acc = warp_sum_x(acc);
+          }
+          if (ln == held) {
+            mine = acc;
+            mine_v = v;
+          }
+          if (++held == kWarp) {
+            finish(mine_v, mine, part[mine_v]);
+            held = 0;
+          }
+        }
+        if (ln < held) finish(mine_v, mine, part[mine_v]);
+        if (L == deepest) {
+          for (int i = lvl[1][L] + tid; i < b1; i += T) {
+            const int v = q[nw + i];
+            finish(v, xf_zero(), part[v]);
+          }
+        } else {
+          int i, len = 0;
+          uint32_t v = 0, e = 0;
+          uint2 c = make_uint2(0u, 0u);
+          fetch(b1, i, v, e, len, c);
+          while (i - ln < b1) {
+            const uint32_t u = v, at = e;
+            const bool on = i < b1;
+            const int groups = on ? len : 0;
+            ulonglong2 sum = make_ulonglong2(0ull, 0ull);
+            if (on) sum = part[u];
+            uint2 x = c;
+            fetch(b1, i, v, e, len, c);
+            xg64 a = sum_zero();
+            for (int j = 1; j <= groups; ++j) {
+              uint2 nx = x;
+              if (j < groups) nx = col[at + 32u * j];
+              pull4(lo_s, hi_s, x, a);
+              if ((j & 7) == 0) xg_norm(a);
+              x = nx;
+            }
+            if (on) finish(u, sum_value(a), sum);
+          }
+        }
+        __syncthreads();
+        // the level is complete: its psi are what the next level sums
+        if (tid == 0 && L < deepest) s_next = lvl[1][L - 1];
+        for (int i = lvl[0][L] + tid; i < a1; i += T) hi[q[i]] &= ~kClosed;
+        for (int i = lvl[1][L] + tid; i < b1; i += T) hi[q[nw + i]] &= ~kClosed;
+        __syncthreads();
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// out[orig] = the sum of a graph's partial vectors, in item order.  A block
+// takes 32 vertices of graph blockIdx.y; its warps sum interleaved items,
+// then warp 0 sums those.
+__global__ void __launch_bounds__(256) k_small_sums(const SmallGraph* graphs, const SmallSum* sums,
+                                                   const ulonglong2* part, double* out) {
+  __shared__ uint64_t sm_m[8][kWarp];
+  __shared__ int sm_e[8][kWarp];
+  const SmallSum S = sums[blockIdx.y];
+  const SmallGraph G = graphs[S.graph];
+  if (blockIdx.x * kWarp >= G.n) return;
+  const int ln = lane_id(), wid = threadIdx.x >> 5;
+  const int v = blockIdx.x * kWarp + ln;
+  xf64 a = xf_zero();
+  if (v < G.n)
+    for (int i = wid; i < S.items; i += 8) {
+      const ulonglong2 o = part[S.part + static_cast<int64_t>(i) * G.n + v];
+      a = xf_add(a, xf64{o.x, static_cast<int32_t>(o.y)});
+    }
+  sm_m[wid][ln] = a.m;
+  sm_e[wid][ln] = a.e;
+  __syncthreads();
+  if (wid || v >= G.n) return;
+  for (int i = 1; i < 8; ++i) a = xf_add(a, xf64{sm_m[i][ln], sm_e[i][ln]});
+  double x = __longlong_as_double(static_cast<long long>(xf_to_bits(a)));
+  if (S.active >= 0) {
+    x += static_cast<double>(S.active);
+    if (v < S.active) x += static_cast<double>(G.n) - 2.0;
+  }
+  out[S.out + G.orig[v]] = x;
+}
+
+// CSRs that no handle has validated: one block per graph.
+__global__ void __launch_bounds__(256) k_small_check(const SmallGraph* graphs, int* bad) {
+  const SmallGraph G = graphs[blockIdx.x];
+  const int64_t nnz = G.rowptr[G.n];
+  int f = 0;
+  for (int v = threadIdx.x; v < G.n; v += blockDim.x) {
+    const int64_t d = G.rowptr[v + 1] - G.rowptr[v];
+    f |= d < 0 ? 1 : (d > G.n ? 4 : 0);
+  }
+  for (int64_t e = threadIdx.x; e < nnz; e += blockDim.x)
+    f |= G.colidx[e] < 0 || G.colidx[e] >= G.n ? 2 : 0;
+  if (f) atomicOr(bad + blockIdx.x, f);
+}
+
+}  // namespace
+
+size_t small_smem(int64_t n) {
+  return (2 * static_cast<size_t>(n + 1) + static_cast<size_t>((n + 31) / 32)) * 4 +
+         ((static_cast<size_t>(n) * 2 + 15) & ~size_t(15));
+}
+
+// Rows rounded up to groups, and each chunk's rows to its longest: since the
+// lengths decrease, that adds at most the first chunk's.
+int64_t small_col_groups(int64_t n, int64_t nnz) {
+  return (nnz + 3 * n) / 4 + kWarp * (kSmallWarpGroups + 1);
+}
+
+int small_configure(size_t max_dyn_smem) {
+  cudaFuncAttributes fa{};
+  if (cudaFuncGetAttributes(&fa, k_small_brandes) != cudaSuccess) return 0;
+  const size_t room = max_dyn_smem > fa.sharedSizeBytes ? max_dyn_smem - fa.sharedSizeBytes : 0;
+  cudaFuncSetAttribute(k_small_brandes, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(room));
+  cudaFuncSetAttribute(k_small_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(max_dyn_smem / 2));
+  int64_t n = std::min<int64_t>(kSmallMaxN, static_cast<int64_t>(room / 10));
+  while (n > 0 && small_smem(n) > room) --n;
+  return static_cast<int>(n);
+}
+
+int small_plan(cudaStream_t s, const SmallGraph* graphs, int count, int64_t max_n) {
+  const size_t bins = static_cast<size_t>((max_n + 3) / 4 + 1);
+  k_small_plan<<<count, 1024, 3 * bins * sizeof(int), s>>>(graphs);
+  return 1;
+}
+
+SmallShape small_shape(const LaunchCfg& c, int64_t max_n, int64_t items) {
+  SmallShape sh{};
+  const size_t smem = small_smem(max_n);
+  // as many warps as the registers allow, split over the blocks that fit and
+  // that there are items for
+  int64_t blocks = std::min<int64_t>(16, static_cast<int64_t>((227 * 1024) / (smem + 4096)));
+  blocks = std::max<int64_t>(1, std::min(blocks, (items + c.sms - 1) / c.sms));
+  int threads = static_cast<int>(kSmallMaxThreads / blocks);
+  threads = std::max(64, std::min(threads, static_cast<int>((2 * max_n + 31) & ~int64_t(31))));
+  threads &= ~31;
+  // a warp lists at most 32 chunks of 32 vertices
+  const int chunks = static_cast<int>((max_n + kWarp - 1) / kWarp);
+  threads = std::max(threads, (chunks + kWarp - 1) / kWarp * kWarp);
+  int resident = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_small_brandes, threads, smem) != cudaSuccess ||
+      resident < 1)
+    resident = 1;
+  sh.threads = threads;
+  sh.grid = c.sms * resident;
+  return sh;
+}
+
+int small_brandes(cudaStream_t s, const SmallShape& sh, const SmallRun& run, int64_t max_n) {
+  const int grid = std::min(sh.grid, run.nitems);
+  k_small_brandes<<<grid, sh.threads, small_smem(max_n), s>>>(run);
+  return 1;
+}
+
+int small_check(cudaStream_t s, const SmallGraph* graphs, int count, int* bad) {
+  k_small_check<<<count, 256, 0, s>>>(graphs, bad);
+  return 1;
+}
+
+int small_sums(cudaStream_t s, const SmallGraph* graphs, const SmallSum* sums, int count, int64_t max_n,
+               const ulonglong2* part, double* out) {
+  const dim3 grid(static_cast<unsigned>((max_n + kWarp - 1) / kWarp), static_cast<unsigned>(count));
+  k_small_sums<<<grid, 256, 0, s>>>(graphs, sums, part, out);
+  return 1;
+}
+
+}  // namespace lgbc

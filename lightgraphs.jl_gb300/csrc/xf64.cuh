@@ -249,4 +249,25 @@ __host__ __device__ __forceinline__ void xg_norm(xg64& a) {
 // The extended value of a normalised gather accumulator.
 __host__ __device__ __forceinline__ xf64 xg_to_xf(xg64 a) { return xf64{a.m << 5, a.e}; }
 
+#ifdef __CUDACC__
+// Sum over the warp (zeros allowed): every value is aligned to the largest
+// exponent and the 63-bit significands are added exactly as four 16-bit
+// pieces by redux (each piece sum < 2^21); the total (< 2^68) keeps its top
+// 63 bits.  Relative error < 2^-56.
+__device__ __forceinline__ xf64 warp_sum_x(xf64 a) {
+  const int E = static_cast<int>(__reduce_max_sync(0xffffffffu, static_cast<unsigned>(a.e)));
+  if (E == 0) return xf_zero();  // every value is zero (warp-uniform)
+  const uint64_t m = xf_shr(a.m, static_cast<uint32_t>(E - a.e));
+  const uint32_t lo = static_cast<uint32_t>(m), hi = static_cast<uint32_t>(m >> 32);
+  const uint64_t s0 = __reduce_add_sync(0xffffffffu, lo & 0xFFFFu);
+  const uint64_t s1 = __reduce_add_sync(0xffffffffu, lo >> 16);
+  const uint64_t s2 = __reduce_add_sync(0xffffffffu, hi & 0xFFFFu);
+  const uint64_t s3 = __reduce_add_sync(0xffffffffu, hi >> 16);
+  // total >> 5 = s3 2^43 + s2 2^27 + s1 2^11 + s0 2^-5 < 2^63
+  const uint64_t t = (s3 << 43) + (s2 << 27) + (s1 << 11) + (s0 >> 5);
+  const int lz = xf_clz(t) - 1;  // 0..5: the largest value alone is >= 2^57 after the shift
+  return xf64{t << lz, E + 5 - lz};
+}
+#endif
+
 }  // namespace lgbc

@@ -1,0 +1,133 @@
+"""The per-source betweenness kernel of small graphs (small.cu) against the
+oracle where it can go wrong: chunk and warp edges of the vertex count, rows
+at the lengths where threads hand over to warps, every row long, levels at the
+depth cap, path counts around 2^16, 2^32 and 2^48, sources nothing enters,
+repeats, weights, and the sizes on both sides of the shared-memory limit."""
+import numpy as np
+import pytest
+
+import lgbc
+from lgbc import generators as G
+from lgbc.learned import betweenness_raw_weighted
+from conftest import csr_args
+from oracle import oracle
+from test_gpu_parity import assert_bc_close, oracle_bc
+
+pytestmark = pytest.mark.gpu
+
+
+def random_graph(n, m, seed, directed=False):
+    e = np.random.default_rng(seed).integers(0, n, (2, m))
+    return (lgbc.SimpleDiGraph if directed else lgbc.SimpleGraph).from_edge_arrays(n, e[0], e[1])
+
+
+def path(n):
+    return lgbc.SimpleGraph.from_edge_arrays(n, np.arange(n - 1), np.arange(1, n))
+
+
+def layers(count, width):
+    """Complete bipartite steps between consecutive layers: width^L paths to layer L + 1."""
+    e = [(l * width + i, (l + 1) * width + j) for l in range(count - 1) for i in range(width)
+         for j in range(width)]
+    return lgbc.SimpleGraph.from_edge_arrays(count * width, *np.asarray(e).T)
+
+
+def fan(n, degree):
+    """A vertex of the given degree among short rows."""
+    ring = np.arange(n)
+    return lgbc.SimpleGraph.from_edge_arrays(
+        n, np.concatenate([ring, np.zeros(degree, int)]),
+        np.concatenate([(ring + 1) % n, 1 + np.arange(degree)]))
+
+
+def check(g, sources=None, endpoints=False):
+    vs = None if sources is None else np.asarray(sources) + 1
+    got = lgbc.betweenness_centrality(g, vs, normalize=False, endpoints=endpoints)
+    assert_bc_close(got, oracle_bc(g, sources, normalize=False, endpoints=endpoints, nthreads=8))
+
+
+@pytest.mark.parametrize("directed", [False, True])
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 32, 33, 63, 64, 65, 300, 1023, 1025])
+@pytest.mark.parametrize("degree", [1, 5, 80])
+def test_vertex_counts(n, degree, directed):
+    # degree 80: every row is walked by a warp and the last chunk is ragged
+    check(random_graph(n, n * degree // (1 if directed else 2) + 1, n + degree, directed),
+          endpoints=n % 2 == 0)
+
+
+@pytest.mark.parametrize("degree", [60, 61, 62, 63, 64, 65, 128, 129, 1500])
+def test_row_lengths(degree):
+    # with its two ring edges the first vertex's row crosses 64 entries at 62
+    check(fan(2000, degree), np.arange(0, 2000, 13))
+
+
+@pytest.mark.parametrize("n", [126, 127, 128, 129, 130, 131, 400])
+def test_depths(n):
+    check(path(n))
+
+
+@pytest.mark.parametrize("count,width", [(10, 4), (17, 4), (18, 4), (12, 8), (13, 8), (24, 4), (26, 4)])
+def test_path_counts(count, width):
+    # 2^16, 2^32 and 2^48 paths lie between these depths
+    check(layers(count, width), np.arange(0, count * width, 3))
+
+
+def test_sources_nothing_enters_and_other_components():
+    n = 500
+    e = np.random.default_rng(5).integers(50, 400, (2, 900))
+    src = np.concatenate([e[0], np.arange(50)])
+    dst = np.concatenate([e[1], np.random.default_rng(6).integers(50, 400, 50)])
+    g = lgbc.SimpleDiGraph.from_edge_arrays(n, src, dst)
+    check(g)
+    check(g, [0, 0, 49, 60, 60, 450, 499])
+
+
+@pytest.mark.parametrize("n", [10000, 22000, 24000])
+def test_shared_memory_limit(n):
+    check(random_graph(n, 3 * n, n), np.arange(0, n, n // 40))
+    check(G.barabasi_albert(n, 3, seed=n), np.arange(0, n, n // 40))
+
+
+def test_weights_and_repeats():
+    g = G.rmat(10, 8, seed=2)
+    rp, ci, _ = csr_args(g)
+    rng = np.random.default_rng(3)
+    src = rng.integers(0, g.nv(), 700).astype(np.int32)
+    w = rng.random(700) * np.where(rng.random(700) < 0.1, 0.0, 10.0)
+    _, want = oracle.dependency(rp, ci, src, w)
+    np.testing.assert_allclose(betweenness_raw_weighted(g, src, w), want, rtol=1e-9)
+
+
+@pytest.mark.parametrize("endpoints", [False, True])
+def test_many_mixed(endpoints):
+    # size classes, a refused depth, refused counts, isolated vertices, and a
+    # graph beyond the limit in one call
+    graphs = [G.barabasi_albert(n, 3, seed=n) for n in (30, 1500, 3000, 5000, 12000)]
+    graphs += [path(400), layers(26, 4), lgbc.SimpleGraph(0), lgbc.SimpleGraph(7),
+               random_graph(2000, 900, 8), random_graph(300, 12000, 9), path(2)]
+    small = [g for g in graphs if g.nv() <= 5000]
+    for g, z in zip(small, lgbc.betweenness_centrality_many(small, normalize=False, endpoints=endpoints)):
+        assert_bc_close(z, oracle_bc(g, normalize=False, endpoints=endpoints, nthreads=8))
+    big = [graphs[4], G.erdos_renyi_nm(24000, 12000, seed=1)]
+    for g, z in zip(big, lgbc.betweenness_centrality_many(big, normalize=False, endpoints=endpoints)):
+        assert_bc_close(z, lgbc.betweenness_centrality(g, normalize=False, endpoints=endpoints))
+
+
+def test_many_rejects_what_it_did():
+    good = path(5)
+    bad = lgbc.SimpleGraph.from_csr([0, 1, 2, 2], [1, 3])
+    with pytest.raises(lgbc.ArgumentError, match="column index"):
+        lgbc.betweenness_centrality_many([good, bad])
+    drop = lgbc.SimpleGraph.from_csr([0, 2, 1, 2], [1, 2])
+    with pytest.raises(lgbc.ArgumentError, match="rowptr"):
+        lgbc.betweenness_centrality_many([good, drop])
+
+
+def test_repeated_entries_take_the_batches():
+    # a row longer than n (repeated entries): accepted as before
+    g = lgbc.SimpleGraph.from_csr([0, 4, 7, 8], [1, 1, 1, 1, 0, 0, 2, 1])
+    h = lgbc.SimpleGraph.from_csr([0, 4, 7, 8], [1, 1, 1, 1, 0, 0, 2, 1])
+    h.device_handle().set_tuning(stack_vertices=0)
+    a, b = (lgbc.betweenness_centrality(x, normalize=False) for x in (g, h))
+    np.testing.assert_allclose(a, b, rtol=1e-12)
+    np.testing.assert_allclose(lgbc.betweenness_centrality_many([g], normalize=False)[0], b, rtol=1e-12)
