@@ -167,6 +167,8 @@ int lgbc_graph_stats(const lgbc_graph *g, lgbc_stats *out);
  * vertices, at most 2^20 stored entries) runs one thread block per source
  * instead, unless a search is deeper than 126 levels or a path count reaches
  * 2^48; lgbc_stats.batches then counts the blocks' shares of the sources.
+ * Distances and distance statistics of such graphs (about 18,900 vertices)
+ * run 32 sources per thread block in the same way.
  *   alpha, beta   direction switch: go bottom-up when the frontier's edges
  *                 exceed (unvisited edges)/alpha; return top-down when the
  *                 frontier has fewer than n/beta vertices.

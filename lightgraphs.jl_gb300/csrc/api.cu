@@ -1010,46 +1010,76 @@ bool same_tuning(const lgbc_tuning& a, const lgbc_tuning& b) {
          a.dependency_df32 == b.dependency_df32;
 }
 
-// Whether the per-source kernel takes this handle's betweenness calls.  The
-// vertex state of one source must fit an SM's shared memory and a row's
-// length must not exceed n (the plan's bins).  A handle whose tuning was
-// changed asks for batches of that shape and keeps them.
-bool small_applies(const lgbc_graph* g) {
-  return g->n > 0 && g->n <= g->small_max_n && g->max_out <= g->n && g->nnz <= kSmallMaxNnz && !g->small.refused &&
+// Whether the shared-memory kernels take this handle's calls.  A row's length
+// must not exceed n (the plan's bins).  A handle whose tuning was changed asks
+// for batches (and single searches) of that shape and keeps them.
+bool small_graph(const lgbc_graph* g) {
+  return g->n > 0 && g->max_out <= g->n && g->max_in <= g->n && g->nnz <= kSmallMaxNnz &&
          same_tuning(g->tune, kDefaultTuning);
 }
 
-int ensure_small(lgbc_graph* g) {
-  SmallWorkspace& w = g->small;
-  if (w.built) return LGBC_OK;
-  w.release();
+// The vertex state of one source must fit an SM's shared memory.
+bool small_applies(const lgbc_graph* g) {
+  return small_graph(g) && g->n <= g->small_max_n && !g->small.refused;
+}
+
+// A block walks every unfinished vertex's edges once a level: with 64 sources
+// or fewer (two blocks at most) the batches' whole grid catches up between
+// 0.43M entries (R-MAT 14: 391 against 399 us) and 0.9M (305 against 269 us);
+// 500 sources took 312 against 1,743 us there.
+bool small_bfs_applies(const lgbc_graph* g, int64_t nsrc) {
+  return small_graph(g) && g->n <= g->small_bfs_max_n && nsrc <= INT32_MAX &&
+         (nsrc > kMaxLanes || g->nnz <= int64_t(1) << 19);
+}
+
+// The plan of one of g's two CSRs (an undirected graph has one).
+int ensure_plan(lgbc_graph* g, SmallPlan* p, const int64_t* rowptr, const int32_t* colidx,
+                const int64_t* in_rowptr) {
+  if (p->graph) return LGBC_OK;
+  p->release();
   const size_t n = static_cast<size_t>(g->n);
-  w.view.n = static_cast<int>(g->n);
-  w.view.rowptr = g->d_rowptr;
-  w.view.colidx = g->d_colidx;
-  LGBC_TRY(dev_alloc(&w.view.rank, n));
-  LGBC_TRY(dev_alloc(&w.view.orig, n));
-  LGBC_TRY(dev_alloc(&w.view.row, n + 1));
-  LGBC_TRY(dev_alloc(&w.view.chunk, (n + 31) / 32));
-  LGBC_TRY(dev_alloc(&w.view.col, static_cast<size_t>(small_col_groups(g->n, g->nnz))));
-  LGBC_TRY(dev_alloc(&w.graph, 1));
-  LGBC_TRY(dev_alloc(&w.sum, 1));
-  LGBC_TRY(dev_alloc(&w.counters, 4));
-  w.view.in_rowptr = g->d_in_rowptr;
-  w.view.nwarp = w.counters;
-  w.view.nlive = w.counters + 3;
-  LGBC_CUDA(cudaMemsetAsync(w.counters, 0, 4 * sizeof(int), g->stream));
-  LGBC_CUDA(cudaMemcpyAsync(w.graph, &w.view, sizeof w.view, cudaMemcpyHostToDevice, g->stream));
-  g->launches += small_plan(g->stream, w.graph, 1, g->n);
-  LGBC_TRY(check_launch(g));
-  w.built = true;
+  SmallGraph& v = p->view;
+  v.n = static_cast<int>(g->n);
+  v.rowptr = rowptr;
+  v.colidx = colidx;
+  v.in_rowptr = in_rowptr;
+  LGBC_TRY(dev_alloc(&v.rank, n));
+  LGBC_TRY(dev_alloc(&v.orig, n));
+  LGBC_TRY(dev_alloc(&v.row, n + 1));
+  LGBC_TRY(dev_alloc(&v.chunk, (n + 31) / 32));
+  LGBC_TRY(dev_alloc(&v.col, static_cast<size_t>(small_col_groups(g->n, g->nnz))));
+  LGBC_TRY(dev_alloc(&p->counters, 2));
+  v.nwarp = p->counters;
+  v.nlive = p->counters + 1;
+  SmallGraph* d = nullptr;
+  LGBC_TRY(dev_alloc(&d, 1));
+  cudaMemsetAsync(p->counters, 0, 2 * sizeof(int), g->stream);
+  cudaMemcpyAsync(d, &v, sizeof v, cudaMemcpyHostToDevice, g->stream);
+  g->launches += small_plan(g->stream, d, 1, g->n);
+  const int rc = check_launch(g);
+  if (rc != LGBC_OK) {
+    cudaFree(d);
+    return rc;
+  }
+  p->graph = d;
   return LGBC_OK;
+}
+
+int run_small_bfs(lgbc_graph* g, SmallBfs run) {
+  // the kernel pulls over in-lists
+  SmallPlan* p = g->directed ? &g->small.in : &g->small.out;
+  LGBC_TRY(ensure_plan(g, p, g->d_in_rowptr, g->d_in_colidx, g->d_rowptr));
+  run.graph = p->graph;
+  g->launches += small_bfs(g->cfg, g->stream, run, g->n);
+  return check_launch(g);
 }
 
 // Brandes over g->d_src[0, k) by the per-source kernel; 1 when it refuses.
 int run_small(lgbc_graph* g, int64_t k, double* bc_dev, const double* d_w) {
-  LGBC_TRY(ensure_small(g));
   SmallWorkspace& w = g->small;
+  LGBC_TRY(ensure_plan(g, &w.out, g->d_rowptr, g->d_colidx, g->d_in_rowptr));
+  if (!w.counters) LGBC_TRY(dev_alloc(&w.counters, 2));
+  if (!w.sum) LGBC_TRY(dev_alloc(&w.sum, 1));
   const SmallShape sh = small_shape(g->cfg, g->n, k);
   const int64_t items = std::min<int64_t>(k, sh.grid);
   if (items * g->n > w.part_cap) {
@@ -1064,20 +1094,20 @@ int run_small(lgbc_graph* g, int64_t k, double* bc_dev, const double* d_w) {
     w.items = items;
   }
   SmallRun run{};
-  run.graphs = w.graph;
+  run.graphs = w.out.graph;
   run.nitems = static_cast<int>(items);
   run.nsrc = static_cast<int>(k);
-  run.next = w.counters + 1;
-  run.refused = w.counters + 2;
+  run.next = w.counters;
+  run.refused = w.counters + 1;
   run.src = g->d_src;
   run.weight = d_w;
   run.part = w.part;
-  LGBC_CUDA(cudaMemsetAsync(w.counters + 1, 0, 2 * sizeof(int), g->stream));
+  LGBC_CUDA(cudaMemsetAsync(w.counters, 0, 2 * sizeof(int), g->stream));
   g->launches += small_brandes(g->stream, sh, run, g->n);
-  g->launches += small_sums(g->stream, w.graph, w.sum, 1, g->n, w.part, bc_dev);
+  g->launches += small_sums(g->stream, w.out.graph, w.sum, 1, g->n, w.part, bc_dev);
   LGBC_TRY(check_launch(g));
   int* refused = reinterpret_cast<int*>(g->h_ctl);
-  LGBC_CUDA(cudaMemcpyAsync(refused, w.counters + 2, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+  LGBC_CUDA(cudaMemcpyAsync(refused, w.counters + 1, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
   LGBC_CUDA(cudaStreamSynchronize(g->stream));
   if (*refused) {
     w.refused = true;
@@ -1137,6 +1167,7 @@ int init_handle(lgbc_graph* g, int64_t n, int directed) {
   g->max_smem = prop.sharedMemPerBlockOptin;
   bfs_configure(g->max_smem);
   g->small_max_n = small_configure(g->max_smem);
+  g->small_bfs_max_n = small_bfs_configure(g->max_smem);
   LGBC_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
   LGBC_CUDA(cudaEventCreate(&g->ev_start));
   LGBC_CUDA(cudaEventCreate(&g->ev_stop));
@@ -1237,6 +1268,7 @@ void degree_pass(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr)
     mi = std::max(mi, max_in[static_cast<size_t>(p)]);
     all.insert(all.end(), tops[static_cast<size_t>(p)].begin(), tops[static_cast<size_t>(p)].end());
   }
+  g->max_in = mi;
   g->sigma_limit = ~0ull / static_cast<unsigned long long>(mi + 1);
   std::sort(all.begin(), all.end());
   g->landmarks.clear();
@@ -1403,8 +1435,21 @@ int lgbc_gdistances(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* di
   LGBC_TRY(check_sources(g, src, nsrc));
   reset_stats(g);
   if (g->n == 0) return LGBC_OK;
-  LGBC_TRY(prepare_bfs(g, src, nsrc));
-  LGBC_TRY(run_bfs(g, g->dev(), nsrc));
+  if (nsrc > 0 && small_bfs_applies(g, 1)) {
+    LGBC_TRY(ensure_dist(g, g->n));
+    LGBC_TRY(ensure_src(g, nsrc));
+    LGBC_CUDA(cudaMemcpyAsync(g->d_src, src, static_cast<size_t>(nsrc) * 4, cudaMemcpyHostToDevice,
+                              g->stream));
+    SmallBfs run{};
+    run.src = g->d_src;
+    run.nsrc = static_cast<int>(nsrc);
+    run.together = 1;
+    run.dist = g->d_dist;
+    LGBC_TRY(run_small_bfs(g, run));
+  } else {
+    LGBC_TRY(prepare_bfs(g, src, nsrc));
+    LGBC_TRY(run_bfs(g, g->dev(), nsrc));
+  }
   LGBC_CUDA(cudaMemcpyAsync(dist_out, g->d_dist, static_cast<size_t>(g->n) * 4,
                             cudaMemcpyDeviceToHost, g->stream));
   LGBC_CUDA(cudaStreamSynchronize(g->stream));
@@ -1420,10 +1465,29 @@ int lgbc_gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32
   if (nsrc > 0 && g->n > 0 && !dist_out) return fail(LGBC_EINVAL, "null output");
   reset_stats(g);
   if (nsrc == 0 || g->n == 0) return LGBC_OK;
-  LGBC_TRY(ensure_ms(g, false));
   LGBC_TRY(ensure_src(g, nsrc));
   LGBC_CUDA(cudaMemcpyAsync(g->d_src, src, static_cast<size_t>(nsrc) * 4, cudaMemcpyHostToDevice,
                             g->stream));
+  if (small_bfs_applies(g, nsrc)) {
+    // at most 2^26 distances on the device at a time
+    const int64_t rows = std::min<int64_t>(nsrc, std::max<int64_t>(kWarp, (int64_t(1) << 26) / g->n / kWarp * kWarp));
+    LGBC_TRY(ensure_dist(g, rows * g->n));
+    for (int64_t s0 = 0; s0 < nsrc; s0 += rows) {
+      SmallBfs run{};
+      run.src = g->d_src + s0;
+      run.nsrc = static_cast<int>(std::min(rows, nsrc - s0));
+      run.dist = g->d_dist;
+      LGBC_TRY(run_small_bfs(g, run));
+      LGBC_CUDA(cudaMemcpyAsync(dist_out + s0 * g->n, g->d_dist,
+                                static_cast<size_t>(run.nsrc) * static_cast<size_t>(g->n) * 4,
+                                cudaMemcpyDeviceToHost, g->stream));
+      g->stats.batches++;
+    }
+    LGBC_CUDA(cudaStreamSynchronize(g->stream));
+    finish_stats(g);
+    return LGBC_OK;
+  }
+  LGBC_TRY(ensure_ms(g, false));
   const int lanes = kMaxLanes;
   LGBC_TRY(ensure_dist(g, static_cast<int64_t>(lanes) * g->n));
   for (int64_t s0 = 0; s0 < nsrc; s0 += lanes) {

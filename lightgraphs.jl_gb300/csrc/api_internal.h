@@ -206,17 +206,11 @@ struct LearnedWorkspace {
   }
 };
 
-// Plan and workspace of the per-source kernel for small graphs (small.cu).
-struct SmallWorkspace {
+// The relabelled rows of a small graph's out-CSR or in-CSR (small.cu).
+struct SmallPlan {
   SmallGraph view{};                // host copy of *graph
   SmallGraph* graph = nullptr;
-  SmallSum* sum = nullptr;
-  int64_t items = 0;                // parts of a call that *sum was written for
-  int* counters = nullptr;          // [0] warp-walked ids, [1] next item, [2] refused, [3] live vertices
-  ulonglong2* part = nullptr;       // partial sums, one n-vector per item
-  int64_t part_cap = 0;
-  bool built = false;
-  bool refused = false;             // too deep or counts too large: the batches take this graph
+  int* counters = nullptr;          // [0] warp-walked ids, [1] live vertices
   void release() {
     dev_free(view.rank);
     dev_free(view.orig);
@@ -224,12 +218,27 @@ struct SmallWorkspace {
     dev_free(view.chunk);
     dev_free(view.col);
     dev_free(graph);
+    dev_free(counters);
+  }
+};
+
+// Plans and workspace of the shared-memory kernels for small graphs.
+struct SmallWorkspace {
+  SmallPlan out, in;                // in: digraphs only
+  SmallSum* sum = nullptr;
+  int64_t items = 0;                // parts of a call that *sum was written for
+  int* counters = nullptr;          // [0] next item, [1] refused
+  ulonglong2* part = nullptr;       // partial sums, one n-vector per item
+  int64_t part_cap = 0;
+  bool refused = false;             // too deep or counts too large: the batches take this graph
+  void release() {
+    out.release();
+    in.release();
     dev_free(sum);
     items = 0;
     dev_free(counters);
     dev_free(part);
     part_cap = 0;
-    built = false;
   }
 };
 
@@ -311,7 +320,8 @@ struct lgbc_graph {
   lgbc::api::LearnedWorkspace learned;
   lgbc::api::SmallWorkspace small;
   int64_t small_max_n = 0;          // largest graph of the per-source kernel on this device
-  int64_t max_out = 0;              // largest out-list
+  int64_t small_bfs_max_n = 0;      // and of the distance kernel
+  int64_t max_out = 0, max_in = 0;  // largest out- and in-list
   int32_t* d_src = nullptr;         // device copy of a call's source list
   int64_t d_src_cap = 0;
   double* d_bc = nullptr;           // device result buffer for host-buffer calls
@@ -396,6 +406,10 @@ int init_handle(lgbc_graph* g, int64_t n, int directed);
 // from the device when the hub items need them).
 int finish_handle(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr,
                   const int32_t* colidx = nullptr, const int32_t* in_colidx = nullptr);
+// Whether the shared-memory distance kernel takes nsrc searches, and the call
+// (run: everything but the graph).
+bool small_bfs_applies(const lgbc_graph* g, int64_t nsrc);
+int run_small_bfs(lgbc_graph* g, SmallBfs run);
 int run_bfs(lgbc_graph* g, const DevGraph& dg, int64_t nsrc);
 int prepare_bfs(lgbc_graph* g, const int32_t* src, int64_t nsrc);
 

@@ -94,7 +94,8 @@ int distance_stats(lgbc_graph* g, const int32_t* src, int64_t nsrc,
   dsum->assign(static_cast<size_t>(nsrc), 0ull);
   dmax->assign(static_cast<size_t>(nsrc), 0);
   if (nsrc == 0) return LGBC_OK;
-  LGBC_TRY(ensure_ms(g, false));
+  const bool small = small_bfs_applies(g, nsrc);
+  if (!small) LGBC_TRY(ensure_ms(g, false));
   LGBC_TRY(ensure_src(g, nsrc));
   unsigned long long* buf = nullptr;  // cnt | dsum | dmax (as int)
   LGBC_TRY(dev_alloc(&buf, static_cast<size_t>(nsrc) * 3));
@@ -104,7 +105,17 @@ int distance_stats(lgbc_graph* g, const int32_t* src, int64_t nsrc,
   LGBC_CUDA(cudaMemcpyAsync(g->d_src, src, static_cast<size_t>(nsrc) * 4, cudaMemcpyHostToDevice,
                             g->stream));
   int* dm = reinterpret_cast<int*>(buf + 2 * nsrc);
-  for (int64_t s0 = 0; s0 < nsrc; s0 += kMaxLanes) {
+  if (small) {
+    SmallBfs run{};
+    run.src = g->d_src;
+    run.nsrc = static_cast<int>(nsrc);
+    run.cnt = buf;
+    run.dsum = buf + nsrc;
+    run.dmax = dm;
+    LGBC_TRY(run_small_bfs(g, run));
+    g->stats.batches++;
+  }
+  for (int64_t s0 = 0; !small && s0 < nsrc; s0 += kMaxLanes) {
     const int nl = static_cast<int>(std::min<int64_t>(kMaxLanes, nsrc - s0));
     const LevelStats st{buf + s0, buf + nsrc + s0, dm + s0};
     LGBC_TRY(run_ms_batch(g, g->d_src + s0, nl, kSigmaNone, nullptr, nullptr, 0, Seeds(), nullptr,

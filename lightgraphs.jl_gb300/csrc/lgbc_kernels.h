@@ -230,6 +230,20 @@ struct SmallSum {
   int64_t part;            // items x n
   int64_t out;
 };
+// Distances on a small graph, 32 sources per block (or one set of sources).
+struct SmallBfs {
+  const SmallGraph* graph;   // plan of the in-CSR
+  const int32_t* src;        // graph's own ids
+  int nsrc;
+  int together;              // 1: one search from all the sources
+  int32_t* dist;             // nsrc (or 1) x n, every entry written; or null
+  unsigned long long* cnt;   // per source: vertices reached at levels >= 1, or null
+  unsigned long long* dsum;  //   and the sum
+  int* dmax;                 //   and maximum of their levels
+};
+// The largest n of the kernel on this device (opts it into the shared memory).
+int small_bfs_configure(size_t max_dyn_smem);
+int small_bfs(const LaunchCfg& c, cudaStream_t s, const SmallBfs& run, int64_t n);
 size_t small_smem(int64_t n);
 int64_t small_col_groups(int64_t n, int64_t nnz);
 // Opt the kernels into the device's shared memory; the largest n they take.

@@ -1,5 +1,5 @@
-"""The per-source betweenness kernel of small graphs (small.cu) against the
-oracle where it can go wrong: chunk and warp edges of the vertex count, rows
+"""The shared-memory betweenness and distance kernels of small graphs (small.cu)
+against the oracle where it can go wrong: chunk and warp edges of the vertex count, rows
 at the lengths where threads hand over to warps, every row long, levels at the
 depth cap, path counts around 2^16, 2^32 and 2^48, sources nothing enters,
 repeats, weights, and the sizes on both sides of the shared-memory limit."""
@@ -111,6 +111,33 @@ def test_many_mixed(endpoints):
     big = [graphs[4], G.erdos_renyi_nm(24000, 12000, seed=1)]
     for g, z in zip(big, lgbc.betweenness_centrality_many(big, normalize=False, endpoints=endpoints)):
         assert_bc_close(z, lgbc.betweenness_centrality(g, normalize=False, endpoints=endpoints))
+
+
+@pytest.mark.parametrize("directed", [False, True])
+@pytest.mark.parametrize("n", [1, 2, 32, 33, 300, 1025, 18800, 19200])
+@pytest.mark.parametrize("k", [1, 31, 32, 33, 70])
+def test_distances(n, k, directed):
+    # lanes at the edges of a block's 32, both sides of the size limit, long rows at n = 300
+    g = random_graph(n, n * (80 if n == 300 else 2), n + k, directed)
+    rp, ci, _ = csr_args(g)
+    src = np.random.default_rng(k).integers(0, n, k).astype(np.int32)
+    want = np.stack([oracle.gdistances(rp, ci, [s]) for s in src]).astype(np.int64)
+    far = want == oracle.UNREACHED32
+    top = np.iinfo(g.eltype).max
+    assert np.array_equal(lgbc.multi_gdistances(g, src + 1), np.where(far, top, want))
+    reached, dsum, dmax = lgbc.distance.distance_stats(g, src)
+    assert np.array_equal(reached, (~far).sum(1))
+    assert np.array_equal(dsum, np.where(far, 0, want).sum(1))
+    assert np.array_equal(dmax, np.where(far, 0, want).max(1))
+    nearest = np.where(far, top, want).min(0)
+    assert np.array_equal(lgbc.gdistances(g, src + 1), nearest)
+
+
+def test_distances_along_a_path():
+    g = path(3000)
+    d = lgbc.multi_gdistances(g, [1, 1500, 3000])
+    i = np.arange(3000)
+    assert np.array_equal(d, np.stack([i, abs(i - 1499), 2999 - i]))
 
 
 def test_many_rejects_what_it_did():
