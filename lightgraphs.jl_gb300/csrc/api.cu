@@ -109,16 +109,18 @@ int grow_ms_lists(lgbc_graph* g) {
   return LGBC_OK;
 }
 
+// Words of one bitmap: whole 16-byte pieces, each bitmap on its own boundary.
+size_t bfs_words(const lgbc_graph* g) { return (static_cast<size_t>(g->n + 31) / 32 + 3) & ~size_t(3); }
+size_t bfs_big(const lgbc_graph* g) { return static_cast<size_t>(g->nnz / kBfsChunk + 1); }
+
 int ensure_bfs(lgbc_graph* g) {
   BfsWorkspace& w = g->bfs;
-  if (w.queue) return LGBC_OK;
-  const size_t n = static_cast<size_t>(g->n);
-  const size_t words = (n + 31) / 32 + 4;
-  LGBC_TRY(dev_alloc(&w.queue, n + 1));
-  LGBC_TRY(dev_alloc(&w.large, n + 1));
-  LGBC_TRY(dev_alloc(&w.bm0, words));
-  LGBC_TRY(dev_alloc(&w.bm1, words));
-  LGBC_TRY(dev_alloc(&w.ctl, 1));
+  if (w.state) return LGBC_OK;
+  w.release();
+  LGBC_TRY(dev_alloc(&w.queue, static_cast<size_t>(g->n) + 1));
+  LGBC_TRY(dev_alloc(&w.bits, 4 * bfs_words(g)));
+  LGBC_TRY(dev_alloc(&w.big, 2 * bfs_big(g)));
+  LGBC_TRY(dev_alloc(&w.state, 1));
   return LGBC_OK;
 }
 
@@ -1165,7 +1167,7 @@ int init_handle(lgbc_graph* g, int64_t n, int directed) {
   g->cfg.block = 256;
   g->cfg.grid = prop.multiProcessorCount * 8;
   g->max_smem = prop.sharedMemPerBlockOptin;
-  bfs_configure(g->max_smem);
+  g->bfs_room = bfs_configure(g->max_smem);
   g->small_max_n = small_configure(g->max_smem);
   g->small_bfs_max_n = small_bfs_configure(g->max_smem);
   LGBC_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
@@ -1378,40 +1380,40 @@ int lgbc_graph_info(const lgbc_graph* g, int64_t* n, int64_t* nnz, int* directed
 
 namespace lgbc::api {
 
-// Level-synchronous BFS over dg from d_src[0, nsrc) into d_dist, which the
-// caller has filled (kUnreached, and any other value on vertices the search
-// must treat as already visited).
-int run_bfs(lgbc_graph* g, const DevGraph& dg, int64_t nsrc) {
-  BfsBuffers b{g->bfs.queue, {g->bfs.bm0, g->bfs.bm1}, g->bfs.ctl, g->bfs.large};
-  g->launches += bfs_init(g->cfg, g->stream, dg, b, g->d_src, nsrc, g->d_dist);
+int run_bfs(lgbc_graph* g, const DevGraph& dg, int64_t nsrc, bool prefilled) {
+  BfsWorkspace& w = g->bfs;
+  BfsRun r{};
+  r.dist = g->d_dist;
+  r.src = g->d_src;
+  r.nsrc = nsrc;
+  r.prefilled = prefilled ? 1 : 0;
+  r.queue = w.queue;
+  r.visited = w.bits;
+  r.words = static_cast<int64_t>(bfs_words(g));
+  r.big = w.big;
+  r.big_cap = static_cast<int64_t>(bfs_big(g));
+  r.state = w.state;
+  r.alpha = g->tune.alpha;
+  r.beta = g->tune.beta;
+  g->launches += bfs_run(g->cfg, g->stream, dg, r, g->bfs_room);
   LGBC_TRY(check_launch(g));
-  LGBC_TRY(read_ctl(g, b.ctl));
-  const size_t bm_bytes = static_cast<size_t>(((g->n + 31) / 32 + 3) & ~int64_t(3)) * 4;
-  const int stage = bm_bytes <= g->max_smem ? 1 : 0;
-  bool bu = false;
-  while (!g->h_ctl->done) {
-    const BatchCtl& c = *g->h_ctl;
-    const double mf = static_cast<double>(c.mf_cur);
-    const double mu = static_cast<double>(g->nnz) - static_cast<double>(c.mu_done);
-    const double nf = static_cast<double>(c.hi - c.lo);
-    bu = bu ? (nf >= static_cast<double>(g->n) / g->tune.beta) : (mf > mu / g->tune.alpha);
-    if (bu) {
-      g->launches += bfs_bottomup(g->cfg, g->stream, dg, b, g->d_dist, stage);
-      g->stats.bottomup_levels++;
-    } else {
-      g->launches += bfs_topdown(g->cfg, g->stream, dg, b, g->d_dist);
-      g->stats.topdown_levels++;
-    }
-    g->launches += bfs_advance(g->stream, b);
-    LGBC_TRY(check_launch(g));
-    LGBC_TRY(read_ctl(g, b.ctl));
-    g->stats.levels++;
-    if (g->stats.levels > g->n + 1) return fail(LGBC_ETIMEOUT, "BFS exceeded n + 1 levels");
-  }
+  static_assert(sizeof(BfsState) <= sizeof(BatchCtl), "h_ctl holds either");
+  LGBC_CUDA(cudaMemcpyAsync(g->h_ctl, w.state, sizeof(BfsState), cudaMemcpyDeviceToHost, g->stream));
   return LGBC_OK;
 }
 
-// Upload nsrc sources and fill the distance buffer with kUnreached.
+int finish_bfs(lgbc_graph* g) {
+  LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  const BfsState* st = reinterpret_cast<const BfsState*>(g->h_ctl);
+  if (st->failed) return fail(LGBC_ETIMEOUT, "BFS: a grid barrier ran out");
+  g->stats.topdown_levels += st->td_levels;
+  g->stats.bottomup_levels += st->bu_levels;
+  g->stats.levels += st->td_levels + st->bu_levels;
+  if (g->stats.levels > g->n + 1) return fail(LGBC_ETIMEOUT, "BFS exceeded n + 1 levels");
+  return LGBC_OK;
+}
+
+// The workspace of a BFS, and its sources on the device.
 int prepare_bfs(lgbc_graph* g, const int32_t* src, int64_t nsrc) {
   LGBC_TRY(ensure_bfs(g));
   LGBC_TRY(ensure_dist(g, g->n));
@@ -1419,15 +1421,14 @@ int prepare_bfs(lgbc_graph* g, const int32_t* src, int64_t nsrc) {
   if (nsrc > 0)
     LGBC_CUDA(cudaMemcpyAsync(g->d_src, src, static_cast<size_t>(nsrc) * 4, cudaMemcpyHostToDevice,
                               g->stream));
-  g->launches += fill_i32(g->cfg, g->stream, g->d_dist, g->n, kUnreached);
   return LGBC_OK;
 }
 
-}  // namespace lgbc::api
+// One search on one SM against the whole grid with a barrier per level: equal
+// at 144,000 entries (104 against 107 us), 55 against 107 us at 96,000.
+constexpr int64_t kSmallSingleNnz = int64_t(1) << 17;
 
-extern "C" {
-
-int lgbc_gdistances(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* dist_out) {
+int gdistances(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* dist_out) {
   LGBC_TRY(check_graph(g));
   std::lock_guard<std::mutex> lock(g->mu);
   LGBC_TRY(use_device(g));
@@ -1435,7 +1436,8 @@ int lgbc_gdistances(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* di
   LGBC_TRY(check_sources(g, src, nsrc));
   reset_stats(g);
   if (g->n == 0) return LGBC_OK;
-  if (nsrc > 0 && small_bfs_applies(g, 1)) {
+  const bool small = nsrc > 0 && small_bfs_applies(g, 1) && g->nnz <= kSmallSingleNnz;
+  if (small) {
     LGBC_TRY(ensure_dist(g, g->n));
     LGBC_TRY(ensure_src(g, nsrc));
     LGBC_CUDA(cudaMemcpyAsync(g->d_src, src, static_cast<size_t>(nsrc) * 4, cudaMemcpyHostToDevice,
@@ -1453,11 +1455,12 @@ int lgbc_gdistances(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* di
   LGBC_CUDA(cudaMemcpyAsync(dist_out, g->d_dist, static_cast<size_t>(g->n) * 4,
                             cudaMemcpyDeviceToHost, g->stream));
   LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  if (!small) LGBC_TRY(finish_bfs(g));
   finish_stats(g);
   return LGBC_OK;
 }
 
-int lgbc_gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* dist_out) {
+int gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* dist_out) {
   LGBC_TRY(check_graph(g));
   std::lock_guard<std::mutex> lock(g->mu);
   LGBC_TRY(use_device(g));
@@ -1502,6 +1505,18 @@ int lgbc_gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32
   LGBC_CUDA(cudaStreamSynchronize(g->stream));
   finish_stats(g);
   return LGBC_OK;
+}
+
+}  // namespace lgbc::api
+
+extern "C" {
+
+int lgbc_gdistances(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* dist_out) {
+  return gdistances(g, src, nsrc, dist_out);
+}
+
+int lgbc_gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* dist_out) {
+  return gdistances_batch(g, src, nsrc, dist_out);
 }
 
 int lgbc_betweenness_dev(lgbc_graph* g, const int32_t* src, int64_t nsrc, int endpoints,

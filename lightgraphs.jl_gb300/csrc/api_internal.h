@@ -142,16 +142,14 @@ struct HubTable {
 
 struct BfsWorkspace {
   int32_t* queue = nullptr;
-  uint32_t* bm0 = nullptr;
-  uint32_t* bm1 = nullptr;
-  BatchCtl* ctl = nullptr;
-  int32_t* large = nullptr;
+  uint32_t* bits = nullptr;     // the visited bitmap and the three level bitmaps
+  int2* big = nullptr;          // the two lists of long out-lists
+  BfsState* state = nullptr;
   void release() {
-    dev_free(large);
     dev_free(queue);
-    dev_free(bm0);
-    dev_free(bm1);
-    dev_free(ctl);
+    dev_free(bits);
+    dev_free(big);
+    dev_free(state);
   }
 };
 
@@ -333,6 +331,7 @@ struct lgbc_graph {
   int64_t launches_at_start = 0;
   lgbc::LaunchCfg cfg{};
   size_t max_smem = 0;
+  size_t bfs_room = 0;              // shared memory the BFS may stage its bitmap in
   unsigned long long sigma_limit = ~0ull;  // (2^64 - 1) / (max in-degree + 1)
   lgbc_stats stats{};
   lgbc_tuning tune = lgbc::api::kDefaultTuning;
@@ -410,7 +409,12 @@ int finish_handle(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr
 // (run: everything but the graph).
 bool small_bfs_applies(const lgbc_graph* g, int64_t nsrc);
 int run_small_bfs(lgbc_graph* g, SmallBfs run);
-int run_bfs(lgbc_graph* g, const DevGraph& dg, int64_t nsrc);
+// Level-synchronous BFS over dg from g->d_src[0, nsrc) into g->d_dist.
+// prefilled: the caller has filled it (kUnreached, and any other value on
+// vertices the search must treat as already visited).  finish_bfs waits for
+// the stream and checks the search.
+int run_bfs(lgbc_graph* g, const DevGraph& dg, int64_t nsrc, bool prefilled = false);
+int finish_bfs(lgbc_graph* g);
 int prepare_bfs(lgbc_graph* g, const int32_t* src, int64_t nsrc);
 
 }  // namespace lgbc::api

@@ -256,7 +256,7 @@ extern "C" int lgbc_bfs_parents(lgbc_graph* g, int32_t s, int dir, int32_t* pare
   LGBC_TRY(check_launch(g));
   LGBC_CUDA(cudaMemcpyAsync(parents_out, d_par, static_cast<size_t>(g->n) * 4,
                             cudaMemcpyDeviceToHost, g->stream));
-  LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  LGBC_TRY(finish_bfs(g));
   finish_stats(g);
   return LGBC_OK;
 }
@@ -281,6 +281,7 @@ extern "C" int lgbc_has_path(lgbc_graph* g, int32_t u, int32_t v, const int32_t*
     return LGBC_OK;
   }
   LGBC_TRY(prepare_bfs(g, &u, 1));
+  if (nexclude > 0) g->launches += fill_i32(g->cfg, g->stream, g->d_dist, g->n, kUnreached);
   int32_t* d_ex = nullptr;
   if (nexclude > 0) {
     // excluded vertices count as visited from the start (a distance the BFS
@@ -291,10 +292,10 @@ extern "C" int lgbc_has_path(lgbc_graph* g, int32_t u, int32_t v, const int32_t*
     g->launches += scatter_i32(g->cfg, g->stream, g->d_dist, d_ex, nexclude, -2);
   }
   std::unique_ptr<int32_t, void (*)(int32_t*)> guard(d_ex, [](int32_t* q) { if (q) cudaFree(q); });
-  LGBC_TRY(run_bfs(g, g->dev(), 1));
+  LGBC_TRY(run_bfs(g, g->dev(), 1, nexclude > 0));
   int32_t dv = kUnreached;
   LGBC_CUDA(cudaMemcpyAsync(&dv, g->d_dist + v, 4, cudaMemcpyDeviceToHost, g->stream));
-  LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  LGBC_TRY(finish_bfs(g));
   *result = dv != kUnreached ? 1 : 0;
   finish_stats(g);
   return LGBC_OK;

@@ -6,17 +6,24 @@
 // INT32_MAX where nothing reaches it.  The per-level sort of the reference
 // (bfs.jl:121) only fixes visiting order and does not change any distance.
 //
-// Top-down levels expand the frontier queue over out-edges with degree-binned
-// thread mapping: a warp takes 32 frontier vertices and streams their
-// concatenated out-lists 32 edges at a time, so a lane never idles on a short
-// list; a vertex with more than kBfsLarge out-edges (an R-MAT hub has 65K) is
-// deferred to a list whose edges the whole grid expands in a second kernel.
-// atomicCAS on the distance claims a vertex once.
-// Bottom-up levels give each unvisited vertex one thread that scans its
-// in-edges and stops at the first in-neighbour in the frontier bitmap; the
-// bitmap is staged in shared memory when it fits, and a warp owns 32
-// consecutive vertices, so it writes one bitmap word of the next frontier
-// (its ballot) without atomics and appends its discoveries with one atomic.
+// A handle's search is one cooperative launch (k_bfs_run): one block per SM
+// runs every level, with a grid barrier between levels in place of three or
+// four launches and a host round trip.  Top-down levels expand the frontier
+// queue over out-edges: a warp streams the concatenated out-lists of up to 32
+// frontier vertices (fewer when the frontier is small, so that every warp has
+// some), and a vertex with more than kBfsChunk out-edges is cut into pieces of
+// that many edges which the whole grid shares.  The visited bitmap (n / 8
+// bytes) is tested before any atomic.  Bottom-up levels give each unvisited
+// vertex one thread that scans its in-edges and stops at the first
+// in-neighbour in the frontier bitmap, staged in shared memory when it fits; a
+// warp owns 32 consecutive vertices, hence one word of the visited and next
+// bitmaps, and needs no atomics at all: the queue of the new frontier is only
+// built when the next level goes top-down.
+// Bound: latency of the barriers and of dependent loads on the small levels,
+// in-edge sectors from HBM on the bottom-up ones.
+//
+// The kernels with one launch per level serve lgbc_gdistances_noalloc, whose
+// fixed scratch holds a queue and two bitmaps.
 #include <algorithm>
 
 #include "lgbc_kernels.h"
@@ -53,7 +60,6 @@ __global__ void k_bfs_ctl_reset(BatchCtl* c) {
   c->overflow_list = 0;
   c->overflow_sigma = 0;
   c->mode = 0;
-  c->large = 0;
 }
 
 // Level 0: claim each source once (duplicates in the source list are
@@ -86,11 +92,9 @@ __global__ void k_bfs_seed_done(BatchCtl* c) {
   }
 }
 
-// Zero the bitmap that the coming top-down level fills with atomicOr, and the
-// level's deferred-vertex count.
+// Zero the bitmap that the coming top-down level fills with atomicOr.
 __global__ void k_bfs_clear_next(BfsBuffers b, int64_t nwords) {
   uint32_t* nbm = bm_at(b, b.ctl->level + 1);
-  if (blockIdx.x == 0 && threadIdx.x == 0) b.ctl->large = 0;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < nwords;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
     nbm[i] = 0u;
@@ -117,11 +121,10 @@ __device__ __forceinline__ void bfs_flush_counts(BatchCtl* c, unsigned long long
   }
 }
 
-// Top-down level: lane j of a warp holds frontier entry base + j.  Vertices
-// with more than kBfsLarge out-edges go to b.large (when there is one); the
-// others' out-lists are walked as one concatenation, edge k of it by lane
-// k % 32 (the owning vertex found by a binary search over the warp's
-// inclusive degree scan).
+// Top-down level: lane j of a warp holds frontier entry base + j.  The 32
+// out-lists are walked as one concatenation, edge k of it by lane k % 32 (the
+// owning vertex found by a binary search over the warp's inclusive degree
+// scan).
 __global__ void __launch_bounds__(256) k_bfs_td(DevGraph g, BfsBuffers b, int32_t* dist) {
   BatchCtl* c = b.ctl;
   const unsigned long long lo = c->lo, hi = c->hi;
@@ -139,10 +142,7 @@ __global__ void __launch_bounds__(256) k_bfs_td(DevGraph g, BfsBuffers b, int32_
       e0 = g.rowptr[v];
       deg = g.rowptr[v + 1] - e0;
     }
-    const bool defer = b.large != nullptr && deg > kBfsLarge;
-    const unsigned long long slot = warp_append(defer, &c->large);
-    if (defer) b.large[slot] = v;
-    const int d = defer ? 0 : static_cast<int>(deg);
+    const int d = static_cast<int>(deg);
     int incl = d;
 #pragma unroll
     for (int o = 1; o < kWarp; o <<= 1) {
@@ -165,34 +165,6 @@ __global__ void __launch_bounds__(256) k_bfs_td(DevGraph g, BfsBuffers b, int32_
       int32_t w = 0;
       if (k < total) {
         w = g.colidx[ej + (k - oj)];
-        app = bfs_claim(g, nbm, dist, w, nl, mf, mu);
-      }
-      const unsigned long long q = warp_append(app, &c->tail);
-      if (app) b.queue[q] = w;
-    }
-  }
-  bfs_flush_counts(c, mf, mu);
-}
-
-// The deferred high-degree frontier vertices: for each in turn, the whole
-// grid walks its out-list (a warp takes 32 consecutive edges).
-__global__ void __launch_bounds__(256) k_bfs_td_large(DevGraph g, BfsBuffers b, int32_t* dist) {
-  BatchCtl* c = b.ctl;
-  const unsigned long long nlarge = c->large;
-  if (nlarge == 0) return;
-  const int32_t nl = c->level + 1;
-  uint32_t* nbm = bm_at(b, nl);
-  const int ln = lane_id();
-  unsigned long long mf = 0, mu = 0;
-  for (unsigned long long h = 0; h < nlarge; ++h) {
-    const int32_t v = b.large[h];
-    const int64_t e0 = g.rowptr[v], e1 = g.rowptr[v + 1];
-    for (int64_t e = e0 + gwarp() * kWarp; e < e1; e += nwarps() * kWarp) {
-      const int64_t idx = e + ln;
-      bool app = false;
-      int32_t w = 0;
-      if (idx < e1) {
-        w = g.colidx[idx];
         app = bfs_claim(g, nbm, dist, w, nl, mf, mu);
       }
       const unsigned long long q = warp_append(app, &c->tail);
@@ -267,6 +239,284 @@ __global__ void k_bfs_advance(BatchCtl* c) {
   c->mf = 0;
 }
 
+// ---------------------------------------------------------------------------
+// The whole search in one cooperative launch.
+// ---------------------------------------------------------------------------
+
+// Grid barrier: every block adds one to an ever-growing count and waits until
+// all have.  The wait is bounded: a block that gives up, or sees that another
+// has, reports it, and the kernel returns.  All blocks are resident (the
+// launch is cooperative), so that happens only if the GPU is wedged.
+constexpr unsigned kBarrierPolls = 1u << 23;  // some seconds
+
+__device__ __forceinline__ bool grid_barrier(BfsState* st, unsigned long long& goal, int* ok) {
+  __syncthreads();
+  goal += gridDim.x;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(&st->arrived, 1ull);
+    unsigned polls = 0;
+    while (*reinterpret_cast<volatile unsigned long long*>(&st->arrived) < goal &&
+           *reinterpret_cast<volatile int*>(&st->failed) == 0) {
+      if (++polls > kBarrierPolls) atomicExch(&st->failed, 1);
+    }
+    __threadfence();
+    *ok = *reinterpret_cast<volatile int*>(&st->failed) == 0;
+  }
+  __syncthreads();
+  return *ok != 0;
+}
+
+// What a thread has found in this level.
+struct BfsFound {
+  unsigned count = 0;
+  unsigned long long mf = 0, mu = 0;
+};
+
+// List w (claimed by this thread) for the next level; `lists` false: count it only.
+__device__ __forceinline__ void bfs_list(const DevGraph& g, const BfsRun& r, BfsSlot* slot,
+                                         unsigned long long base, int parity, bool claimed, int32_t w,
+                                         bool lists, BfsFound& f) {
+  int64_t d = 0;
+  if (claimed) {
+    d = g.rowptr[w + 1] - g.rowptr[w];
+    f.count += 1;
+    f.mf += static_cast<unsigned long long>(d);
+    f.mu += static_cast<unsigned long long>(g.in_rowptr[w + 1] - g.in_rowptr[w]);
+  }
+  if (!lists) return;
+  const bool big = d > kBfsChunk;
+  const unsigned long long at = warp_append(claimed && !big, &slot->queued);
+  if (claimed && !big) r.queue[base + at] = w;
+  if (big) {
+    // one atomic hands out the entry (high word) and its first chunk (low
+    // word), so the list is sorted by first chunk
+    const unsigned chunks = static_cast<unsigned>((d + kBfsChunk - 1) / kBfsChunk);
+    const unsigned long long p = atomicAdd(&slot->big, (1ull << 32) | chunks);
+    r.big[parity * r.big_cap + static_cast<int64_t>(p >> 32)] = make_int2(static_cast<int>(p & 0xFFFFFFFFu), w);
+  }
+}
+
+__device__ __forceinline__ bool bfs_take(const BfsRun& r, uint32_t* next, int32_t w, int32_t level) {
+  const uint32_t bit = 1u << (w & 31);
+  // a stale cached word can only lack bits, which the atomic then finds set
+  if (r.visited[w >> 5] & bit) return false;
+  if (atomicOr(r.visited + (w >> 5), bit) & bit) return false;
+  atomicOr(next + (w >> 5), bit);
+  r.dist[w] = level;
+  return true;
+}
+
+__global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
+  extern __shared__ uint32_t sbm[];
+  __shared__ int s_ok;
+  __shared__ unsigned long long s_sum[3];
+  BfsState* st = r.state;
+  const int ln = lane_id();
+  const int64_t n = g.n, nwords = (n + 31) >> 5;
+  const int64_t tid = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int64_t threads = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  const long long warp = gwarp(), warps = nwarps();
+  unsigned long long goal = 0;
+  auto bitmap = [&](int32_t level) { return r.visited + (1 + level % 3) * r.words; };
+
+  // fold a level's findings into its slot, one set of atomics per block
+  auto report = [&](BfsSlot* slot, const BfsFound& f) {
+    if (threadIdx.x < 3) s_sum[threadIdx.x] = 0ull;
+    __syncthreads();
+    const unsigned c = __reduce_add_sync(kFull, f.count);
+    const unsigned long long mf = warp_sum_u64(f.mf), mu = warp_sum_u64(f.mu);
+    if (ln == 0 && c) {
+      atomicAdd(&s_sum[0], static_cast<unsigned long long>(c));
+      atomicAdd(&s_sum[1], mf);
+      atomicAdd(&s_sum[2], mu);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_sum[0]) {
+      atomicAdd(&slot->count, s_sum[0]);
+      atomicAdd(&slot->mf, s_sum[1]);
+      atomicAdd(&slot->mu, s_sum[2]);
+    }
+  };
+
+  // distances, bitmaps (prefilled: distances other than kUnreached are
+  // vertices the search must leave alone)
+  for (int64_t w0 = warp * kWarp; w0 < nwords * kWarp; w0 += warps * kWarp) {
+    const int64_t v = w0 + ln;
+    bool seen = v >= n;
+    if (v < n) {
+      if (r.prefilled) seen = r.dist[v] != kUnreached;
+      else r.dist[v] = kUnreached;
+    }
+    const unsigned bal = __ballot_sync(kFull, seen);
+    if (ln == 0) {
+      r.visited[w0 >> 5] = bal;
+      bitmap(0)[w0 >> 5] = 0u;
+      bitmap(1)[w0 >> 5] = 0u;
+    }
+  }
+  if (!grid_barrier(st, goal, &s_ok)) return;
+  {
+    BfsFound f;
+    for (int64_t i0 = tid - ln; i0 < r.nsrc; i0 += threads) {
+      const int64_t i = i0 + ln;
+      const int32_t s = i < r.nsrc ? r.src[i] : 0;
+      const bool claimed = i < r.nsrc && bfs_take(r, bitmap(0), s, 0);
+      bfs_list(g, r, &st->slot[0], 0, 0, claimed, s, true, f);
+    }
+    report(&st->slot[0], f);
+  }
+  if (!grid_barrier(st, goal, &s_ok)) return;
+
+  unsigned long long lo = 0, mu_done = 0;
+  bool bu = false;
+  long long td_levels = 0, bu_levels = 0;
+  for (int32_t level = 0;; ++level) {
+    // a slot is reused three levels later, by when every block has read it
+    const BfsSlot* cur = &st->slot[level % 3];
+    BfsSlot* nxt = &st->slot[(level + 1) % 3];
+    const unsigned long long nf = __ldcg(&cur->count), mf = __ldcg(&cur->mf);
+    unsigned long long queued = __ldcg(&cur->queued), big = __ldcg(&cur->big);
+    mu_done += __ldcg(&cur->mu);
+    if (nf == 0 || level > n) break;
+    const bool was = bu;
+    const double left = static_cast<double>(g.nnz) - static_cast<double>(mu_done);
+    bu = was ? static_cast<double>(nf) >= static_cast<double>(n) / r.beta
+             : static_cast<double>(mf) > left / r.alpha;
+    uint32_t* front = bitmap(level);
+    uint32_t* next = bitmap(level + 1);
+    uint32_t* stale = bitmap(level + 2);
+    if (was && !bu) {
+      // the frontier exists only as a bitmap: list it, in this level's own slot
+      BfsSlot* own = &st->slot[level % 3];
+      BfsFound ignored;
+      for (int64_t w0 = warp * kWarp; w0 < nwords; w0 += warps * kWarp) {
+        uint32_t bits = w0 + ln < nwords ? __ldcg(front + w0 + ln) : 0u;
+        while (__any_sync(kFull, bits != 0u)) {
+          const bool has = bits != 0u;
+          const int32_t v = static_cast<int32_t>((w0 + ln) * kWarp + (has ? __ffs(bits) - 1 : 0));
+          bits &= bits - 1u;
+          bfs_list(g, r, own, lo, level & 1, has, v, true, ignored);
+        }
+      }
+      if (!grid_barrier(st, goal, &s_ok)) return;
+      queued = __ldcg(&own->queued);
+      big = __ldcg(&own->big);
+    }
+    // what the level after next will fill
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      BfsSlot* z = &st->slot[(level + 2) % 3];
+      z->count = z->mf = z->mu = z->queued = z->big = 0ull;
+    }
+    for (int64_t i = tid; i < nwords; i += threads) stale[i] = 0u;
+    const unsigned long long hi = lo + queued;
+    BfsFound f;
+    if (bu) {
+      ++bu_levels;
+      const uint32_t* fbm = front;
+      if (r.stage) {
+        const uint4* src4 = reinterpret_cast<const uint4*>(front);
+        uint4* dst4 = reinterpret_cast<uint4*>(sbm);
+        for (int64_t i = threadIdx.x; i < (nwords + 3) >> 2; i += blockDim.x) dst4[i] = __ldcg(src4 + i);
+        __syncthreads();
+        fbm = sbm;
+      }
+      for (int64_t w0 = warp; w0 < nwords; w0 += warps) {
+        const uint32_t seen = __ldcg(r.visited + w0);
+        if (seen == ~0u) {
+          if (ln == 0) next[w0] = 0u;
+          continue;
+        }
+        const int64_t v = (w0 << 5) + ln;
+        bool found = false;
+        if (!((seen >> ln) & 1u)) {
+          const int64_t e1 = g.in_rowptr[v + 1];
+          for (int64_t e = g.in_rowptr[v]; e < e1; ++e) {
+            const int32_t u = g.in_colidx[e];
+            const uint32_t word = r.stage ? fbm[u >> 5] : __ldcg(fbm + (u >> 5));
+            if ((word >> (u & 31)) & 1u) {
+              found = true;
+              break;
+            }
+          }
+        }
+        const unsigned bal = __ballot_sync(kFull, found);
+        if (ln == 0) {
+          next[w0] = bal;
+          if (bal) r.visited[w0] = seen | bal;
+        }
+        if (found) r.dist[v] = level + 1;
+        bfs_list(g, r, nxt, hi, (level + 1) & 1, found, static_cast<int32_t>(v), false, f);
+      }
+    } else {
+      ++td_levels;
+      // vertices a warp takes at a time: all warps get some
+      int per = static_cast<int>((queued + static_cast<unsigned long long>(warps) - 1) /
+                                 static_cast<unsigned long long>(warps));
+      per = per < 1 ? 1 : (per > kWarp ? kWarp : per);
+      for (unsigned long long base = lo + static_cast<unsigned long long>(warp) * per; base < hi;
+           base += static_cast<unsigned long long>(warps) * per) {
+        const unsigned long long i = base + ln;
+        int64_t e0 = 0;
+        int d = 0;
+        if (ln < per && i < hi) {
+          const int32_t v = __ldcg(r.queue + i);
+          e0 = g.rowptr[v];
+          d = static_cast<int>(g.rowptr[v + 1] - e0);
+        }
+        int incl = d;
+#pragma unroll
+        for (int o = 1; o < kWarp; o <<= 1) {
+          const int y = __shfl_up_sync(kFull, incl, o);
+          if (ln >= o) incl += y;
+        }
+        const int total = __shfl_sync(kFull, incl, kWarp - 1);
+        const int off = incl - d;
+        for (int k0 = 0; k0 < total; k0 += kWarp) {
+          const int k = k0 + ln;
+          int j = 0;  // the lane whose list holds concatenated edge k
+#pragma unroll
+          for (int step = 16; step >= 1; step >>= 1) {
+            const int iv = __shfl_sync(kFull, incl, j + step - 1);
+            if (iv <= k) j += step;
+          }
+          const int64_t ej = shfl_i64(e0, j);
+          const int oj = __shfl_sync(kFull, off, j);
+          const int32_t w = k < total ? g.colidx[ej + (k - oj)] : 0;
+          const bool claimed = k < total && bfs_take(r, next, w, level + 1);
+          if (__any_sync(kFull, claimed)) bfs_list(g, r, nxt, hi, (level + 1) & 1, claimed, w, true, f);
+        }
+      }
+      const long long entries = static_cast<long long>(big >> 32), chunks = static_cast<long long>(big & 0xFFFFFFFFull);
+      const int2* list = r.big + (level & 1) * r.big_cap;
+      for (long long c = warp; c < chunks; c += warps) {
+        long long a = 0, b = entries - 1;  // the last entry whose first chunk is at most c
+        while (a < b) {
+          const long long mid = (a + b + 1) >> 1;
+          if (__ldcg(&list[mid]).x <= c) a = mid;
+          else b = mid - 1;
+        }
+        const int2 en = __ldcg(&list[a]);
+        const int64_t e0 = g.rowptr[en.y] + (c - en.x) * kBfsChunk;
+        const int64_t e1 = min(e0 + kBfsChunk, g.rowptr[en.y + 1]);
+        for (int64_t e = e0; e < e1; e += kWarp) {
+          const int64_t idx = e + ln;
+          const int32_t w = idx < e1 ? g.colidx[idx] : 0;
+          const bool claimed = idx < e1 && bfs_take(r, next, w, level + 1);
+          if (__any_sync(kFull, claimed)) bfs_list(g, r, nxt, hi, (level + 1) & 1, claimed, w, true, f);
+        }
+      }
+    }
+    report(nxt, f);
+    lo = hi;
+    if (!grid_barrier(st, goal, &s_ok)) return;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->td_levels = td_levels;
+    st->bu_levels = bu_levels;
+  }
+}
+
 // _bfs_parents (src/traversals/bfs.jl:40-66) visits each level in sorted
 // vertex order and gives a newly reached vertex the first level vertex that
 // lists it, i.e. the smallest in-neighbour one level closer; the source is
@@ -310,10 +560,26 @@ __global__ void k_scatter_i32(int32_t* p, const int32_t* idx, int64_t count, int
 
 }  // namespace
 
-int bfs_configure(size_t max_dyn_smem) {
+size_t bfs_configure(size_t max_dyn_smem) {
   cudaFuncSetAttribute(k_bfs_bu<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        static_cast<int>(max_dyn_smem));
-  return 0;
+  cudaFuncAttributes fa{};
+  size_t room = 0;
+  if (cudaFuncGetAttributes(&fa, k_bfs_run) == cudaSuccess && max_dyn_smem > fa.sharedSizeBytes)
+    room = max_dyn_smem - fa.sharedSizeBytes;
+  cudaFuncSetAttribute(k_bfs_run, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(room));
+  return room;
+}
+
+int bfs_run(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, BfsRun r, size_t room) {
+  cudaMemsetAsync(r.state, 0, sizeof(BfsState), s);
+  const size_t bytes = static_cast<size_t>((((g.n + 31) >> 5) + 3) & ~int64_t(3)) * 4;
+  r.stage = bytes <= room ? 1 : 0;
+  DevGraph dg = g;
+  void* args[] = {&dg, &r};
+  cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_bfs_run), dim3(static_cast<unsigned>(c.sms)), dim3(1024),
+                              args, r.stage ? bytes : 0, s);
+  return 1;
 }
 
 int bfs_init(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, const BfsBuffers& b,
@@ -337,9 +603,7 @@ int bfs_topdown(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, const Bfs
   const int64_t nwords = (g.n + 31) >> 5;
   k_bfs_clear_next<<<c.grid, c.block, 0, s>>>(b, nwords);
   k_bfs_td<<<c.grid, c.block, 0, s>>>(g, b, dist);
-  if (!b.large) return 2;
-  k_bfs_td_large<<<c.grid, c.block, 0, s>>>(g, b, dist);
-  return 3;
+  return 2;
 }
 
 int bfs_bottomup(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, const BfsBuffers& b,

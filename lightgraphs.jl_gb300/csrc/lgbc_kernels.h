@@ -259,14 +259,42 @@ int small_sums(cudaStream_t s, const SmallGraph* graphs, const SmallSum* sums, i
                const ulonglong2* part, double* out);
 
 // ---- single multi-source BFS (gdistances): bfs.cu ------------------------
+// One level per launch (lgbc_gdistances_noalloc).
 struct BfsBuffers {
   int32_t* queue;               // n: every level, concatenated
   uint32_t* bm[2];              // (n + 31) / 32 words each: frontier bitmaps
   BatchCtl* ctl;
-  int32_t* large = nullptr;     // n or null: frontier vertices with more than kBfsLarge
-                                // out-edges, expanded by the whole grid (null: by one warp)
 };
-constexpr int kBfsLarge = 1024;
+// A whole search in one cooperative launch.
+constexpr int kBfsChunk = 256;  // out-edges a warp takes of a long list
+struct BfsSlot {                // one level's frontier, rotating over three
+  unsigned long long count, mf, mu;  // vertices, their out-edges and in-edges
+  unsigned long long queued;         // those listed in the queue
+  unsigned long long big;            // entries << 32 | chunks of the list of long out-lists
+};
+struct BfsState {               // zeroed before the launch
+  unsigned long long arrived;   // grid barrier
+  int failed;
+  BfsSlot slot[3];
+  long long td_levels, bu_levels;
+};
+struct BfsRun {
+  int32_t* dist;                // n
+  const int32_t* src;
+  int64_t nsrc;
+  int prefilled;                // 1: the caller filled dist (kUnreached, or another value where
+                                // the search must not go); 0: filled here
+  int32_t* queue;               // n
+  uint32_t* visited;            // the visited bitmap and three level bitmaps of `words` words
+  int64_t words;                //   (a multiple of 4, at least (n + 31) / 32)
+  int2* big;                    // two lists of big_cap entries: (first chunk, vertex)
+  int64_t big_cap;              // at least nnz / kBfsChunk + 1
+  BfsState* state;
+  double alpha, beta;
+  int stage;                    // set by bfs_run: the frontier bitmap fits shared memory
+};
+// room: bfs_configure's result.
+int bfs_run(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, BfsRun r, size_t room);
 int bfs_init(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, const BfsBuffers& b,
              const int32_t* src, int64_t nsrc, int32_t* dist);
 int bfs_topdown(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, const BfsBuffers& b,
@@ -281,8 +309,8 @@ int bfs_parents(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, const int
 // p[idx[i]] = value for i < count.
 int scatter_i32(const LaunchCfg& c, cudaStream_t s, int32_t* p, const int32_t* idx, int64_t count,
                 int32_t value);
-// Largest dynamic shared memory the bottom-up kernel may stage (bytes).
-int bfs_configure(size_t max_dyn_smem);
+// Opt the kernels into the device's shared memory; the bytes k_bfs_run may stage.
+size_t bfs_configure(size_t max_dyn_smem);
 
 // Set the thread-local message returned by lgbc_last_error() (api.cu).
 void set_last_error(const char* msg);
