@@ -79,6 +79,11 @@ int lgbc_graph_info(const lgbc_graph *g, int64_t *n, int64_t *nnz, int *directed
 int lgbc_gdistances(lgbc_graph *g, const int32_t *src, int64_t nsrc,
                     int32_t *dist_out /* n */);
 
+/* The same in 64 bits, INT64_MAX where no source reaches: gdistances of a
+ * graph with Int64 vertex ids (typemax(T), src/traversals/bfs.jl:141). */
+int lgbc_gdistances64(lgbc_graph* g, const int32_t* src, int64_t nsrc,
+                      int64_t* dist_out /* n */);
+
 /* nsrc independent single-source gdistances, one per source, written as
  * dist_out[i * n + v] (row i = source i).  Runs sources as bit lanes of a
  * multi-source BFS that shares every edge read. */

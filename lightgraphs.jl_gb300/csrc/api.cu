@@ -1358,6 +1358,7 @@ int lgbc_graph_destroy(lgbc_graph* g) {
   dev_free(g->d_src);
   dev_free(g->d_bc);
   dev_free(g->d_dist);
+  dev_free(g->d_wide);
   dev_free(g->d_lmdist);
   dev_free(g->d_lw_fixed);
   if (g->h_ctl) cudaFreeHost(g->h_ctl);
@@ -1424,11 +1425,31 @@ int prepare_bfs(lgbc_graph* g, const int32_t* src, int64_t nsrc) {
   return LGBC_OK;
 }
 
+// g->d_dist[0, count) to out[at, at + count) on the host: as it is, or in 64
+// bits with typemax(Int64) where nothing reaches.
+int copy_dist(lgbc_graph* g, void* out, int64_t at, int64_t count, bool wide) {
+  const size_t bytes = static_cast<size_t>(count) * (wide ? 8 : 4);
+  const void* from = g->d_dist;
+  if (wide) {
+    if (count > g->d_wide_cap) {
+      dev_free(g->d_wide);
+      g->d_wide_cap = 0;
+      LGBC_TRY(dev_alloc(&g->d_wide, static_cast<size_t>(count)));
+      g->d_wide_cap = count;
+    }
+    g->launches += widen_dist(g->cfg, g->stream, g->d_dist, count, g->d_wide);
+    from = g->d_wide;
+  }
+  LGBC_CUDA(cudaMemcpyAsync(static_cast<char*>(out) + at * (wide ? 8 : 4), from, bytes, cudaMemcpyDeviceToHost,
+                            g->stream));
+  return LGBC_OK;
+}
+
 // One search on one SM against the whole grid with a barrier per level: equal
 // at 144,000 entries (104 against 107 us), 55 against 107 us at 96,000.
 constexpr int64_t kSmallSingleNnz = int64_t(1) << 17;
 
-int gdistances(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* dist_out) {
+int gdistances(lgbc_graph* g, const int32_t* src, int64_t nsrc, void* dist_out, bool wide) {
   LGBC_TRY(check_graph(g));
   std::lock_guard<std::mutex> lock(g->mu);
   LGBC_TRY(use_device(g));
@@ -1452,15 +1473,14 @@ int gdistances(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* dist_ou
     LGBC_TRY(prepare_bfs(g, src, nsrc));
     LGBC_TRY(run_bfs(g, g->dev(), nsrc));
   }
-  LGBC_CUDA(cudaMemcpyAsync(dist_out, g->d_dist, static_cast<size_t>(g->n) * 4,
-                            cudaMemcpyDeviceToHost, g->stream));
+  LGBC_TRY(copy_dist(g, dist_out, 0, g->n, wide));
   LGBC_CUDA(cudaStreamSynchronize(g->stream));
   if (!small) LGBC_TRY(finish_bfs(g));
   finish_stats(g);
   return LGBC_OK;
 }
 
-int gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* dist_out) {
+int gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, void* dist_out, bool wide) {
   LGBC_TRY(check_graph(g));
   std::lock_guard<std::mutex> lock(g->mu);
   LGBC_TRY(use_device(g));
@@ -1481,9 +1501,7 @@ int gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* d
       run.nsrc = static_cast<int>(std::min(rows, nsrc - s0));
       run.dist = g->d_dist;
       LGBC_TRY(run_small_bfs(g, run));
-      LGBC_CUDA(cudaMemcpyAsync(dist_out + s0 * g->n, g->d_dist,
-                                static_cast<size_t>(run.nsrc) * static_cast<size_t>(g->n) * 4,
-                                cudaMemcpyDeviceToHost, g->stream));
+      LGBC_TRY(copy_dist(g, dist_out, s0 * g->n, run.nsrc * g->n, wide));
       g->stats.batches++;
     }
     LGBC_CUDA(cudaStreamSynchronize(g->stream));
@@ -1497,9 +1515,7 @@ int gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* d
     const int nl = static_cast<int>(std::min<int64_t>(lanes, nsrc - s0));
     g->launches += fill_i32(g->cfg, g->stream, g->d_dist, static_cast<int64_t>(nl) * g->n, kUnreached);
     LGBC_TRY(run_ms_batch(g, g->d_src + s0, nl, kSigmaNone, nullptr, g->d_dist, g->n));
-    LGBC_CUDA(cudaMemcpyAsync(dist_out + s0 * g->n, g->d_dist,
-                              static_cast<size_t>(nl) * static_cast<size_t>(g->n) * 4,
-                              cudaMemcpyDeviceToHost, g->stream));
+    LGBC_TRY(copy_dist(g, dist_out, s0 * g->n, nl * g->n, wide));
     g->stats.batches++;
   }
   LGBC_CUDA(cudaStreamSynchronize(g->stream));
@@ -1512,11 +1528,19 @@ int gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* d
 extern "C" {
 
 int lgbc_gdistances(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* dist_out) {
-  return gdistances(g, src, nsrc, dist_out);
+  return gdistances(g, src, nsrc, dist_out, false);
+}
+
+int lgbc_gdistances64(lgbc_graph* g, const int32_t* src, int64_t nsrc, int64_t* dist_out) {
+  return gdistances(g, src, nsrc, dist_out, true);
 }
 
 int lgbc_gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, int32_t* dist_out) {
-  return gdistances_batch(g, src, nsrc, dist_out);
+  return gdistances_batch(g, src, nsrc, dist_out, false);
+}
+
+int lgbc_gdistances_batch64(lgbc_graph* g, const int32_t* src, int64_t nsrc, int64_t* dist_out) {
+  return gdistances_batch(g, src, nsrc, dist_out, true);
 }
 
 int lgbc_betweenness_dev(lgbc_graph* g, const int32_t* src, int64_t nsrc, int endpoints,

@@ -325,6 +325,8 @@ struct lgbc_graph {
   double* d_bc = nullptr;           // device result buffer for host-buffer calls
   int32_t* d_dist = nullptr;        // device distance buffer (gdistances)
   int64_t d_dist_cap = 0;
+  int64_t* d_wide = nullptr;        // the same in 64 bits
+  int64_t d_wide_cap = 0;
   lgbc::BatchCtl* h_ctl = nullptr;        // pinned mirror of a control block
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   int64_t launches = 0;             // running count of kernels launched

@@ -320,6 +320,8 @@ void set_last_error(const char* msg);
 // [0, n), 4 = rowptr[0] != 0 or rowptr[n] != nnz.
 int validate_csr(const LaunchCfg& c, cudaStream_t s, const int64_t* rowptr, const int32_t* colidx,
                  int64_t n, int64_t nnz, int* bad);
+// out[i] = in[i] in 64 bits, INT64_MAX where in[i] is kUnreached (16-byte aligned arrays).
+int widen_dist(const LaunchCfg& c, cudaStream_t s, const int32_t* in, int64_t count, int64_t* out);
 int fill_i32(const LaunchCfg& c, cudaStream_t s, int32_t* p, int64_t count, int32_t value);
 // The CSR of a disjoint union of `copies` copies of an n-vertex graph (copy
 // r = vertices [r n, (r + 1) n)): rp1[copies n + 1], c1[copies nnz]; n > 0.

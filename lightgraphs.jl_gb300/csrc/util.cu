@@ -1,4 +1,6 @@
 // util.cu -- fills and the endpoint terms of the betweenness accumulation.
+#include <algorithm>
+
 #include "lgbc_kernels.h"
 
 namespace lgbc {
@@ -150,6 +152,30 @@ int sum_copies(const LaunchCfg& c, cudaStream_t s, const double* stacked, int64_
                double* out) {
   if (n <= 0) return 0;
   k_sum_copies<<<c.grid, c.block, 0, s>>>(stacked, n, copies, out);
+  return 1;
+}
+
+namespace {
+// Distances in 64 bits, typemax(Int64) where kUnreached (both arrays start on
+// 16-byte boundaries; a stream, bound by HBM).
+__global__ void k_widen_dist(const int32_t* __restrict__ in, int64_t count, long long* __restrict__ out) {
+  const int64_t quads = count >> 2;
+  auto wide = [](int32_t d) { return d == kUnreached ? INT64_MAX : static_cast<long long>(d); };
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < quads;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int4 d = reinterpret_cast<const int4*>(in)[i];
+    reinterpret_cast<longlong2*>(out)[2 * i] = make_longlong2(wide(d.x), wide(d.y));
+    reinterpret_cast<longlong2*>(out)[2 * i + 1] = make_longlong2(wide(d.z), wide(d.w));
+  }
+  const int64_t t = (quads << 2) + threadIdx.x;
+  if (blockIdx.x == 0 && t < count) out[t] = wide(in[t]);
+}
+}  // namespace
+
+int widen_dist(const LaunchCfg& c, cudaStream_t s, const int32_t* in, int64_t count, int64_t* out) {
+  if (count <= 0) return 0;
+  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(c.grid, (count / 4 + c.block - 1) / c.block));
+  k_widen_dist<<<static_cast<int>(blocks), c.block, 0, s>>>(in, count, reinterpret_cast<long long*>(out));
   return 1;
 }
 

@@ -88,7 +88,9 @@ def _declare(lib) -> None:
         "lgbc_graph_info": ([p, ctypes.POINTER(i64), ctypes.POINTER(i64),
                              ctypes.POINTER(c_int)], c_int),
         "lgbc_gdistances": ([p, p, i64, p], c_int),
+        "lgbc_gdistances64": ([p, p, i64, p], c_int),
         "lgbc_gdistances_batch": ([p, p, i64, p], c_int),
+        "lgbc_gdistances_batch64": ([p, p, i64, p], c_int),
         "lgbc_betweenness": ([p, p, i64, c_int, p], c_int),
         "lgbc_path_counts": ([p, p, i64, p, p], c_int),
         "lgbc_betweenness_dev": ([p, p, i64, c_int, p], c_int),

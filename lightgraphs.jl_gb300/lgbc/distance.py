@@ -47,13 +47,12 @@ def closeness_centrality(g, distmx=None, *, normalize: bool = True) -> np.ndarra
     out = np.zeros(n, np.float64)
     act = np.flatnonzero(g.degrees() > 0).astype(np.int32)
     reached, dsum, _ = distance_stats(g, act)
-    for u, r, s in zip(act.tolist(), reached.tolist(), dsum.tolist()):
-        l = r - 1
-        if s > 0:
-            c = l / s
-            if normalize:
-                c *= l / (n - 1)
-            out[u] = c
+    far = dsum > 0
+    l = (reached[far] - 1).astype(np.float64)  # exact, as the sums are below 2^53
+    c = l / dsum[far]
+    if normalize:
+        c *= l / (n - 1)
+    out[act[far]] = c
     return out
 
 

@@ -33,18 +33,27 @@ def _as_sources(g, source) -> np.ndarray:
     return _sources0(g, source)
 
 
-def _device_levels(g, src0: np.ndarray) -> np.ndarray:
-    """int32 levels from the GPU BFS; INT32_MAX marks unreached."""
-    out = np.empty(g.nv(), np.int32)
+def _device_levels(g, src0: np.ndarray, dtype=np.int32) -> np.ndarray:
+    """Levels from the GPU BFS in int32 or int64; its typemax marks unreached."""
+    out = np.empty(g.nv(), dtype)
     if g.nv() == 0:
         return out
     h = g.device_handle()
     src = np.ascontiguousarray(src0, np.int32)
-    _lib.check(_lib.lib().lgbc_gdistances(h.handle, _lib.ptr(src), len(src), _lib.ptr(out)))
+    lib = _lib.lib()
+    call = lib.lgbc_gdistances64 if out.dtype == np.int64 else lib.lgbc_gdistances
+    _lib.check(call(h.handle, _lib.ptr(src), len(src), _lib.ptr(out)))
     return out
 
 
+def _device_type(dtype):
+    """The type the library writes distances in for a graph of this eltype."""
+    return np.int64 if np.dtype(dtype) == np.int64 else np.int32
+
+
 def _to_eltype(levels: np.ndarray, dtype) -> np.ndarray:
+    if levels.dtype == np.dtype(dtype):  # unreached is typemax already
+        return levels
     out = levels.astype(dtype)
     out[levels == _lib.UNREACHED] = _typemax(dtype)
     return out
@@ -52,7 +61,7 @@ def _to_eltype(levels: np.ndarray, dtype) -> np.ndarray:
 
 def gdistances(g, source, *, sort_alg=None) -> np.ndarray:
     """Drop-in for LightGraphs.gdistances (bfs.jl:141)."""
-    lv = _device_levels(g, _as_sources(g, source))
+    lv = _device_levels(g, _as_sources(g, source), _device_type(g.eltype))
     return _to_eltype(lv, g.eltype)
 
 
@@ -74,11 +83,12 @@ def multi_gdistances(g, sources) -> np.ndarray:
     them as bit lanes of one BFS (lgbc_gdistances_batch)."""
     src = _sources0(g, sources)
     n = g.nv()
-    out = np.empty((len(src), n), np.int32)
+    out = np.empty((len(src), n), _device_type(g.eltype))
     if len(src) and n:
         h = g.device_handle()
-        _lib.check(_lib.lib().lgbc_gdistances_batch(h.handle, _lib.ptr(src), len(src),
-                                                    _lib.ptr(out)))
+        lib = _lib.lib()
+        call = lib.lgbc_gdistances_batch64 if out.dtype == np.int64 else lib.lgbc_gdistances_batch
+        _lib.check(call(h.handle, _lib.ptr(src), len(src), _lib.ptr(out)))
     return _to_eltype(out, g.eltype)
 
 
