@@ -46,6 +46,28 @@ __device__ __forceinline__ long long nwarps() {
   return (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
 }
 
+// Work of a gather kernel, handed out to warps in pieces as they come free:
+// rows differ by the hundredfold in cost, and with a fixed share per warp the
+// SMs held 23 of their 32 warps on average.  The next piece is asked for
+// before the current one is worked on.
+struct WorkQueue {
+  unsigned long long* next;
+  unsigned long long step, ahead;
+  __device__ __forceinline__ WorkQueue(unsigned long long* counter, unsigned step_) : next(counter), step(step_) {
+    ask();
+  }
+  __device__ __forceinline__ void ask() {
+    ahead = 0;
+    if (step && lane_id() == 0) ahead = atomicAdd(next, step);
+  }
+  // First item of the next piece (warp-uniform).
+  __device__ __forceinline__ unsigned long long take() {
+    const unsigned long long at = shfl_u64(ahead, 0);
+    ask();
+    return at;
+  }
+};
+
 // Level-parity buffer select (a runtime index into the by-value array would
 // force the parameter struct into local memory).
 __device__ __forceinline__ uint64_t* mb_at(const MsBuffers& b, int level) {
@@ -853,6 +875,7 @@ __global__ void __launch_bounds__(kWideLanes) k_ms_init(DevGraph g, MsBuffers b,
   c->td_levels = 0;
   c->bu_levels = 0;
   c->runaway = 0;
+  c->work[0] = c->work[1] = 0ull;
   for (int j = 0; j < kMaxWords; ++j) {
     c->front_union[j] = j < W ? act.w[j % W] : 0ull;
     c->next_union[j] = 0ull;
@@ -944,7 +967,8 @@ __global__ void __launch_bounds__(256, W == 4 ? 3 : 4) k_ms_td_settle(DevGraph g
   Lanes<W>* visit = lanes_of<W>(b.visit);
   const int ln = lane_id();
   unsigned long long mf = 0, mu = 0, smax = 0;
-  for (unsigned long long i = lo + gwarp(); i < hi; i += nwarps()) {
+  WorkQueue wq(&c->work[0], 1);
+  for (unsigned long long i = lo + wq.take(); i < hi; i = lo + wq.take()) {
     const int32_t w = b.qv[i];
     const Lanes<W> mask = next[w];
     const int64_t e0 = g.in_rowptr[w], e1 = g.in_rowptr[w + 1];
@@ -1003,7 +1027,8 @@ __global__ void __launch_bounds__(256, W == 4 ? 3 : 4) k_ms_bu(DevGraph g, MsBuf
     if (threadIdx.x == 0) live = frontier_lanes<W>(c);
     __syncthreads();
   }
-  for (int64_t base = gwarp() * kWarp; base < n; base += nwarps() * kWarp) {
+  WorkQueue wq(&c->work[0], kWarp);
+  for (int64_t base = static_cast<int64_t>(wq.take()); base < n; base = static_cast<int64_t>(wq.take())) {
     const int64_t wme = base + ln;
     bool cand = false;
     my_found[ln] = lz<W>();
@@ -1072,7 +1097,10 @@ __global__ void __launch_bounds__(256, W == 4 ? 3 : 4) k_ms_hub_pull(DevGraph g,
   Lanes<W>* visit = lanes_of<W>(b.visit);
   const int ln = lane_id();
   unsigned long long mf = 0, mu = 0, smax = 0;
-  for (long long it = gwarp(); it < hd.n_in; it += nwarps()) {
+  // top-down few hubs take part and most items only look: fixed shares
+  WorkQueue wq(&c->work[1], BU ? 1 : 0);
+  for (long long it = BU ? static_cast<long long>(wq.take()) : gwarp(); it < hd.n_in;
+       it = BU ? static_cast<long long>(wq.take()) : it + nwarps()) {
     const HubItem I = hd.in_items[it];
     const int32_t h = I.v;
     Lanes<W> vis = lz<W>(), want;
@@ -1231,12 +1259,14 @@ __global__ void k_loop_back_arm(MsBuffers b, LoopParams lp) {
 __global__ void k_loop_back_advance(MsBuffers b, LoopParams lp) {
   BatchCtl* c = b.ctl;
   c->level -= 1;
+  c->work[0] = c->work[1] = 0ull;
   cudaGraphSetConditional(lp.loop, c->level >= 0 ? 1u : 0u);
 }
 
 __device__ __forceinline__ void advance_step(const MsBuffers& b, int64_t n) {
   BatchCtl* c = b.ctl;
   const int L = c->level;
+  c->work[0] = c->work[1] = 0ull;
   b.lvl_off[L + 2] = c->tail;
   // every count of level L + 1 is a sum of at most max-in-degree counts of
   // level L; once a level's largest count passes the limit, the next level
@@ -1294,7 +1324,8 @@ __global__ void __launch_bounds__(256, W == 1 ? 5 : (W == 2 ? 4 : 3)) k_ms_delta
   const Lanes<W>* qm = lanes_of<W>(b.qm);
   Lanes<W>* visit = lanes_of<W>(b.visit);
   const int ln = lane_id();
-  for (unsigned long long i = lo + gwarp(); i < hi; i += nwarps()) {
+  WorkQueue wq(&c->work[0], 1);
+  for (unsigned long long i = lo + wq.take(); i < hi; i = lo + wq.take()) {
     const int32_t v = b.qv[i];
     const Lanes<W> F = qm[i];
     if (ln == 0) {
@@ -1347,7 +1378,8 @@ __global__ void __launch_bounds__(256, W == 1 ? 5 : (W == 2 ? 4 : 3)) k_ms_hub_d
   const Lanes<W>* __restrict__ succ = mbw<W>(b, L + 1);
   const Lanes<W>* __restrict__ cur = mbw<W>(b, L);
   const int ln = lane_id();
-  for (long long it = gwarp(); it < hd.n_out; it += nwarps()) {
+  WorkQueue wq(&c->work[1], 1);
+  for (long long it = static_cast<long long>(wq.take()); it < hd.n_out; it = static_cast<long long>(wq.take())) {
     const HubItem I = hd.out_items[it];
     const int32_t h = I.v;
     const Lanes<W> F = cur[h];
@@ -1763,7 +1795,10 @@ __global__ void __launch_bounds__(256) k_st_hub_count(DevGraph g, MsBuffers b, H
   }
 }
 
-__global__ void k_ms_back_advance(MsBuffers b) { b.ctl->level -= 1; }
+__global__ void k_ms_back_advance(MsBuffers b) {
+  b.ctl->level -= 1;
+  b.ctl->work[0] = b.ctl->work[1] = 0ull;
+}
 
 // End of a Brandes batch: the backward sweep cleared visit for every listed
 // vertex; clear the dense masks of levels 0 and 1 that remain.
@@ -1981,6 +2016,7 @@ __global__ void k_ms_init_seeds_ctl(MsBuffers b, long long nseeds, unsigned long
   c->td_levels = 0;
   c->bu_levels = 0;
   c->runaway = 0;
+  c->work[0] = c->work[1] = 0ull;
   for (int j = 0; j < kMaxWords; ++j) {
     c->front_union[j] = ~0ull;  // every lane may be seeded
     c->next_union[j] = 0ull;
