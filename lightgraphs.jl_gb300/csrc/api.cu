@@ -74,20 +74,11 @@ int ensure_ms(lgbc_graph* g, bool need_sigma, int words) {
   if (need_sigma && w.sigma_words < words) {
     LGBC_CUDA(cudaStreamSynchronize(g->stream));
     if (w.sigma) cudaFree(w.sigma);
-    if (w.psi) cudaFree(w.psi);
-    w.sigma = w.psi = nullptr;
+    w.sigma = nullptr;
     w.sigma_words = 0;
-    const size_t row = static_cast<size_t>(64) * static_cast<size_t>(words);
     unsigned long long* s = nullptr;
-    unsigned long long* p = nullptr;
-    LGBC_TRY(dev_alloc(&s, n * row));
-    int rc = dev_alloc(&p, n * row);
-    if (rc != LGBC_OK) {
-      cudaFree(s);
-      return rc;
-    }
+    LGBC_TRY(dev_alloc(&s, n * static_cast<size_t>(64) * static_cast<size_t>(words)));
     w.sigma = s;
-    w.psi = p;
     w.sigma_words = words;
   }
   return LGBC_OK;
@@ -315,7 +306,7 @@ MsBuffers ms_buffers(lgbc_graph* g, const int32_t* lane_src, const double* lane_
   b.mb[0] = w.mb0;
   b.mb[1] = w.mb1;
   b.sigma = w.sigma;
-  b.psi = w.psi;
+  b.psi = w.sigma;  // the backward sweep turns each path count into its psi in place
   b.qv = w.qv;
   b.qm = w.qm;
   b.lvl_off = w.lvl_off;

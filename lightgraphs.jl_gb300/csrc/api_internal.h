@@ -83,13 +83,12 @@ int parallel_parts(int64_t n, F&& f) {
 }
 
 // Multi-source workspace (msbfs.cu): lane sets sized for two words per
-// vertex / list entry; path-count and psi rows for `sigma_words` words.
+// vertex / list entry; path-count / psi rows for `sigma_words` words.
 struct MsWorkspace {
   uint64_t* visit = nullptr;
   uint64_t* mb0 = nullptr;
   uint64_t* mb1 = nullptr;
   void* sigma = nullptr;
-  void* psi = nullptr;
   int32_t* qv = nullptr;
   uint64_t* qm = nullptr;
   unsigned long long* lvl_off = nullptr;
@@ -103,8 +102,7 @@ struct MsWorkspace {
     dev_free(mb0);
     dev_free(mb1);
     if (sigma) cudaFree(sigma);
-    if (psi) cudaFree(psi);
-    sigma = psi = nullptr;
+    sigma = nullptr;
     dev_free(qv);
     dev_free(qm);
     dev_free(lvl_off);
