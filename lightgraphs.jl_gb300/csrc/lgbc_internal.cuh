@@ -54,6 +54,7 @@ struct BatchCtl {
   // outside it discovers nothing at level L + 1, so bottom-up scans skip it
   unsigned long long front_union[kMaxWords];
   unsigned long long work[2];     // next piece of the level's list or vertex range / hub items
+  int hubs;                       // a hub takes part in this level (bottom-up, backward)
   unsigned long long next_union[kMaxWords];  // lanes of Q_{L+1}, accumulated after its appends
 };
 

@@ -325,9 +325,11 @@ template <class A, int K> __device__ __forceinline__ void zero_accs(A (&a)[K]) {
 }
 
 // Per-warp staging of one chunk's contributing edges (compacted).
-template <int W> struct ChunkStage {
-  Lanes<W> f[kWarp];
-  int32_t v[kWarp];
+// The walks read a few entries at a time: kStageTail empty ones may follow.
+constexpr int kStageTail = 4;
+template <int W> struct alignas(16) ChunkStage {
+  Lanes<W> f[kWarp + kStageTail];
+  int32_t v[kWarp + kStageTail];
   int32_t j[kWarp];  // owner segment (seg_gather)
 };
 constexpr int kWarpsPerBlock = 8;  // every gather kernel runs 256-thread blocks
@@ -366,25 +368,55 @@ __device__ __forceinline__ void gather_chunk(int32_t nb, const Lanes<W>& f, cons
       st.v[r] = nb;
       st.f[r] = f;
     }
+    if (std::is_same<T, A>::value && ln < G) {
+      st.v[S + ln] = 0;
+      st.f[S + ln] = lz<W>();
+    }
     __syncwarp();
-    for (int r = 0; r < S; r += G) {
-      T x[G][2 * W];
-      unsigned my[G];
+    if constexpr (std::is_same<T, A>::value) {
+      // short adds (path counts): the set's bits are tested in place, one
+      // instruction each
+      const unsigned me = 1u << ln;
+      for (int r = 0; r < S; r += G) {
+        T x[G][2 * W];
+        unsigned h[G][2 * W];  // the set's halves: testing one against `me` is one instruction
 #pragma unroll
-      for (int q = 0; q < G; ++q) {
-        const bool ok = r + q < S;
-        const Lanes<W> fj = ok ? st.f[r + q] : lz<W>();
-        const int64_t off = static_cast<int64_t>(ok ? st.v[r + q] : 0) * RS;
-        my[q] = my_bits(fj);
+        for (int q = 0; q < G; ++q) {
+          const unsigned* fw = reinterpret_cast<const unsigned*>(&st.f[r + q]);
+          const T* row = r0 + static_cast<int64_t>(st.v[r + q]) * RS;
 #pragma unroll
-        for (int k = 0; k < 2 * W; ++k)  // x[q][k] is read below only under the same bit
-          if (my[q] & (1u << k)) x[q][k] = r0[off + 32 * k];
+          for (int k = 0; k < 2 * W; ++k) h[q][k] = fw[k];
+#pragma unroll
+          for (int k = 0; k < 2 * W; ++k)  // x[q][k] is read below only under the same bit
+            if (h[q][k] & me) x[q][k] = row[32 * k];
+        }
+#pragma unroll
+        for (int q = 0; q < G; ++q)
+#pragma unroll
+          for (int k = 0; k < 2 * W; ++k)
+            if (h[q][k] & me) acc_slot<T, A, W>(acc[k], x[q][k], k);
       }
+    } else {
+      // long adds (dependency sums): the bits are packed once per edge
+      for (int r = 0; r < S; r += G) {
+        T x[G][2 * W];
+        unsigned my[G];
 #pragma unroll
-      for (int q = 0; q < G; ++q)
+        for (int q = 0; q < G; ++q) {
+          const bool ok = r + q < S;
+          const Lanes<W> fj = ok ? st.f[r + q] : lz<W>();
+          const int64_t off = static_cast<int64_t>(ok ? st.v[r + q] : 0) * RS;
+          my[q] = my_bits(fj);
 #pragma unroll
-        for (int k = 0; k < 2 * W; ++k)
-          if (my[q] & (1u << k)) acc_slot<T, A, W>(acc[k], x[q][k], k);
+          for (int k = 0; k < 2 * W; ++k)  // x[q][k] is read below only under the same bit
+            if (my[q] & (1u << k)) x[q][k] = r0[off + 32 * k];
+        }
+#pragma unroll
+        for (int q = 0; q < G; ++q)
+#pragma unroll
+          for (int k = 0; k < 2 * W; ++k)
+            if (my[q] & (1u << k)) acc_slot<T, A, W>(acc[k], x[q][k], k);
+      }
     }
     chunk_end<W>(acc);
     __syncwarp();
@@ -876,6 +908,7 @@ __global__ void __launch_bounds__(kWideLanes) k_ms_init(DevGraph g, MsBuffers b,
   c->bu_levels = 0;
   c->runaway = 0;
   c->work[0] = c->work[1] = 0ull;
+  c->hubs = 0;
   for (int j = 0; j < kMaxWords; ++j) {
     c->front_union[j] = j < W ? act.w[j % W] : 0ull;
     c->next_union[j] = 0ull;
@@ -1034,8 +1067,9 @@ __global__ void __launch_bounds__(256, W == 4 ? 3 : 4) k_ms_bu(DevGraph g, MsBuf
     my_found[ln] = lz<W>();
     if (wme < n) {
       const int64_t d = g.in_rowptr[wme + 1] - g.in_rowptr[wme];
-      cand = (LF ? lany(land(lminus(act, visit[wme]), live)) : !leq(visit[wme], act)) && d > 0 &&
-             d <= hd.hub_degree;
+      const bool open = LF ? lany(land(lminus(act, visit[wme]), live)) : !leq(visit[wme], act);
+      cand = open && d > 0 && d <= hd.hub_degree;
+      if (open && d > hd.hub_degree) c->hubs = 1;  // for k_ms_hub_pull
     }
     unsigned cb = __ballot_sync(kFull, cand);
     __syncwarp();
@@ -1098,6 +1132,9 @@ __global__ void __launch_bounds__(256, W == 4 ? 3 : 4) k_ms_hub_pull(DevGraph g,
   const int ln = lane_id();
   unsigned long long mf = 0, mu = 0, smax = 0;
   // top-down few hubs take part and most items only look: fixed shares
+  // bottom-up: k_ms_bu saw whether a hub is left to finish (52,000 items that
+  // only look were 72 us of atomics on the one counter)
+  if (BU && c->hubs == 0) return;
   WorkQueue wq(&c->work[1], BU ? 1 : 0);
   for (long long it = BU ? static_cast<long long>(wq.take()) : gwarp(); it < hd.n_in;
        it = BU ? static_cast<long long>(wq.take()) : it + nwarps()) {
@@ -1260,6 +1297,7 @@ __global__ void k_loop_back_advance(MsBuffers b, LoopParams lp) {
   BatchCtl* c = b.ctl;
   c->level -= 1;
   c->work[0] = c->work[1] = 0ull;
+  c->hubs = 0;
   cudaGraphSetConditional(lp.loop, c->level >= 0 ? 1u : 0u);
 }
 
@@ -1267,6 +1305,7 @@ __device__ __forceinline__ void advance_step(const MsBuffers& b, int64_t n) {
   BatchCtl* c = b.ctl;
   const int L = c->level;
   c->work[0] = c->work[1] = 0ull;
+  c->hubs = 0;
   b.lvl_off[L + 2] = c->tail;
   // every count of level L + 1 is a sum of at most max-in-degree counts of
   // level L; once a level's largest count passes the limit, the next level
@@ -1334,7 +1373,10 @@ __global__ void __launch_bounds__(256, W == 1 ? 5 : (W == 2 ? 4 : 3)) k_ms_delta
     }
     if (L == 0) continue;
     const int64_t e0 = g.rowptr[v], e1 = g.rowptr[v + 1];
-    if (e1 - e0 > hd.hub_degree) continue;  // k_ms_hub_delta
+    if (e1 - e0 > hd.hub_degree) {  // k_ms_hub_delta
+      if (ln == 0) c->hubs = 1;
+      continue;
+    }
     const unsigned mine = my_bits(F);
     if (SK == kSigmaU64) {
       df32 acc[2 * W];
@@ -1378,6 +1420,7 @@ __global__ void __launch_bounds__(256, W == 1 ? 5 : (W == 2 ? 4 : 3)) k_ms_hub_d
   const Lanes<W>* __restrict__ succ = mbw<W>(b, L + 1);
   const Lanes<W>* __restrict__ cur = mbw<W>(b, L);
   const int ln = lane_id();
+  if (c->hubs == 0) return;  // k_ms_delta met none in the level's list
   WorkQueue wq(&c->work[1], 1);
   for (long long it = static_cast<long long>(wq.take()); it < hd.n_out; it = static_cast<long long>(wq.take())) {
     const HubItem I = hd.out_items[it];
@@ -1518,7 +1561,9 @@ __global__ void __launch_bounds__(256, W == 1 ? 3 : 2) k_ms_bu_seg(DevGraph g, M
       vis = visit[wme];
       e0 = g.in_rowptr[wme];
       deg = g.in_rowptr[wme + 1] - e0;
-      cand = lany(land(lminus(act, vis), fl)) && deg > 0 && deg <= hd.hub_degree;
+      const bool open = lany(land(lminus(act, vis), fl));
+      cand = open && deg > 0 && deg <= hd.hub_degree;
+      if (open && deg > hd.hub_degree) c->hubs = 1;  // for k_ms_hub_pull
     }
     Lanes<W> my_nm = lz<W>();
     seg_gather<T, T, false, W>(cand, e0, static_cast<int>(cand ? deg : 0), land(lminus(act, vis), fl),
@@ -1580,6 +1625,7 @@ __global__ void __launch_bounds__(256, W == 1 ? 3 : 2) k_ms_delta_seg(DevGraph g
     }
     if (L == 0) continue;
     const bool mine = ve && deg <= hd.hub_degree;  // hubs: k_ms_hub_delta
+    if (ve && !mine) c->hubs = 1;
     const int dg = static_cast<int>(mine ? deg : 0);
     if (SK == kSigmaU64) {
       seg_gather<float2, df32, true, W>(mine, e0, dg, F, g.colidx, succ,
@@ -1798,6 +1844,7 @@ __global__ void __launch_bounds__(256) k_st_hub_count(DevGraph g, MsBuffers b, H
 __global__ void k_ms_back_advance(MsBuffers b) {
   b.ctl->level -= 1;
   b.ctl->work[0] = b.ctl->work[1] = 0ull;
+  b.ctl->hubs = 0;
 }
 
 // End of a Brandes batch: the backward sweep cleared visit for every listed
@@ -2017,6 +2064,7 @@ __global__ void k_ms_init_seeds_ctl(MsBuffers b, long long nseeds, unsigned long
   c->bu_levels = 0;
   c->runaway = 0;
   c->work[0] = c->work[1] = 0ull;
+  c->hubs = 0;
   for (int j = 0; j < kMaxWords; ++j) {
     c->front_union[j] = ~0ull;  // every lane may be seeded
     c->next_union[j] = 0ull;
