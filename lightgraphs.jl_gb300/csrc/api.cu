@@ -1110,6 +1110,37 @@ int run_small(lgbc_graph* g, int64_t k, double* bc_dev, const double* d_w) {
   return LGBC_OK;
 }
 
+int run_small_stress(lgbc_graph* g, unsigned long long* d_stress) {
+  SmallWorkspace& w = g->small;
+  const int64_t k = static_cast<int64_t>(g->h_active.size());
+  if (k == 0 || !small_graph(g) || g->n > g->small_stress_max_n || w.stress_refused) return 1;
+  LGBC_TRY(upload_sources(g));
+  LGBC_TRY(ensure_plan(g, &w.out, g->d_rowptr, g->d_colidx, g->d_in_rowptr));
+  if (!w.counters) LGBC_TRY(dev_alloc(&w.counters, 2));
+  const SmallShape sh = small_stress_shape(g->cfg, g->n, k);
+  SmallRun run{};
+  run.graphs = w.out.graph;
+  run.nitems = static_cast<int>(std::min<int64_t>(k, 4 * static_cast<int64_t>(sh.grid)));
+  run.nsrc = static_cast<int>(k);
+  run.next = w.counters;
+  run.refused = w.counters + 1;
+  run.src = g->d_src;
+  run.stress = d_stress;
+  LGBC_CUDA(cudaMemsetAsync(w.counters, 0, 2 * sizeof(int), g->stream));
+  g->launches += small_stress(g->stream, sh, run, g->n);
+  LGBC_TRY(check_launch(g));
+  int* refused = reinterpret_cast<int*>(g->h_ctl);
+  LGBC_CUDA(cudaMemcpyAsync(refused, w.counters + 1, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+  LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  if (!*refused) {
+    g->stats.batches += run.nitems;
+    return LGBC_OK;
+  }
+  w.stress_refused = true;
+  LGBC_CUDA(cudaMemsetAsync(d_stress, 0, static_cast<size_t>(g->n) * 8, g->stream));
+  return 1;
+}
+
 int accumulate_active(lgbc_graph* g, int endpoints, double* bc_dev) {
   const int64_t k = static_cast<int64_t>(g->h_active.size());
   double* d_w = nullptr;
@@ -1161,6 +1192,7 @@ int init_handle(lgbc_graph* g, int64_t n, int directed) {
   g->bfs_room = bfs_configure(g->max_smem);
   g->small_max_n = small_configure(g->max_smem);
   g->small_bfs_max_n = small_bfs_configure(g->max_smem);
+  g->small_stress_max_n = small_stress_configure(g->max_smem);
   LGBC_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
   LGBC_CUDA(cudaEventCreate(&g->ev_start));
   LGBC_CUDA(cudaEventCreate(&g->ev_stop));

@@ -227,6 +227,7 @@ struct SmallWorkspace {
   ulonglong2* part = nullptr;       // partial sums, one n-vector per item
   int64_t part_cap = 0;
   bool refused = false;             // too deep or counts too large: the batches take this graph
+  bool stress_refused = false;      // too deep, in a stress call
   void release() {
     out.release();
     in.release();
@@ -316,7 +317,7 @@ struct lgbc_graph {
   lgbc::api::LearnedWorkspace learned;
   lgbc::api::SmallWorkspace small;
   int64_t small_max_n = 0;          // largest graph of the per-source kernel on this device
-  int64_t small_bfs_max_n = 0;      // and of the distance kernel
+  int64_t small_stress_max_n = 0, small_bfs_max_n = 0;  // and of the stress and distance kernels
   int64_t max_out = 0, max_in = 0;  // largest out- and in-list
   int32_t* d_src = nullptr;         // device copy of a call's source list
   int64_t d_src_cap = 0;
@@ -409,6 +410,10 @@ int finish_handle(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr
 // (run: everything but the graph).
 bool small_bfs_applies(const lgbc_graph* g, int64_t nsrc);
 int run_small_bfs(lgbc_graph* g, SmallBfs run);
+// Stress over g->h_active into d_stress (zeroed by the caller) by the
+// per-source kernel: 1 when it does not take the graph (d_stress zero again).
+int run_small_stress(lgbc_graph* g, unsigned long long* d_stress);
+int upload_sources(lgbc_graph* g);
 // Level-synchronous BFS over dg from g->d_src[0, nsrc) into g->d_dist.
 // prefilled: the caller has filled it (kUnreached, and any other value on
 // vertices the search must treat as already visited).  finish_bfs waits for

@@ -155,14 +155,19 @@ extern "C" int lgbc_stress(lgbc_graph* g, const int32_t* src, int64_t nsrc, int6
   if (!stress_out && g->n > 0) return fail(LGBC_EINVAL, "null output");
   reset_stats(g);
   LGBC_TRY(filter_sources(g, src, nsrc));
-  LGBC_TRY(order_sources(g));
-  const int64_t k_act = static_cast<int64_t>(g->h_active.size());
   if (g->n == 0) return LGBC_OK;
   unsigned long long* d_st = nullptr;
   LGBC_TRY(dev_alloc(&d_st, static_cast<size_t>(g->n)));
   std::unique_ptr<unsigned long long, void (*)(unsigned long long*)> guard(
       d_st, [](unsigned long long* q) { cudaFree(q); });
   LGBC_CUDA(cudaMemsetAsync(d_st, 0, static_cast<size_t>(g->n) * 8, g->stream));
+  const int rc = run_small_stress(g, d_st);
+  if (rc != LGBC_OK && rc != 1) return rc;
+  int64_t k_act = 0;
+  if (rc == 1) {
+    LGBC_TRY(order_sources(g));
+    k_act = static_cast<int64_t>(g->h_active.size());
+  }
   if (k_act > 0) LGBC_TRY(ensure_ms(g, true));  // the path-count rows hold E
   for (int64_t s0 = 0; s0 < k_act; s0 += kMaxLanes) {
     const int nl = static_cast<int>(std::min<int64_t>(kMaxLanes, k_act - s0));

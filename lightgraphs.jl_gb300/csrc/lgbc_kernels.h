@@ -217,6 +217,7 @@ struct SmallRun {
   const int32_t* src;      // sources as the graph's own ids, or null
   const double* weight;    // weights of the sources in src, or null
   ulonglong2* part;        // extended-format sums (xf64.cuh): significand, exponent
+  unsigned long long* stress;  // stress: n results of graph 0, added to
 };
 struct SmallShape {
   int grid, threads;
@@ -244,7 +245,6 @@ struct SmallBfs {
 // The largest n of the kernel on this device (opts it into the shared memory).
 int small_bfs_configure(size_t max_dyn_smem);
 int small_bfs(const LaunchCfg& c, cudaStream_t s, const SmallBfs& run, int64_t n);
-size_t small_smem(int64_t n);
 int64_t small_col_groups(int64_t n, int64_t nnz);
 // Opt the kernels into the device's shared memory; the largest n they take.
 int small_configure(size_t max_dyn_smem);
@@ -252,6 +252,10 @@ int small_plan(cudaStream_t s, const SmallGraph* graphs, int count, int64_t max_
 // Launch shape for `items` items of graphs of up to max_n vertices.
 SmallShape small_shape(const LaunchCfg& c, int64_t max_n, int64_t items);
 int small_brandes(cudaStream_t s, const SmallShape& sh, const SmallRun& run, int64_t max_n);
+// Stress centrality (run.stress) likewise.
+int small_stress_configure(size_t max_dyn_smem);
+SmallShape small_stress_shape(const LaunchCfg& c, int64_t n, int64_t items);
+int small_stress(cudaStream_t s, const SmallShape& sh, const SmallRun& run, int64_t n);
 // ORs into bad[i] for graph i: 1 = rowptr decreases, 2 = a column outside
 // [0, n), 4 = a row longer than n.
 int small_check(cudaStream_t s, const SmallGraph* graphs, int count, int* bad);

@@ -160,90 +160,254 @@ __global__ void __launch_bounds__(1024) k_small_plan(const SmallGraph* graphs) {
 // Sweeps
 // ---------------------------------------------------------------------------
 
-// Path count (chi : clo) of a frontier vertex to four neighbours, except those
-// that are closed.  64-bit shared atomics are compare-and-swap loops, so the
-// words are added apart.  With every count of the frontier below 2^16 no sum
-// over fewer than 2^15 predecessors passes 2^31: the adds need no answer and
-// nothing waits for them (NARROW).  Otherwise the low word's old value gives
-// the carry.
-//
-// The shared accesses are written out with predicates: as branches around
-// each of the four they cost more instructions than the adds themselves.
+// The shared accesses of a group of four neighbours are written out with
+// predicates: as branches around each of the four they cost more instructions
+// than the adds themselves.
 __device__ __forceinline__ uint32_t lds(uint32_t at) {
   uint32_t x;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(x) : "r"(at));
   return x;
 }
-// Byte offsets of a group's four state words.
-__device__ __forceinline__ void offsets(uint2 c, uint32_t (&w)[4]) {
-  w[0] = (c.x << 2) & 0x3FFFCu;
-  w[1] = (c.x >> 14) & 0x3FFFCu;
-  w[2] = (c.y << 2) & 0x3FFFCu;
-  w[3] = (c.y >> 14) & 0x3FFFCu;
+// *at += add if the sign of h is clear.
+__device__ __forceinline__ void red_if_open(uint32_t at, uint32_t add, uint32_t h) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ge.s32 p, %2, 0;\n\t"
+      "@p red.shared.add.u32 [%0], %1;\n\t}"
+      ::"r"(at), "r"(add), "r"(h) : "memory");
+}
+// x = *at if h > 0 as a signed number.
+__device__ __forceinline__ void lds_if_done(uint32_t& x, uint32_t at, uint32_t h) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.gt.s32 p, %2, 0;\n\t"
+      "@p ld.shared.u32 %0, [%1];\n\t}"
+      : "+r"(x) : "r"(at), "r"(h));
+}
+__device__ __forceinline__ uint32_t shared_at(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-template <bool NARROW>
-__device__ __forceinline__ void push4(uint32_t lo, uint32_t hi, uint2 c, uint32_t clo, uint32_t chi) {
-  uint32_t w[4], h[4];
-  offsets(c, w);
+// ---- Brandes: path counts, then psi, in two words per vertex ---------------
+struct BrandesState {
+  using Sum = xg64;           // of psi, while a row is walked
+  using Value = xf64;         // the finished sum
+  using Early = ulonglong2;   // a vertex's partial sum, loaded ahead of its row
+  struct Count {
+    uint32_t lo, hi;
+  };
+  uint32_t *lo, *hi;
+  uint32_t lo_s, hi_s;
+  int n;
+  ulonglong2* part;
+  const double* weight;
+  xf64 w;
+
+  static __host__ __device__ size_t words(int64_t n) { return 2 * static_cast<size_t>(n + 1); }
+  __device__ __forceinline__ BrandesState(uint32_t* sm, const SmallRun& run, const SmallItem& I, const SmallGraph& G)
+      : lo(sm), hi(sm + G.n + 1), lo_s(shared_at(lo)), hi_s(shared_at(hi)), n(G.n), part(run.part + I.part),
+        weight(run.weight), w(xf_zero()) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) part[i] = make_ulonglong2(0ull, 0ull);
+  }
+  __device__ __forceinline__ void clear(int si) {
+    for (int i = threadIdx.x; i <= 2 * n + 1; i += blockDim.x) lo[i] = 0u;
+    if (weight) w = xf_from_bits(static_cast<uint64_t>(__double_as_longlong(weight[si])));
+  }
+  __device__ __forceinline__ void seed(int s) {
+    hi[n] = kClosed;
+    lo[s] = 1u;
+    hi[s] = kClosed;
+  }
+  __device__ __forceinline__ Count count(int v) const { return Count{lo[v], hi[v] & ~kClosed}; }
+
+  // A frontier vertex's path count to four neighbours, except those that are
+  // closed.  64-bit shared atomics are compare-and-swap loops, so the words
+  // are added apart.  With every count of the frontier below 2^16 no sum over
+  // fewer than 2^15 predecessors passes 2^31: the adds need no answer and
+  // nothing waits for them (NARROW).  Otherwise the low word's old value
+  // gives the carry.
+  template <bool NARROW> __device__ __forceinline__ void push4(uint2 c, Count f) const {
+    // byte offsets of the four state words
+    const uint32_t at[4] = {(c.x << 2) & 0x3FFFCu, (c.x >> 14) & 0x3FFFCu, (c.y << 2) & 0x3FFFCu,
+                            (c.y >> 14) & 0x3FFFCu};
+    uint32_t h[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) h[k] = lds(hi + w[k]);
-  if (NARROW) {
+    for (int k = 0; k < 4; ++k) h[k] = lds(hi_s + at[k]);
+    if (NARROW) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+      for (int k = 0; k < 4; ++k) red_if_open(lo_s + at[k], f.lo, h[k]);
+      return;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      uint32_t old = 0u;
       asm volatile(
           "{\n\t.reg .pred p;\n\t"
-          "setp.ge.s32 p, %2, 0;\n\t"
-          "@p red.shared.add.u32 [%0], %1;\n\t}"
-          ::"r"(lo + w[k]), "r"(clo), "r"(h[k]) : "memory");
-    return;
+          "setp.ge.s32 p, %3, 0;\n\t"
+          "@p atom.shared.add.u32 %0, [%1], %2;\n\t}"
+          : "+r"(old) : "r"(lo_s + at[k]), "r"(f.lo), "r"(h[k]) : "memory");
+      const uint32_t up = f.hi + (old > ~f.lo ? 1u : 0u);
+      if (static_cast<int>(h[k]) >= 0 && up)
+        asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(hi_s + at[k]), "r"(up) : "memory");
+    }
   }
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    uint32_t old = 0u;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ge.s32 p, %3, 0;\n\t"
-        "@p atom.shared.add.u32 %0, [%1], %2;\n\t}"
-        : "+r"(old) : "r"(lo + w[k]), "r"(clo), "r"(h[k]) : "memory");
-    const uint32_t up = chi + (old > ~clo ? 1u : 0u);
-    if (static_cast<int>(h[k]) >= 0 && up)
-      asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(hi + w[k]), "r"(up) : "memory");
+  // The same for one neighbour (narrow counts); true for its first add.
+  __device__ __forceinline__ bool first(uint32_t v, Count f) const {
+    return static_cast<int>(hi[v]) >= 0 && atomicAdd(lo + v, f.lo) == 0u;
   }
-}
+  __device__ __forceinline__ bool close(int v) const {  // true: the count is 2^16 or more
+    hi[v] = kClosed;
+    return (lo[v] >> 16) != 0u;
+  }
+  // Close v if this level counted it; returns whether it did.
+  __device__ __forceinline__ bool close_fresh(int v, int* wide, int* stop) const {
+    const uint32_t h = hi[v], l = lo[v];
+    if (static_cast<int>(h) < 0 || (h | l) == 0u) return false;
+    hi[v] = h | kClosed;
+    if (h | (l >> 16)) *wide = 1;
+    if (h >= kCountLimitHi) *stop = 1;
+    return true;
+  }
 
-// psi of the successors among four neighbours into the sum.  Any other
-// neighbour adds a zero of exponent 0, far below every sum's (sum_zero).
-__device__ __forceinline__ void pull4(uint32_t lo, uint32_t hi, uint2 c, xg64& a) {
-  uint32_t w[4], h[4], l[4];
-  offsets(c, w);
+  // An empty sum whose exponent shifts a term of exponent 0 out entirely (psi
+  // is at least 2^-48, so its exponent field is above 900).
+  static __device__ __forceinline__ Sum zero() { return xg64{0ull, 128}; }
+  // psi of the successors among four neighbours into the sum; any other
+  // neighbour adds a zero of exponent 0.
+  __device__ __forceinline__ void pull4(uint2 c, Sum& a) const {
+    const uint32_t at[4] = {(c.x << 2) & 0x3FFFCu, (c.x >> 14) & 0x3FFFCu, (c.y << 2) & 0x3FFFCu,
+                            (c.y >> 14) & 0x3FFFCu};
+    uint32_t h[4], l[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) h[k] = lds(hi + w[k]);
+    for (int k = 0; k < 4; ++k) h[k] = lds(hi_s + at[k]);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    l[k] = 0u;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.gt.s32 p, %2, 0;\n\t"
-        "@p ld.shared.u32 %0, [%1];\n\t}"
-        : "+r"(l[k]) : "r"(lo + w[k]), "r"(h[k]));
-    h[k] = static_cast<uint32_t>(max(static_cast<int>(h[k]), 0));
+    for (int k = 0; k < 4; ++k) {
+      l[k] = 0u;
+      lds_if_done(l[k], lo_s + at[k], h[k]);
+      h[k] = static_cast<uint32_t>(max(static_cast<int>(h[k]), 0));
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) xg_add_bits(a, (static_cast<uint64_t>(h[k]) << 32) | l[k]);
   }
+  static __device__ __forceinline__ void after32(Sum& a) { xg_norm(a); }
+  static __device__ __forceinline__ Value value(Sum a) {
+    xg_norm(a);
+    return a.m ? xg_to_xf(a) : xf_zero();
+  }
+  static __device__ __forceinline__ Value none() { return xf_zero(); }
+  static __device__ __forceinline__ Value warp_sum(Value x) { return warp_sum_x(x); }
+  __device__ __forceinline__ Early early(int v) const { return part[v]; }
+  // psi = 1 / sigma + acc replaces the count; sigma * acc is the dependency.
+  __device__ __forceinline__ void finish(int v, Value acc, Early sum) const {
+    const uint64_t s = (static_cast<uint64_t>(hi[v] & ~kClosed) << 32) | lo[v];
+    const uint64_t p = xf_to_bits(xf_add(acc, xf_recip_u64(s)));
+    lo[v] = static_cast<uint32_t>(p);
+    hi[v] = static_cast<uint32_t>(p >> 32) | kClosed;
+    if (acc.m == 0) return;
+    xf64 d = xf_mul_u64(acc, s);
+    if (weight) d = xf_mul(d, w);
+    const xf64 t = xf_add(d, xf64{sum.x, static_cast<int32_t>(sum.y)});
+    part[v] = make_ulonglong2(t.m, static_cast<unsigned long long>(t.e));
+  }
+  __device__ __forceinline__ void open(int v) const { hi[v] &= ~kClosed; }
+};
+
+// ---- Stress (src/centrality/stress.jl:51-77; the recursion of k_st_delta in
+// msbfs.cu): predecessor counts P in 16 bits, bit 15 in the part of bit 31
+// above, and E = 1 + sum of the successors' E in two words, wrapping.  The
+// sum times P goes to the result with one 64-bit atomic, whose order cannot
+// show.  P < 2^15, as every in-list is shorter.  300 sources on R-MAT 14:
+// 2.31 ms as batches, 0.40 ms here.
+struct StressState {
+  using Sum = unsigned long long;
+  using Value = unsigned long long;
+  using Early = int;          // the vertex's own id
+  struct Count {};
+  uint16_t* st;
+  uint32_t *lo, *hi;
+  uint32_t st_s, lo_s, hi_s;
+  int n;
+  const int32_t* orig;
+  unsigned long long* out;
+
+  static __host__ __device__ size_t words(int64_t n) { return 2 * static_cast<size_t>(n + 1) + static_cast<size_t>(n + 2) / 2; }
+  __device__ __forceinline__ StressState(uint32_t* sm, const SmallRun& run, const SmallItem&, const SmallGraph& G)
+      : st(reinterpret_cast<uint16_t*>(sm + 2 * (G.n + 1))), lo(sm), hi(sm + G.n + 1), st_s(shared_at(st)),
+        lo_s(shared_at(lo)), hi_s(shared_at(hi)), n(G.n), orig(G.orig), out(run.stress) {}
+  __device__ __forceinline__ void clear(int) {
+    uint32_t* w = reinterpret_cast<uint32_t*>(st);
+    for (int i = threadIdx.x; i < (n + 2) / 2; i += blockDim.x) w[i] = 0u;
+  }
+  __device__ __forceinline__ void seed(int s) {
+    st[n] = 0x8000u;
+    st[s] = 0x8000u;
+  }
+  __device__ __forceinline__ Count count(int) const { return Count(); }
+  template <bool NARROW> __device__ __forceinline__ void push4(uint2 c, Count) const {
+    const uint32_t id[4] = {c.x & 0xFFFFu, c.x >> 16, c.y & 0xFFFFu, c.y >> 16};
+    uint32_t h[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) xg_add_bits(a, (static_cast<uint64_t>(h[k]) << 32) | l[k]);
-}
-// An empty sum whose exponent shifts a term of exponent 0 out entirely (psi
-// is at least 2^-48, so its exponent field is above 900).
-__device__ __forceinline__ xg64 sum_zero() { return xg64{0ull, 128}; }
-__device__ __forceinline__ xf64 sum_value(xg64 a) {
-  xg_norm(a);
-  return a.m ? xg_to_xf(a) : xf_zero();
-}
+    for (int k = 0; k < 4; ++k) {  // the half in the upper 16 bits
+      h[k] = lds(st_s + ((id[k] << 1) & ~3u));
+      h[k] <<= (~id[k] & 1u) << 4;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) red_if_open(st_s + ((id[k] << 1) & ~3u), (id[k] & 1u) ? 0x10000u : 1u, h[k]);
+  }
+  __device__ __forceinline__ bool first(uint32_t v, Count) const {
+    if (st[v] & 0x8000u) return false;
+    const uint32_t sh = (v & 1u) << 4;
+    return ((atomicAdd(reinterpret_cast<uint32_t*>(st) + (v >> 1), 1u << sh) >> sh) & 0xFFFFu) == 0u;
+  }
+  __device__ __forceinline__ bool close(int v) const {
+    st[v] |= 0x8000u;
+    return false;
+  }
+  __device__ __forceinline__ bool close_fresh(int v, int*, int*) const {
+    const uint16_t p = st[v];
+    if (p == 0u || (p & 0x8000u)) return false;
+    st[v] = static_cast<uint16_t>(p | 0x8000u);
+    return true;
+  }
+  static __device__ __forceinline__ Sum zero() { return 0ull; }
+  __device__ __forceinline__ void pull4(uint2 c, Sum& a) const {
+    const uint32_t id[4] = {c.x & 0xFFFFu, c.x >> 16, c.y & 0xFFFFu, c.y >> 16};
+    uint32_t h[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      h[k] = lds(st_s + ((id[k] << 1) & ~3u));
+      h[k] <<= (~id[k] & 1u) << 4;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      // an unfinished neighbour carries bit 15 (so its upper half is negative)
+      const uint32_t done = (h[k] >> 16) ? h[k] | 1u : 0u;
+      uint32_t l = 0u, u = 0u;
+      lds_if_done(l, lo_s + 4u * id[k], done);
+      lds_if_done(u, hi_s + 4u * id[k], done);
+      a += (static_cast<unsigned long long>(u) << 32) | l;
+    }
+  }
+  static __device__ __forceinline__ void after32(Sum&) {}
+  static __device__ __forceinline__ Value value(Sum a) { return a; }
+  static __device__ __forceinline__ Value none() { return 0ull; }
+  static __device__ __forceinline__ Value warp_sum(Value x) { return warp_sum_u64(x); }
+  __device__ __forceinline__ Early early(int v) const { return orig[v]; }
+  __device__ __forceinline__ void finish(int v, Value acc, Early own) const {
+    const unsigned long long e = acc + 1ull;
+    lo[v] = static_cast<uint32_t>(e);
+    hi[v] = static_cast<uint32_t>(e >> 32);
+    const unsigned long long x = acc * (st[v] & 0x7FFFu);
+    if (x) atomicAdd(out + own, x);
+  }
+  __device__ __forceinline__ void open(int v) const { st[v] &= 0x7FFFu; }
+};
 
 // One block per item (a range of sources of one graph).  Each source: count
-// paths level by level, then sweep the levels back, adding the dependencies
-// to the item's partial sums.
-__global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_brandes(SmallRun run) {
+// paths (or predecessors) level by level, then sweep the levels back, adding
+// to the item's partial sums (or the result).
+template <class S>
+__global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun run) {
   extern __shared__ uint32_t sm[];
   __shared__ int lvl[2][kSmallMaxLevels + 2];  // level starts: [0] warp-walked vertices, [1] the others
   __shared__ int s_count[kWarp];
@@ -272,18 +436,13 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_brandes(SmallRun 
     }
     const SmallGraph G = run.graphs[I.graph];
     const int n = G.n;
-    uint32_t* lo = sm;
-    uint32_t* hi = sm + (n + 1);
-    const uint32_t lo_s = static_cast<uint32_t>(__cvta_generic_to_shared(lo));
-    const uint32_t hi_s = static_cast<uint32_t>(__cvta_generic_to_shared(hi));
-    uint32_t* chunk = sm + 2 * (n + 1);
+    S st(sm, run, I, G);
+    uint32_t* chunk = sm + S::words(n);
     uint16_t* q = reinterpret_cast<uint16_t*>(chunk + (n + 31) / 32);
     const uint2* const col = G.col;
     // warp-walked ids [0, nw): whole chunks of 32, so that a chunk's
     // discoveries go to one list
     const int nw = (*G.nwarp + 31) & ~31;
-    ulonglong2* part = run.part + I.part;
-    for (int i = tid; i < n; i += T) part[i] = make_ulonglong2(0ull, 0ull);
     for (int c = nw / kWarp + tid; c * kWarp < n; c += T) chunk[c] = G.chunk[c];
     // the row of a thread-walked vertex: its first group and their number
     auto row_of = [&](uint32_t v, uint32_t& e, int& len) {
@@ -308,8 +467,9 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_brandes(SmallRun 
       constexpr bool N = decltype(narrow)::value;
       for (int i = a0 + wid; i < a1; i += W) {
         const int v = q[i];
-        const uint32_t clo = lo[v], chi = hi[v] & ~kClosed, g1 = G.row[v + 1];
-        for (uint32_t e = G.row[v] + ln; e < g1; e += kWarp) push4<N>(lo_s, hi_s, col[e], clo, chi);
+        const typename S::Count f = st.count(v);
+        const uint32_t g1 = G.row[v + 1];
+        for (uint32_t e = G.row[v] + ln; e < g1; e += kWarp) st.template push4<N>(col[e], f);
       }
       int i, len = 0;
       uint32_t v = 0, e = 0;
@@ -317,26 +477,25 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_brandes(SmallRun 
       fetch(b1, i, v, e, len, c);
       while (i - ln < b1) {
         const bool on = i < b1;
-        const uint32_t clo = on ? lo[v] : 0u, chi = on ? hi[v] & ~kClosed : 0u, at = e;
+        const typename S::Count f = st.count(on ? v : n);
+        const uint32_t at = e;
         const int groups = on ? len : 0;
         uint2 x = c;
         fetch(b1, i, v, e, len, c);
         for (int j = 1; j <= groups; ++j) {
           uint2 nx = x;
           if (j < groups) nx = col[at + 32u * j];
-          push4<N>(lo_s, hi_s, x, clo, chi);
+          st.template push4<N>(x, f);
           x = nx;
         }
       }
     };
     for (int si = I.begin; si < I.end && !s_stop; ++si) {
-      for (int i = tid; i <= 2 * n + 1; i += T) sm[i] = 0u;
+      st.clear(si);
       __syncthreads();
       if (tid == 0) {
         const int s = run.src ? G.rank[run.src[si]] : si;
-        hi[n] = kClosed;
-        lo[s] = 1u;
-        hi[s] = kClosed;
+        st.seed(s);
         const int k = s < nw ? 0 : 1;
         const int own = G.orig[s];
         s_goal = *G.nlive + (G.in_rowptr[own + 1] == G.in_rowptr[own] ? 1 : 0);
@@ -359,7 +518,8 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_brandes(SmallRun 
           if (tid < 2) s_count[tid] = 0;
           __syncthreads();
           for (int i = lvl[1][L] + wid; i < b1; i += W) {
-            const uint32_t v = q[nw + i], clo = lo[v];
+            const uint32_t v = q[nw + i];
+            const typename S::Count f = st.count(v);
             uint32_t e;
             int len;
             row_of(v, e, len);
@@ -369,7 +529,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_brandes(SmallRun 
 #pragma unroll
               for (int k = 0; k < 4; ++k) {
                 const uint32_t w = ids[k];
-                if (static_cast<int>(hi[w]) < 0 || atomicAdd(lo + w, clo) != 0u) continue;
+                if (!st.first(w, f)) continue;
                 const int t = w < static_cast<uint32_t>(nw) ? 0 : 1;
                 q[(t ? nw + b1 : a1) + atomicAdd(&s_count[t], 1)] = static_cast<uint16_t>(w);
               }
@@ -379,8 +539,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_brandes(SmallRun 
           const int ta = a1 + s_count[0], tb = b1 + s_count[1];
           if (ta == a1 && tb == b1) break;
           auto close = [&](int v) {
-            hi[v] = kClosed;
-            if (lo[v] >> 16) s_wide[(L + 1) & 1] = 1;
+            if (st.close(v)) s_wide[(L + 1) & 1] = 1;
           };
           for (int i = a1 + tid; i < ta; i += T) close(q[i]);
           for (int i = b1 + tid; i < tb; i += T) close(q[nw + i]);
@@ -415,19 +574,9 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_brandes(SmallRun 
         unsigned bits = 0;
         for (int j = 0; j < mine_c; ++j) {
           const int v = (c0 + j) * kWarp + ln;
-          uint32_t h = kClosed, l = 0;
-          if (v < n) {
-            h = hi[v];
-            l = lo[v];
-          }
-          const bool fresh = static_cast<int>(h) >= 0 && (h | l) != 0u;
+          const bool fresh = v < n && st.close_fresh(v, &s_wide[(L + 1) & 1], &s_stop);
           const unsigned bal = __ballot_sync(kFull, fresh);
           if (ln == j) bits = bal;
-          if (fresh) {
-            hi[v] = h | kClosed;
-            if (h | (l >> 16)) s_wide[(L + 1) & 1] = 1;
-            if (h >= kCountLimitHi) s_stop = 1;
-          }
         }
         // counts of both lists in one word: they stay below 2^16
         const int cnt = __popc(bits) << (c0 + ln < nw / kWarp ? 0 : 16);
@@ -472,55 +621,40 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_brandes(SmallRun 
         }
         __syncthreads();
       }
-      const xf64 w = run.weight ? xf_from_bits(__double_as_longlong(run.weight[si])) : xf_zero();
-      // psi = 1 / sigma + acc replaces the count; sigma * acc is the dependency
-      // (sum: v's partial sum, loaded early)
-      auto finish = [&](int v, xf64 acc, ulonglong2 sum) {
-        const uint64_t s = (static_cast<uint64_t>(hi[v] & ~kClosed) << 32) | lo[v];
-        const uint64_t p = xf_to_bits(xf_add(acc, xf_recip_u64(s)));
-        lo[v] = static_cast<uint32_t>(p);
-        hi[v] = static_cast<uint32_t>(p >> 32) | kClosed;
-        if (acc.m == 0) return;
-        xf64 d = xf_mul_u64(acc, s);
-        if (run.weight) d = xf_mul(d, w);
-        const xf64 t = xf_add(d, xf64{sum.x, static_cast<int32_t>(sum.y)});
-        part[v] = make_ulonglong2(t.m, static_cast<unsigned long long>(t.e));
-      };
       const int deepest = L;
       if (tid == 0) s_next = lvl[1][max(L - 1, 0)];  // the deepest level is not fetched
       for (; L > 0; --L) {
         const int a1 = lvl[0][L + 1], b1 = lvl[1][L + 1];
         int held = 0, mine_v = 0;
-        xf64 mine = xf_zero();  // lane j keeps the j-th sum of the warp, to finish 32 at once
+        typename S::Value mine = S::none();  // lane j keeps the j-th sum of the warp, to finish 32 at once
         for (int i = lvl[0][L] + wid; i < a1; i += W) {
           const int v = q[i];
-          xf64 acc = xf_zero();
+          typename S::Value acc = S::none();
           if (L < deepest) {
-            xg64 a = sum_zero();
+            typename S::Sum a = S::zero();
             const uint32_t g1 = G.row[v + 1];
             uint32_t e = G.row[v] + ln;
             while (e < g1) {
 #pragma unroll 1
-              for (int k = 0; k < 8 && e < g1; ++k, e += kWarp) pull4(lo_s, hi_s, col[e], a);
-              xg_norm(a);
+              for (int k = 0; k < 8 && e < g1; ++k, e += kWarp) st.pull4(col[e], a);
+              S::after32(a);
             }
-            acc = sum_value(a);
-            acc = warp_sum_x(acc);
+            acc = S::warp_sum(S::value(a));
           }
           if (ln == held) {
             mine = acc;
             mine_v = v;
           }
           if (++held == kWarp) {
-            finish(mine_v, mine, part[mine_v]);
+            st.finish(mine_v, mine, st.early(mine_v));
             held = 0;
           }
         }
-        if (ln < held) finish(mine_v, mine, part[mine_v]);
+        if (ln < held) st.finish(mine_v, mine, st.early(mine_v));
         if (L == deepest) {
           for (int i = lvl[1][L] + tid; i < b1; i += T) {
             const int v = q[nw + i];
-            finish(v, xf_zero(), part[v]);
+            st.finish(v, S::none(), st.early(v));
           }
         } else {
           int i, len = 0;
@@ -531,26 +665,26 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_brandes(SmallRun 
             const uint32_t u = v, at = e;
             const bool on = i < b1;
             const int groups = on ? len : 0;
-            ulonglong2 sum = make_ulonglong2(0ull, 0ull);
-            if (on) sum = part[u];
+            typename S::Early early{};
+            if (on) early = st.early(u);
             uint2 x = c;
             fetch(b1, i, v, e, len, c);
-            xg64 a = sum_zero();
+            typename S::Sum a = S::zero();
             for (int j = 1; j <= groups; ++j) {
               uint2 nx = x;
               if (j < groups) nx = col[at + 32u * j];
-              pull4(lo_s, hi_s, x, a);
-              if ((j & 7) == 0) xg_norm(a);
+              st.pull4(x, a);
+              if ((j & 7) == 0) S::after32(a);
               x = nx;
             }
-            if (on) finish(u, sum_value(a), sum);
+            if (on) st.finish(u, S::value(a), early);
           }
         }
         __syncthreads();
         // the level is complete: its psi are what the next level sums
         if (tid == 0 && L < deepest) s_next = lvl[1][L - 1];
-        for (int i = lvl[0][L] + tid; i < a1; i += T) hi[q[i]] &= ~kClosed;
-        for (int i = lvl[1][L] + tid; i < b1; i += T) hi[q[nw + i]] &= ~kClosed;
+        for (int i = lvl[0][L] + tid; i < a1; i += T) st.open(q[i]);
+        for (int i = lvl[1][L] + tid; i < b1; i += T) st.open(q[nw + i]);
         __syncthreads();
       }
       __syncthreads();
@@ -732,10 +866,50 @@ __global__ void __launch_bounds__(256) k_small_check(const SmallGraph* graphs, i
 
 }  // namespace
 
-size_t small_smem(int64_t n) {
-  return (2 * static_cast<size_t>(n + 1) + static_cast<size_t>((n + 31) / 32)) * 4 +
-         ((static_cast<size_t>(n) * 2 + 15) & ~size_t(15));
+namespace {
+// State, chunk words and level lists of an n-vertex graph.
+template <class S> size_t sweep_smem(int64_t n) {
+  return (S::words(n) + static_cast<size_t>((n + 31) / 32)) * 4 + ((static_cast<size_t>(n) * 2 + 15) & ~size_t(15));
 }
+
+template <class S> int sweep_configure(size_t max_dyn_smem) {
+  cudaFuncAttributes fa{};
+  if (cudaFuncGetAttributes(&fa, k_small_sweeps<S>) != cudaSuccess) return 0;
+  const size_t room = max_dyn_smem > fa.sharedSizeBytes ? max_dyn_smem - fa.sharedSizeBytes : 0;
+  cudaFuncSetAttribute(k_small_sweeps<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(room));
+  int64_t n = std::min<int64_t>(kSmallMaxN, static_cast<int64_t>(room / 10));
+  while (n > 0 && sweep_smem<S>(n) > room) --n;
+  return static_cast<int>(n);
+}
+
+template <class S> SmallShape sweep_shape(const LaunchCfg& c, int64_t max_n, int64_t items) {
+  SmallShape sh{};
+  const size_t smem = sweep_smem<S>(max_n);
+  // as many warps as the registers allow, split over the blocks that fit and
+  // that there are items for
+  int64_t blocks = std::min<int64_t>(16, static_cast<int64_t>((227 * 1024) / (smem + 4096)));
+  blocks = std::max<int64_t>(1, std::min(blocks, (items + c.sms - 1) / c.sms));
+  int threads = static_cast<int>(kSmallMaxThreads / blocks);
+  threads = std::max(64, std::min(threads, static_cast<int>((2 * max_n + 31) & ~int64_t(31))));
+  threads &= ~31;
+  // a warp lists at most 32 chunks of 32 vertices
+  const int chunks = static_cast<int>((max_n + kWarp - 1) / kWarp);
+  threads = std::max(threads, (chunks + kWarp - 1) / kWarp * kWarp);
+  int resident = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_small_sweeps<S>, threads, smem) != cudaSuccess ||
+      resident < 1)
+    resident = 1;
+  sh.threads = threads;
+  sh.grid = c.sms * resident;
+  return sh;
+}
+
+template <class S> int sweep(cudaStream_t s, const SmallShape& sh, const SmallRun& run, int64_t max_n) {
+  const int grid = std::min(sh.grid, run.nitems);
+  k_small_sweeps<S><<<grid, sh.threads, sweep_smem<S>(max_n), s>>>(run);
+  return 1;
+}
+}  // namespace
 
 // Rows rounded up to groups, and each chunk's rows to its longest: since the
 // lengths decrease, that adds at most the first chunk's.
@@ -769,15 +943,10 @@ int small_bfs(const LaunchCfg& c, cudaStream_t s, const SmallBfs& run, int64_t n
 }
 
 int small_configure(size_t max_dyn_smem) {
-  cudaFuncAttributes fa{};
-  if (cudaFuncGetAttributes(&fa, k_small_brandes) != cudaSuccess) return 0;
-  const size_t room = max_dyn_smem > fa.sharedSizeBytes ? max_dyn_smem - fa.sharedSizeBytes : 0;
-  cudaFuncSetAttribute(k_small_brandes, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(room));
   cudaFuncSetAttribute(k_small_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(max_dyn_smem / 2));
-  int64_t n = std::min<int64_t>(kSmallMaxN, static_cast<int64_t>(room / 10));
-  while (n > 0 && small_smem(n) > room) --n;
-  return static_cast<int>(n);
+  return sweep_configure<BrandesState>(max_dyn_smem);
 }
+int small_stress_configure(size_t max_dyn_smem) { return sweep_configure<StressState>(max_dyn_smem); }
 
 int small_plan(cudaStream_t s, const SmallGraph* graphs, int count, int64_t max_n) {
   const size_t bins = static_cast<size_t>((max_n + 3) / 4 + 1);
@@ -786,31 +955,16 @@ int small_plan(cudaStream_t s, const SmallGraph* graphs, int count, int64_t max_
 }
 
 SmallShape small_shape(const LaunchCfg& c, int64_t max_n, int64_t items) {
-  SmallShape sh{};
-  const size_t smem = small_smem(max_n);
-  // as many warps as the registers allow, split over the blocks that fit and
-  // that there are items for
-  int64_t blocks = std::min<int64_t>(16, static_cast<int64_t>((227 * 1024) / (smem + 4096)));
-  blocks = std::max<int64_t>(1, std::min(blocks, (items + c.sms - 1) / c.sms));
-  int threads = static_cast<int>(kSmallMaxThreads / blocks);
-  threads = std::max(64, std::min(threads, static_cast<int>((2 * max_n + 31) & ~int64_t(31))));
-  threads &= ~31;
-  // a warp lists at most 32 chunks of 32 vertices
-  const int chunks = static_cast<int>((max_n + kWarp - 1) / kWarp);
-  threads = std::max(threads, (chunks + kWarp - 1) / kWarp * kWarp);
-  int resident = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_small_brandes, threads, smem) != cudaSuccess ||
-      resident < 1)
-    resident = 1;
-  sh.threads = threads;
-  sh.grid = c.sms * resident;
-  return sh;
+  return sweep_shape<BrandesState>(c, max_n, items);
 }
-
 int small_brandes(cudaStream_t s, const SmallShape& sh, const SmallRun& run, int64_t max_n) {
-  const int grid = std::min(sh.grid, run.nitems);
-  k_small_brandes<<<grid, sh.threads, small_smem(max_n), s>>>(run);
-  return 1;
+  return sweep<BrandesState>(s, sh, run, max_n);
+}
+SmallShape small_stress_shape(const LaunchCfg& c, int64_t n, int64_t items) {
+  return sweep_shape<StressState>(c, n, items);
+}
+int small_stress(cudaStream_t s, const SmallShape& sh, const SmallRun& run, int64_t n) {
+  return sweep<StressState>(s, sh, run, n);
 }
 
 int small_check(cudaStream_t s, const SmallGraph* graphs, int count, int* bad) {

@@ -140,6 +140,25 @@ def test_distances_along_a_path():
     assert np.array_equal(d, np.stack([i, abs(i - 1499), 2999 - i]))
 
 
+@pytest.mark.parametrize("directed", [False, True])
+@pytest.mark.parametrize("n,degree", [(1, 1), (2, 1), (33, 5), (300, 80), (1025, 3), (16384, 6), (18900, 2), (19200, 2)])
+def test_stress(n, degree, directed):
+    # odd and even vertex counts (two counts share a word), long rows, both
+    # sides of the size limit; whole numbers, compared exactly
+    g = random_graph(n, n * degree // (1 if directed else 2) + 1, n, directed)
+    rp, ci, kw = csr_args(g)
+    src = np.random.default_rng(n).integers(0, n, min(n, 60)).astype(np.int32)
+    want = oracle.stress(rp, ci, src, **kw)
+    assert np.array_equal(lgbc.stress_centrality(g, src + 1), want)
+
+
+def test_stress_wraps_and_depths():
+    for g in (layers(40, 4), path(126), path(400), fan(2000, 1500)):
+        rp, ci, kw = csr_args(g)
+        src = np.arange(0, g.nv(), 3, dtype=np.int32)
+        assert np.array_equal(lgbc.stress_centrality(g, src + 1), oracle.stress(rp, ci, src, **kw))
+
+
 def test_many_rejects_what_it_did():
     good = path(5)
     bad = lgbc.SimpleGraph.from_csr([0, 1, 2, 2], [1, 3])
