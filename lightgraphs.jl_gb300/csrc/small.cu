@@ -34,14 +34,15 @@
 //
 // State of vertex v, two words lo / hi (separate arrays: a 4-byte access uses
 // all 32 banks):
-//   0                       not reached
-//   path count, hi bit 31 = 0   being counted (the level after the frontier)
-//   path count | hi bit 31      counted; the forward sweep leaves it alone
-//   binary64 psi | hi bit 31    finished while its level is swept back
-//   binary64 psi, hi > 0        finished, its level complete
-// A vertex of level L has successors only at level L + 1, and every other
-// neighbour carries bit 31 while level L is swept, so the sign of hi decides
-// in both sweeps and no level is stored per vertex.
+//   0                           not reached
+//   path count, bits 31 = 0     being counted (the level after the frontier)
+//   path count, bit 31          counted; the forward sweep leaves it alone
+//   psi, bit 30 = level & 1     finished by the backward sweep
+// psi lies in (2^-48, 2^15], so 6 bits of exponent (bits 29..24 of hi) leave
+// 56 for the significand: 3 more than binary64.  A vertex of level L has
+// successors only at level L + 1, and every other neighbour is a path count
+// still or finished with the other parity while level L is swept, so the two
+// top bits of hi decide in both sweeps and no level is stored per vertex.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -189,13 +190,25 @@ __device__ __forceinline__ uint32_t shared_at(const void* p) {
 }
 
 // ---- Brandes: path counts, then psi, in two words per vertex ---------------
+// psi = M 2^(b - 103) with M in [2^55, 2^56), b the 6-bit exponent; a sum is
+// m 2^(e - 103) and takes up to 255 terms before m must be brought below 2^56
+// again.  Each add truncates less than 2^-55 of the largest term so far.
+struct PsiSum {
+  uint64_t m;
+  int32_t e;
+};
+// Reciprocals of the path counts below this come from a table in shared
+// memory (most are a handful; the rest are computed).
+constexpr int kRecipTable = 512;
+
 struct BrandesState {
-  using Sum = xg64;           // of psi, while a row is walked
+  using Sum = PsiSum;         // of psi, while a row is walked
   using Value = xf64;         // the finished sum
   using Early = ulonglong2;   // a vertex's partial sum, loaded ahead of its row
   struct Count {
     uint32_t lo, hi;
   };
+  const uint64_t* recip;      // significands of 1 / s, s < kRecipTable
   uint32_t *lo, *hi;
   uint32_t lo_s, hi_s;
   int n;
@@ -203,10 +216,13 @@ struct BrandesState {
   const double* weight;
   xf64 w;
 
-  static __host__ __device__ size_t words(int64_t n) { return 2 * static_cast<size_t>(n + 1); }
+  static __host__ __device__ size_t words(int64_t n) { return 2 * kRecipTable + 2 * static_cast<size_t>(n + 1); }
   __device__ __forceinline__ BrandesState(uint32_t* sm, const SmallRun& run, const SmallItem& I, const SmallGraph& G)
-      : lo(sm), hi(sm + G.n + 1), lo_s(shared_at(lo)), hi_s(shared_at(hi)), n(G.n), part(run.part + I.part),
-        weight(run.weight), w(xf_zero()) {
+      : recip(reinterpret_cast<uint64_t*>(sm)), lo(sm + 2 * kRecipTable), hi(lo + G.n + 1), lo_s(shared_at(lo)),
+        hi_s(shared_at(hi)), n(G.n), part(run.part + I.part), weight(run.weight), w(xf_zero()) {
+    uint64_t* t = reinterpret_cast<uint64_t*>(sm);
+    for (int i = threadIdx.x; i < kRecipTable; i += blockDim.x)
+      t[i] = xf_recip_u64(static_cast<uint64_t>(i > 0 ? i : 1)).m;
     for (int i = threadIdx.x; i < n; i += blockDim.x) part[i] = make_ulonglong2(0ull, 0ull);
   }
   __device__ __forceinline__ void clear(int si) {
@@ -269,52 +285,88 @@ struct BrandesState {
     return true;
   }
 
-  // An empty sum whose exponent shifts a term of exponent 0 out entirely (psi
-  // is at least 2^-48, so its exponent field is above 900).
-  static __device__ __forceinline__ Sum zero() { return xg64{0ull, 128}; }
-  // psi of the successors among four neighbours into the sum; any other
-  // neighbour adds a zero of exponent 0.
-  __device__ __forceinline__ void pull4(uint2 c, Sum& a) const {
+  static __device__ __forceinline__ Sum zero() { return PsiSum{0ull, 0}; }
+  // psi of the successors among four neighbours of a vertex of level L into
+  // the sum; any other neighbour adds zero.
+  __device__ __forceinline__ void pull4(uint2 c, int L, Sum& a) const {
     const uint32_t at[4] = {(c.x << 2) & 0x3FFFCu, (c.x >> 14) & 0x3FFFCu, (c.y << 2) & 0x3FFFCu,
                             (c.y >> 14) & 0x3FFFCu};
+    const uint32_t parity = static_cast<uint32_t>((L + 1) & 1) << 30;
     uint32_t h[4], l[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) h[k] = lds(hi_s + at[k]);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      l[k] = 0u;
-      lds_if_done(l[k], lo_s + at[k], h[k]);
-      h[k] = static_cast<uint32_t>(max(static_cast<int>(h[k]), 0));
-    }
+    for (int k = 0; k < 4; ++k)
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t.reg .u32 x;\n\t"
+          "xor.b32 x, %0, %2;\n\t"
+          "setp.lt.u32 p, x, 0x40000000;\n\t"
+          "selp.u32 %0, x, 0, p;\n\t"
+          "mov.u32 %1, 0;\n\t"
+          "@p ld.shared.u32 %1, [%3];\n\t}"
+          : "+r"(h[k]), "=&r"(l[k]) : "r"(parity), "r"(lo_s + at[k]));
 #pragma unroll
-    for (int k = 0; k < 4; ++k) xg_add_bits(a, (static_cast<uint64_t>(h[k]) << 32) | l[k]);
+    for (int k = 0; k < 4; ++k) {
+      const int b = static_cast<int>(h[k] >> 24);
+      const uint64_t M = (static_cast<uint64_t>(h[k] & 0xFFFFFFu) << 32) | l[k];
+      const int E = a.e > b ? a.e : b;
+      a.m = xf_shr(a.m, static_cast<uint32_t>(E - a.e)) + xf_shr(M, static_cast<uint32_t>(E - b));
+      a.e = E;
+    }
   }
-  static __device__ __forceinline__ void after32(Sum& a) { xg_norm(a); }
+  static __device__ __forceinline__ void after32(Sum& a) {
+    const int sh = max(0, 8 - xf_clz(a.m));
+    a.m >>= sh;
+    a.e += sh;
+  }
   static __device__ __forceinline__ Value value(Sum a) {
-    xg_norm(a);
-    return a.m ? xg_to_xf(a) : xf_zero();
+    if (a.m == 0) return xf_zero();
+    after32(a);
+    const int lz = xf_clz(a.m);  // at least 8
+    return xf64{a.m << (lz - 1), a.e + 983 - lz};
   }
   static __device__ __forceinline__ Value none() { return xf_zero(); }
   static __device__ __forceinline__ Value warp_sum(Value x) { return warp_sum_x(x); }
   __device__ __forceinline__ Early early(int v) const { return part[v]; }
   // psi = 1 / sigma + acc replaces the count; sigma * acc is the dependency.
-  __device__ __forceinline__ void finish(int v, Value acc, Early sum) const {
-    const uint64_t s = (static_cast<uint64_t>(hi[v] & ~kClosed) << 32) | lo[v];
-    const uint64_t p = xf_to_bits(xf_add(acc, xf_recip_u64(s)));
-    lo[v] = static_cast<uint32_t>(p);
-    hi[v] = static_cast<uint32_t>(p >> 32) | kClosed;
+  __device__ __forceinline__ void finish(int v, int L, Value acc, Early sum) const {
+    const uint32_t slo = lo[v], shi = hi[v] & ~kClosed;
+    const uint64_t s = (static_cast<uint64_t>(shi) << 32) | slo;
+    xf64 r;
+    if (shi == 0u && slo < kRecipTable) {
+      r.m = recip[slo];
+      r.e = 991 + __clz(static_cast<int>(slo)) + (r.m == (1ull << 62) ? 1 : 0);
+    } else {
+      r = xf_recip_u64(s);
+    }
+    const xf64 psi = xf_add(acc, r);
+    uint64_t M = (psi.m + 63u + ((psi.m >> 7) & 1u)) >> 7;  // to 56 bits, ties to even
+    const uint32_t up = static_cast<uint32_t>(M >> 56);
+    M >>= up;
+    lo[v] = static_cast<uint32_t>(M);
+    hi[v] = static_cast<uint32_t>(M >> 32) | static_cast<uint32_t>(psi.e - 975 + static_cast<int>(up)) << 24 |
+            static_cast<uint32_t>(L & 1) << 30;
     if (acc.m == 0) return;
-    xf64 d = xf_mul_u64(acc, s);
+    xf64 d;
+    if (shi == 0u) {  // 63 x 32 bits
+      const uint64_t p0 = static_cast<uint64_t>(static_cast<uint32_t>(acc.m)) * slo;
+      const uint64_t p1 = (acc.m >> 32) * slo + (p0 >> 32);  // below 2^63, at least 2^30
+      const int sh = 33 - xf_clz(p1);                        // 0..32
+      d.m = (p1 << (32 - sh)) | (static_cast<uint64_t>(static_cast<uint32_t>(p0)) >> sh);
+      d.e = acc.e + sh;
+    } else {
+      d = xf_mul_u64(acc, s);
+    }
     if (weight) d = xf_mul(d, w);
     const xf64 t = xf_add(d, xf64{sum.x, static_cast<int32_t>(sum.y)});
     part[v] = make_ulonglong2(t.m, static_cast<unsigned long long>(t.e));
   }
-  __device__ __forceinline__ void open(int v) const { hi[v] &= ~kClosed; }
 };
 
 // ---- Stress (src/centrality/stress.jl:51-77; the recursion of k_st_delta in
 // msbfs.cu): predecessor counts P in 16 bits, bit 15 in the part of bit 31
-// above, and E = 1 + sum of the successors' E in two words, wrapping.  The
+// above and 1 + (level & 1) once finished, and E = 1 + sum of the successors'
+// E in two words, wrapping.  The
 // sum times P goes to the result with one 64-bit atomic, whose order cannot
 // show.  P < 2^15, as every in-list is shorter.  300 sources on R-MAT 14:
 // 2.31 ms as batches, 0.40 ms here.
@@ -370,8 +422,9 @@ struct StressState {
     return true;
   }
   static __device__ __forceinline__ Sum zero() { return 0ull; }
-  __device__ __forceinline__ void pull4(uint2 c, Sum& a) const {
+  __device__ __forceinline__ void pull4(uint2 c, int L, Sum& a) const {
     const uint32_t id[4] = {c.x & 0xFFFFu, c.x >> 16, c.y & 0xFFFFu, c.y >> 16};
+    const uint32_t mark = 1u + static_cast<uint32_t>((L + 1) & 1);
     uint32_t h[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -380,8 +433,7 @@ struct StressState {
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      // an unfinished neighbour carries bit 15 (so its upper half is negative)
-      const uint32_t done = (h[k] >> 16) ? h[k] | 1u : 0u;
+      const uint32_t done = (h[k] >> 16) == mark ? 1u : 0u;
       uint32_t l = 0u, u = 0u;
       lds_if_done(l, lo_s + 4u * id[k], done);
       lds_if_done(u, hi_s + 4u * id[k], done);
@@ -393,14 +445,14 @@ struct StressState {
   static __device__ __forceinline__ Value none() { return 0ull; }
   static __device__ __forceinline__ Value warp_sum(Value x) { return warp_sum_u64(x); }
   __device__ __forceinline__ Early early(int v) const { return orig[v]; }
-  __device__ __forceinline__ void finish(int v, Value acc, Early own) const {
+  __device__ __forceinline__ void finish(int v, int L, Value acc, Early own) const {
     const unsigned long long e = acc + 1ull;
     lo[v] = static_cast<uint32_t>(e);
     hi[v] = static_cast<uint32_t>(e >> 32);
     const unsigned long long x = acc * (st[v] & 0x7FFFu);
+    st[v] = static_cast<uint16_t>(1 + (L & 1));
     if (x) atomicAdd(out + own, x);
   }
-  __device__ __forceinline__ void open(int v) const { st[v] &= 0x7FFFu; }
 };
 
 // One block per item (a range of sources of one graph).  Each source: count
@@ -411,7 +463,8 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
   extern __shared__ uint32_t sm[];
   __shared__ int lvl[2][kSmallMaxLevels + 2];  // level starts: [0] warp-walked vertices, [1] the others
   __shared__ int s_count[kWarp];
-  __shared__ int s_item, s_stop, s_next, s_goal;
+  __shared__ int s_item, s_stop, s_goal;
+  __shared__ int s_next[2];                    // [L & 1]: next entry of level L's second list
   __shared__ int s_wide[2];                    // [L & 1]: a count of level L is 2^16 or more
   const int tid = threadIdx.x, T = blockDim.x, ln = lane_id(), wid = tid >> 5, W = T >> 5;
   for (;;) {
@@ -453,9 +506,9 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
     // A warp's next 32 entries of the level's list: the lists are roughly by
     // decreasing row length, so taking them as warps come free evens the
     // warps out.  (i: the lane's entry; its vertex, row and first group.)
-    auto fetch = [&](int end, int& i, uint32_t& v, uint32_t& e, int& len, uint2& c) {
+    auto fetch = [&](int L, int end, int& i, uint32_t& v, uint32_t& e, int& len, uint2& c) {
       int at = 0;
-      if (ln == 0) at = atomicAdd(&s_next, kWarp);
+      if (ln == 0) at = atomicAdd(&s_next[L & 1], kWarp);
       i = __shfl_sync(kFull, at, 0) + ln;
       if (i >= end) return;
       v = q[nw + i];
@@ -463,7 +516,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
       if (len > 0) c = col[e];
     };
     // Every count of a level to its successors.
-    auto push_level = [&](auto narrow, int a0, int a1, int b1) {
+    auto push_level = [&](auto narrow, int L, int a0, int a1, int b1) {
       constexpr bool N = decltype(narrow)::value;
       for (int i = a0 + wid; i < a1; i += W) {
         const int v = q[i];
@@ -474,14 +527,14 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
       int i, len = 0;
       uint32_t v = 0, e = 0;
       uint2 c = make_uint2(0u, 0u);
-      fetch(b1, i, v, e, len, c);
+      fetch(L, b1, i, v, e, len, c);
       while (i - ln < b1) {
         const bool on = i < b1;
         const typename S::Count f = st.count(on ? v : n);
         const uint32_t at = e;
         const int groups = on ? len : 0;
         uint2 x = c;
-        fetch(b1, i, v, e, len, c);
+        fetch(L, b1, i, v, e, len, c);
         for (int j = 1; j <= groups; ++j) {
           uint2 nx = x;
           if (j < groups) nx = col[at + 32u * j];
@@ -503,7 +556,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
         lvl[0][0] = lvl[1][0] = 0;
         lvl[0][1] = 1 - k;
         lvl[1][1] = k;
-        s_next = s_wide[0] = s_wide[1] = 0;
+        s_next[0] = s_wide[0] = s_wide[1] = 0;
       }
       __syncthreads();
       int L = 0;
@@ -556,15 +609,15 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
           if (tid == 0) {
             lvl[0][L + 1] = ta;
             lvl[1][L + 1] = tb;
-            s_next = lvl[1][L];
+            s_next[L & 1] = lvl[1][L];
           }
           __syncthreads();
           continue;
         }
         if (s_wide[L & 1])
-          push_level(std::false_type(), lvl[0][L], a1, b1);
+          push_level(std::false_type(), L, lvl[0][L], a1, b1);
         else
-          push_level(std::true_type(), lvl[0][L], a1, b1);
+          push_level(std::true_type(), L, lvl[0][L], a1, b1);
         __syncthreads();
         // Close the vertices counted in this level and list them in id order:
         // each warp takes consecutive chunks (32 at most) and keeps chunk j's
@@ -617,13 +670,15 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
         if (tid == 0) {
           lvl[0][L + 1] = ta;
           lvl[1][L + 1] = tb;
-          s_next = lvl[1][L];
+          s_next[L & 1] = lvl[1][L];
         }
         __syncthreads();
       }
       const int deepest = L;
-      if (tid == 0) s_next = lvl[1][max(L - 1, 0)];  // the deepest level is not fetched
       for (; L > 0; --L) {
+        // for the level after this one (its parity's counter was last used
+        // before the previous barrier)
+        if (tid == 0) s_next[(L - 1) & 1] = lvl[1][L - 1];
         const int a1 = lvl[0][L + 1], b1 = lvl[1][L + 1];
         int held = 0, mine_v = 0;
         typename S::Value mine = S::none();  // lane j keeps the j-th sum of the warp, to finish 32 at once
@@ -636,7 +691,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
             uint32_t e = G.row[v] + ln;
             while (e < g1) {
 #pragma unroll 1
-              for (int k = 0; k < 8 && e < g1; ++k, e += kWarp) st.pull4(col[e], a);
+              for (int k = 0; k < 8 && e < g1; ++k, e += kWarp) st.pull4(col[e], L, a);
               S::after32(a);
             }
             acc = S::warp_sum(S::value(a));
@@ -646,21 +701,21 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
             mine_v = v;
           }
           if (++held == kWarp) {
-            st.finish(mine_v, mine, st.early(mine_v));
+            st.finish(mine_v, L, mine, st.early(mine_v));
             held = 0;
           }
         }
-        if (ln < held) st.finish(mine_v, mine, st.early(mine_v));
+        if (ln < held) st.finish(mine_v, L, mine, st.early(mine_v));
         if (L == deepest) {
           for (int i = lvl[1][L] + tid; i < b1; i += T) {
             const int v = q[nw + i];
-            st.finish(v, S::none(), st.early(v));
+            st.finish(v, L, S::none(), st.early(v));
           }
         } else {
           int i, len = 0;
           uint32_t v = 0, e = 0;
           uint2 c = make_uint2(0u, 0u);
-          fetch(b1, i, v, e, len, c);
+          fetch(L, b1, i, v, e, len, c);
           while (i - ln < b1) {
             const uint32_t u = v, at = e;
             const bool on = i < b1;
@@ -668,23 +723,18 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
             typename S::Early early{};
             if (on) early = st.early(u);
             uint2 x = c;
-            fetch(b1, i, v, e, len, c);
+            fetch(L, b1, i, v, e, len, c);
             typename S::Sum a = S::zero();
             for (int j = 1; j <= groups; ++j) {
               uint2 nx = x;
               if (j < groups) nx = col[at + 32u * j];
-              st.pull4(x, a);
+              st.pull4(x, L, a);
               if ((j & 7) == 0) S::after32(a);
               x = nx;
             }
-            if (on) st.finish(u, S::value(a), early);
+            if (on) st.finish(u, L, S::value(a), early);
           }
         }
-        __syncthreads();
-        // the level is complete: its psi are what the next level sums
-        if (tid == 0 && L < deepest) s_next = lvl[1][L - 1];
-        for (int i = lvl[0][L] + tid; i < a1; i += T) st.open(q[i]);
-        for (int i = lvl[1][L] + tid; i < b1; i += T) st.open(q[nw + i]);
         __syncthreads();
       }
       __syncthreads();
