@@ -27,6 +27,10 @@ struct DevGraph {
   const int32_t* in_colidx;
 };
 
+// Work counters of a gather kernel (WorkShare in msbfs.cu), each on a line of its own.
+constexpr int kWorkQueues = 8;
+constexpr int kWorkStride = 16;
+
 // Per-batch control block, resident in device memory.  Kernels read the
 // current frontier range from it, so a level's launches are identical from
 // level to level and the host never has to patch arguments.
@@ -53,7 +57,8 @@ struct BatchCtl {
   // lanes present in the current frontier Q_L (a superset is allowed): a lane
   // outside it discovers nothing at level L + 1, so bottom-up scans skip it
   unsigned long long front_union[kMaxWords];
-  unsigned long long work[2];     // next piece of the level's list or vertex range / hub items
+  // next units of the level's list or vertex range, and of the hub items
+  unsigned long long work[2][kWorkQueues * kWorkStride];
   int hubs;                       // a hub takes part in this level (bottom-up, backward)
   unsigned long long next_union[kMaxWords];  // lanes of Q_{L+1}, accumulated after its appends
 };

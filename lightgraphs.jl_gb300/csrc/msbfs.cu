@@ -46,27 +46,65 @@ __device__ __forceinline__ long long nwarps() {
   return (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
 }
 
-// Work of a gather kernel, handed out to warps in pieces as they come free:
-// rows differ by the hundredfold in cost, and with a fixed share per warp the
-// SMs held 23 of their 32 warps on average.  The next piece is asked for
-// before the current one is worked on.
-struct WorkQueue {
-  unsigned long long* next;
-  unsigned long long step, ahead;
-  __device__ __forceinline__ WorkQueue(unsigned long long* counter, unsigned step_) : next(counter), step(step_) {
-    ask();
+// Work of a gather kernel, handed out to warps one unit at a time as they come
+// free: rows differ by the hundredfold in cost, and with fixed shares the SMs
+// held 23 of their 32 warps on average.  Larger pieces spread the rows in
+// flight over more of the graph and were slower (2 / 4 / 8 entries: +0.2, +0.9,
+// +3.8 % on R-MAT 20).  One counter serves an atomic about every 1.4 ns, too
+// slow for the cheap rows of batches with few sources, so the units are dealt
+// out in turn to kWorkQueues counters; a warp whose counter has run out looks
+// at all of them at once and goes on with one that has not.  Few units are
+// taken as fixed shares, without atomics.  The next unit is asked for before
+// the current one is worked on.
+// (Units fit 32 bits: a level lists a vertex once, and hub items hold up to
+// kHubChunk entries each.)
+template <int KIND, bool QUEUE = true> struct WorkShare {
+  uint32_t total, ahead;
+  int q;  // the warp's counter; -1: fixed shares
+  __device__ __forceinline__ WorkShare(BatchCtl* c, unsigned long long total_) : total(static_cast<uint32_t>(total_)) {
+    q = -1;
+    ahead = static_cast<uint32_t>(gwarp());
+    if (QUEUE && total > 2u * static_cast<uint32_t>(nwarps())) {
+      q = static_cast<int>(blockIdx.x % kWorkQueues);
+      ask(c);
+    }
   }
-  __device__ __forceinline__ void ask() {
-    ahead = 0;
-    if (step && lane_id() == 0) ahead = atomicAdd(next, step);
+  __device__ __forceinline__ void ask(BatchCtl* c) {
+    if (lane_id() == 0) ahead = static_cast<uint32_t>(atomicAdd(&c->work[KIND][q * kWorkStride], 1ull));
   }
-  // First item of the next piece (warp-uniform).
-  __device__ __forceinline__ unsigned long long take() {
-    const unsigned long long at = shfl_u64(ahead, 0);
-    ask();
-    return at;
+  // The next unit; false when there is none (warp-uniform).
+  __device__ __forceinline__ bool take(BatchCtl* c, uint32_t& unit) {
+    if (!QUEUE || q < 0) {
+      unit = ahead;
+      ahead += static_cast<uint32_t>(nwarps());
+      return unit < total;
+    }
+    for (;;) {
+      unit = __shfl_sync(kFull, ahead, 0) * kWorkQueues + static_cast<uint32_t>(q);
+      if (unit < total) {
+        ask(c);
+        return true;
+      }
+      const uint32_t ln = static_cast<uint32_t>(lane_id());
+      bool left = false;
+      if (ln < kWorkQueues)
+        left = static_cast<uint32_t>(*reinterpret_cast<volatile unsigned long long*>(
+                   &c->work[KIND][ln * kWorkStride])) * kWorkQueues + ln < total;
+      const unsigned some = __ballot_sync(kFull, left);
+      if (!some) return false;
+      // the first at or after the own one, so that warps spread; a counter
+      // only grows, so each is tried again at most until it has run out
+      const unsigned after = some & ~((1u << q) - 1u);
+      q = __ffs(static_cast<int>(after ? after : some)) - 1;
+      ask(c);
+    }
   }
 };
+
+__device__ __forceinline__ void reset_work(BatchCtl* c) {
+  for (int i = 0; i < kWorkQueues; ++i) c->work[0][i * kWorkStride] = c->work[1][i * kWorkStride] = 0ull;
+  c->hubs = 0;
+}
 
 // Level-parity buffer select (a runtime index into the by-value array would
 // force the parameter struct into local memory).
@@ -907,8 +945,7 @@ __global__ void __launch_bounds__(kWideLanes) k_ms_init(DevGraph g, MsBuffers b,
   c->td_levels = 0;
   c->bu_levels = 0;
   c->runaway = 0;
-  c->work[0] = c->work[1] = 0ull;
-  c->hubs = 0;
+  reset_work(c);
   for (int j = 0; j < kMaxWords; ++j) {
     c->front_union[j] = j < W ? act.w[j % W] : 0ull;
     c->next_union[j] = 0ull;
@@ -1000,8 +1037,9 @@ __global__ void __launch_bounds__(256, W == 4 ? 3 : 4) k_ms_td_settle(DevGraph g
   Lanes<W>* visit = lanes_of<W>(b.visit);
   const int ln = lane_id();
   unsigned long long mf = 0, mu = 0, smax = 0;
-  WorkQueue wq(&c->work[0], 1);
-  for (unsigned long long i = lo + wq.take(); i < hi; i = lo + wq.take()) {
+  WorkShare<0> share(c, hi - lo);
+  for (uint32_t unit; share.take(c, unit);) {
+    const unsigned long long i = lo + unit;
     const int32_t w = b.qv[i];
     const Lanes<W> mask = next[w];
     const int64_t e0 = g.in_rowptr[w], e1 = g.in_rowptr[w + 1];
@@ -1060,8 +1098,9 @@ __global__ void __launch_bounds__(256, W == 4 ? 3 : 4) k_ms_bu(DevGraph g, MsBuf
     if (threadIdx.x == 0) live = frontier_lanes<W>(c);
     __syncthreads();
   }
-  WorkQueue wq(&c->work[0], kWarp);
-  for (int64_t base = static_cast<int64_t>(wq.take()); base < n; base = static_cast<int64_t>(wq.take())) {
+  WorkShare<0> share(c, static_cast<unsigned long long>((n + kWarp - 1) / kWarp));
+  for (uint32_t unit; share.take(c, unit);) {
+    const int64_t base = static_cast<int64_t>(unit) * kWarp;
     const int64_t wme = base + ln;
     bool cand = false;
     my_found[ln] = lz<W>();
@@ -1135,9 +1174,8 @@ __global__ void __launch_bounds__(256, W == 4 ? 3 : 4) k_ms_hub_pull(DevGraph g,
   // bottom-up: k_ms_bu saw whether a hub is left to finish (52,000 items that
   // only look were 72 us of atomics on the one counter)
   if (BU && c->hubs == 0) return;
-  WorkQueue wq(&c->work[1], BU ? 1 : 0);
-  for (long long it = BU ? static_cast<long long>(wq.take()) : gwarp(); it < hd.n_in;
-       it = BU ? static_cast<long long>(wq.take()) : it + nwarps()) {
+  WorkShare<1, BU> share(c, static_cast<unsigned long long>(hd.n_in));
+  for (uint32_t it; share.take(c, it);) {
     const HubItem I = hd.in_items[it];
     const int32_t h = I.v;
     Lanes<W> vis = lz<W>(), want;
@@ -1296,16 +1334,14 @@ __global__ void k_loop_back_arm(MsBuffers b, LoopParams lp) {
 __global__ void k_loop_back_advance(MsBuffers b, LoopParams lp) {
   BatchCtl* c = b.ctl;
   c->level -= 1;
-  c->work[0] = c->work[1] = 0ull;
-  c->hubs = 0;
+  reset_work(c);
   cudaGraphSetConditional(lp.loop, c->level >= 0 ? 1u : 0u);
 }
 
 __device__ __forceinline__ void advance_step(const MsBuffers& b, int64_t n) {
   BatchCtl* c = b.ctl;
   const int L = c->level;
-  c->work[0] = c->work[1] = 0ull;
-  c->hubs = 0;
+  reset_work(c);
   b.lvl_off[L + 2] = c->tail;
   // every count of level L + 1 is a sum of at most max-in-degree counts of
   // level L; once a level's largest count passes the limit, the next level
@@ -1363,8 +1399,9 @@ __global__ void __launch_bounds__(256, W == 1 ? 5 : (W == 2 ? 4 : 3)) k_ms_delta
   const Lanes<W>* qm = lanes_of<W>(b.qm);
   Lanes<W>* visit = lanes_of<W>(b.visit);
   const int ln = lane_id();
-  WorkQueue wq(&c->work[0], 1);
-  for (unsigned long long i = lo + wq.take(); i < hi; i = lo + wq.take()) {
+  WorkShare<0> share(c, hi - lo);
+  for (uint32_t unit; share.take(c, unit);) {
+    const unsigned long long i = lo + unit;
     const int32_t v = b.qv[i];
     const Lanes<W> F = qm[i];
     if (ln == 0) {
@@ -1421,8 +1458,8 @@ __global__ void __launch_bounds__(256, W == 1 ? 5 : (W == 2 ? 4 : 3)) k_ms_hub_d
   const Lanes<W>* __restrict__ cur = mbw<W>(b, L);
   const int ln = lane_id();
   if (c->hubs == 0) return;  // k_ms_delta met none in the level's list
-  WorkQueue wq(&c->work[1], 1);
-  for (long long it = static_cast<long long>(wq.take()); it < hd.n_out; it = static_cast<long long>(wq.take())) {
+  WorkShare<1> share(c, static_cast<unsigned long long>(hd.n_out));
+  for (uint32_t it; share.take(c, it);) {
     const HubItem I = hd.out_items[it];
     const int32_t h = I.v;
     const Lanes<W> F = cur[h];
@@ -1843,8 +1880,7 @@ __global__ void __launch_bounds__(256) k_st_hub_count(DevGraph g, MsBuffers b, H
 
 __global__ void k_ms_back_advance(MsBuffers b) {
   b.ctl->level -= 1;
-  b.ctl->work[0] = b.ctl->work[1] = 0ull;
-  b.ctl->hubs = 0;
+  reset_work(b.ctl);
 }
 
 // End of a Brandes batch: the backward sweep cleared visit for every listed
@@ -2063,8 +2099,7 @@ __global__ void k_ms_init_seeds_ctl(MsBuffers b, long long nseeds, unsigned long
   c->td_levels = 0;
   c->bu_levels = 0;
   c->runaway = 0;
-  c->work[0] = c->work[1] = 0ull;
-  c->hubs = 0;
+  reset_work(c);
   for (int j = 0; j < kMaxWords; ++j) {
     c->front_union[j] = ~0ull;  // every lane may be seeded
     c->next_union[j] = 0ull;
