@@ -1429,7 +1429,7 @@ int run_bfs(lgbc_graph* g, const DevGraph& dg, int64_t nsrc, bool prefilled) {
 int finish_bfs(lgbc_graph* g) {
   LGBC_CUDA(cudaStreamSynchronize(g->stream));
   const BfsState* st = reinterpret_cast<const BfsState*>(g->h_ctl);
-  if (st->failed) return fail(LGBC_ETIMEOUT, "BFS: a grid barrier ran out");
+  if (st->barrier.failed) return fail(LGBC_ETIMEOUT, "BFS: a grid barrier ran out");
   g->stats.topdown_levels += st->td_levels;
   g->stats.bottomup_levels += st->bu_levels;
   g->stats.levels += st->td_levels + st->bu_levels;

@@ -154,16 +154,7 @@ struct BfsWorkspace {
 // Learned-proposal state of a graph (learned.cu): core numbers, features,
 // scores, the proposal p and its CDF, and scan scratch.
 struct LearnedWorkspace {
-  int32_t* core = nullptr;
-  uint8_t* flag = nullptr;
-  int32_t* list = nullptr;
-  int32_t* large = nullptr;                // hubs deferred by a core pass
-  int32_t* log_v = nullptr;                // vertices lowered by a core pass
-  int32_t* log_old = nullptr;              //   and their values before it
-  int32_t* hub_v = nullptr;                // the same for the hubs
-  int32_t* hub_old = nullptr;
-  unsigned long long* counters = nullptr;  // [0] self-loop flag, [1] lowered this pass,
-                                           // [2] list size, [3] deferred hubs, [4] lowered hubs
+  CoreRun run{};                           // core numbers and the lists of their passes
   float4* feat = nullptr;
   float* y = nullptr;
   float* fscr = nullptr;
@@ -178,15 +169,18 @@ struct LearnedWorkspace {
   bool built = false;
   int64_t core_passes = 0;
   void release() {
-    dev_free(core);
-    dev_free(flag);
-    dev_free(list);
-    dev_free(large);
-    dev_free(log_v);
-    dev_free(log_old);
-    dev_free(hub_v);
-    dev_free(hub_old);
-    dev_free(counters);
+    dev_free(run.core);
+    dev_free(run.flag);
+    for (int i = 0; i < 2; ++i) {
+      dev_free(run.small[i]);
+      dev_free(run.hubs[i]);
+    }
+    dev_free(run.all_hubs);
+    dev_free(run.log_v);
+    dev_free(run.log_old);
+    dev_free(run.hub_v);
+    dev_free(run.hub_old);
+    dev_free(run.state);
     dev_free(feat);
     dev_free(y);
     dev_free(fscr);

@@ -12,18 +12,25 @@ namespace lgbc::api {
 
 int ensure_learned(lgbc_graph* g) {
   LearnedWorkspace& w = g->learned;
-  if (w.core) return LGBC_OK;
+  if (w.cdf) return LGBC_OK;  // allocated last
+  w.release();
   const size_t n = static_cast<size_t>(g->n);
   const size_t tiles = static_cast<size_t>(proposal_tiles(g->n));
-  LGBC_TRY(dev_alloc(&w.core, n));
-  LGBC_TRY(dev_alloc(&w.flag, n));
-  LGBC_TRY(dev_alloc(&w.list, n));
-  LGBC_TRY(dev_alloc(&w.large, n));
-  LGBC_TRY(dev_alloc(&w.log_v, n));
-  LGBC_TRY(dev_alloc(&w.log_old, n));
-  LGBC_TRY(dev_alloc(&w.hub_v, n));
-  LGBC_TRY(dev_alloc(&w.hub_old, n));
-  LGBC_TRY(dev_alloc(&w.counters, 5));
+  const size_t hubs = static_cast<size_t>(core_hub_cap(g->nnz, g->directed));
+  CoreRun& r = w.run;
+  LGBC_TRY(dev_alloc(&r.core, n));
+  LGBC_TRY(dev_alloc(&r.flag, (n + 31) / 32));
+  for (int i = 0; i < 2; ++i) {
+    LGBC_TRY(dev_alloc(&r.small[i], n));
+    LGBC_TRY(dev_alloc(&r.hubs[i], hubs));
+  }
+  LGBC_TRY(dev_alloc(&r.all_hubs, hubs));
+  LGBC_TRY(dev_alloc(&r.log_v, n));
+  LGBC_TRY(dev_alloc(&r.log_old, n));
+  LGBC_TRY(dev_alloc(&r.hub_v, hubs));
+  LGBC_TRY(dev_alloc(&r.hub_old, hubs));
+  LGBC_TRY(dev_alloc(&r.state, 1));
+  r.max_passes = g->nnz + 2;  // every pass with work lowers some value by at least one
   LGBC_TRY(dev_alloc(&w.feat, n));
   LGBC_TRY(dev_alloc(&w.y, n));
   LGBC_TRY(dev_alloc(&w.fscr, tiles + 1));
@@ -32,56 +39,40 @@ int ensure_learned(lgbc_graph* g) {
   LGBC_TRY(dev_alloc(&w.scal, 1));
   LGBC_TRY(dev_alloc(&w.p, n));
   LGBC_TRY(dev_alloc(&w.cdf, n));
-  LGBC_CUDA(cudaMemsetAsync(w.flag, 0, n, g->stream));
   return LGBC_OK;
 }
 
-unsigned long long read_counter(lgbc_graph* g, int i, int* rc) {
-  unsigned long long v = 0;
-  cudaError_t e = cudaMemcpyAsync(&v, g->learned.counters + i, 8, cudaMemcpyDeviceToHost, g->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-  *rc = e == cudaSuccess ? LGBC_OK : cuda_fail(e, "reading a device counter");
-  return v;
-}
-
-// Core numbers into learned.core: degrees without self-loops, then h-index
-// passes over the flagged vertices until none is lowered.  strict: a
-// self-loop is an error (core_number's ArgumentError).
-int compute_core(lgbc_graph* g, bool strict) {
+// Core numbers into learned.run.core: degrees without self-loops, then
+// h-index passes until none lowers a value.  Queued; finish_core checks them.
+int queue_core(lgbc_graph* g) {
   LearnedWorkspace& w = g->learned;
   const DevGraph dg = g->dev();
-  LGBC_CUDA(cudaMemsetAsync(w.counters, 0, 5 * 8, g->stream));
-  g->launches += core_degree(g->cfg, g->stream, dg, w.core, reinterpret_cast<int*>(w.counters));
-  LGBC_TRY(check_launch(g));
-  int rc = LGBC_OK;
-  const unsigned long long loops = read_counter(g, 0, &rc);
-  LGBC_TRY(rc);
-  if (strict && (loops & 0xffffffffull))
-    return fail(LGBC_EINVAL, "core_number: graph must not have self-loops");
-  const int32_t* list = nullptr;
-  int64_t nlist = g->n;
-  w.core_passes = 0;
-  while (nlist > 0) {
-    const CorePassBuffers cb{w.counters + 1, w.counters + 4, w.counters + 3, w.log_v,
-                             w.log_old,      w.hub_v,        w.hub_old,      w.large};
-    g->launches += core_pass(g->cfg, g->stream, dg, list, nlist, w.core, w.flag, cb);
-    LGBC_CUDA(cudaMemsetAsync(w.counters + 2, 0, 8, g->stream));
-    g->launches += core_compact(g->cfg, g->stream, g->n, w.flag, w.list, w.counters + 2);
-    LGBC_TRY(check_launch(g));
-    nlist = static_cast<int64_t>(read_counter(g, 2, &rc));
-    LGBC_TRY(rc);
-    list = w.list;
-    // every pass with work lowers some value by at least one; the values
-    // start at the degrees, so more passes than stored entries means a fault
-    if (++w.core_passes > g->nnz + 2) return fail(LGBC_ETIMEOUT, "core iteration did not settle");
-  }
+  LGBC_CUDA(cudaMemsetAsync(w.run.state, 0, sizeof(CoreState), g->stream));
+  g->launches += core_degree(g->cfg, g->stream, dg, w.run.core, &w.run.state->loops);
+  g->launches += core_run(g->cfg, g->stream, dg, w.run);
+  static_assert(sizeof(CoreState) <= sizeof(BatchCtl), "h_ctl holds either");
+  LGBC_CUDA(cudaMemcpyAsync(g->h_ctl, w.run.state, sizeof(CoreState), cudaMemcpyDeviceToHost, g->stream));
+  return check_launch(g);
+}
+
+// Waits for the stream.  strict: a self-loop is an error (core_number's
+// ArgumentError).
+int finish_core(lgbc_graph* g, bool strict) {
+  LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  const CoreState* st = reinterpret_cast<const CoreState*>(g->h_ctl);
+  if (st->barrier.failed) return fail(LGBC_ETIMEOUT, "core numbers: a grid barrier ran out");
+  if (strict && st->loops) return fail(LGBC_EINVAL, "core_number: graph must not have self-loops");
+  g->learned.core_passes = st->passes;
+  if (st->passes > g->learned.run.max_passes) return fail(LGBC_ETIMEOUT, "core iteration did not settle");
   return LGBC_OK;
 }
 
 int compute_features(lgbc_graph* g) {
   LGBC_TRY(ensure_learned(g));
-  LGBC_TRY(compute_core(g, false));
-  g->launches += features(g->cfg, g->stream, g->dev(), g->learned.core, g->learned.feat);
+  LGBC_TRY(queue_core(g));
+  LearnedWorkspace& w = g->learned;
+  // (e is the softmax's scratch, free until then)
+  g->launches += features(g->cfg, g->stream, g->dev(), w.run, reinterpret_cast<float2*>(w.e), w.feat);
   return check_launch(g);
 }
 
@@ -149,8 +140,9 @@ int lgbc_core_number(lgbc_graph* g, int32_t* core_out) {
   reset_stats(g);
   if (g->n == 0) return LGBC_OK;
   LGBC_TRY(ensure_learned(g));
-  LGBC_TRY(compute_core(g, true));
-  LGBC_CUDA(cudaMemcpyAsync(core_out, g->learned.core, static_cast<size_t>(g->n) * 4,
+  LGBC_TRY(queue_core(g));
+  LGBC_TRY(finish_core(g, true));
+  LGBC_CUDA(cudaMemcpyAsync(core_out, g->learned.run.core, static_cast<size_t>(g->n) * 4,
                             cudaMemcpyDeviceToHost, g->stream));
   LGBC_CUDA(cudaStreamSynchronize(g->stream));
   g->stats.levels = g->learned.core_passes;
@@ -169,7 +161,7 @@ int lgbc_features(lgbc_graph* g, float* feat_out) {
   LGBC_TRY(compute_features(g));
   LGBC_CUDA(cudaMemcpyAsync(feat_out, g->learned.feat, static_cast<size_t>(g->n) * 16,
                             cudaMemcpyDeviceToHost, g->stream));
-  LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  LGBC_TRY(finish_core(g, false));
   g->stats.levels = g->learned.core_passes;
   finish_stats(g);
   return LGBC_OK;
@@ -280,7 +272,7 @@ int lgbc_proposal_build(lgbc_graph* g, lgbc_mlp* m, double eps, double* p_out) {
   if (p_out)
     LGBC_CUDA(cudaMemcpyAsync(p_out, w.p, static_cast<size_t>(g->n) * 8, cudaMemcpyDeviceToHost,
                               g->stream));
-  LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  LGBC_TRY(finish_core(g, false));
   w.built = true;
   g->stats.levels = w.core_passes;
   finish_stats(g);

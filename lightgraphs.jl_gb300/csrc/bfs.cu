@@ -245,30 +245,6 @@ __global__ void k_bfs_advance(BatchCtl* c) {
 // The whole search in one cooperative launch.
 // ---------------------------------------------------------------------------
 
-// Grid barrier: every block adds one to an ever-growing count and waits until
-// all have.  The wait is bounded: a block that gives up, or sees that another
-// has, reports it, and the kernel returns.  All blocks are resident (the
-// launch is cooperative), so that happens only if the GPU is wedged.
-constexpr unsigned kBarrierPolls = 1u << 23;  // some seconds
-
-__device__ __forceinline__ bool grid_barrier(BfsState* st, unsigned long long& goal, int* ok) {
-  __syncthreads();
-  goal += gridDim.x;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(&st->arrived, 1ull);
-    unsigned polls = 0;
-    while (*reinterpret_cast<volatile unsigned long long*>(&st->arrived) < goal &&
-           *reinterpret_cast<volatile int*>(&st->failed) == 0) {
-      if (++polls > kBarrierPolls) atomicExch(&st->failed, 1);
-    }
-    __threadfence();
-    *ok = *reinterpret_cast<volatile int*>(&st->failed) == 0;
-  }
-  __syncthreads();
-  return *ok != 0;
-}
-
 // What a thread has found in this level.
 struct BfsFound {
   unsigned count = 0;
@@ -357,7 +333,7 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
       bitmap(1)[w0 >> 5] = 0u;
     }
   }
-  if (!grid_barrier(st, goal, &s_ok)) return;
+  if (!grid_barrier(&st->barrier, goal, &s_ok)) return;
   {
     BfsFound f;
     for (int64_t i0 = tid - ln; i0 < r.nsrc; i0 += threads) {
@@ -368,7 +344,7 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
     }
     report(&st->slot[0], f);
   }
-  if (!grid_barrier(st, goal, &s_ok)) return;
+  if (!grid_barrier(&st->barrier, goal, &s_ok)) return;
 
   unsigned long long lo = 0, mu_done = 0;
   bool bu = false;
@@ -401,7 +377,7 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
           bfs_list(g, r, own, lo, level & 1, has, v, true, ignored);
         }
       }
-      if (!grid_barrier(st, goal, &s_ok)) return;
+      if (!grid_barrier(&st->barrier, goal, &s_ok)) return;
       queued = __ldcg(&own->queued);
       big = __ldcg(&own->big);
     }
@@ -511,7 +487,7 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
     }
     report(nxt, f);
     lo = hi;
-    if (!grid_barrier(st, goal, &s_ok)) return;
+    if (!grid_barrier(&st->barrier, goal, &s_ok)) return;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->td_levels = td_levels;

@@ -60,30 +60,40 @@ __global__ void __launch_bounds__(256) k_core_degree(DevGraph g, int32_t* deg, i
 }
 
 // ---- h-index passes ------------------------------------------------------------
-// One pass computes, for every vertex of the list (all vertices at first), the
+// One pass computes, for every vertex to be searched (all at first), the
 // h-index of its neighbours' values -- the largest h <= c (its own value) with
 // #{neighbour entries u != v : core[u] >= h} >= h -- and lowers core[v] to it.
 // Updates are in place; a value read while a neighbour is being lowered is at
 // least that neighbour's core number, so every stored value stays >= the core
-// number.  Each lowered vertex is logged with its old value; after the pass,
-// k_core_flag flags the neighbours u whose count at their own value the drop
-// can have changed: lo < core[u] <= c_old (a neighbour that did not count for
-// u before, or still counts, cannot change u's h-index).  Only flagged
-// vertices are searched again; a pass that lowers nothing is the fixed point,
-// the core numbers.
+// number.  Each lowered vertex is logged with its old value; after the pass
+// the neighbours u whose count at their own value the drop can have changed,
+// lo < core[u] <= c_old (a neighbour that did not count for u before, or still
+// counts, cannot change u's h-index), are listed for the next.  A pass that
+// lowers nothing is the fixed point, the core numbers.
+//
+// All passes run in one cooperative launch with two grid barriers a pass, in
+// place of five kernels, four memsets and a read-back.  Most of the 13 to 45
+// passes touch little, so what bounds them is latency: the serial chain of a
+// warp's vertices (fewer per warp on short lists) and of a long row (several
+// entries per thread in flight).  core_number: R-MAT of 2,178 / 16,384 /
+// 131,072 / 1,048,576 vertices 838 / 1,115 / 2,587 / 7,329 us launched one by
+// one, 244 / 407 / 1,427 / 6,919 us here.  Values are read past L1, which
+// keeps lines from earlier passes.
 struct CoreLog {
   unsigned long long* count;  // lowered vertices this pass
-  int32_t* v;                 // n entries: the vertex
-  int32_t* old;               // n entries: its value before the pass
+  int32_t* v;                 // the vertex
+  int32_t* old;               // its value before the pass
 };
 
 // A vertex with at most kCoreCached neighbour entries keeps their values
 // (capped at c) in registers, entry k * 32 + lane in slot k of that lane, so
-// the search reads memory once; larger lists go to k_core_pass_large.
+// the search reads memory once; larger lists (hubs) take a block.
 constexpr int kCoreSlots = 8;
-constexpr int kCoreCached = kCoreSlots * kWarp;
+static_assert(kCoreCached == kCoreSlots * kWarp, "a warp's registers hold a row");
 // A vertex with at most kCoreThread entries is searched by one thread.
 constexpr int kCoreThread = 16;
+// Entries of a long row that a thread has in flight.
+constexpr int kCoreAhead = 8;
 
 __device__ __forceinline__ int core_entries(const DevGraph& g, int32_t v) {
   int64_t d = g.rowptr[v + 1] - g.rowptr[v];
@@ -112,7 +122,7 @@ __device__ __forceinline__ int32_t core_search_thread(const DevGraph& g, int32_t
     if (k < ent) {
       const int32_t u = core_entry(g, v, o0, n0, k);
       if (u >= 0 && u != v) {
-        const int32_t cu = core[u];
+        const int32_t cu = __ldcg(core + u);
         x[k] = cu < c ? cu : c;
       }
     }
@@ -139,7 +149,7 @@ __device__ __forceinline__ int32_t core_search_warp(const DevGraph& g, int32_t v
     x[k] = -1;
     const int32_t u = core_entry(g, v, o0, n0, static_cast<int64_t>(k) * kWarp + ln);
     if (u >= 0 && u != v) {
-      const int32_t cu = core[u];
+      const int32_t cu = __ldcg(core + u);
       x[k] = cu < c ? cu : c;
     }
   }
@@ -165,21 +175,25 @@ __device__ __forceinline__ void core_log(const CoreLog& lg, unsigned long long a
   lg.old[at] = old;
 }
 
-// One pass: lane j of a warp takes list entry base + j.  Vertices with at
-// most kCoreThread entries are searched by their own lane; the others, one at
-// a time, by the whole warp, or deferred to `large` (more than kCoreCached
-// entries) for k_core_pass_large.
-__global__ void __launch_bounds__(256) k_core_pass(DevGraph g, const int32_t* list, long long nlist,
-                                                  int32_t* core, CoreLog lg, int32_t* large,
-                                                  unsigned long long* nlarge) {
+// Lane j of a warp takes entry base + j of the list (all vertices when it is
+// null; hubs are passed over there).  Vertices with at most kCoreThread
+// entries are searched by their own lane; the others, one at a time, by the
+// whole warp.
+__device__ __forceinline__ void core_search_small(const DevGraph& g, const int32_t* list, long long nlist,
+                                                  uint32_t* flag, int32_t* core, CoreLog lg) {
   const int ln = lane_id();
-  for (long long base = gwarp() * kWarp; base < nlist; base += nwarps() * kWarp) {
-    const long long i = base + ln;
+  // 32 entries a warp at most, fewer on a short list: a vertex that takes the
+  // whole warp is three dependent round trips, one after the other
+  const long long share = (nlist + nwarps() - 1) / nwarps();
+  const int per = static_cast<int>(min(max(share, 1ll), static_cast<long long>(kWarp)));
+  for (long long base = gwarp() * per; base < nlist; base += nwarps() * per) {
+    const long long i = ln < per ? base + ln : nlist;
     int32_t v = 0, c = 0;
     int ent = 0;
     if (i < nlist) {
-      v = list ? list[i] : static_cast<int32_t>(i);
-      c = core[v];
+      v = list ? __ldcg(list + i) : static_cast<int32_t>(i);
+      if (list) atomicAnd(flag + (v >> 5), ~(1u << (v & 31)));
+      c = __ldcg(core + v);
       if (c > 0) ent = core_entries(g, v);
     }
     int32_t h = c;
@@ -188,17 +202,12 @@ __global__ void __launch_bounds__(256) k_core_pass(DevGraph g, const int32_t* li
     if (lowered) core[v] = h;
     const unsigned long long at = warp_append(lowered, lg.count);
     if (lowered) core_log(lg, at, v, c);
-    unsigned rest = __ballot_sync(kFull, c > 0 && ent > kCoreThread);
+    unsigned rest = __ballot_sync(kFull, c > 0 && ent > kCoreThread && ent <= kCoreCached);
     while (rest) {
       const int j = __ffs(rest) - 1;
       rest &= rest - 1u;
       const int32_t vj = __shfl_sync(kFull, v, j);
       const int32_t cj = __shfl_sync(kFull, c, j);
-      const int entj = __shfl_sync(kFull, ent, j);
-      if (entj > kCoreCached) {
-        if (ln == 0) large[atomicAdd(nlarge, 1ull)] = vj;
-        continue;
-      }
       const int32_t hj = core_search_warp(g, vj, cj, core);
       if (hj < cj && ln == 0) {
         core[vj] = hj;
@@ -231,45 +240,49 @@ __device__ __forceinline__ int block_count_at_least(const DevGraph& g, int32_t v
   int c = 0;
   for (int64_t e = g.rowptr[v] + threadIdx.x; e < g.rowptr[v + 1]; e += blockDim.x) {
     const int32_t u = g.colidx[e];
-    c += (u != v && core[u] >= h) ? 1 : 0;
+    c += (u != v && __ldcg(core + u) >= h) ? 1 : 0;
   }
   if (is_digraph(g))
     for (int64_t e = g.in_rowptr[v] + threadIdx.x; e < g.in_rowptr[v + 1]; e += blockDim.x) {
       const int32_t u = g.in_colidx[e];
-      c += (u != v && core[u] >= h) ? 1 : 0;
+      c += (u != v && __ldcg(core + u) >= h) ? 1 : 0;
     }
   return block_sum_int(c, red);
 }
 
-__global__ void __launch_bounds__(256) k_core_pass_large(DevGraph g, const int32_t* large,
-                                                        const unsigned long long* nlarge,
-                                                        int32_t* core, CoreLog lg) {
-  // lg: the hubs' own log (their neighbours are flagged by k_core_flag_large)
+__device__ __forceinline__ void core_search_hubs(const DevGraph& g, const int32_t* hubs, unsigned long long nl,
+                                                 uint32_t* flag, int32_t* core, CoreLog lg) {
   __shared__ int hist[kCoreHist + 1];
   __shared__ int red[8];
   __shared__ int s_h;
-  const unsigned long long nl = *nlarge;
   const bool dir = is_digraph(g);
   for (unsigned long long i = blockIdx.x; i < nl; i += gridDim.x) {
-    const int32_t v = large[i];
-    const int32_t c = core[v];
+    const int32_t v = __ldcg(hubs + i);
+    const int32_t c = __ldcg(core + v);
+    if (threadIdx.x == 0) atomicAnd(flag + (v >> 5), ~(1u << (v & 31)));
     const int cap = c < kCoreHist ? c : kCoreHist;
     for (int b = threadIdx.x; b <= cap; b += blockDim.x) hist[b] = 0;
     __syncthreads();
-    // lanes with the same bin add their count with one atomic
+    // Lanes with the same bin add their count with one atomic.  A thread has
+    // kCoreAhead entries in flight: one at a time the longest row of R-MAT 17
+    // took 80 dependent round trips, 60 us, in every pass that searched it.
     auto bin_list = [&](const int32_t* ci, int64_t e0, int64_t e1) {
-      for (int64_t b0 = e0 + (threadIdx.x & ~(kWarp - 1)); b0 < e1; b0 += blockDim.x) {
-        const int64_t e = b0 + lane_id();
-        int bin = -1;
-        if (e < e1) {
-          const int32_t u = ci[e];
-          if (u != v) {
-            const int32_t cu = core[u];
-            bin = cu < cap ? cu : cap;
-          }
+      for (int64_t b0 = e0 + (threadIdx.x & ~(kWarp - 1)); b0 < e1; b0 += kCoreAhead * static_cast<int64_t>(blockDim.x)) {
+        int bin[kCoreAhead];
+#pragma unroll
+        for (int q = 0; q < kCoreAhead; ++q) {
+          const int64_t e = b0 + q * static_cast<int64_t>(blockDim.x) + lane_id();
+          bin[q] = -1;
+          if (e < e1) bin[q] = ci[e];
         }
-        const unsigned peers = __match_any_sync(kFull, bin);
-        if (bin >= 0 && lane_id() == __ffs(peers) - 1) atomicAdd(&hist[bin], __popc(peers));
+#pragma unroll
+        for (int q = 0; q < kCoreAhead; ++q)
+          if (bin[q] >= 0) bin[q] = bin[q] == v ? -1 : min(__ldcg(core + bin[q]), cap);
+#pragma unroll
+        for (int q = 0; q < kCoreAhead; ++q) {
+          const unsigned peers = __match_any_sync(kFull, bin[q]);
+          if (bin[q] >= 0 && lane_id() == __ffs(peers) - 1) atomicAdd(&hist[bin[q]], __popc(peers));
+        }
       }
     };
     bin_list(g.colidx, g.rowptr[v], g.rowptr[v + 1]);
@@ -319,70 +332,94 @@ __global__ void __launch_bounds__(256) k_core_pass_large(DevGraph g, const int32
   }
 }
 
-// After a pass: for each logged vertex v (value c_old -> lo), flag the
-// neighbours u with lo < core[u] <= c_old.  A warp per logged vertex (lists
-// of at most kCoreCached entries); k_core_flag_large gives each logged hub a
-// block.
-__global__ void __launch_bounds__(256) k_core_flag(DevGraph g, const int32_t* core, uint8_t* flag,
-                                                  CoreLog lg) {
-  const unsigned long long nlog = *lg.count;
+// List u for the next pass, once, where `ok` (lo < core[u] <= old) and its flag
+// was clear.
+__device__ __forceinline__ void core_list(const DevGraph& g, const CoreRun& r, CoreSlot* nxt, int parity, bool ok,
+                                          int32_t u) {
+  if (!__any_sync(kFull, ok)) return;
+  const uint32_t bit = 1u << (u & 31);
+  const bool take = ok && !(atomicOr(r.flag + (u >> 5), bit) & bit);
+  const bool hub = take && core_entries(g, u) > kCoreCached;
+  const unsigned long long a = warp_append(take && !hub, &nxt->small);
+  if (take && !hub) (parity ? r.small[1] : r.small[0])[a] = u;
+  const unsigned long long b = warp_append(hub, &nxt->hubs);
+  if (hub) (parity ? r.hubs[1] : r.hubs[0])[b] = u;
+}
+
+// The neighbours of one lowered vertex (value old -> lo), AHEAD * 32 entries a
+// step; `first` / `step`: the warp's share of the list.
+template <int AHEAD>
+__device__ __forceinline__ void core_list_neighbours(const DevGraph& g, const CoreRun& r, CoreSlot* nxt, int parity,
+                                                     int32_t v, int32_t lo, int32_t old, int first, int step) {
   const int ln = lane_id();
-  for (unsigned long long i = gwarp(); i < nlog; i += nwarps()) {
-    const int32_t v = lg.v[i];
-    const int32_t c_old = lg.old[i];
-    const int32_t lo = core[v];
-    for (int64_t e = g.rowptr[v] + ln; e < g.rowptr[v + 1]; e += kWarp) {
-      const int32_t u = g.colidx[e];
-      const int32_t cu = core[u];
-      if (u != v && cu > lo && cu <= c_old) flag[u] = 1;
-    }
-    if (is_digraph(g))
-      for (int64_t e = g.in_rowptr[v] + ln; e < g.in_rowptr[v + 1]; e += kWarp) {
-        const int32_t u = g.in_colidx[e];
-        const int32_t cu = core[u];
-        if (u != v && cu > lo && cu <= c_old) flag[u] = 1;
+  for (int side = 0; side < (is_digraph(g) ? 2 : 1); ++side) {
+    const int64_t* rp = side ? g.in_rowptr : g.rowptr;
+    const int32_t* ci = side ? g.in_colidx : g.colidx;
+    const int64_t e1 = rp[v + 1];
+    for (int64_t e = rp[v] + first * AHEAD * kWarp; e < e1; e += static_cast<int64_t>(step) * AHEAD * kWarp) {
+      int32_t u[AHEAD];
+      bool ok[AHEAD];
+#pragma unroll
+      for (int q = 0; q < AHEAD; ++q) {
+        const int64_t i = e + q * kWarp + ln;
+        u[q] = i < e1 ? ci[i] : v;
       }
+#pragma unroll
+      for (int q = 0; q < AHEAD; ++q) {
+        const int32_t cu = u[q] != v ? __ldcg(r.core + u[q]) : lo;
+        ok[q] = cu > lo && cu <= old;
+      }
+#pragma unroll
+      for (int q = 0; q < AHEAD; ++q) core_list(g, r, nxt, parity, ok[q], u[q]);
+    }
   }
 }
 
-__global__ void __launch_bounds__(256) k_core_flag_large(DevGraph g, const int32_t* core,
-                                                        uint8_t* flag, CoreLog lg) {
-  const unsigned long long nlog = *lg.count;
-  for (unsigned long long i = blockIdx.x; i < nlog; i += gridDim.x) {
-    const int32_t v = lg.v[i];
-    const int32_t c_old = lg.old[i];
-    const int32_t lo = core[v];
-    for (int64_t e = g.rowptr[v] + threadIdx.x; e < g.rowptr[v + 1]; e += blockDim.x) {
-      const int32_t u = g.colidx[e];
-      const int32_t cu = core[u];
-      if (u != v && cu > lo && cu <= c_old) flag[u] = 1;
-    }
-    if (is_digraph(g))
-      for (int64_t e = g.in_rowptr[v] + threadIdx.x; e < g.in_rowptr[v + 1]; e += blockDim.x) {
-        const int32_t u = g.in_colidx[e];
-        const int32_t cu = core[u];
-        if (u != v && cu > lo && cu <= c_old) flag[u] = 1;
-      }
-  }
-}
-
-// Gather the flagged vertices into `list` (and clear the flags).
-__global__ void k_core_compact(int64_t n, uint8_t* flag, int32_t* list, unsigned long long* count) {
+__global__ void __launch_bounds__(256) k_core_run(DevGraph g, CoreRun r) {
+  __shared__ int s_ok;
+  CoreState* st = r.state;
   const int ln = lane_id();
-  for (long long base = static_cast<long long>(blockIdx.x) * blockDim.x; base < n;
-       base += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long v = base + threadIdx.x;
-    const bool f = v < n && flag[v];
-    const unsigned bal = __ballot_sync(kFull, f);
-    if (!bal) continue;
-    unsigned long long at = 0;
-    if (ln == 0) at = atomicAdd(count, static_cast<unsigned long long>(__popc(bal)));
-    at = __shfl_sync(kFull, at, 0);
-    if (f) {
-      flag[v] = 0;
-      list[at + __popc(bal & ((1u << ln) - 1u))] = static_cast<int32_t>(v);
-    }
+  const int wid = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+  unsigned long long goal = 0;
+  for (long long base = gwarp() * kWarp; base < g.n; base += nwarps() * kWarp) {
+    const long long v = base + ln;
+    if (ln == 0) r.flag[base >> 5] = 0u;
+    const bool hub = v < g.n && core_entries(g, static_cast<int32_t>(v)) > kCoreCached;
+    if (!__any_sync(kFull, hub)) continue;
+    const unsigned long long at = warp_append(hub, &st->all_hubs);
+    if (hub) r.all_hubs[at] = static_cast<int32_t>(v);
   }
+  if (!grid_barrier(&st->barrier, goal, &s_ok)) return;
+  long long pass = 0;
+  for (;; ++pass) {
+    // a slot is reused three passes later, by when every block has read it
+    CoreSlot* cur = &st->slot[pass % 3];
+    CoreSlot* nxt = &st->slot[(pass + 1) % 3];
+    const long long nsmall = pass ? static_cast<long long>(__ldcg(&cur->small)) : g.n;
+    const unsigned long long nhubs = pass ? __ldcg(&cur->hubs) : __ldcg(&st->all_hubs);
+    if ((nsmall == 0 && nhubs == 0) || pass > r.max_passes) break;
+    const int from = static_cast<int>(pass & 1), to = from ^ 1;
+    core_search_hubs(g, pass ? (from ? r.hubs[1] : r.hubs[0]) : r.all_hubs, nhubs, r.flag, r.core,
+                     CoreLog{&cur->hub_log, r.hub_v, r.hub_old});
+    core_search_small(g, pass ? (from ? r.small[1] : r.small[0]) : nullptr, nsmall, r.flag, r.core,
+                      CoreLog{&cur->log, r.log_v, r.log_old});
+    if (!grid_barrier(&st->barrier, goal, &s_ok)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      CoreSlot* z = &st->slot[(pass + 2) % 3];
+      z->small = z->hubs = z->log = z->hub_log = 0ull;
+    }
+    const unsigned long long nhl = __ldcg(&cur->hub_log), nl = __ldcg(&cur->log);
+    for (unsigned long long i = blockIdx.x; i < nhl; i += gridDim.x) {
+      const int32_t v = __ldcg(r.hub_v + i);
+      core_list_neighbours<kCoreAhead>(g, r, nxt, to, v, __ldcg(r.core + v), __ldcg(r.hub_old + i), wid, wpb);
+    }
+    for (unsigned long long i = gwarp(); i < nl; i += nwarps()) {
+      const int32_t v = __ldcg(r.log_v + i);
+      core_list_neighbours<2>(g, r, nxt, to, v, __ldcg(r.core + v), __ldcg(r.log_old + i), 0, 1);
+    }
+    if (!grid_barrier(&st->barrier, goal, &s_ok)) return;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) st->passes = pass;
 }
 
 // ---------------------------------------------------------------------------
@@ -390,31 +427,82 @@ __global__ void k_core_compact(int64_t n, uint8_t* flag, int32_t* list, unsigned
 // neighbours u, log(1 + sum of the neighbours' degrees)).  Degrees here are
 // CSR row lengths (a self-loop counts once, as length(fadjlist[v])).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_features(DevGraph g, const int32_t* core, float4* feat) {
+// The two terms a neighbour adds, once per vertex: log(1 + deg) and deg.
+__global__ void k_feature_terms(DevGraph g, float2* terms) {
+  for (int64_t v = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; v < g.n;
+       v += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t d = g.rowptr[v + 1] - g.rowptr[v];
+    terms[v] = make_float2(log1pf(static_cast<float>(d)), __int_as_float(static_cast<int>(d)));
+  }
+}
+
+// Lane sums to the vertex's features (every lane of the warp takes part).
+__device__ __forceinline__ void put_features(int64_t v, int64_t d, const int32_t* core, float sl,
+                                             unsigned long long sd, float4* feat) {
+  for (int o = 16; o > 0; o >>= 1) {
+    sl += __shfl_xor_sync(kFull, sl, o);
+    sd += __shfl_xor_sync(kFull, sd, o);
+  }
+  if (lane_id() == 0) {
+    float4 f;
+    f.x = log1pf(static_cast<float>(d));
+    f.y = log1pf(static_cast<float>(core[v]));
+    f.z = d > 0 ? sl / static_cast<float>(d) : 0.f;
+    f.w = log1pf(static_cast<float>(sd));
+    feat[v] = f;
+  }
+}
+
+// One warp per vertex, lane j adding entries j, j + 32, ... in that order
+// (hubs: k_features_hubs, with the same sums).
+__global__ void __launch_bounds__(256) k_features(DevGraph g, const int32_t* core, const float2* terms,
+                                                  float4* feat) {
   const int ln = lane_id();
   for (long long v = gwarp(); v < g.n; v += nwarps()) {
     const int64_t e0 = g.rowptr[v], e1 = g.rowptr[v + 1];
+    if (e1 - e0 > kCoreCached) continue;
     float sl = 0.f;
     unsigned long long sd = 0;
+#pragma unroll 4
     for (int64_t e = e0 + ln; e < e1; e += kWarp) {
-      const int32_t u = g.colidx[e];
-      const int64_t du = g.rowptr[u + 1] - g.rowptr[u];
-      sl += log1pf(static_cast<float>(du));
-      sd += static_cast<unsigned long long>(du);
+      const float2 t = terms[g.colidx[e]];
+      sl += t.x;
+      sd += static_cast<unsigned long long>(__float_as_int(t.y));
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      sl += __shfl_xor_sync(kFull, sl, o);
-      sd += __shfl_xor_sync(kFull, sd, o);
+    put_features(v, e1 - e0, core, sl, sd, feat);
+  }
+}
+
+// A block per hub: all warps bring the terms into shared memory, the first
+// adds them up in the order one warp alone would (the longest row of R-MAT 17
+// kept a single warp busy for 200 us).
+__global__ void __launch_bounds__(256) k_features_hubs(DevGraph g, const int32_t* core, const float2* terms,
+                                                       const int32_t* hubs, const unsigned long long* count,
+                                                       float4* feat) {
+  constexpr int kPiece = 2048;
+  __shared__ float2 part[kPiece];
+  const unsigned long long nh = *count;
+  for (unsigned long long i = blockIdx.x; i < nh; i += gridDim.x) {
+    const int32_t v = hubs[i];
+    const int64_t e0 = g.rowptr[v], e1 = g.rowptr[v + 1];
+    float sl = 0.f;
+    unsigned long long sd = 0;
+    for (int64_t p = e0; p < e1; p += kPiece) {
+      const int m = static_cast<int>(min(static_cast<int64_t>(kPiece), e1 - p));
+#pragma unroll
+      for (int q = 0; q < kPiece / 256; ++q) {
+        const int k = q * 256 + static_cast<int>(threadIdx.x);
+        if (k < m) part[k] = terms[g.colidx[p + k]];
+      }
+      __syncthreads();
+      if (threadIdx.x < kWarp)
+        for (int k = static_cast<int>(threadIdx.x); k < m; k += kWarp) {
+          sl += part[k].x;
+          sd += static_cast<unsigned long long>(__float_as_int(part[k].y));
+        }
+      __syncthreads();
     }
-    if (ln == 0) {
-      const int64_t d = e1 - e0;
-      float4 f;
-      f.x = log1pf(static_cast<float>(d));
-      f.y = log1pf(static_cast<float>(core[v]));
-      f.z = d > 0 ? sl / static_cast<float>(d) : 0.f;
-      f.w = log1pf(static_cast<float>(sd));
-      feat[v] = f;
-    }
+    if (threadIdx.x < kWarp) put_features(v, e1 - e0, core, sl, sd, feat);
   }
 }
 
@@ -869,33 +957,27 @@ int core_degree(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, int32_t* 
   return 1;
 }
 
-int core_pass(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, const int32_t* list,
-              int64_t nlist, int32_t* core, uint8_t* flag, const CorePassBuffers& b) {
-  if (nlist <= 0) return 0;
-  const int64_t want = (nlist + 255) / 256;  // a warp takes 32 entries, a block 256
-  const int grid = static_cast<int>(want < c.grid ? want : c.grid);
-  const CoreLog lg{b.changed, b.log_v, b.log_old};
-  const CoreLog lh{b.changed_hubs, b.hub_v, b.hub_old};
-  cudaMemsetAsync(b.changed, 0, sizeof(unsigned long long), s);
-  cudaMemsetAsync(b.changed_hubs, 0, sizeof(unsigned long long), s);
-  cudaMemsetAsync(b.nlarge, 0, sizeof(unsigned long long), s);
-  k_core_pass<<<grid, 256, 0, s>>>(g, list, nlist, core, lg, b.large, b.nlarge);
-  k_core_pass_large<<<c.grid, 256, 0, s>>>(g, b.large, b.nlarge, core, lh);
-  k_core_flag<<<c.grid, 256, 0, s>>>(g, core, flag, lg);
-  k_core_flag_large<<<c.grid, 256, 0, s>>>(g, core, flag, lh);
-  return 4;
-}
-
-int core_compact(const LaunchCfg& c, cudaStream_t s, int64_t n, uint8_t* flag, int32_t* list,
-                 unsigned long long* count) {
-  k_core_compact<<<c.grid, c.block, 0, s>>>(n, flag, list, count);
+int core_run(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, const CoreRun& r) {
+  int per_sm = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_core_run, 256, 0) != cudaSuccess || per_sm < 1)
+    per_sm = 1;
+  // the barrier costs more with more blocks: some hundred entries for each
+  const int64_t want = g.nnz / 512 + 1;
+  const int64_t most = static_cast<int64_t>(c.sms) * (per_sm < 4 ? per_sm : 4);
+  DevGraph dg = g;
+  CoreRun rr = r;
+  void* args[] = {&dg, &rr};
+  cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_core_run),
+                              dim3(static_cast<unsigned>(want < most ? want : most)), dim3(256), args, 0, s);
   return 1;
 }
 
-int features(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, const int32_t* core,
+int features(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, const CoreRun& r, float2* terms,
              float4* feat) {
-  k_features<<<c.grid, c.block, 0, s>>>(g, core, feat);
-  return 1;
+  k_feature_terms<<<c.grid, c.block, 0, s>>>(g, terms);
+  k_features_hubs<<<c.grid, 256, 0, s>>>(g, r.core, terms, r.all_hubs, &r.state->all_hubs, feat);
+  k_features<<<c.grid, c.block, 0, s>>>(g, r.core, terms, feat);
+  return 3;
 }
 
 int mlp_forward(const LaunchCfg& c, cudaStream_t s, const float4* x, int64_t rows,

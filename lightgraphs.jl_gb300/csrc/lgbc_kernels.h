@@ -277,8 +277,7 @@ struct BfsSlot {                // one level's frontier, rotating over three
   unsigned long long big;            // entries << 32 | chunks of the list of long out-lists
 };
 struct BfsState {               // zeroed before the launch
-  unsigned long long arrived;   // grid barrier
-  int failed;
+  GridBarrier barrier;
   BfsSlot slot[3];
   long long td_levels, bu_levels;
 };
@@ -352,27 +351,36 @@ int add_endpoints_many(const LaunchCfg& c, cudaStream_t s, double* bc, const int
 // ---- learned source proposal: learned.cu ----------------------------------
 // deg[v] = neighbours other than v; *loops |= 1 if v has a self-loop.
 int core_degree(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, int32_t* deg, int* loops);
-// One h-index pass over list[0, nlist) (all vertices when list is null):
-// lowered vertices are logged (vertex, old value) -- those with more than 256
-// neighbour entries ("hubs", deferred to `large` and searched by a block each)
-// in the hub log -- and then their neighbours whose count can have changed
-// are flagged.  Every array holds n entries.
-struct CorePassBuffers {
-  unsigned long long* changed;       // lowered non-hub vertices this pass
-  unsigned long long* changed_hubs;  // lowered hubs this pass
-  unsigned long long* nlarge;        // hubs deferred this pass
-  int32_t* log_v;
-  int32_t* log_old;
-  int32_t* hub_v;
-  int32_t* hub_old;
-  int32_t* large;
+// Core numbers from the degrees in core (h-index passes until none is
+// lowered), in one cooperative launch.
+constexpr int kCoreCached = 256;       // vertices with more neighbour entries are hubs
+struct CoreSlot {                      // one pass, rotating over three
+  unsigned long long small, hubs;      // vertices to search
+  unsigned long long log, hub_log;     // vertices lowered
 };
-int core_pass(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, const int32_t* list,
-              int64_t nlist, int32_t* core, uint8_t* flag, const CorePassBuffers& b);
-// list <- flagged vertices (flags cleared), *count += their number.
-int core_compact(const LaunchCfg& c, cudaStream_t s, int64_t n, uint8_t* flag, int32_t* list,
-                 unsigned long long* count);
-int features(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, const int32_t* core,
+struct CoreState {                     // zeroed before the launch
+  GridBarrier barrier;
+  CoreSlot slot[3];
+  unsigned long long all_hubs;         // entries of CoreRun::all_hubs
+  long long passes;
+  int loops;                           // a vertex has a self-loop (core_degree)
+};
+struct CoreRun {
+  int32_t* core;                       // n
+  uint32_t* flag;                      // (n + 31) / 32 words
+  int32_t* small[2];                   // n each
+  int32_t* hubs[2];                    // hub_cap each
+  int32_t* all_hubs;                   // hub_cap
+  int32_t *log_v, *log_old;            // n
+  int32_t *hub_v, *hub_old;            // hub_cap
+  CoreState* state;
+  long long max_passes;                // more means a fault
+};
+// At most this many vertices have more than kCoreCached entries.
+inline int64_t core_hub_cap(int64_t nnz, int directed) { return (directed ? 2 * nnz : nnz) / kCoreCached + 1; }
+int core_run(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, const CoreRun& r);
+// terms: n float2 of scratch; all_hubs / state: as core_run left them.
+int features(const LaunchCfg& c, cudaStream_t s, const DevGraph& g, const CoreRun& r, float2* terms,
              float4* feat);
 
 // MLP parameter layout (floats): W1[64][4], b1[64], W2[64][64], b2[64], W3[64], b3.

@@ -326,3 +326,22 @@ def test_core_number_hubs(name):
     np.testing.assert_array_equal(got, oracle.core_number(rp, ci, **kw))
     if name == "clique1100_with_tail":
         assert got[:1100].min() == 1099
+
+
+@pytest.mark.parametrize("degree", [16, 17, 255, 256, 257, 2047, 2048, 2049, 5000])
+def test_core_numbers_and_features_at_row_lengths(degree):
+    # rows on both sides of the lengths that a thread, a warp and a block take,
+    # and of a block's pieces, over a random graph whose values settle slowly
+    n = max(600, degree + 100)
+    rng = np.random.default_rng(degree)
+    e = rng.integers(0, n, (2, 3 * n))
+    src = np.concatenate([e[0], np.full(degree, n)])
+    dst = np.concatenate([e[1], rng.choice(n, degree, replace=False)])
+    keep = src != dst
+    g = lgbc.SimpleGraph.from_edge_arrays(n + 1, src[keep], dst[keep])
+    rp, ci = g.csr()
+    assert rp[n + 1] - rp[n] == degree
+    np.testing.assert_array_equal(lgbc.core_number(g), oracle.core_number(rp, ci))
+    # a lane adds degree / 32 terms one after the other, then five pairs
+    rtol = (degree / 32 + 8) * 2.0**-24 + 4 * 2.0**-24
+    np.testing.assert_allclose(lgbc.features(g), oracle.features(rp, ci), rtol=rtol, atol=rtol)
