@@ -980,14 +980,21 @@ int filter_sources(lgbc_graph* g, const int32_t* src, int64_t nsrc) {
   return LGBC_OK;
 }
 
-// g->h_active to g->d_src (a pageable copy: staged before the call returns).
+// A call's source list to g->d_src (short ones through pinned memory).
+int copy_sources(lgbc_graph* g, const int32_t* src, int64_t k) {
+  LGBC_TRY(ensure_src(g, k));
+  if (k <= 0) return LGBC_OK;
+  if (k <= kPinnedSources) {
+    std::memcpy(g->h_src, src, static_cast<size_t>(k) * 4);
+    src = g->h_src;
+  }
+  LGBC_CUDA(cudaMemcpyAsync(g->d_src, src, static_cast<size_t>(k) * 4, cudaMemcpyHostToDevice, g->stream));
+  return LGBC_OK;
+}
+
 int upload_sources(lgbc_graph* g) {
   const int64_t k = static_cast<int64_t>(g->h_active.size());
-  LGBC_TRY(ensure_src(g, k));
-  if (k > 0)
-    LGBC_CUDA(cudaMemcpyAsync(g->d_src, g->h_active.data(), static_cast<size_t>(k) * sizeof(int32_t),
-                              cudaMemcpyHostToDevice, g->stream));
-  return LGBC_OK;
+  return copy_sources(g, g->h_active.data(), k);
 }
 
 int order_sources(lgbc_graph* g) {
@@ -1067,11 +1074,21 @@ int run_small_bfs(lgbc_graph* g, SmallBfs run) {
   return check_launch(g);
 }
 
-// Brandes over g->d_src[0, k) by the per-source kernel; 1 when it refuses.
-int run_small(lgbc_graph* g, int64_t k, double* bc_dev, const double* d_w) {
+// Device counters of the per-source kernels, zero when first allocated.
+int ensure_small_counters(lgbc_graph* g) {
+  SmallWorkspace& w = g->small;
+  if (w.counters) return LGBC_OK;
+  LGBC_TRY(dev_alloc(&w.counters, 4));
+  LGBC_CUDA(cudaMemsetAsync(w.counters, 0, 4 * sizeof(int), g->stream));
+  return LGBC_OK;
+}
+
+// Brandes over the k sources at src (device or pinned memory) by the
+// per-source kernel into out (likewise); waits for the stream; 1 when it refuses.
+int run_small(lgbc_graph* g, const int32_t* src, int64_t k, double* out, const double* d_w) {
   SmallWorkspace& w = g->small;
   LGBC_TRY(ensure_plan(g, &w.out, g->d_rowptr, g->d_colidx, g->d_in_rowptr));
-  if (!w.counters) LGBC_TRY(dev_alloc(&w.counters, 2));
+  LGBC_TRY(ensure_small_counters(g));
   if (!w.sum) LGBC_TRY(dev_alloc(&w.sum, 1));
   const SmallShape sh = small_shape(g->cfg, g->n, k);
   const int64_t items = std::min<int64_t>(k, sh.grid);
@@ -1092,15 +1109,17 @@ int run_small(lgbc_graph* g, int64_t k, double* bc_dev, const double* d_w) {
   run.nsrc = static_cast<int>(k);
   run.next = w.counters;
   run.refused = w.counters + 1;
-  run.src = g->d_src;
+  run.src = src;
   run.weight = d_w;
   run.part = w.part;
-  LGBC_CUDA(cudaMemsetAsync(w.counters, 0, 2 * sizeof(int), g->stream));
-  g->launches += small_brandes(g->stream, sh, run, g->n);
-  g->launches += small_sums(g->stream, w.out.graph, w.sum, 1, g->n, w.part, bc_dev);
-  LGBC_TRY(check_launch(g));
   int* refused = reinterpret_cast<int*>(g->h_ctl);
-  LGBC_CUDA(cudaMemcpyAsync(refused, w.counters + 1, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+  g->launches += small_brandes(g->stream, sh, run, g->n);
+  g->launches += small_sums(g->stream, w.out.graph, w.sum, 1, g->n, w.part, out, w.counters, refused);
+  const int rc = check_launch(g);
+  if (rc != LGBC_OK) {
+    dev_free(w.counters);  // the sums may not have zeroed them
+    return rc;
+  }
   LGBC_CUDA(cudaStreamSynchronize(g->stream));
   if (*refused) {
     w.refused = true;
@@ -1116,21 +1135,21 @@ int run_small_stress(lgbc_graph* g, unsigned long long* d_stress) {
   if (k == 0 || !small_graph(g) || g->n > g->small_stress_max_n || w.stress_refused) return 1;
   LGBC_TRY(upload_sources(g));
   LGBC_TRY(ensure_plan(g, &w.out, g->d_rowptr, g->d_colidx, g->d_in_rowptr));
-  if (!w.counters) LGBC_TRY(dev_alloc(&w.counters, 2));
+  LGBC_TRY(ensure_small_counters(g));
   const SmallShape sh = small_stress_shape(g->cfg, g->n, k);
   SmallRun run{};
   run.graphs = w.out.graph;
   run.nitems = static_cast<int>(std::min<int64_t>(k, 4 * static_cast<int64_t>(sh.grid)));
   run.nsrc = static_cast<int>(k);
-  run.next = w.counters;
-  run.refused = w.counters + 1;
+  run.next = w.counters + 2;
+  run.refused = w.counters + 3;
   run.src = g->d_src;
   run.stress = d_stress;
-  LGBC_CUDA(cudaMemsetAsync(w.counters, 0, 2 * sizeof(int), g->stream));
+  LGBC_CUDA(cudaMemsetAsync(w.counters + 2, 0, 2 * sizeof(int), g->stream));
   g->launches += small_stress(g->stream, sh, run, g->n);
   LGBC_TRY(check_launch(g));
   int* refused = reinterpret_cast<int*>(g->h_ctl);
-  LGBC_CUDA(cudaMemcpyAsync(refused, w.counters + 1, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+  LGBC_CUDA(cudaMemcpyAsync(refused, w.counters + 3, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
   LGBC_CUDA(cudaStreamSynchronize(g->stream));
   if (!*refused) {
     g->stats.batches += run.nitems;
@@ -1141,7 +1160,11 @@ int run_small_stress(lgbc_graph* g, unsigned long long* d_stress) {
   return 1;
 }
 
-int accumulate_active(lgbc_graph* g, int endpoints, double* bc_dev) {
+// Sources that the kernel fetches from pinned memory, one round trip for each
+// (beyond, a copy of all is shorter).
+constexpr int64_t kDirectSources = 256;
+
+int accumulate_active(lgbc_graph* g, int endpoints, double* bc_dev, double* host_out) {
   const int64_t k = static_cast<int64_t>(g->h_active.size());
   double* d_w = nullptr;
   std::unique_ptr<double, void (*)(double*)> guard(nullptr, [](double* q) { if (q) cudaFree(q); });
@@ -1155,19 +1178,42 @@ int accumulate_active(lgbc_graph* g, int endpoints, double* bc_dev) {
                               cudaMemcpyHostToDevice, g->stream));
     return LGBC_OK;
   };
+  auto to_host = [&]() -> int {
+    if (!host_out) return LGBC_OK;
+    LGBC_CUDA(cudaMemcpyAsync(host_out, bc_dev, static_cast<size_t>(g->n) * 8, cudaMemcpyDeviceToHost, g->stream));
+    LGBC_CUDA(cudaStreamSynchronize(g->stream));
+    return LGBC_OK;
+  };
   if (k > 0 && small_applies(g)) {
-    LGBC_TRY(upload_sources(g));
+    // A call of few sources and a short result moves both through pinned
+    // memory that the kernels read and write themselves: two launches and one
+    // wait (a 50-vertex graph 56 us with four copies and two waits, 31 us so).
+    const size_t bytes = static_cast<size_t>(g->n) * 8;
+    const bool direct = host_out && !endpoints && bytes <= kPinnedOut;
+    const int32_t* src = g->h_src;
+    if (k <= kDirectSources && !endpoints)
+      std::memcpy(g->h_src, g->h_active.data(), static_cast<size_t>(k) * 4);
+    else {
+      LGBC_TRY(upload_sources(g));
+      src = g->d_src;
+    }
     LGBC_TRY(upload_weights());
-    const int rc = run_small(g, k, bc_dev, d_w);
+    const int rc = run_small(g, src, k, direct ? reinterpret_cast<double*>(g->h_out) : bc_dev, d_w);
+    if (rc == LGBC_OK && direct) {
+      std::memcpy(host_out, g->h_out, bytes);
+      return LGBC_OK;
+    }
     if (rc == LGBC_OK) {
       if (endpoints) g->launches += add_endpoints(g->cfg, g->stream, bc_dev, g->n, g->d_src, k);
-      return check_launch(g);
+      LGBC_TRY(check_launch(g));
+      return to_host();
     }
     if (rc != 1) return rc;
   }
   LGBC_TRY(order_sources(g));
   LGBC_TRY(upload_weights());
-  return run_betweenness(g, k, endpoints, bc_dev, d_w);
+  LGBC_TRY(run_betweenness(g, k, endpoints, bc_dev, d_w));
+  return to_host();
 }
 
 void reset_stats(lgbc_graph* g) {
@@ -1183,12 +1229,12 @@ int init_handle(lgbc_graph* g, int64_t n, int directed) {
   LGBC_CUDA(cudaGetDevice(&g->device));
   g->n = n;
   g->directed = directed ? 1 : 0;
-  cudaDeviceProp prop;
-  LGBC_CUDA(cudaGetDeviceProperties(&prop, g->device));
-  g->cfg.sms = prop.multiProcessorCount;
+  int smem = 0;
+  LGBC_CUDA(cudaDeviceGetAttribute(&g->cfg.sms, cudaDevAttrMultiProcessorCount, g->device));
+  LGBC_CUDA(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, g->device));
   g->cfg.block = 256;
-  g->cfg.grid = prop.multiProcessorCount * 8;
-  g->max_smem = prop.sharedMemPerBlockOptin;
+  g->cfg.grid = g->cfg.sms * 8;
+  g->max_smem = static_cast<size_t>(smem);
   g->bfs_room = bfs_configure(g->max_smem);
   g->small_max_n = small_configure(g->max_smem);
   g->small_bfs_max_n = small_bfs_configure(g->max_smem);
@@ -1196,7 +1242,11 @@ int init_handle(lgbc_graph* g, int64_t n, int directed) {
   LGBC_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
   LGBC_CUDA(cudaEventCreate(&g->ev_start));
   LGBC_CUDA(cudaEventCreate(&g->ev_stop));
-  LGBC_CUDA(cudaMallocHost(reinterpret_cast<void**>(&g->h_ctl), sizeof(BatchCtl)));
+  unsigned char* pin = nullptr;
+  LGBC_CUDA(cudaMallocHost(reinterpret_cast<void**>(&pin), kPinnedCtl + kPinnedOut + kPinnedSources * 4));
+  g->h_ctl = reinterpret_cast<BatchCtl*>(pin);
+  g->h_out = pin + kPinnedCtl;
+  g->h_src = reinterpret_cast<int32_t*>(pin + kPinnedCtl + kPinnedOut);
   return LGBC_OK;
 }
 
@@ -1382,6 +1432,7 @@ int lgbc_graph_destroy(lgbc_graph* g) {
   dev_free(g->d_bc);
   dev_free(g->d_dist);
   dev_free(g->d_wide);
+  dev_free(g->d_stats);
   dev_free(g->d_lmdist);
   dev_free(g->d_lw_fixed);
   if (g->h_ctl) cudaFreeHost(g->h_ctl);
@@ -1441,10 +1492,15 @@ int finish_bfs(lgbc_graph* g) {
 int prepare_bfs(lgbc_graph* g, const int32_t* src, int64_t nsrc) {
   LGBC_TRY(ensure_bfs(g));
   LGBC_TRY(ensure_dist(g, g->n));
-  LGBC_TRY(ensure_src(g, nsrc));
-  if (nsrc > 0)
-    LGBC_CUDA(cudaMemcpyAsync(g->d_src, src, static_cast<size_t>(nsrc) * 4, cudaMemcpyHostToDevice,
-                              g->stream));
+  return copy_sources(g, src, nsrc);
+}
+
+int ensure_wide(lgbc_graph* g, int64_t count) {
+  if (count <= g->d_wide_cap) return LGBC_OK;
+  dev_free(g->d_wide);
+  g->d_wide_cap = 0;
+  LGBC_TRY(dev_alloc(&g->d_wide, static_cast<size_t>(count)));
+  g->d_wide_cap = count;
   return LGBC_OK;
 }
 
@@ -1456,6 +1512,7 @@ int copy_dist(lgbc_graph* g, void* out, int64_t at, int64_t count, bool wide) {
   if (wide) {
     if (count > g->d_wide_cap) {
       dev_free(g->d_wide);
+  dev_free(g->d_stats);
       g->d_wide_cap = 0;
       LGBC_TRY(dev_alloc(&g->d_wide, static_cast<size_t>(count)));
       g->d_wide_cap = count;
@@ -1472,6 +1529,45 @@ int copy_dist(lgbc_graph* g, void* out, int64_t at, int64_t count, bool wide) {
 // at 144,000 entries (104 against 107 us), 55 against 107 us at 96,000.
 constexpr int64_t kSmallSingleNnz = int64_t(1) << 17;
 
+// Whether `rows` distance rows go through the pinned result buffer.
+bool direct_dist(const lgbc_graph* g, int64_t rows, bool wide) {
+  return static_cast<size_t>(rows) * static_cast<size_t>(g->n) * (wide ? 8 : 4) <= kPinnedOut;
+}
+
+// The shared-memory searches `run` from src into `rows` rows, written in their
+// final type: short ones to the pinned result buffer (take_direct, after the
+// wait), others to the device and from there to out.
+int small_distances(lgbc_graph* g, SmallBfs run, const int32_t* src, int64_t rows, void* out, bool wide) {
+  if (run.nsrc <= kSmallFew) {
+    std::memcpy(run.few, src, static_cast<size_t>(run.nsrc) * 4);
+  } else {
+    LGBC_TRY(copy_sources(g, src, run.nsrc));
+    run.src = g->d_src;
+  }
+  const int64_t count = rows * g->n;
+  const bool direct = direct_dist(g, rows, wide);
+  if (direct) {
+    if (wide) run.dist64 = reinterpret_cast<long long*>(g->h_out);
+    else run.dist = reinterpret_cast<int32_t*>(g->h_out);
+  } else if (wide) {
+    LGBC_TRY(ensure_wide(g, count));
+    run.dist64 = reinterpret_cast<long long*>(g->d_wide);
+  } else {
+    LGBC_TRY(ensure_dist(g, count));
+    run.dist = g->d_dist;
+  }
+  LGBC_TRY(run_small_bfs(g, run));
+  if (!direct)
+    LGBC_CUDA(cudaMemcpyAsync(out, wide ? static_cast<void*>(g->d_wide) : static_cast<void*>(g->d_dist),
+                              static_cast<size_t>(count) * (wide ? 8 : 4), cudaMemcpyDeviceToHost, g->stream));
+  return LGBC_OK;
+}
+
+void take_direct(lgbc_graph* g, int64_t rows, void* out, bool wide) {
+  if (direct_dist(g, rows, wide))
+    std::memcpy(out, g->h_out, static_cast<size_t>(rows) * static_cast<size_t>(g->n) * (wide ? 8 : 4));
+}
+
 int gdistances(lgbc_graph* g, const int32_t* src, int64_t nsrc, void* dist_out, bool wide) {
   LGBC_TRY(check_graph(g));
   std::lock_guard<std::mutex> lock(g->mu);
@@ -1482,23 +1578,18 @@ int gdistances(lgbc_graph* g, const int32_t* src, int64_t nsrc, void* dist_out, 
   if (g->n == 0) return LGBC_OK;
   const bool small = nsrc > 0 && small_bfs_applies(g, 1) && g->nnz <= kSmallSingleNnz;
   if (small) {
-    LGBC_TRY(ensure_dist(g, g->n));
-    LGBC_TRY(ensure_src(g, nsrc));
-    LGBC_CUDA(cudaMemcpyAsync(g->d_src, src, static_cast<size_t>(nsrc) * 4, cudaMemcpyHostToDevice,
-                              g->stream));
     SmallBfs run{};
-    run.src = g->d_src;
     run.nsrc = static_cast<int>(nsrc);
     run.together = 1;
-    run.dist = g->d_dist;
-    LGBC_TRY(run_small_bfs(g, run));
+    LGBC_TRY(small_distances(g, run, src, 1, dist_out, wide));
+    LGBC_CUDA(cudaStreamSynchronize(g->stream));
+    take_direct(g, 1, dist_out, wide);
   } else {
     LGBC_TRY(prepare_bfs(g, src, nsrc));
     LGBC_TRY(run_bfs(g, g->dev(), nsrc));
+    LGBC_TRY(copy_dist(g, dist_out, 0, g->n, wide));
+    LGBC_TRY(finish_bfs(g));
   }
-  LGBC_TRY(copy_dist(g, dist_out, 0, g->n, wide));
-  LGBC_CUDA(cudaStreamSynchronize(g->stream));
-  if (!small) LGBC_TRY(finish_bfs(g));
   finish_stats(g);
   return LGBC_OK;
 }
@@ -1511,26 +1602,22 @@ int gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, void* dist
   if (nsrc > 0 && g->n > 0 && !dist_out) return fail(LGBC_EINVAL, "null output");
   reset_stats(g);
   if (nsrc == 0 || g->n == 0) return LGBC_OK;
-  LGBC_TRY(ensure_src(g, nsrc));
-  LGBC_CUDA(cudaMemcpyAsync(g->d_src, src, static_cast<size_t>(nsrc) * 4, cudaMemcpyHostToDevice,
-                            g->stream));
   if (small_bfs_applies(g, nsrc)) {
     // at most 2^26 distances on the device at a time
     const int64_t rows = std::min<int64_t>(nsrc, std::max<int64_t>(kWarp, (int64_t(1) << 26) / g->n / kWarp * kWarp));
-    LGBC_TRY(ensure_dist(g, rows * g->n));
     for (int64_t s0 = 0; s0 < nsrc; s0 += rows) {
       SmallBfs run{};
-      run.src = g->d_src + s0;
       run.nsrc = static_cast<int>(std::min(rows, nsrc - s0));
-      run.dist = g->d_dist;
-      LGBC_TRY(run_small_bfs(g, run));
-      LGBC_TRY(copy_dist(g, dist_out, s0 * g->n, run.nsrc * g->n, wide));
+      void* out = static_cast<char*>(dist_out) + s0 * g->n * (wide ? 8 : 4);
+      LGBC_TRY(small_distances(g, run, src + s0, run.nsrc, out, wide));
+      LGBC_CUDA(cudaStreamSynchronize(g->stream));
+      take_direct(g, run.nsrc, out, wide);
       g->stats.batches++;
     }
-    LGBC_CUDA(cudaStreamSynchronize(g->stream));
     finish_stats(g);
     return LGBC_OK;
   }
+  LGBC_TRY(copy_sources(g, src, nsrc));
   LGBC_TRY(ensure_ms(g, false));
   const int lanes = kMaxLanes;
   LGBC_TRY(ensure_dist(g, static_cast<int64_t>(lanes) * g->n));
@@ -1574,7 +1661,7 @@ int lgbc_betweenness_dev(lgbc_graph* g, const int32_t* src, int64_t nsrc, int en
   if (!bc_raw_dev && g->n > 0) return fail(LGBC_EINVAL, "null output");
   reset_stats(g);
   LGBC_TRY(filter_sources(g, src, nsrc));
-  LGBC_TRY(accumulate_active(g, endpoints, bc_raw_dev));
+  LGBC_TRY(accumulate_active(g, endpoints, bc_raw_dev, nullptr));
   finish_stats(g);
   return LGBC_OK;
 }
@@ -1589,10 +1676,7 @@ int lgbc_betweenness(lgbc_graph* g, const int32_t* src, int64_t nsrc, int endpoi
   LGBC_TRY(filter_sources(g, src, nsrc));
   if (g->n == 0) return LGBC_OK;
   if (!g->d_bc) LGBC_TRY(dev_alloc(&g->d_bc, static_cast<size_t>(g->n)));
-  LGBC_TRY(accumulate_active(g, endpoints, g->d_bc));
-  LGBC_CUDA(cudaMemcpyAsync(bc_raw_out, g->d_bc, static_cast<size_t>(g->n) * 8,
-                            cudaMemcpyDeviceToHost, g->stream));
-  LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  LGBC_TRY(accumulate_active(g, endpoints, g->d_bc, bc_raw_out));
   finish_stats(g);
   return LGBC_OK;
 }

@@ -217,7 +217,7 @@ struct SmallWorkspace {
   SmallPlan out, in;                // in: digraphs only
   SmallSum* sum = nullptr;
   int64_t items = 0;                // parts of a call that *sum was written for
-  int* counters = nullptr;          // [0] next item, [1] refused
+  int* counters = nullptr;          // [0] next item, [1] refused (zero between calls); [2, 3] for stress
   ulonglong2* part = nullptr;       // partial sums, one n-vector per item
   int64_t part_cap = 0;
   bool refused = false;             // too deep or counts too large: the batches take this graph
@@ -290,6 +290,10 @@ struct PathExport {
 }  // namespace lgbc::api
 
 namespace lgbc::api {
+constexpr size_t kPinnedCtl = 4096;      // room for the control block mirror
+constexpr size_t kPinnedOut = size_t(1) << 16;
+constexpr int64_t kPinnedSources = 4096;
+static_assert(sizeof(BatchCtl) + 16 <= kPinnedCtl, "pinned layout");
 constexpr lgbc_tuning kDefaultTuning{14.0, 24.0, 256, 128, 32, 0, 1, 1, 1 << 21, 2, 0};
 }
 
@@ -320,7 +324,13 @@ struct lgbc_graph {
   int64_t d_dist_cap = 0;
   int64_t* d_wide = nullptr;        // the same in 64 bits
   int64_t d_wide_cap = 0;
-  lgbc::BatchCtl* h_ctl = nullptr;        // pinned mirror of a control block
+  unsigned long long* d_stats = nullptr;  // distance statistics of a call's sources
+  int64_t d_stats_cap = 0;
+  // pinned host memory, one allocation: the mirror of a control block, then
+  // what small calls exchange with their kernels without a copy
+  lgbc::BatchCtl* h_ctl = nullptr;
+  unsigned char* h_out = nullptr;         // kPinnedOut bytes of results
+  int32_t* h_src = nullptr;               // kPinnedSources source ids
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   int64_t launches = 0;             // running count of kernels launched
   int64_t launches_at_start = 0;
@@ -387,8 +397,9 @@ inline int dep_kind(const lgbc_graph* g) {
 int run_betweenness(lgbc_graph* g, int64_t k_act, int endpoints, double* bc_dev,
                     const double* d_w = nullptr);
 // Brandes over g->h_active (with g->h_weights unless empty), in the order that
-// suits the path taken, into bc_dev.
-int accumulate_active(lgbc_graph* g, int endpoints, double* bc_dev);
+// suits the path taken, into bc_dev; host_out, when given, receives the result
+// (bc_dev is then scratch) and the call is blocking.
+int accumulate_active(lgbc_graph* g, int endpoints, double* bc_dev, double* host_out);
 // Validate and keep the sources of degree > 0 (betweenness.jl:58) in g->h_active.
 int filter_sources(lgbc_graph* g, const int32_t* src, int64_t nsrc);
 // Order g->h_active (and g->h_weights) for batches and copy the sources to g->d_src.
@@ -408,6 +419,8 @@ int run_small_bfs(lgbc_graph* g, SmallBfs run);
 // per-source kernel: 1 when it does not take the graph (d_stress zero again).
 int run_small_stress(lgbc_graph* g, unsigned long long* d_stress);
 int upload_sources(lgbc_graph* g);
+// A call's source list to g->d_src; the next one waits until the stream has it.
+int copy_sources(lgbc_graph* g, const int32_t* src, int64_t k);
 // Level-synchronous BFS over dg from g->d_src[0, nsrc) into g->d_dist.
 // prefilled: the caller has filled it (kUnreached, and any other value on
 // vertices the search must treat as already visited).  finish_bfs waits for

@@ -87,14 +87,15 @@ int distance_stats(lgbc_graph* g, const int32_t* src, int64_t nsrc,
   if (nsrc == 0) return LGBC_OK;
   const bool small = small_bfs_applies(g, nsrc);
   if (!small) LGBC_TRY(ensure_ms(g, false));
-  LGBC_TRY(ensure_src(g, nsrc));
-  unsigned long long* buf = nullptr;  // cnt | dsum | dmax (as int)
-  LGBC_TRY(dev_alloc(&buf, static_cast<size_t>(nsrc) * 3));
-  std::unique_ptr<unsigned long long, void (*)(unsigned long long*)> guard(
-      buf, [](unsigned long long* q) { cudaFree(q); });
-  LGBC_CUDA(cudaMemsetAsync(buf, 0, static_cast<size_t>(nsrc) * 24, g->stream));
-  LGBC_CUDA(cudaMemcpyAsync(g->d_src, src, static_cast<size_t>(nsrc) * 4, cudaMemcpyHostToDevice,
-                            g->stream));
+  if (nsrc > g->d_stats_cap) {
+    dev_free(g->d_stats);
+    g->d_stats_cap = 0;
+    LGBC_TRY(dev_alloc(&g->d_stats, static_cast<size_t>(nsrc) * 3));
+    g->d_stats_cap = nsrc;
+  }
+  unsigned long long* buf = g->d_stats;  // cnt | dsum | dmax (as int)
+  if (!small) LGBC_CUDA(cudaMemsetAsync(buf, 0, static_cast<size_t>(nsrc) * 24, g->stream));
+  LGBC_TRY(copy_sources(g, src, nsrc));
   int* dm = reinterpret_cast<int*>(buf + 2 * nsrc);
   if (small) {
     SmallBfs run{};
@@ -113,13 +114,18 @@ int distance_stats(lgbc_graph* g, const int32_t* src, int64_t nsrc,
                           &st));
     g->stats.batches++;
   }
-  LGBC_CUDA(cudaMemcpyAsync(cnt->data(), buf, static_cast<size_t>(nsrc) * 8, cudaMemcpyDeviceToHost,
-                            g->stream));
-  LGBC_CUDA(cudaMemcpyAsync(dsum->data(), buf + nsrc, static_cast<size_t>(nsrc) * 8,
-                            cudaMemcpyDeviceToHost, g->stream));
-  LGBC_CUDA(cudaMemcpyAsync(dmax->data(), dm, static_cast<size_t>(nsrc) * 4, cudaMemcpyDeviceToHost,
-                            g->stream));
+  const size_t bytes = static_cast<size_t>(nsrc) * 20;
+  std::vector<unsigned char> res;
+  unsigned char* to = g->h_out;
+  if (bytes > kPinnedOut) {
+    res.resize(bytes);
+    to = res.data();
+  }
+  LGBC_CUDA(cudaMemcpyAsync(to, buf, bytes, cudaMemcpyDeviceToHost, g->stream));
   LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  std::memcpy(cnt->data(), to, static_cast<size_t>(nsrc) * 8);
+  std::memcpy(dsum->data(), to + static_cast<size_t>(nsrc) * 8, static_cast<size_t>(nsrc) * 8);
+  std::memcpy(dmax->data(), to + static_cast<size_t>(nsrc) * 16, static_cast<size_t>(nsrc) * 4);
   return LGBC_OK;
 }
 
@@ -244,10 +250,7 @@ int lgbc_betweenness_weighted(lgbc_graph* g, const int32_t* src, const double* w
   g->h_active.swap(act);
   g->h_weights.swap(aw);
   if (!g->d_bc) LGBC_TRY(dev_alloc(&g->d_bc, static_cast<size_t>(g->n)));
-  LGBC_TRY(accumulate_active(g, 0, g->d_bc));
-  LGBC_CUDA(cudaMemcpyAsync(bc_raw_out, g->d_bc, static_cast<size_t>(g->n) * 8,
-                            cudaMemcpyDeviceToHost, g->stream));
-  LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  LGBC_TRY(accumulate_active(g, 0, g->d_bc, bc_raw_out));
   finish_stats(g);
   return LGBC_OK;
 }

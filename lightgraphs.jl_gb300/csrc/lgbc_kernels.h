@@ -231,13 +231,16 @@ struct SmallSum {
   int64_t part;            // items x n
   int64_t out;
 };
+constexpr int kSmallFew = 8;  // sources that travel with the launch
 // Distances on a small graph, 32 sources per block (or one set of sources).
 struct SmallBfs {
   const SmallGraph* graph;   // plan of the in-CSR
-  const int32_t* src;        // graph's own ids
+  const int32_t* src;        // graph's own ids, or null: the first nsrc of few
+  int32_t few[kSmallFew];
   int nsrc;
   int together;              // 1: one search from all the sources
   int32_t* dist;             // nsrc (or 1) x n, every entry written; or null
+  long long* dist64;         // the same in 64 bits, INT64_MAX where not reached; or null
   unsigned long long* cnt;   // per source: vertices reached at levels >= 1, or null
   unsigned long long* dsum;  //   and the sum
   int* dmax;                 //   and maximum of their levels
@@ -259,8 +262,11 @@ int small_stress(cudaStream_t s, const SmallShape& sh, const SmallRun& run, int6
 // ORs into bad[i] for graph i: 1 = rowptr decreases, 2 = a column outside
 // [0, n), 4 = a row longer than n.
 int small_check(cudaStream_t s, const SmallGraph* graphs, int count, int* bad);
+// counters, when given, are those of a single-graph run: its refusal goes to
+// *refused (which may be pinned host memory, as out may) and both are zeroed
+// for the next run.
 int small_sums(cudaStream_t s, const SmallGraph* graphs, const SmallSum* sums, int count, int64_t max_n,
-               const ulonglong2* part, double* out);
+               const ulonglong2* part, double* out, int* counters = nullptr, int* refused = nullptr);
 
 // ---- single multi-source BFS (gdistances): bfs.cu ------------------------
 // One level per launch (lgbc_gdistances_noalloc).

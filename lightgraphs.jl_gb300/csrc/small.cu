@@ -771,7 +771,14 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_bfs(SmallBfs run)
   const int first = blockIdx.x * kWarp;
   const int nl = run.together ? 1 : min(kWarp, run.nsrc - first);
   const uint32_t full = nl == kWarp ? ~0u : (1u << nl) - 1u;
-  int32_t* dist = run.dist ? run.dist + static_cast<int64_t>(first) * n : nullptr;
+  const int64_t row0 = static_cast<int64_t>(first) * n;
+  int32_t* dist = run.dist ? run.dist + row0 : nullptr;
+  long long* dist64 = run.dist64 ? run.dist64 + row0 : nullptr;
+  const bool put_dist = dist || dist64;
+  auto put = [&](int64_t at, int32_t d) {
+    if (dist) dist[at] = d;
+    if (dist64) dist64[at] = d == kUnreached ? INT64_MAX : static_cast<long long>(d);
+  };
   for (int i = tid; i < 3 * (n + 1); i += T) sm[i] = 0u;
   for (int c = nw / kWarp + tid; c < nc; c += T) chunk[c] = G.chunk[c];
   if (tid < kWarp) {
@@ -780,11 +787,11 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_bfs(SmallBfs run)
   }
   __syncthreads();
   for (int i = tid; i < (run.together ? run.nsrc : nl); i += T) {
-    const int own = run.src[first + i], r = G.rank[own];
+    const int own = run.src ? run.src[first + i] : run.few[first + i], r = G.rank[own];
     const uint32_t bit = run.together ? 1u : 1u << i;
     atomicOr(vis + r, bit);
     atomicOr(front + r, bit);
-    if (dist) dist[static_cast<int64_t>(run.together ? 0 : i) * n + own] = 0;
+    put(static_cast<int64_t>(run.together ? 0 : i) * n + own, 0);
   }
   __syncthreads();
   // lane b of every warp counts what the warp's vertices add to source b
@@ -794,9 +801,9 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_bfs(SmallBfs run)
   const uint2* const col = G.col;
   for (int level = 1;; ++level) {
     unsigned fresh = 0;  // vertices the level adds to source `ln`
-    auto put = [&](uint32_t bits, int v) {
+    auto put_level = [&](uint32_t bits, int v) {
       const int own = G.orig[v];
-      for (; bits; bits &= bits - 1u) dist[static_cast<int64_t>(__ffs(bits) - 1) * n + own] = level;
+      for (; bits; bits &= bits - 1u) put(static_cast<int64_t>(__ffs(bits) - 1) * n + own, level);
     };
     for (int v = wid; v < min(nw, n); v += W) {
       const uint32_t want = full & ~vis[v];
@@ -811,7 +818,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_bfs(SmallBfs run)
       if (ln == 0) {
         next[v] = got;
         if (got) vis[v] |= got;
-        if (got && dist) put(got, v);
+        if (got && put_dist) put_level(got, v);
       }
       fresh += (got >> ln) & 1u;
     }
@@ -835,7 +842,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_bfs(SmallBfs run)
           fresh += __popc(warp_transpose32(got));
           if (got) {
             vis[v] |= got;
-            if (dist) put(got, v);
+            if (put_dist) put_level(got, v);
           }
         }
       }
@@ -849,11 +856,11 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_bfs(SmallBfs run)
     front = next;
     next = t;
   }
-  if (dist)
+  if (put_dist)
     for (int v = tid; v < n; v += T) {
       const int own = G.orig[v];
       for (uint32_t miss = full & ~vis[v]; miss; miss &= miss - 1u)
-        dist[static_cast<int64_t>(__ffs(miss) - 1) * n + own] = kUnreached;
+        put(static_cast<int64_t>(__ffs(miss) - 1) * n + own, kUnreached);
     }
   if (!run.cnt) return;
   if (cnt) {
@@ -873,9 +880,14 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_bfs(SmallBfs run)
 // takes 32 vertices of graph blockIdx.y; its warps sum interleaved items,
 // then warp 0 sums those.
 __global__ void __launch_bounds__(256) k_small_sums(const SmallGraph* graphs, const SmallSum* sums,
-                                                   const ulonglong2* part, double* out) {
+                                                   const ulonglong2* part, double* out, int* counters,
+                                                   int* refused) {
   __shared__ uint64_t sm_m[8][kWarp];
   __shared__ int sm_e[8][kWarp];
+  if (counters && blockIdx.x == 0 && threadIdx.x == 0) {
+    *refused = counters[1];
+    counters[0] = counters[1] = 0;
+  }
   const SmallSum S = sums[blockIdx.y];
   const SmallGraph G = graphs[S.graph];
   if (blockIdx.x * kWarp >= G.n) return;
@@ -1023,9 +1035,9 @@ int small_check(cudaStream_t s, const SmallGraph* graphs, int count, int* bad) {
 }
 
 int small_sums(cudaStream_t s, const SmallGraph* graphs, const SmallSum* sums, int count, int64_t max_n,
-               const ulonglong2* part, double* out) {
+               const ulonglong2* part, double* out, int* counters, int* refused) {
   const dim3 grid(static_cast<unsigned>((max_n + kWarp - 1) / kWarp), static_cast<unsigned>(count));
-  k_small_sums<<<grid, 256, 0, s>>>(graphs, sums, part, out);
+  k_small_sums<<<grid, 256, 0, s>>>(graphs, sums, part, out, counters, refused);
   return 1;
 }
 

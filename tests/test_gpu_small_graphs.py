@@ -177,3 +177,18 @@ def test_repeated_entries_take_the_batches():
     a, b = (lgbc.betweenness_centrality(x, normalize=False) for x in (g, h))
     np.testing.assert_allclose(a, b, rtol=1e-12)
     np.testing.assert_allclose(lgbc.betweenness_centrality_many([g], normalize=False)[0], b, rtol=1e-12)
+
+
+@pytest.mark.parametrize("n", [8191, 8192, 8193])
+@pytest.mark.parametrize("k", [8, 9, 256, 257])
+def test_results_and_sources_at_the_sizes_of_the_pinned_areas(n, k):
+    # n 8-byte results fill the pinned 64 KB at 8192; 8 sources travel with a
+    # search's launch, 256 sources are read where the host wrote them
+    g = random_graph(n, 2 * n, n + k)
+    src = np.random.default_rng(k).choice(n, k, replace=False)
+    for _ in range(2):  # the second call finds the first one's counters and areas
+        check(g, src)
+    rp, ci, _ = csr_args(g)
+    want = oracle.gdistances(rp, ci, src.astype(np.int32)).astype(np.int64)
+    want[want == oracle.UNREACHED32] = np.iinfo(g.eltype).max
+    assert np.array_equal(lgbc.gdistances(g, src + 1), want)
