@@ -300,47 +300,51 @@ __device__ __forceinline__ df32 acc_done(df32 acc) { return fast_two_sum(acc.hi,
 
 template <class T, class A> __device__ __forceinline__ void acc_row(A& acc, T x);
 template <> __device__ __forceinline__ void acc_row(unsigned long long& acc, unsigned long long x) { acc += x; }
-// FP64 dependencies: psi rows hold binary64 bits, summed by the gather
-// accumulator (renormalised at the end of every 32-edge chunk).  In a
-// two-word batch the first NF slots (lanes 0 .. 32 NF - 1) add on the FP64
-// pipe instead (binary64 running sums, their bits kept in m) while the other
-// slots add on the integer pipes: the two units work in parallel and neither
-// carries all the adds.  NF is a property of the accumulator type, chosen per
-// kernel from its measured FP64-pipe load.
-template <int NF> struct XgAcc : xg64 {};
+// FP64 dependencies: psi rows hold 64-bit words in the format that the gather
+// accumulator adds at least cost (xg_pack; as binary64 bits, unpacked at each
+// add, R-MAT 20 from 4,096 sources took 155.3 ms instead of 150.0).  In a
+// two-word batch the first of every four slots (lanes 0 .. 31 of 128) holds
+// binary64 and adds on the FP64 pipe instead (its running sum's bits kept in
+// m) while the others add on the integer pipes: the two units work in
+// parallel and neither carries all the adds (none on the FP64 pipe: 156 ms).
+struct XgAcc : xg64 {};
+template <int W> constexpr int kFp64Slots = W / 2;
 
-template <class A, int W> struct Fp64Slots {
-  static constexpr int value = 0;
-};
-template <int NF, int W> struct Fp64Slots<XgAcc<NF>, W> {
-  static constexpr int value = W == 1 ? 0 : NF * (W / 2);  // NF of every four slots
-};
-
+// up: 1 for every other edge (xg_add_packed)
 template <class T, class A, int W>
-__device__ __forceinline__ void acc_slot(A& acc, T x, int k) {
-  if constexpr (std::is_same<A, XgAcc<1>>::value || std::is_same<A, XgAcc<2>>::value) {
-    if (k < Fp64Slots<A, W>::value)
+__device__ __forceinline__ void acc_slot(A& acc, T x, int k, uint32_t up) {
+  if constexpr (std::is_same<A, XgAcc>::value) {
+    if (k < kFp64Slots<W>)
       acc.m = static_cast<unsigned long long>(__double_as_longlong(
           __longlong_as_double(static_cast<long long>(acc.m)) +
           __longlong_as_double(static_cast<long long>(x))));
     else
-      xg_add_bits(acc, x);
+      xg_add_packed(acc, x, up);
   } else {
     acc_row<T, A>(acc, x);
   }
 }
 
-template <class A> __device__ __forceinline__ void acc_chunk_end(A&) {}
-template <int NF> __device__ __forceinline__ void acc_chunk_end(XgAcc<NF>& a) { xg_norm(a); }
-template <int W, class A, int K> __device__ __forceinline__ void chunk_end(A (&a)[K]) {
+// Brings the accumulators below 2^58, so that 32 edges more fit.  (Only when
+// the edges added since would not fit cost 1.7 % on R-MAT 20: the count takes
+// a register more than there are.)
+template <int W, class A> __device__ __forceinline__ void make_room(A (&a)[2 * W]) {
+  if constexpr (std::is_same<A, XgAcc>::value) {
 #pragma unroll
-  for (int k = 0; k < K; ++k)
-    if (k >= Fp64Slots<A, W>::value) acc_chunk_end(a[k]);
+    for (int k = kFp64Slots<W>; k < 2 * W; ++k) xg_norm(a[k]);
+  }
 }
 
-// The extended value of slot k of a normalised gather accumulator.
-template <int W, class A> __device__ __forceinline__ xf64 gather_value(const A& a, int k) {
-  return k < Fp64Slots<A, W>::value ? xf_from_bits(a.m) : xg_to_xf(a);
+// The extended value of slot k of a gather accumulator.
+template <int W> __device__ __forceinline__ xf64 gather_value(XgAcc a, int k) {
+  if (k < kFp64Slots<W>) return xf_from_bits(a.m);
+  xg_norm(a);
+  return xg_packed_sum(a);
+}
+
+// The word of an extended psi that goes to slot k of a row.
+template <int W> __device__ __forceinline__ unsigned long long psi_word(xf64 x, int k) {
+  return k < kFp64Slots<W> ? xf_to_bits(x) : xg_pack(x);
 }
 template <> __device__ __forceinline__ void acc_row(double& acc, double x) { acc += x; }
 template <> __device__ __forceinline__ void acc_row(df32& acc, float2 x) { acc_add(acc, x.x, x.y); }
@@ -354,8 +358,7 @@ template <class A> __device__ __forceinline__ A zero_acc();
 template <> __device__ __forceinline__ unsigned long long zero_acc() { return 0ull; }
 template <> __device__ __forceinline__ double zero_acc() { return 0.0; }
 template <> __device__ __forceinline__ df32 zero_acc() { return df32{0.f, 0.f}; }
-template <> __device__ __forceinline__ XgAcc<1> zero_acc() { return XgAcc<1>{}; }
-template <> __device__ __forceinline__ XgAcc<2> zero_acc() { return XgAcc<2>{}; }
+template <> __device__ __forceinline__ XgAcc zero_acc() { return XgAcc{}; }
 
 template <class A, int K> __device__ __forceinline__ void zero_accs(A (&a)[K]) {
 #pragma unroll
@@ -399,6 +402,7 @@ __device__ __forceinline__ void gather_chunk(int32_t nb, const Lanes<W>& f, cons
   if (bal == 0) return;
   const T* r0 = rows + ln;
   const int S = __popc(bal);
+  make_room<W, A>(acc);
   if (S <= dense) {
     ChunkStage<W>& st = my_stage<W>();
     if (lany(f)) {
@@ -432,7 +436,7 @@ __device__ __forceinline__ void gather_chunk(int32_t nb, const Lanes<W>& f, cons
         for (int q = 0; q < G; ++q)
 #pragma unroll
           for (int k = 0; k < 2 * W; ++k)
-            if (h[q][k] & me) acc_slot<T, A, W>(acc[k], x[q][k], k);
+            if (h[q][k] & me) acc_slot<T, A, W>(acc[k], x[q][k], k, (r + q) & 1);
       }
     } else {
       // long adds (dependency sums): the bits are packed once per edge
@@ -453,10 +457,9 @@ __device__ __forceinline__ void gather_chunk(int32_t nb, const Lanes<W>& f, cons
         for (int q = 0; q < G; ++q)
 #pragma unroll
           for (int k = 0; k < 2 * W; ++k)
-            if (my[q] & (1u << k)) acc_slot<T, A, W>(acc[k], x[q][k], k);
+            if (my[q] & (1u << k)) acc_slot<T, A, W>(acc[k], x[q][k], k, (r + q) & 1);
       }
     }
-    chunk_end<W>(acc);
     __syncwarp();
     return;
   }
@@ -487,10 +490,9 @@ __device__ __forceinline__ void gather_chunk(int32_t nb, const Lanes<W>& f, cons
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (ok[q]) acc_slot<T, A, W>(acc[k], x[q], k);
+        if (ok[q]) acc_slot<T, A, W>(acc[k], x[q], k, q & 1);
     }
   }
-  chunk_end<W>(acc);
 }
 
 // Path-count gather over in-edges [e0, e1) of one vertex: for every
@@ -514,23 +516,18 @@ __device__ __forceinline__ Lanes<W> pull_range(const int32_t* __restrict__ ci, i
     }
     return lwarp_or(found);
   }
-  // software-pipelined: the next chunk's neighbour ids and masks are loaded
-  // before the current chunk's rows are gathered
+  // software-pipelined: the next chunk's masks and the ids of the one after
+  // are loaded before the current chunk's rows are gathered
   using T = typename Sig<SK>::T;
-  int32_t v = 0;
+  int32_t v = 0, vn = 0;
   Lanes<W> f = lz<W>();
-  if (e0 + ln < e1) {
-    v = ci[e0 + ln];
-    f = land(front[v], want);
-  }
+  if (e0 + ln < e1) v = ci[e0 + ln];
+  if (e0 + ln < e1) f = land(front[v], want);
   for (int64_t e = e0; e < e1; e += kWarp) {
     const int64_t nidx = e + kWarp + ln;
-    int32_t vn = 0;
+    vn = 0;
     Lanes<W> fn = lz<W>();
-    if (nidx < e1) {
-      vn = ci[nidx];
-      fn = land(front[vn], want);
-    }
+    if (nidx < e1) { vn = ci[nidx]; fn = land(front[vn], want); }
     found = lor(found, f);
     gather_chunk<T, T, W>(v, f, reinterpret_cast<const T*>(sigma), dense, a);
     v = vn;
@@ -551,20 +548,15 @@ __device__ __forceinline__ void psi_range(const int32_t* __restrict__ ci, int64_
                                           const void* __restrict__ psi, int dense,
                                           A (&acc)[2 * W]) {
   const int ln = lane_id();
-  int32_t w = 0;
+  int32_t w = 0, wn = 0;
   Lanes<W> gm = lz<W>();
-  if (e0 + ln < e1) {
-    w = ci[e0 + ln];
-    gm = land(succ[w], F);
-  }
+  if (e0 + ln < e1) w = ci[e0 + ln];
+  if (e0 + ln < e1) gm = land(succ[w], F);
   for (int64_t e = e0; e < e1; e += kWarp) {
     const int64_t nidx = e + kWarp + ln;
-    int32_t wn = 0;
+    wn = 0;
     Lanes<W> gn = lz<W>();
-    if (nidx < e1) {
-      wn = ci[nidx];
-      gn = land(succ[wn], F);
-    }
+    if (nidx < e1) { wn = ci[nidx]; gn = land(succ[wn], F); }
     gather_chunk<T, A, W>(w, gm, reinterpret_cast<const T*>(psi), dense, acc);
     w = wn;
     gm = gn;
@@ -589,14 +581,14 @@ __device__ __forceinline__ void psi_range_f64(const int32_t* __restrict__ ci, in
   psi_range<double, double, W>(ci, e0, e1, F, succ, psi, dense, acc);
 }
 
-template <int W, int NF = 1>
+template <int W>
 __device__ __forceinline__ void psi_range_x(const int32_t* __restrict__ ci, int64_t e0, int64_t e1,
                                             const Lanes<W>& F, const Lanes<W>* __restrict__ succ,
                                             const void* __restrict__ psi, int dense,
                                             xf64 (&acc)[2 * W]) {
-  XgAcc<NF> a[2 * W];
+  XgAcc a[2 * W];
   zero_accs(a);
-  psi_range<unsigned long long, XgAcc<NF>, W>(ci, e0, e1, F, succ, psi, dense, a);
+  psi_range<unsigned long long, XgAcc, W>(ci, e0, e1, F, succ, psi, dense, a);
 #pragma unroll
   for (int k = 0; k < 2 * W; ++k) acc[k] = gather_value<W>(a[k], k);
 }
@@ -669,6 +661,7 @@ __device__ __forceinline__ void seg_gather(bool valid, int64_t e0, int deg, cons
     }
     __syncwarp();
     const int S = __popc(bal);
+    make_room<W, A>(acc);
     for (int r = 0; r < S; r += G) {
       T xr[G][2 * W];
       unsigned my[G];
@@ -702,10 +695,9 @@ __device__ __forceinline__ void seg_gather(bool valid, int64_t e0, int deg, cons
         nm = lor(nm, fq[q]);
 #pragma unroll
         for (int k = 0; k < 2 * W; ++k)
-          if (my[q] & (1u << k)) acc_slot<T, A, W>(acc[k], xr[q][k], k);
+          if (my[q] & (1u << k)) acc_slot<T, A, W>(acc[k], xr[q][k], k, (r + q) & 1);
       }
     }
-    chunk_end<W>(acc);
     __syncwarp();
   }
   if (cur >= 0) {
@@ -779,12 +771,14 @@ __device__ __forceinline__ double finish_f64(void* psi, const void* sigma, int32
 
 // FP64 dependencies from an extended psi sum (kSigmaU64F64): with acc =
 // sum of the successors' psi = delta / sigma, psi = 1 / sigma + acc (the
-// reference's coeff, (1 + delta) / sigma) is stored as binary64 and
+// reference's coeff, (1 + delta) / sigma) is stored as a row word and
 // delta = sigma * acc is returned; the path count stays an exact integer.
+template <int W>
 __device__ __forceinline__ xf64 finish_lane_x(const unsigned long long* srow,
-                                              unsigned long long* prow, int l, xf64 acc) {
+                                              unsigned long long* prow, int k, xf64 acc) {
+  const int l = 32 * k + lane_id();
   const unsigned long long sv = srow[l];
-  prow[l] = xf_to_bits(xf_add(acc, xf_recip_u64(sv)));
+  prow[l] = psi_word<W>(xf_add(acc, xf_recip_u64(sv)), k);
   return xf_mul_u64(acc, sv);
 }
 
@@ -802,7 +796,7 @@ __device__ __forceinline__ xf64 finish_x(void* psi, const void* sigma, int32_t v
 #pragma unroll
   for (int k = 0; k < 2 * W; ++k)
     if (mine & (1u << k)) {
-      xf64 d = finish_lane_x(srow, prow, 32 * k + ln, acc[k]);
+      xf64 d = finish_lane_x<W>(srow, prow, k, acc[k]);
       if (lw) d = xf_mul(d, xf_from_bits(__double_as_longlong(lw[32 * k + ln])));
       contrib = xf_add(contrib, d);
     }
@@ -1678,17 +1672,13 @@ __global__ void __launch_bounds__(256, W == 1 ? 3 : 2) k_ms_delta_seg(DevGraph g
                                           if (ln == 0 && contrib.hi != 0.f) bc[vj] += df_to_double(contrib);
                                         });
     } else if (SK == kSigmaU64F64) {
-      seg_gather<unsigned long long, XgAcc<1>, true, W>(
+      seg_gather<unsigned long long, XgAcc, true, W>(
           mine, e0, dg, F, g.colidx, succ, reinterpret_cast<const unsigned long long*>(b.psi),
-          [&](int j, const Lanes<W>&, const XgAcc<1> (&a)[2 * W]) {
+          [&](int j, const Lanes<W>&, const XgAcc (&a)[2 * W]) {
             const int32_t vj = __shfl_sync(kFull, v, j);
             xf64 d[2 * W];
 #pragma unroll
-            for (int k = 0; k < 2 * W; ++k) {
-              XgAcc<1> t = a[k];  // flushed mid-chunk: renormalise first
-              if (k >= Fp64Slots<XgAcc<1>, W>::value) xg_norm(t);
-              d[k] = gather_value<W>(t, k);
-            }
+            for (int k = 0; k < 2 * W; ++k) d[k] = gather_value<W>(a[k], k);
             const xf64 contrib =
                 warp_sum_x(finish_x<W>(b.psi, b.sigma, vj, my_bits(lshfl(F, j)), d, nullptr));
             if (ln == 0) bc_add_x(bc, vj, contrib);

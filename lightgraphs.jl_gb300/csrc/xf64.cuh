@@ -214,8 +214,8 @@ __host__ __device__ __forceinline__ xf64 xf_recip_u64(uint64_t s) {
 //
 //   xg{m, e}  =  m * 2^(e - 1080),   m in [2^57, 2^58) after xg_norm (or 0, e = 0),
 //
-// terms enter as (53-bit significand << 5) in [2^57, 2^58) and after k adds
-// m < (k + 1) 2^58 < 2^64 for k <= 32.  Each add truncates less than one unit
+// terms enter in [2^57, 2^58) and after k adds m < (k + 1) 2^58 < 2^64 for
+// k <= 32.  Each add truncates less than one unit
 // of the 58-bit scale (relative error < 2^-57, against binary64's 2^-53).
 struct xg64 {
   uint64_t m;
@@ -244,6 +244,36 @@ __host__ __device__ __forceinline__ void xg_norm(xg64& a) {
   const int sh = top > 57 ? top - 57 : 0;
   a.m >>= sh;
   a.e += sh;
+}
+
+// ---- packed terms ------------------------------------------------------------
+// The terms of the gathers as 64-bit words that enter the accumulator without
+// unpacking: w 2^(b - 186), where b = the low byte of w and the whole word is
+// the significand (top bit set, or just below it).  The word nearest to a value is
+// within 2^-56 of it, against binary64's 2^-53.  psi = (1 + delta) / sigma lies
+// in [2^-64, 2^32), so b stays in [59, 156].  An accumulator of packed terms
+// holds exponents less kXgPackBias.
+constexpr int kXgPackBias = 900;
+
+__host__ __device__ __forceinline__ uint64_t xg_pack(xf64 x) {
+  const uint32_t b = static_cast<uint32_t>(x.e - kXgPackBias);
+  const uint64_t s = (x.m << 1) - b;
+  const uint64_t r = s + 128u;
+  return ((r < s ? s : r) & ~255ull) | b;  // no carry out of the top: truncated there
+}
+
+// a += the packed term w.  The shifts drop half a unit on average: with `up`
+// (every other term) a whole one is added, so that long sums are not biased.
+__host__ __device__ __forceinline__ void xg_add_packed(xg64& a, uint64_t w, uint32_t up) {
+  const int ex = static_cast<int>(static_cast<uint32_t>(w) & 255u);
+  const int E = a.e > ex ? a.e : ex;
+  a.m = xg_shr(a.m, static_cast<uint32_t>(E - a.e)) + xg_shr(w, static_cast<uint32_t>(E + 6 - ex)) + up;
+  a.e = E;
+}
+
+// The extended value of a normalised accumulator of packed terms.
+__host__ __device__ __forceinline__ xf64 xg_packed_sum(xg64 a) {
+  return xf64{a.m << 5, a.m ? a.e + kXgPackBias : 0};
 }
 
 // The extended value of a normalised gather accumulator.
