@@ -245,12 +245,12 @@ int build_hubs(lgbc_graph* g, const int64_t* rowptr, const int32_t* colidx, cons
     g->hubs.n_in = g->hubs.n_out;
   }
   // accumulators for the widest batch: 64 * kMaxWords lanes, kMaxWords mask words
-  LGBC_TRY(dev_alloc(&g->hubs.acc, static_cast<size_t>(nslots) * kWideLanes));
-  LGBC_TRY(dev_alloc(&g->hubs.mask, static_cast<size_t>(nslots) * kMaxWords));
-  LGBC_TRY(dev_alloc(&g->hubs.cnt, static_cast<size_t>(nslots)));
-  LGBC_CUDA(cudaMemset(g->hubs.acc, 0, static_cast<size_t>(nslots) * kWideLanes * 8));
-  LGBC_CUDA(cudaMemset(g->hubs.mask, 0, static_cast<size_t>(nslots) * kMaxWords * 8));
-  LGBC_CUDA(cudaMemset(g->hubs.cnt, 0, static_cast<size_t>(nslots) * 4));
+  // and a counter, in one allocation
+  const size_t words = static_cast<size_t>(nslots) * (kWideLanes + kMaxWords + 1);
+  LGBC_TRY(dev_alloc(&g->hubs.acc, words));
+  g->hubs.mask = g->hubs.acc + nslots * kWideLanes;
+  g->hubs.cnt = reinterpret_cast<unsigned int*>(g->hubs.mask + nslots * kMaxWords);
+  LGBC_CUDA(cudaMemset(g->hubs.acc, 0, words * 8));
   return LGBC_OK;
 }
 

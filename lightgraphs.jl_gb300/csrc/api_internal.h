@@ -119,7 +119,7 @@ struct HubTable {
   int64_t n_out = 0;
   HubItem* in_items = nullptr;   // == out_items for undirected graphs
   int64_t n_in = 0;
-  unsigned long long* acc = nullptr;
+  unsigned long long* acc = nullptr;  // one allocation with mask and cnt
   unsigned long long* mask = nullptr;
   unsigned int* cnt = nullptr;
   int64_t nslots = 0;
@@ -130,8 +130,8 @@ struct HubTable {
     dev_free(out_items);
     in_items = nullptr;
     dev_free(acc);
-    dev_free(mask);
-    dev_free(cnt);
+    mask = nullptr;
+    cnt = nullptr;
     n_out = n_in = nslots = 0;
     built_for = -1;
     built_order = -1;

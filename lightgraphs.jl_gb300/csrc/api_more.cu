@@ -311,147 +311,64 @@ extern "C" int lgbc_has_path(lgbc_graph* g, int32_t u, int32_t v, const int32_t*
 // ---------------------------------------------------------------------------
 namespace lgbc::api {
 
-// Sort `count` keys (owned: keys / alt swap), keep the first copy of each, and
-// emit the CSR rows into colidx (allocated here) and rowptr.  With `sorted_out`
-// the kept keys are also returned compacted.
-int build_rows(lgbc_graph* g, unsigned long long*& keys, unsigned long long*& alt, int64_t count,
-               int B, int32_t** colidx, int64_t* rowptr_dev, int64_t* nnz,
-               unsigned long long** sorted_out) {
-  cudaStream_t s = g->stream;
-  const int64_t cells = radix_scratch_words(count);
-  const int64_t nsums = std::max<int64_t>(std::max(scan_tiles(cells), scan_tiles(count)),
-                                          scan_tiles(g->n)) + 1;
-  uint32_t* hist = nullptr;
-  int64_t* off = nullptr;
-  int64_t* sums = nullptr;
-  uint8_t* keep = nullptr;
-  int64_t* pos = nullptr;
-  unsigned int* deg = nullptr;
-  int64_t* d_nkept = nullptr;
-  auto cleanup = [&]() {
-    cudaFree(hist); cudaFree(off); cudaFree(sums); cudaFree(keep); cudaFree(pos); cudaFree(deg);
-    cudaFree(d_nkept);
-  };
-  int rc = LGBC_OK;
-  if ((rc = dev_alloc(&hist, static_cast<size_t>(cells))) || (rc = dev_alloc(&off, static_cast<size_t>(cells))) ||
-      (rc = dev_alloc(&sums, static_cast<size_t>(nsums))) || (rc = dev_alloc(&keep, static_cast<size_t>(count))) ||
-      (rc = dev_alloc(&pos, static_cast<size_t>(count))) || (rc = dev_alloc(&deg, static_cast<size_t>(g->n))) ||
-      (rc = dev_alloc(&d_nkept, 1))) {
-    cleanup();
-    return rc;
-  }
-  g->launches += radix_sort(s, keys, alt, count, 2 * B, hist, off, sums);
-  g->launches += ingest_unique(g->cfg, s, keys, count, keep, pos, sums, d_nkept);
-  int64_t nk = 0;
-  cudaError_t e = cudaMemcpyAsync(&nk, d_nkept, 8, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) {
-    cleanup();
-    return cuda_fail(e, "ingest: unique arcs");
-  }
-  if (count == 0) nk = 0;
-  *nnz = nk;
-  if ((rc = dev_alloc(colidx, static_cast<size_t>(std::max<int64_t>(nk, 1))))) {
-    cleanup();
-    return rc;
-  }
-  cudaMemsetAsync(deg, 0, static_cast<size_t>(g->n) * 4, s);
-  g->launches += ingest_emit(g->cfg, s, keys, count, keep, pos, B, *colidx, deg);
-  g->launches += ingest_rowptr(s, deg, g->n, sums, rowptr_dev);
-  if (g->n == 0) cudaMemsetAsync(rowptr_dev, 0, 8, s);
-  if (sorted_out) {
-    *sorted_out = alt;  // reuse the spare buffer for the compacted keys
-    alt = nullptr;
-    g->launches += ingest_compact(g->cfg, s, keys, count, keep, pos, *sorted_out);
-  }
-  e = cudaStreamSynchronize(s);
-  cleanup();
-  if (e != cudaSuccess) return cuda_fail(e, "ingest: rows");
-  return check_launch(g);
-}
-
 int create_from_edges_impl(lgbc_graph* g, int64_t n, int64_t m, const int32_t* src,
                            const int32_t* dst, int directed) {
   LGBC_TRY(init_handle(g, n, directed));
   cudaStream_t s = g->stream;
   const int B = ingest_bits(n);
   const int64_t count = directed ? m : 2 * m;
-  int32_t* d_edges = nullptr;
-  unsigned long long* keys = nullptr;
-  unsigned long long* alt = nullptr;
-  int* d_bad = nullptr;
-  auto cleanup = [&]() { cudaFree(d_edges); cudaFree(keys); cudaFree(alt); cudaFree(d_bad); };
-  int rc = LGBC_OK;
-  if ((rc = dev_alloc(&d_edges, static_cast<size_t>(2 * std::max<int64_t>(m, 1)))) ||
-      (rc = dev_alloc(&keys, static_cast<size_t>(std::max<int64_t>(count, 1)))) ||
-      (rc = dev_alloc(&alt, static_cast<size_t>(std::max<int64_t>(count, 1)))) ||
-      (rc = dev_alloc(&d_bad, 1))) {
-    cleanup();
-    return rc;
-  }
-  cudaMemsetAsync(d_bad, 0, 4, s);
+  // One allocation for what the build needs for a while (17 of them, with
+  // their frees, were a third of the call): {bad, kept} | scratch | keys |
+  // keys of the next pass, which hold the endpoints until there are keys.
+  const int64_t words = 2 + ingest_scratch_words(count) + 2 * std::max<int64_t>(count, m);
+  int64_t* arena = nullptr;
+  LGBC_TRY(dev_alloc(&arena, static_cast<size_t>(words)));
+  std::unique_ptr<int64_t, cudaError_t (*)(void*)> guard(arena, cudaFree);
+  int64_t* status = arena;
+  int64_t* scratch = arena + 2;
+  unsigned long long* keys = reinterpret_cast<unsigned long long*>(scratch + ingest_scratch_words(count));
+  unsigned long long* alt = keys + std::max<int64_t>(count, m);
+  int32_t* d_edges = reinterpret_cast<int32_t*>(alt);
+  LGBC_CUDA(cudaMemsetAsync(status, 0, 16, s));
   if (m > 0) {
     LGBC_CUDA(cudaMemcpyAsync(d_edges, src, static_cast<size_t>(m) * 4, cudaMemcpyHostToDevice, s));
     LGBC_CUDA(cudaMemcpyAsync(d_edges + m, dst, static_cast<size_t>(m) * 4, cudaMemcpyHostToDevice, s));
   }
-  g->launches += ingest_make_keys(g->cfg, s, d_edges, d_edges + m, m, n, B, directed, keys, d_bad);
-  int bad = 0;
-  LGBC_CUDA(cudaMemcpyAsync(&bad, d_bad, 4, cudaMemcpyDeviceToHost, s));
+  g->launches += ingest_make_keys(g->cfg, s, d_edges, d_edges + m, m, n, B, directed, keys,
+                                  reinterpret_cast<int*>(status));
+  g->launches += radix_sort(s, keys, alt, count, 0, 2 * B, scratch);
+  g->launches += ingest_count(s, keys, count, scratch, status + 1);
+  LGBC_TRY(check_launch(g));
+  int64_t* found = reinterpret_cast<int64_t*>(g->h_ctl);
+  LGBC_CUDA(cudaMemcpyAsync(found, status, 16, cudaMemcpyDeviceToHost, s));
+  // what does not depend on the arcs, while they are sorted
+  LGBC_TRY(dev_alloc(&g->d_rowptr, static_cast<size_t>(n + 1)));
+  if (directed) LGBC_TRY(dev_alloc(&g->d_in_rowptr, static_cast<size_t>(n + 1)));
+  std::vector<int64_t> rp(static_cast<size_t>(n + 1)), irp(directed ? static_cast<size_t>(n + 1) : 0);
   LGBC_CUDA(cudaStreamSynchronize(s));
-  if (bad) {
-    cleanup();
-    return fail(LGBC_EINVAL, "edge endpoint outside [0, n)");
-  }
-  cudaFree(d_edges);
-  d_edges = nullptr;
-  if ((rc = dev_alloc(&g->d_rowptr, static_cast<size_t>(n + 1)))) {
-    cleanup();
-    return rc;
-  }
-  unsigned long long* sorted = nullptr;
-  int64_t nnz = 0;
-  rc = build_rows(g, keys, alt, count, B, &g->d_colidx, g->d_rowptr, &nnz, directed ? &sorted : nullptr);
-  if (rc != LGBC_OK) {
-    cudaFree(sorted);
-    cleanup();
-    return rc;
-  }
+  if (found[0]) return fail(LGBC_EINVAL, "edge endpoint outside [0, n)");
+  const int64_t nnz = found[1];
   g->nnz = nnz;
-  std::vector<int64_t> rp(static_cast<size_t>(n + 1)), irp;
+  const size_t cols = static_cast<size_t>(std::max<int64_t>(nnz, 1));
+  LGBC_TRY(dev_alloc(&g->d_colidx, cols));
+  g->launches += ingest_emit(s, keys, count, scratch, B, g->d_colidx, alt);
+  g->launches += ingest_rows(g->cfg, s, alt, nnz, n, B, g->d_rowptr);
+  LGBC_CUDA(cudaMemcpyAsync(rp.data(), g->d_rowptr, rp.size() * 8, cudaMemcpyDeviceToHost, s));
   if (directed) {
-    // in-CSR: the kept arcs with their ends swapped, sorted again
-    cudaFree(keys);
-    keys = nullptr;
-    unsigned long long* ikeys = nullptr;
-    if ((rc = dev_alloc(&ikeys, static_cast<size_t>(std::max<int64_t>(nnz, 1))))) {
-      cudaFree(sorted);
-      cleanup();
-      return rc;
-    }
-    g->launches += ingest_swap_keys(g->cfg, s, sorted, nnz, B, ikeys);
-    unsigned long long* ialt = sorted;
-    if ((rc = dev_alloc(&g->d_in_rowptr, static_cast<size_t>(n + 1)))) {
-      cudaFree(ikeys);
-      cudaFree(ialt);
-      cleanup();
-      return rc;
-    }
-    int64_t innz = 0;
-    rc = build_rows(g, ikeys, ialt, nnz, B, &g->d_in_colidx, g->d_in_rowptr, &innz, nullptr);
-    cudaFree(ikeys);
-    cudaFree(ialt);
-    if (rc != LGBC_OK) {
-      cleanup();
-      return rc;
-    }
-    irp.resize(static_cast<size_t>(n + 1));
-    LGBC_CUDA(cudaMemcpy(irp.data(), g->d_in_rowptr, irp.size() * 8, cudaMemcpyDeviceToHost));
+    // in-CSR: the kept arcs, in order of their tails, with their ends swapped
+    // and sorted by the heads alone
+    LGBC_TRY(dev_alloc(&g->d_in_colidx, cols));
+    g->launches += ingest_swap_keys(g->cfg, s, alt, nnz, B, keys);
+    g->launches += radix_sort(s, keys, alt, nnz, B, 2 * B, scratch);
+    g->launches += ingest_columns(g->cfg, s, keys, nnz, B, g->d_in_colidx);
+    g->launches += ingest_rows(g->cfg, s, keys, nnz, n, B, g->d_in_rowptr);
+    LGBC_CUDA(cudaMemcpyAsync(irp.data(), g->d_in_rowptr, irp.size() * 8, cudaMemcpyDeviceToHost, s));
   } else {
     g->d_in_rowptr = g->d_rowptr;
     g->d_in_colidx = g->d_colidx;
   }
-  cleanup();
-  LGBC_CUDA(cudaMemcpy(rp.data(), g->d_rowptr, rp.size() * 8, cudaMemcpyDeviceToHost));
+  LGBC_TRY(check_launch(g));
+  LGBC_CUDA(cudaStreamSynchronize(s));
   return finish_handle(g, rp.data(), directed ? irp.data() : rp.data());
 }
 

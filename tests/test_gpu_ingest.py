@@ -61,3 +61,15 @@ def test_ingest_large_power_of_two():
     assert len(ci) == len(keys)
     assert np.array_equal(ci, (keys % n).astype(np.int32))
     assert np.array_equal(np.diff(rp), np.bincount(keys // n, minlength=n))
+
+
+@pytest.mark.parametrize("directed", [False, True])
+@pytest.mark.parametrize("n,m", [(2, 1), (255, 127), (256, 128), (257, 129), (1000, 8191), (1000, 8193),
+                                 (40, 16384), (70000, 16385), (66000, 131072), (300, 262145), (200000, 300001)])
+def test_ingest_at_tile_edges(n, m, directed):
+    # sort tiles of 256 to 4,096 keys and their count at 64, the one-block
+    # histogram scan at 64 tiles, digits at 8, 9 and 17 bits, few distinct arcs among many
+    rng = np.random.default_rng(m)
+    src, dst = rng.integers(0, n, (2, m))
+    src[: m // 3] = 0
+    _check(n, src, dst, directed)
