@@ -156,12 +156,13 @@ void make_items(const int64_t* rowptr, const int32_t* colidx, int64_t n, int H, 
         it.v = static_cast<int32_t>(v);
         it.slot = slot_of[static_cast<size_t>(v)];
         it.nitems = nit;
-        it.pad = 0;
-        out.push_back(it);
-        if (!ordered) continue;
         const int64_t mid2 = (lo - e0) + it.hi - e0;  // twice the middle's offset in the row
-        key.push_back(order == 1 ? static_cast<int64_t>(colidx[lo + (it.hi - lo) / 2]) * kBuckets / n
-                                 : mid2 * kBuckets / (2 * (e1 - e0)));
+        const int64_t bucket = !ordered     ? 0
+                               : order == 1 ? static_cast<int64_t>(colidx[lo + (it.hi - lo) / 2]) * kBuckets / n
+                                            : mid2 * kBuckets / (2 * (e1 - e0));
+        it.bucket = static_cast<int32_t>(bucket);
+        out.push_back(it);
+        if (ordered) key.push_back(bucket);
       }
     }
   });
@@ -186,6 +187,18 @@ int upload_items(const std::vector<HubItem>& items, HubItem** out) {
   if (items.empty()) return LGBC_OK;
   LGBC_TRY(dev_alloc(out, items.size()));
   LGBC_CUDA(cudaMemcpy(*out, items.data(), items.size() * sizeof(HubItem), cudaMemcpyHostToDevice));
+  return LGBC_OK;
+}
+
+// Accumulators of every hub for the widest batch: 64 * kMaxWords lanes,
+// kMaxWords mask words and a counter, in one allocation.
+int alloc_hub_sums(lgbc_graph* g) {
+  HubTable& h = g->hubs;
+  const size_t words = static_cast<size_t>(h.nslots) * (kWideLanes + kMaxWords + 1);
+  LGBC_TRY(dev_alloc(&h.acc, words));
+  h.mask = h.acc + h.nslots * kWideLanes;
+  h.cnt = reinterpret_cast<unsigned int*>(h.mask + h.nslots * kMaxWords);
+  LGBC_CUDA(cudaMemsetAsync(h.acc, 0, words * 8, g->stream));
   return LGBC_OK;
 }
 
@@ -244,14 +257,7 @@ int build_hubs(lgbc_graph* g, const int64_t* rowptr, const int32_t* colidx, cons
     g->hubs.in_items = g->hubs.out_items;
     g->hubs.n_in = g->hubs.n_out;
   }
-  // accumulators for the widest batch: 64 * kMaxWords lanes, kMaxWords mask words
-  // and a counter, in one allocation
-  const size_t words = static_cast<size_t>(nslots) * (kWideLanes + kMaxWords + 1);
-  LGBC_TRY(dev_alloc(&g->hubs.acc, words));
-  g->hubs.mask = g->hubs.acc + nslots * kWideLanes;
-  g->hubs.cnt = reinterpret_cast<unsigned int*>(g->hubs.mask + nslots * kMaxWords);
-  LGBC_CUDA(cudaMemset(g->hubs.acc, 0, words * 8));
-  return LGBC_OK;
+  return alloc_hub_sums(g);
 }
 
 // Rebuild the hub table after hub_degree or hub_order changed (rowptr copied back).
@@ -805,24 +811,48 @@ int create_replicated(lgbc_graph* g, int64_t copies, lgbc_graph** out) {
     LGBC_TRY(dev_alloc(&st->d_colidx, static_cast<size_t>(std::max<int64_t>(NNZ, 1))));
     st->launches += replicate_csr(st->cfg, st->stream, g->d_rowptr, g->d_colidx, n, nnz, copies,
                                   st->d_rowptr, st->d_colidx);
-    std::vector<int64_t> rp(static_cast<size_t>(N + 1)), irp;
     if (g->directed) {
       LGBC_TRY(dev_alloc(&st->d_in_rowptr, static_cast<size_t>(N + 1)));
       LGBC_TRY(dev_alloc(&st->d_in_colidx, static_cast<size_t>(std::max<int64_t>(NNZ, 1))));
       st->launches += replicate_csr(st->cfg, st->stream, g->d_in_rowptr, g->d_in_colidx, n, nnz,
                                     copies, st->d_in_rowptr, st->d_in_colidx);
-      irp.resize(rp.size());
-      LGBC_CUDA(cudaMemcpyAsync(irp.data(), st->d_in_rowptr, irp.size() * 8, cudaMemcpyDeviceToHost,
-                                st->stream));
     } else {
       st->d_in_rowptr = st->d_rowptr;
       st->d_in_colidx = st->d_colidx;
     }
-    LGBC_CUDA(cudaMemcpyAsync(rp.data(), st->d_rowptr, rp.size() * 8, cudaMemcpyDeviceToHost,
-                              st->stream));
+    // Degrees and hubs are g's (sources are filtered and ordered there, so
+    // the union keeps neither a degree filter nor landmarks).  Read back and
+    // built on the host, as for a graph that comes from there, they were 7 ms
+    // of the first call for 10 copies of 200,000 vertices.
+    st->max_in = g->max_in;
+    st->max_out = g->max_out;
+    st->sigma_limit = g->sigma_limit;
+    LGBC_TRY(ensure_hubs(g));
+    st->tune = g->tune;
+    const HubTable& from = g->hubs;
+    HubTable& to = st->hubs;
+    to.built_for = from.built_for;
+    to.built_order = from.built_order;
+    to.nslots = copies * from.nslots;
+    if (to.nslots > 0) {
+      const bool buckets = from.built_order == 2;
+      auto items = [&](const HubItem* in, int64_t count, HubItem** out) -> int {
+        if (count == 0) return LGBC_OK;
+        LGBC_TRY(dev_alloc(out, static_cast<size_t>(copies * count)));
+        st->launches += replicate_items(st->cfg, st->stream, in, count, copies, n, nnz, from.nslots, buckets, *out);
+        return LGBC_OK;
+      };
+      to.n_out = copies * from.n_out;
+      LGBC_TRY(items(from.out_items, from.n_out, &to.out_items));
+      to.n_in = copies * from.n_in;
+      if (g->directed)
+        LGBC_TRY(items(from.in_items, from.n_in, &to.in_items));
+      else
+        to.in_items = to.out_items;
+      LGBC_TRY(alloc_hub_sums(st));
+    }
     LGBC_CUDA(cudaStreamSynchronize(st->stream));
-    LGBC_TRY(check_launch(st));
-    return finish_handle(st, rp.data(), g->directed ? irp.data() : rp.data());
+    return check_launch(st);
   };
   const int rc = build();
   if (rc != LGBC_OK) {

@@ -85,7 +85,7 @@ struct HubItem {
   int32_t v;           // the hub vertex
   int32_t slot;        // its accumulator slot
   int32_t nitems;      // items of this hub in this list
-  int32_t pad;
+  int32_t bucket;      // order key (ascending in the list), or 0
 };
 struct HubData {
   const HubItem* out_items;      // items over out-edges (top-down discovery, dependencies)
@@ -336,6 +336,11 @@ int fill_i32(const LaunchCfg& c, cudaStream_t s, int32_t* p, int64_t count, int3
 // r = vertices [r n, (r + 1) n)): rp1[copies n + 1], c1[copies nnz]; n > 0.
 int replicate_csr(const LaunchCfg& c, cudaStream_t s, const int64_t* rp0, const int32_t* c0,
                   int64_t n, int64_t nnz, int64_t copies, int64_t* rp1, int32_t* c1);
+// The hub items of such a union from those of one graph with n vertices, nnz
+// entries and nslots hubs: bucket by bucket and copy by copy in each, as the
+// union's own list is ordered, or copy by copy.
+int replicate_items(const LaunchCfg& c, cudaStream_t s, const HubItem* in, int64_t count, int64_t copies, int64_t n,
+                    int64_t nnz, int64_t nslots, bool buckets, HubItem* out);
 // out[v] = sum over r < copies of stacked[r * n + v] (a fixed order).
 int sum_copies(const LaunchCfg& c, cudaStream_t s, const double* stacked, int64_t n, int64_t copies,
                double* out);

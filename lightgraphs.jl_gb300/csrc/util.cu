@@ -137,7 +137,42 @@ __global__ void k_replicate_cols(const int32_t* c0, int64_t nnz, int64_t n, int6
     c1[i] = static_cast<int32_t>(r * n + c0[i - r * nnz]);
   }
 }
+
+__global__ void k_replicate_items(const HubItem* in, int64_t count, int64_t copies, int64_t n, int64_t nnz,
+                                  int64_t nslots, bool buckets, HubItem* out) {
+  const int64_t total = copies * count;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t r = i / count, j = i - r * count;
+    HubItem it = in[j];
+    int64_t at = i;
+    if (buckets) {  // [b0, b1): the items of j's bucket
+      auto first_from = [&](int32_t key) {
+        int64_t lo = 0, hi = count;
+        while (lo < hi) {
+          const int64_t mid = (lo + hi) >> 1;
+          if (in[mid].bucket < key) lo = mid + 1; else hi = mid;
+        }
+        return lo;
+      };
+      const int64_t b0 = first_from(it.bucket), b1 = first_from(it.bucket + 1);
+      at = copies * b0 + r * (b1 - b0) + (j - b0);
+    }
+    it.lo += r * nnz;
+    it.hi += r * nnz;
+    it.v += static_cast<int32_t>(r * n);
+    it.slot += static_cast<int32_t>(r * nslots);
+    out[at] = it;
+  }
+}
 }  // namespace
+
+int replicate_items(const LaunchCfg& c, cudaStream_t s, const HubItem* in, int64_t count, int64_t copies, int64_t n,
+                    int64_t nnz, int64_t nslots, bool buckets, HubItem* out) {
+  if (count <= 0 || copies <= 0) return 0;
+  k_replicate_items<<<c.grid, c.block, 0, s>>>(in, count, copies, n, nnz, nslots, buckets, out);
+  return 1;
+}
 
 int replicate_csr(const LaunchCfg& c, cudaStream_t s, const int64_t* rp0, const int32_t* c0,
                   int64_t n, int64_t nnz, int64_t copies, int64_t* rp1, int32_t* c1) {

@@ -64,3 +64,17 @@ def test_hub_order_validation():
         h.set_tuning(hub_order=3)
     h.set_tuning(hub_order=0)
     assert h.tuning().hub_order == 0
+
+
+@pytest.mark.parametrize("hub_order", [0, 1, 2])
+@pytest.mark.parametrize("hub_degree", [4, 16, 1 << 20])
+@pytest.mark.parametrize("name", ["rmat10", "rmat10_directed"])
+def test_orders_in_stacked_unions(name, hub_degree, hub_order):
+    # the union's items come from the graph's own, with several in a bucket,
+    # some or no hubs; built again when the hub cut changes
+    g = GRAPHS[name]()
+    src = np.random.default_rng(hub_order).choice(g.nv(), 300, replace=False).astype(np.int32)
+    want = oracle_bc(g, src, normalize=False)
+    for cut in (hub_degree, hub_degree + 3):
+        g.device_handle().set_tuning(lanes=64, hub_degree=cut, hub_order=hub_order, stack_vertices=5 * g.nv())
+        assert_bc_close(lgbc.betweenness_centrality(g, list(src + 1), normalize=False), want)
