@@ -1217,7 +1217,7 @@ int accumulate_active(lgbc_graph* g, int endpoints, double* bc_dev, double* host
   if (k > 0 && small_applies(g)) {
     // A call of few sources and a short result moves both through pinned
     // memory that the kernels read and write themselves: two launches and one
-    // wait (a 50-vertex graph 56 us with four copies and two waits, 31 us so).
+    // wait (a 50-vertex graph 56 us with four copies and two waits, 35 us so).
     const size_t bytes = static_cast<size_t>(g->n) * 8;
     const bool direct = host_out && !endpoints && bytes <= kPinnedOut;
     const int32_t* src = g->h_src;

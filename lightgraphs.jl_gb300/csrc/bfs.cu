@@ -20,9 +20,10 @@
 // bitmaps, and needs no atomics at all: the queue of the new frontier is only
 // built when the next level goes top-down.
 // Bound: latency of the barriers and of dependent loads on the small levels
-// (about 5 us a level), in-edge sectors from HBM on the bottom-up ones.  A
-// single-source call on R-MAT 20, 4 MB of distances included, takes 174 us
-// (host-driven levels: 400 us).
+// (5 to 10 us a level), in-edge sectors from HBM on the bottom-up ones.  A
+// single-source call on R-MAT 20, 4 MB of distances included, takes 139 us
+// (226 us with one edge per thread in flight and every warp reading the
+// level's counters; host-driven levels more than 400 us).
 //
 // The kernels with one launch per level serve lgbc_gdistances_noalloc, whose
 // fixed scratch holds a queue and two bitmaps.
@@ -38,6 +39,12 @@ __device__ __forceinline__ long long gwarp() {
 }
 __device__ __forceinline__ long long nwarps() {
   return (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
+}
+
+__device__ __forceinline__ unsigned long long shfl_up_u64(unsigned long long x, int o) {
+  const unsigned lo = __shfl_up_sync(kFull, static_cast<unsigned>(x), o);
+  const unsigned hi = __shfl_up_sync(kFull, static_cast<unsigned>(x >> 32), o);
+  return (static_cast<unsigned long long>(hi) << 32) | lo;
 }
 
 __device__ __forceinline__ int64_t shfl_i64(int64_t x, int src) {
@@ -251,10 +258,55 @@ struct BfsFound {
   unsigned long long mf = 0, mu = 0;
 };
 
-// List w (claimed by this thread) for the next level; `lists` false: count it only.
+// List the vertices w[q] where ok[q], with rows of d[q] entries, for a level
+// of the given parity: one atomic per warp for the queue and one for the long
+// rows.  That one hands out entries (high word) and their first chunks (low
+// word), so the list is sorted by first chunk; an atomic for every long row
+// was 1.4 ns each on the one address, and neighbours of hubs are often hubs.
+template <int Q>
+__device__ __forceinline__ void bfs_append(const BfsRun& r, BfsSlot* slot, unsigned long long base, int parity,
+                                           const int32_t (&w)[Q], const int64_t (&d)[Q], const bool (&ok)[Q]) {
+  const int ln = lane_id();
+  int at[Q], total = 0;
+  unsigned long long mine = 0;
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const unsigned bal = __ballot_sync(kFull, ok[q] && d[q] <= kBfsChunk);
+    at[q] = total + __popc(bal & ((1u << ln) - 1u));
+    total += __popc(bal);
+    if (ok[q] && d[q] > kBfsChunk) mine += (1ull << 32) | static_cast<unsigned>((d[q] + kBfsChunk - 1) / kBfsChunk);
+  }
+  unsigned long long first = 0;
+  if (ln == 0 && total) first = atomicAdd(&slot->queued, static_cast<unsigned long long>(total));
+  const bool big = __any_sync(kFull, mine != 0ull);
+  unsigned long long p = mine;
+  if (big) {
+#pragma unroll
+    for (int o = 1; o < kWarp; o <<= 1) {
+      const unsigned long long y = shfl_up_u64(p, o);
+      if (ln >= o) p += y;
+    }
+    unsigned long long b0 = 0;
+    if (ln == kWarp - 1) b0 = atomicAdd(&slot->big, p);
+    p = static_cast<unsigned long long>(shfl_i64(static_cast<int64_t>(b0), kWarp - 1)) + p - mine;
+  }
+  first = base + static_cast<unsigned long long>(shfl_i64(static_cast<int64_t>(first), 0));
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    if (!ok[q]) continue;
+    if (d[q] <= kBfsChunk) {
+      r.queue[first + at[q]] = w[q];
+    } else {
+      r.big[parity * r.big_cap + static_cast<int64_t>(p >> 32)] = make_int2(static_cast<int>(p & 0xFFFFFFFFu), w[q]);
+      p += (1ull << 32) | static_cast<unsigned>((d[q] + kBfsChunk - 1) / kBfsChunk);
+    }
+  }
+}
+
+// List w (claimed by this thread) for a level.
 __device__ __forceinline__ void bfs_list(const DevGraph& g, const BfsRun& r, BfsSlot* slot,
                                          unsigned long long base, int parity, bool claimed, int32_t w,
-                                         bool lists, BfsFound& f) {
+                                         BfsFound& f) {
   int64_t d = 0;
   if (claimed) {
     d = g.rowptr[w + 1] - g.rowptr[w];
@@ -262,32 +314,61 @@ __device__ __forceinline__ void bfs_list(const DevGraph& g, const BfsRun& r, Bfs
     f.mf += static_cast<unsigned long long>(d);
     f.mu += static_cast<unsigned long long>(g.in_rowptr[w + 1] - g.in_rowptr[w]);
   }
-  if (!lists) return;
-  const bool big = d > kBfsChunk;
-  const unsigned long long at = warp_append(claimed && !big, &slot->queued);
-  if (claimed && !big) r.queue[base + at] = w;
-  if (big) {
-    // one atomic hands out the entry (high word) and its first chunk (low
-    // word), so the list is sorted by first chunk
-    const unsigned chunks = static_cast<unsigned>((d + kBfsChunk - 1) / kBfsChunk);
-    const unsigned long long p = atomicAdd(&slot->big, (1ull << 32) | chunks);
-    r.big[parity * r.big_cap + static_cast<int64_t>(p >> 32)] = make_int2(static_cast<int>(p & 0xFFFFFFFFu), w);
-  }
+  const int32_t ws[1] = {w};
+  const int64_t ds[1] = {d};
+  const bool oks[1] = {claimed};
+  bfs_append<1>(r, slot, base, parity, ws, ds, oks);
 }
 
-__device__ __forceinline__ bool bfs_take(const BfsRun& r, uint32_t* next, int32_t w, int32_t level) {
-  const uint32_t bit = 1u << (w & 31);
-  // a stale cached word can only lack bits, which the atomic then finds set
-  if (r.visited[w >> 5] & bit) return false;
-  if (atomicOr(r.visited + (w >> 5), bit) & bit) return false;
-  atomicOr(next + (w >> 5), bit);
-  r.dist[w] = level;
-  return true;
+// Take the edges to w[q] where ok[q] for level `level` and list what they
+// reach.  Every step of the chain (visited word, claim, row lengths, queue
+// entry) is a round trip of about a microsecond, so kBfsAhead edges per thread
+// go through it together, with one queue atomic for all of the warp's.
+__device__ __forceinline__ void bfs_expand(const DevGraph& g, const BfsRun& r, uint32_t* next, BfsSlot* slot,
+                                           unsigned long long base, int32_t level, const int32_t (&w)[kBfsAhead],
+                                           bool (&ok)[kBfsAhead], BfsFound& f) {
+  uint32_t word[kBfsAhead];
+#pragma unroll
+  for (int q = 0; q < kBfsAhead; ++q)  // a stale cached word can only lack bits, which the atomic then finds set
+    word[q] = ok[q] ? r.visited[w[q] >> 5] : ~0u;
+#pragma unroll
+  for (int q = 0; q < kBfsAhead; ++q) {
+    const uint32_t bit = 1u << (w[q] & 31);
+    if (!(word[q] & bit)) word[q] = atomicOr(r.visited + (w[q] >> 5), bit);
+  }
+  bool any = false;
+#pragma unroll
+  for (int q = 0; q < kBfsAhead; ++q) {
+    const uint32_t bit = 1u << (w[q] & 31);
+    ok[q] = !(word[q] & bit);
+    any |= ok[q];
+    if (ok[q]) {
+      atomicOr(next + (w[q] >> 5), bit);
+      r.dist[w[q]] = level;
+    }
+  }
+  if (!__any_sync(kFull, any)) return;
+  int64_t d[kBfsAhead];
+#pragma unroll
+  for (int q = 0; q < kBfsAhead; ++q) {
+    d[q] = 0;
+    if (ok[q]) {
+      d[q] = g.rowptr[w[q] + 1] - g.rowptr[w[q]];
+      f.mu += static_cast<unsigned long long>(g.in_rowptr[w[q] + 1] - g.in_rowptr[w[q]]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < kBfsAhead; ++q) {
+    f.count += ok[q] ? 1u : 0u;
+    f.mf += static_cast<unsigned long long>(d[q]);
+  }
+  bfs_append<kBfsAhead>(r, slot, base, level & 1, w, d, ok);
 }
 
 __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
   extern __shared__ uint32_t sbm[];
-  __shared__ int s_ok;
+  __shared__ int s_ok, s_bu;
+  __shared__ unsigned long long s_queued, s_big;
   __shared__ unsigned long long s_sum[3];
   BfsState* st = r.state;
   const int ln = lane_id();
@@ -325,6 +406,9 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
     if (v < n) {
       if (r.prefilled) seen = r.dist[v] != kUnreached;
       else r.dist[v] = kUnreached;
+      // no edge reaches it: else a bottom-up level would come back to it each
+      // time (two fifths of an R-MAT graph)
+      seen |= g.in_rowptr[v + 1] == g.in_rowptr[v];
     }
     const unsigned bal = __ballot_sync(kFull, seen);
     if (ln == 0) {
@@ -339,8 +423,15 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
     for (int64_t i0 = tid - ln; i0 < r.nsrc; i0 += threads) {
       const int64_t i = i0 + ln;
       const int32_t s = i < r.nsrc ? r.src[i] : 0;
-      const bool claimed = i < r.nsrc && bfs_take(r, bitmap(0), s, 0);
-      bfs_list(g, r, &st->slot[0], 0, 0, claimed, s, true, f);
+      // by the frontier's bit: a source that nothing enters has its visited bit
+      const uint32_t bit = 1u << (s & 31);
+      bool claimed = i < r.nsrc && (!r.prefilled || __ldcg(r.dist + s) == kUnreached);
+      if (claimed) claimed = !(atomicOr(bitmap(0) + (s >> 5), bit) & bit);
+      if (claimed) {
+        atomicOr(r.visited + (s >> 5), bit);
+        r.dist[s] = 0;
+      }
+      bfs_list(g, r, &st->slot[0], 0, 0, claimed, s, f);
     }
     report(&st->slot[0], f);
   }
@@ -353,14 +444,24 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
     // a slot is reused three levels later, by when every block has read it
     const BfsSlot* cur = &st->slot[level % 3];
     BfsSlot* nxt = &st->slot[(level + 1) % 3];
-    const unsigned long long nf = __ldcg(&cur->count), mf = __ldcg(&cur->mf);
-    unsigned long long queued = __ldcg(&cur->queued), big = __ldcg(&cur->big);
-    mu_done += __ldcg(&cur->mu);
-    if (nf == 0 || level > n) break;
+    // One thread reads the slot and chooses the direction: the reads of every
+    // warp went to one L2 line (24,000 of them, 10 us a level), and a division
+    // of 1,024 threads keeps the FP64 pipe for some more.
+    if (threadIdx.x == 0) {
+      const unsigned long long count = __ldcg(&cur->count), mf = __ldcg(&cur->mf);
+      s_queued = __ldcg(&cur->queued);
+      s_big = __ldcg(&cur->big);
+      mu_done += __ldcg(&cur->mu);
+      const double left = static_cast<double>(g.nnz) - static_cast<double>(mu_done);
+      s_bu = count == 0 ? -1
+             : bu       ? static_cast<double>(count) >= static_cast<double>(n) / r.beta
+                        : static_cast<double>(mf) > left / r.alpha;
+    }
+    __syncthreads();
     const bool was = bu;
-    const double left = static_cast<double>(g.nnz) - static_cast<double>(mu_done);
-    bu = was ? static_cast<double>(nf) >= static_cast<double>(n) / r.beta
-             : static_cast<double>(mf) > left / r.alpha;
+    if (s_bu < 0 || level > n) break;
+    bu = s_bu != 0;
+    unsigned long long queued = s_queued, big = s_big;
     uint32_t* front = bitmap(level);
     uint32_t* next = bitmap(level + 1);
     uint32_t* stale = bitmap(level + 2);
@@ -374,12 +475,17 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
           const bool has = bits != 0u;
           const int32_t v = static_cast<int32_t>((w0 + ln) * kWarp + (has ? __ffs(bits) - 1 : 0));
           bits &= bits - 1u;
-          bfs_list(g, r, own, lo, level & 1, has, v, true, ignored);
+          bfs_list(g, r, own, lo, level & 1, has, v, ignored);
         }
       }
       if (!grid_barrier(&st->barrier, goal, &s_ok)) return;
-      queued = __ldcg(&own->queued);
-      big = __ldcg(&own->big);
+      if (threadIdx.x == 0) {
+        s_queued = __ldcg(&own->queued);
+        s_big = __ldcg(&own->big);
+      }
+      __syncthreads();
+      queued = s_queued;
+      big = s_big;
     }
     // what the level after next will fill
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -395,36 +501,65 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
       if (r.stage) {
         const uint4* src4 = reinterpret_cast<const uint4*>(front);
         uint4* dst4 = reinterpret_cast<uint4*>(sbm);
-        for (int64_t i = threadIdx.x; i < (nwords + 3) >> 2; i += blockDim.x) dst4[i] = __ldcg(src4 + i);
+        // eight loads in flight
+        const int64_t quads = (nwords + 3) >> 2;
+        for (int64_t i0 = threadIdx.x; i0 < quads; i0 += 8 * blockDim.x) {
+          uint4 x[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if (i0 + q * blockDim.x < quads) x[q] = __ldcg(src4 + i0 + q * blockDim.x);
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if (i0 + q * blockDim.x < quads) dst4[i0 + q * blockDim.x] = x[q];
+        }
         __syncthreads();
         fbm = sbm;
       }
-      for (int64_t w0 = warp; w0 < nwords; w0 += warps) {
-        const uint32_t seen = __ldcg(r.visited + w0);
-        if (seen == ~0u) {
-          if (ln == 0) next[w0] = 0u;
-          continue;
-        }
-        const int64_t v = (w0 << 5) + ln;
-        bool found = false;
-        if (!((seen >> ln) & 1u)) {
-          const int64_t e1 = g.in_rowptr[v + 1];
-          for (int64_t e = g.in_rowptr[v]; e < e1; ++e) {
+      // A warp's words are loaded 32 at a time, and a word's row pointers while
+      // the rows of the word before are looked through: what is left for a word
+      // is its columns' round trips.
+      for (int64_t g0 = warp; g0 < nwords; g0 += warps * kWarp) {
+        const int64_t mine = g0 + ln * warps;
+        const uint32_t words = mine < nwords ? __ldcg(r.visited + mine) : ~0u;
+        if (mine < nwords && words == ~0u) next[mine] = 0u;
+        unsigned todo = __ballot_sync(kFull, words != ~0u);
+        int64_t en = 0, en1 = 0;
+        auto rows_of = [&](int k) {
+          const int64_t v = ((g0 + k * warps) << 5) + ln;
+          en = en1 = 0;
+          if (!((__shfl_sync(kFull, words, k) >> ln) & 1u)) {
+            en = g.in_rowptr[v];
+            en1 = g.in_rowptr[v + 1];
+          }
+        };
+        if (todo) rows_of(__ffs(todo) - 1);
+        while (todo) {
+          const int k = __ffs(todo) - 1;
+          todo &= todo - 1u;
+          const int64_t w0 = g0 + k * warps, v = (w0 << 5) + ln;
+          const uint32_t seen = __shfl_sync(kFull, words, k);
+          int64_t e = en;
+          const int64_t e1 = en1;
+          const unsigned long long din = static_cast<unsigned long long>(e1 - e);
+          if (todo) rows_of(__ffs(todo) - 1);
+          bool found = false;
+          for (; !found && e < e1; ++e) {
             const int32_t u = g.in_colidx[e];
             const uint32_t word = r.stage ? fbm[u >> 5] : __ldcg(fbm + (u >> 5));
-            if ((word >> (u & 31)) & 1u) {
-              found = true;
-              break;
-            }
+            found = ((word >> (u & 31)) & 1u) != 0u;
+          }
+          const unsigned bal = __ballot_sync(kFull, found);
+          if (ln == 0) {
+            next[w0] = bal;
+            if (bal) r.visited[w0] = seen | bal;
+          }
+          if (found) {
+            r.dist[v] = level + 1;
+            f.count += 1;
+            f.mu += din;
+            f.mf += g.rowptr == g.in_rowptr ? din : static_cast<unsigned long long>(g.rowptr[v + 1] - g.rowptr[v]);
           }
         }
-        const unsigned bal = __ballot_sync(kFull, found);
-        if (ln == 0) {
-          next[w0] = bal;
-          if (bal) r.visited[w0] = seen | bal;
-        }
-        if (found) r.dist[v] = level + 1;
-        bfs_list(g, r, nxt, hi, (level + 1) & 1, found, static_cast<int32_t>(v), false, f);
       }
     } else {
       ++td_levels;
@@ -450,19 +585,26 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
         }
         const int total = __shfl_sync(kFull, incl, kWarp - 1);
         const int off = incl - d;
-        for (int k0 = 0; k0 < total; k0 += kWarp) {
-          const int k = k0 + ln;
-          int j = 0;  // the lane whose list holds concatenated edge k
+        for (int k0 = 0; k0 < total; k0 += kBfsAhead * kWarp) {
+          int32_t w[kBfsAhead];
+          bool ok[kBfsAhead];
 #pragma unroll
-          for (int step = 16; step >= 1; step >>= 1) {
-            const int iv = __shfl_sync(kFull, incl, j + step - 1);
-            if (iv <= k) j += step;
+          for (int q = 0; q < kBfsAhead; ++q) {
+            const int k = k0 + q * kWarp + ln;
+            ok[q] = k < total;
+            w[q] = 0;
+            if (k0 + q * kWarp >= total) continue;  // warp-uniform
+            int j = 0;  // the lane whose list holds concatenated edge k
+#pragma unroll
+            for (int step = 16; step >= 1; step >>= 1) {
+              const int iv = __shfl_sync(kFull, incl, j + step - 1);
+              if (iv <= k) j += step;
+            }
+            const int64_t ej = shfl_i64(e0, j);
+            const int oj = __shfl_sync(kFull, off, j);
+            if (ok[q]) w[q] = g.colidx[ej + (k - oj)];
           }
-          const int64_t ej = shfl_i64(e0, j);
-          const int oj = __shfl_sync(kFull, off, j);
-          const int32_t w = k < total ? g.colidx[ej + (k - oj)] : 0;
-          const bool claimed = k < total && bfs_take(r, next, w, level + 1);
-          if (__any_sync(kFull, claimed)) bfs_list(g, r, nxt, hi, (level + 1) & 1, claimed, w, true, f);
+          bfs_expand(g, r, next, nxt, hi, level + 1, w, ok, f);
         }
       }
       const long long entries = static_cast<long long>(big >> 32), chunks = static_cast<long long>(big & 0xFFFFFFFFull);
@@ -477,12 +619,15 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
         const int2 en = __ldcg(&list[a]);
         const int64_t e0 = g.rowptr[en.y] + (c - en.x) * kBfsChunk;
         const int64_t e1 = min(e0 + kBfsChunk, g.rowptr[en.y + 1]);
-        for (int64_t e = e0; e < e1; e += kWarp) {
-          const int64_t idx = e + ln;
-          const int32_t w = idx < e1 ? g.colidx[idx] : 0;
-          const bool claimed = idx < e1 && bfs_take(r, next, w, level + 1);
-          if (__any_sync(kFull, claimed)) bfs_list(g, r, nxt, hi, (level + 1) & 1, claimed, w, true, f);
+        int32_t w[kBfsAhead];
+        bool ok[kBfsAhead];
+#pragma unroll
+        for (int q = 0; q < kBfsAhead; ++q) {
+          const int64_t idx = e0 + q * kWarp + ln;
+          ok[q] = idx < e1;
+          w[q] = ok[q] ? g.colidx[idx] : 0;
         }
+        bfs_expand(g, r, next, nxt, hi, level + 1, w, ok, f);
       }
     }
     report(nxt, f);

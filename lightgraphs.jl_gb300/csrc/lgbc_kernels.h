@@ -276,7 +276,8 @@ struct BfsBuffers {
   BatchCtl* ctl;
 };
 // A whole search in one cooperative launch.
-constexpr int kBfsChunk = 256;  // out-edges a warp takes of a long list
+constexpr int kBfsAhead = 4;               // edges a thread has in flight
+constexpr int kBfsChunk = 32 * kBfsAhead;  // out-edges a warp takes of a long list
 struct BfsSlot {                // one level's frontier, rotating over three
   unsigned long long count, mf, mu;  // vertices, their out-edges and in-edges
   unsigned long long queued;         // those listed in the queue

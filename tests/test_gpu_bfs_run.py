@@ -1,5 +1,5 @@
 """The one-launch BFS (k_bfs_run) against the oracle's gdistances! bit for bit:
-rows around the length that one claim of a warp covers (256 entries), vertex
+rows around the lengths that one claim of a warp covers (128 entries), vertex
 counts around the 32-vertex words of its bitmaps, both directions forced and
 the default choice between them.  A tuning other than the default keeps these
 small graphs on this kernel."""
@@ -26,7 +26,7 @@ def bfs(g, srcs, tuning):
 
 
 @pytest.mark.parametrize("tuning", sorted(TUNINGS))
-@pytest.mark.parametrize("degree", [255, 256, 257, 511, 512, 513, 1500])
+@pytest.mark.parametrize("degree", [31, 33, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1500])
 def test_row_lengths(degree, tuning):
     # a hub, its leaves, and a second hub of one more entry two levels on
     n = 2 * degree + 40
