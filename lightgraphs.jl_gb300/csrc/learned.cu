@@ -377,6 +377,7 @@ __device__ __forceinline__ void core_list_neighbours(const DevGraph& g, const Co
 
 __global__ void __launch_bounds__(256) k_core_run(DevGraph g, CoreRun r) {
   __shared__ int s_ok;
+  __shared__ unsigned long long s_n[4];  // read and written a grid barrier apart
   CoreState* st = r.state;
   const int ln = lane_id();
   const int wid = threadIdx.x >> 5, wpb = blockDim.x >> 5;
@@ -395,8 +396,14 @@ __global__ void __launch_bounds__(256) k_core_run(DevGraph g, CoreRun r) {
     // a slot is reused three passes later, by when every block has read it
     CoreSlot* cur = &st->slot[pass % 3];
     CoreSlot* nxt = &st->slot[(pass + 1) % 3];
-    const long long nsmall = pass ? static_cast<long long>(__ldcg(&cur->small)) : g.n;
-    const unsigned long long nhubs = pass ? __ldcg(&cur->hubs) : __ldcg(&st->all_hubs);
+    // one thread reads the counters: the reads of every warp went to one L2 line
+    if (threadIdx.x == 0) {
+      s_n[0] = pass ? __ldcg(&cur->small) : static_cast<unsigned long long>(g.n);
+      s_n[1] = pass ? __ldcg(&cur->hubs) : __ldcg(&st->all_hubs);
+    }
+    __syncthreads();
+    const long long nsmall = static_cast<long long>(s_n[0]);
+    const unsigned long long nhubs = s_n[1];
     if ((nsmall == 0 && nhubs == 0) || pass > r.max_passes) break;
     const int from = static_cast<int>(pass & 1), to = from ^ 1;
     core_search_hubs(g, pass ? (from ? r.hubs[1] : r.hubs[0]) : r.all_hubs, nhubs, r.flag, r.core,
@@ -408,7 +415,12 @@ __global__ void __launch_bounds__(256) k_core_run(DevGraph g, CoreRun r) {
       CoreSlot* z = &st->slot[(pass + 2) % 3];
       z->small = z->hubs = z->log = z->hub_log = 0ull;
     }
-    const unsigned long long nhl = __ldcg(&cur->hub_log), nl = __ldcg(&cur->log);
+    if (threadIdx.x == 0) {
+      s_n[2] = __ldcg(&cur->hub_log);
+      s_n[3] = __ldcg(&cur->log);
+    }
+    __syncthreads();
+    const unsigned long long nhl = s_n[2], nl = s_n[3];
     for (unsigned long long i = blockIdx.x; i < nhl; i += gridDim.x) {
       const int32_t v = __ldcg(r.hub_v + i);
       core_list_neighbours<kCoreAhead>(g, r, nxt, to, v, __ldcg(r.core + v), __ldcg(r.hub_old + i), wid, wpb);
