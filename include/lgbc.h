@@ -157,7 +157,7 @@ int lgbc_timer_stop(lgbc_graph *g, double *elapsed_ms, int64_t *kernel_launches)
 /* Statistics of the last betweenness / gdistances call on this handle. */
 typedef struct lgbc_stats {
   int64_t kernel_launches;   /* kernels the call launched */
-  int64_t batches;           /* source batches (<= 128 sources each) */
+  int64_t batches;           /* source batches (<= lanes sources each; see below for small graphs) */
   int64_t levels;            /* BFS levels summed over batches */
   int64_t active_sources;    /* sources with degree > 0 */
   int64_t wide_batches;      /* batches replayed in FP64 because a path count exceeded 2^64 */
@@ -168,7 +168,7 @@ int lgbc_graph_stats(const lgbc_graph *g, lgbc_stats *out);
 
 /* Tunables (the autotuner writes these; defaults are used otherwise).  They
  * shape the bit-lane batches.  With every field at its default, betweenness
- * of a graph whose vertex state fits one SM's shared memory (about 22,700
+ * of a graph whose vertex state fits one SM's shared memory (about 22,300
  * vertices, at most 2^20 stored entries) runs one thread block per source
  * instead, unless a search is deeper than 126 levels or a path count reaches
  * 2^48; lgbc_stats.batches then counts the blocks' shares of the sources.

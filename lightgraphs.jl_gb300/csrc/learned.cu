@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(256) k_core_degree(DevGraph g, int32_t* deg, i
 // warp's vertices (fewer per warp on short lists) and of a long row (several
 // entries per thread in flight).  core_number: R-MAT of 2,178 / 16,384 /
 // 131,072 / 1,048,576 vertices 838 / 1,115 / 2,587 / 7,329 us launched one by
-// one, 244 / 407 / 1,427 / 6,919 us here.  Values are read past L1, which
+// one, 238 / 373 / 1,353 / 6,739 us here.  Values are read past L1, which
 // keeps lines from earlier passes.
 struct CoreLog {
   unsigned long long* count;  // lowered vertices this pass

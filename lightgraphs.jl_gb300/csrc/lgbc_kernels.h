@@ -46,7 +46,7 @@ struct MsBuffers {
   uint64_t* visit;     // n lane sets: lanes that have reached v
   uint64_t* mb[2];     // n lane sets each: dense level masks, F_L lives in mb[L & 1]
   void* sigma;         // n rows: uint64 or double path counts
-  void* psi;           // n rows: df32 or double, (1 + delta) / sigma
+  void* psi;           // the rows of sigma: (1 + delta) / sigma takes a count's place
   int32_t* qv;         // cap: concatenated level lists (vertex)
   uint64_t* qm;        // cap lane sets: lanes of that vertex at that level
   unsigned long long* lvl_off;  // n + 3: start of each level's list

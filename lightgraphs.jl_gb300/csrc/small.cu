@@ -9,8 +9,8 @@
 // is instruction issue: 64 % of the issue slots busy with 32 warps per SM
 // (ALU pipe 52 %), the rest barriers and fixed latencies; DRAM is idle.
 // Measured (exact betweenness, batches -> here): G(10,000, 50,000) 11.7 ->
-// 4.24 ms; 24 Barabasi-Albert graphs of up to 20,000 vertices 453 -> 154 ms;
-// a 50-vertex digraph 289 -> 57 us.
+// 4.08 ms; 24 Barabasi-Albert graphs of up to 20,000 vertices 448 -> 150 ms;
+// a 50-vertex digraph 289 -> 36 us.
 //
 // Replaces, per source, dijkstra_shortest_paths(g, s; allpaths, trackvertices)
 // with unit weights (src/shortestpaths/dijkstra.jl:59-141) and
@@ -140,8 +140,8 @@ __global__ void __launch_bounds__(1024) k_small_plan(const SmallGraph* graphs) {
   }
 }
 
-// The columns of the planned rows, a warp per vertex: most of the plan's work,
-// and 380 us of a 430 us plan of 16,384 vertices when one block did it.
+// The columns of the planned rows, a warp per vertex: most of the plan's work.
+// One block's plan of 16,384 vertices took 380 us, the two kernels take 45 + 53.
 __global__ void __launch_bounds__(256) k_small_columns(const SmallGraph* graphs) {
   const SmallGraph G = graphs[blockIdx.y];
   const int n = G.n;
@@ -762,7 +762,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
 // lane has finished is passed over.  Bound: latency of the levels of a few
 // blocks (one source), shared-memory loads (many).  Measured against those
 // paths: distance sums from all 3,000 vertices of G(3,000, 18,000) 11.6 ms ->
-// 82 us, one BFS on G(1,001, 5,003) 222 -> 40 us as a call.
+// 82 us, one BFS on G(1,001, 5,003) 222 -> 29 us as a call.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_bfs(SmallBfs run) {
   extern __shared__ uint32_t sm[];
