@@ -1540,13 +1540,7 @@ int copy_dist(lgbc_graph* g, void* out, int64_t at, int64_t count, bool wide) {
   const size_t bytes = static_cast<size_t>(count) * (wide ? 8 : 4);
   const void* from = g->d_dist;
   if (wide) {
-    if (count > g->d_wide_cap) {
-      dev_free(g->d_wide);
-  dev_free(g->d_stats);
-      g->d_wide_cap = 0;
-      LGBC_TRY(dev_alloc(&g->d_wide, static_cast<size_t>(count)));
-      g->d_wide_cap = count;
-    }
+    LGBC_TRY(ensure_wide(g, count));
     g->launches += widen_dist(g->cfg, g->stream, g->d_dist, count, g->d_wide);
     from = g->d_wide;
   }

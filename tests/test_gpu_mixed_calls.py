@@ -1,0 +1,49 @@
+"""Calls of different kinds in turn on one handle: each keeps a workspace there,
+and growing one must leave the others as they were.  Int64 graphs (distances in
+64 bits pass through a buffer of their own) of more than 2^17 stored entries,
+below and above the vertex count up to which searches run in shared memory."""
+import numpy as np
+import pytest
+
+import lgbc
+from conftest import csr_args
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,m", [(3000, 80000), (19500, 75000)])
+def test_distance_statistics_between_distance_calls(n, m):
+    e = np.random.default_rng(n).integers(0, n, (2, m))
+    g = lgbc.SimpleGraph.from_edge_arrays(n, e[0], e[1])
+    rp, ci, _ = csr_args(g)
+    assert g.eltype == np.int64 and rp[n] > 1 << 17
+    src = np.arange(0, n, n // 90, dtype=np.int32)
+    want = oracle.gdistances_many(rp, ci, src, nthreads=8).astype(np.int64)
+    far = want == oracle.UNREACHED32
+    top = np.iinfo(np.int64).max
+
+    def statistics():
+        reached, dsum, dmax = lgbc.distance.distance_stats(g, src)
+        assert np.array_equal(reached, (~far).sum(1))
+        assert np.array_equal(dsum, np.where(far, 0, want).sum(1))
+        assert np.array_equal(dmax, np.where(far, 0, want).max(1))
+
+    statistics()
+    assert np.array_equal(lgbc.gdistances(g, int(src[0]) + 1), np.where(far, top, want)[0])
+    statistics()
+    assert np.array_equal(lgbc.multi_gdistances(g, src + 1), np.where(far, top, want))
+    statistics()
+    few = src[:3]
+    assert np.array_equal(lgbc.eccentricity(g, list(few + 1)), np.where(far.any(1), top, want.max(1))[:3])
+
+
+def test_closeness_between_distance_calls():
+    n = 3000
+    e = np.random.default_rng(5).integers(0, n, (2, 80000))
+    g = lgbc.SimpleGraph.from_edge_arrays(n, e[0], e[1])
+    rp, ci, _ = csr_args(g)
+    want = oracle.closeness(rp, ci, np.diff(rp))
+    for call in (lambda: lgbc.gdistances(g, 1), lambda: lgbc.multi_gdistances(g, range(1, 200)), lambda: None):
+        assert np.array_equal(lgbc.closeness_centrality(g), want)
+        call()
