@@ -1534,18 +1534,25 @@ int ensure_wide(lgbc_graph* g, int64_t count) {
   return LGBC_OK;
 }
 
+// Distances widened to 64 bits at a time: all 64 rows of a batch at once would
+// take twice the memory of the batch's 32-bit distances on top of them.
+constexpr int64_t kWidePiece = int64_t(1) << 25;
+
 // g->d_dist[0, count) to out[at, at + count) on the host: as it is, or in 64
 // bits with typemax(Int64) where nothing reaches.
 int copy_dist(lgbc_graph* g, void* out, int64_t at, int64_t count, bool wide) {
-  const size_t bytes = static_cast<size_t>(count) * (wide ? 8 : 4);
-  const void* from = g->d_dist;
-  if (wide) {
-    LGBC_TRY(ensure_wide(g, count));
-    g->launches += widen_dist(g->cfg, g->stream, g->d_dist, count, g->d_wide);
-    from = g->d_wide;
+  if (!wide) {
+    LGBC_CUDA(cudaMemcpyAsync(static_cast<int32_t*>(out) + at, g->d_dist, static_cast<size_t>(count) * 4,
+                              cudaMemcpyDeviceToHost, g->stream));
+    return LGBC_OK;
   }
-  LGBC_CUDA(cudaMemcpyAsync(static_cast<char*>(out) + at * (wide ? 8 : 4), from, bytes, cudaMemcpyDeviceToHost,
-                            g->stream));
+  LGBC_TRY(ensure_wide(g, std::min(count, kWidePiece)));
+  for (int64_t p = 0; p < count; p += kWidePiece) {
+    const int64_t c = std::min(kWidePiece, count - p);
+    g->launches += widen_dist(g->cfg, g->stream, g->d_dist + p, c, g->d_wide);
+    LGBC_CUDA(cudaMemcpyAsync(static_cast<int64_t*>(out) + at + p, g->d_wide, static_cast<size_t>(c) * 8,
+                              cudaMemcpyDeviceToHost, g->stream));
+  }
   return LGBC_OK;
 }
 

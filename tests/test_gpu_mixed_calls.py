@@ -47,3 +47,25 @@ def test_closeness_between_distance_calls():
     for call in (lambda: lgbc.gdistances(g, 1), lambda: lgbc.multi_gdistances(g, range(1, 200)), lambda: None):
         assert np.array_equal(lgbc.closeness_centrality(g), want)
         call()
+
+
+def test_wide_distances_take_a_bounded_buffer():
+    # 64 rows of 2^20 vertices: the 64-bit table may cost the device at most
+    # 2^25 entries (256 MB) more than the 32-bit one, and more than one piece
+    # of it is widened
+    torch = pytest.importorskip("torch")
+    n = 1 << 20
+    e = np.random.default_rng(3).integers(0, n, (2, 3 * n // 2))
+    used, rows = {}, {}
+    for dtype in (np.int32, np.int64):
+        g = lgbc.SimpleGraph.from_edge_arrays(n, e[0], e[1], eltype=dtype)
+        g.device_handle()
+        free = torch.cuda.mem_get_info()[0]
+        rows[dtype] = lgbc.multi_gdistances(g, range(1, 65))
+        used[dtype] = free - torch.cuda.mem_get_info()[0]
+        del g
+    assert used[np.int64] - used[np.int32] <= (1 << 28) + (1 << 23)
+    narrow, wide = rows[np.int32], rows[np.int64]
+    far = narrow == np.iinfo(np.int32).max
+    assert far.any() and np.array_equal(far, wide == np.iinfo(np.int64).max)
+    assert np.array_equal(narrow[~far], wide[~far])
