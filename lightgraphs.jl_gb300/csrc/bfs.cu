@@ -377,6 +377,7 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
   const int64_t threads = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const long long warp = gwarp(), warps = nwarps();
   unsigned long long goal = 0;
+  BarrierBeat beat, walked;
   auto bitmap = [&](int32_t level) { return r.visited + (1 + level % 3) * r.words; };
 
   // fold a level's findings into its slot, one set of atomics per block
@@ -547,6 +548,7 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
             const int32_t u = g.in_colidx[e];
             const uint32_t word = r.stage ? fbm[u >> 5] : __ldcg(fbm + (u >> 5));
             found = ((word >> (u & 31)) & 1u) != 0u;
+            if (walked.entry_due()) beat_now(&st->barrier);
           }
           const unsigned bal = __ballot_sync(kFull, found);
           if (ln == 0) {
@@ -586,6 +588,7 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
         const int total = __shfl_sync(kFull, incl, kWarp - 1);
         const int off = incl - d;
         for (int k0 = 0; k0 < total; k0 += kBfsAhead * kWarp) {
+          beat_turn(&st->barrier, beat);
           int32_t w[kBfsAhead];
           bool ok[kBfsAhead];
 #pragma unroll
@@ -610,6 +613,7 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_run(DevGraph g, BfsRun r) {
       const long long entries = static_cast<long long>(big >> 32), chunks = static_cast<long long>(big & 0xFFFFFFFFull);
       const int2* list = r.big + (level & 1) * r.big_cap;
       for (long long c = warp; c < chunks; c += warps) {
+        beat_turn(&st->barrier, beat);
         long long a = 0, b = entries - 1;  // the last entry whose first chunk is at most c
         while (a < b) {
           const long long mid = (a + b + 1) >> 1;

@@ -180,13 +180,15 @@ __device__ __forceinline__ void core_log(const CoreLog& lg, unsigned long long a
 // entries are searched by their own lane; the others, one at a time, by the
 // whole warp.
 __device__ __forceinline__ void core_search_small(const DevGraph& g, const int32_t* list, long long nlist,
-                                                  uint32_t* flag, int32_t* core, CoreLog lg) {
+                                                  uint32_t* flag, int32_t* core, CoreLog lg, GridBarrier* bar,
+                                                  BarrierBeat& beat) {
   const int ln = lane_id();
   // 32 entries a warp at most, fewer on a short list: a vertex that takes the
   // whole warp is three dependent round trips, one after the other
   const long long share = (nlist + nwarps() - 1) / nwarps();
   const int per = static_cast<int>(min(max(share, 1ll), static_cast<long long>(kWarp)));
   for (long long base = gwarp() * per; base < nlist; base += nwarps() * per) {
+    beat_turn(bar, beat);
     const long long i = ln < per ? base + ln : nlist;
     int32_t v = 0, c = 0;
     int ent = 0;
@@ -236,14 +238,17 @@ __device__ __forceinline__ int block_sum_int(int x, int* red) {
 }
 
 __device__ __forceinline__ int block_count_at_least(const DevGraph& g, int32_t v, const int32_t* core,
-                                                    int32_t h, int* red) {
+                                                    int32_t h, int* red, GridBarrier* bar,
+                                                    BarrierBeat& beat) {
   int c = 0;
   for (int64_t e = g.rowptr[v] + threadIdx.x; e < g.rowptr[v + 1]; e += blockDim.x) {
+    beat_turn(bar, beat);
     const int32_t u = g.colidx[e];
     c += (u != v && __ldcg(core + u) >= h) ? 1 : 0;
   }
   if (is_digraph(g))
     for (int64_t e = g.in_rowptr[v] + threadIdx.x; e < g.in_rowptr[v + 1]; e += blockDim.x) {
+      beat_turn(bar, beat);
       const int32_t u = g.in_colidx[e];
       c += (u != v && __ldcg(core + u) >= h) ? 1 : 0;
     }
@@ -251,12 +256,14 @@ __device__ __forceinline__ int block_count_at_least(const DevGraph& g, int32_t v
 }
 
 __device__ __forceinline__ void core_search_hubs(const DevGraph& g, const int32_t* hubs, unsigned long long nl,
-                                                 uint32_t* flag, int32_t* core, CoreLog lg) {
+                                                 uint32_t* flag, int32_t* core, CoreLog lg, GridBarrier* bar,
+                                                 BarrierBeat& beat) {
   __shared__ int hist[kCoreHist + 1];
   __shared__ int red[8];
   __shared__ int s_h;
   const bool dir = is_digraph(g);
   for (unsigned long long i = blockIdx.x; i < nl; i += gridDim.x) {
+    beat_turn(bar, beat);
     const int32_t v = __ldcg(hubs + i);
     const int32_t c = __ldcg(core + v);
     if (threadIdx.x == 0) atomicAnd(flag + (v >> 5), ~(1u << (v & 31)));
@@ -268,6 +275,7 @@ __device__ __forceinline__ void core_search_hubs(const DevGraph& g, const int32_
     // took 80 dependent round trips, 60 us, in every pass that searched it.
     auto bin_list = [&](const int32_t* ci, int64_t e0, int64_t e1) {
       for (int64_t b0 = e0 + (threadIdx.x & ~(kWarp - 1)); b0 < e1; b0 += kCoreAhead * static_cast<int64_t>(blockDim.x)) {
+        beat_turn(bar, beat);
         int bin[kCoreAhead];
 #pragma unroll
         for (int q = 0; q < kCoreAhead; ++q) {
@@ -313,13 +321,13 @@ __device__ __forceinline__ void core_search_hubs(const DevGraph& g, const int32_
     __syncthreads();
     int h = s_h;  // the h-index over values capped at cap: exact when h < kCoreHist
     if (h >= kCoreHist && c > kCoreHist) {
-      if (block_count_at_least(g, v, core, c, red) >= c) {
+      if (block_count_at_least(g, v, core, c, red, bar, beat) >= c) {
         h = c;
       } else {
         int lo = kCoreHist, hi = c - 1;
         while (lo < hi) {
           const int mid = (lo + hi + 1) >> 1;
-          if (block_count_at_least(g, v, core, mid, red) >= mid) lo = mid; else hi = mid - 1;
+          if (block_count_at_least(g, v, core, mid, red, bar, beat) >= mid) lo = mid; else hi = mid - 1;
         }
         h = lo;
       }
@@ -350,13 +358,16 @@ __device__ __forceinline__ void core_list(const DevGraph& g, const CoreRun& r, C
 // step; `first` / `step`: the warp's share of the list.
 template <int AHEAD>
 __device__ __forceinline__ void core_list_neighbours(const DevGraph& g, const CoreRun& r, CoreSlot* nxt, int parity,
-                                                     int32_t v, int32_t lo, int32_t old, int first, int step) {
+                                                     int32_t v, int32_t lo, int32_t old, int first, int step,
+                                                     BarrierBeat& beat) {
   const int ln = lane_id();
+  beat_turn(&r.state->barrier, beat);
   for (int side = 0; side < (is_digraph(g) ? 2 : 1); ++side) {
     const int64_t* rp = side ? g.in_rowptr : g.rowptr;
     const int32_t* ci = side ? g.in_colidx : g.colidx;
     const int64_t e1 = rp[v + 1];
     for (int64_t e = rp[v] + first * AHEAD * kWarp; e < e1; e += static_cast<int64_t>(step) * AHEAD * kWarp) {
+      beat_turn(&r.state->barrier, beat);
       int32_t u[AHEAD];
       bool ok[AHEAD];
 #pragma unroll
@@ -382,7 +393,9 @@ __global__ void __launch_bounds__(256) k_core_run(DevGraph g, CoreRun r) {
   const int ln = lane_id();
   const int wid = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   unsigned long long goal = 0;
+  BarrierBeat beat;
   for (long long base = gwarp() * kWarp; base < g.n; base += nwarps() * kWarp) {
+    beat_turn(&st->barrier, beat);
     const long long v = base + ln;
     if (ln == 0) r.flag[base >> 5] = 0u;
     const bool hub = v < g.n && core_entries(g, static_cast<int32_t>(v)) > kCoreCached;
@@ -407,9 +420,9 @@ __global__ void __launch_bounds__(256) k_core_run(DevGraph g, CoreRun r) {
     if ((nsmall == 0 && nhubs == 0) || pass > r.max_passes) break;
     const int from = static_cast<int>(pass & 1), to = from ^ 1;
     core_search_hubs(g, pass ? (from ? r.hubs[1] : r.hubs[0]) : r.all_hubs, nhubs, r.flag, r.core,
-                     CoreLog{&cur->hub_log, r.hub_v, r.hub_old});
+                     CoreLog{&cur->hub_log, r.hub_v, r.hub_old}, &st->barrier, beat);
     core_search_small(g, pass ? (from ? r.small[1] : r.small[0]) : nullptr, nsmall, r.flag, r.core,
-                      CoreLog{&cur->log, r.log_v, r.log_old});
+                      CoreLog{&cur->log, r.log_v, r.log_old}, &st->barrier, beat);
     if (!grid_barrier(&st->barrier, goal, &s_ok)) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       CoreSlot* z = &st->slot[(pass + 2) % 3];
@@ -423,11 +436,11 @@ __global__ void __launch_bounds__(256) k_core_run(DevGraph g, CoreRun r) {
     const unsigned long long nhl = s_n[2], nl = s_n[3];
     for (unsigned long long i = blockIdx.x; i < nhl; i += gridDim.x) {
       const int32_t v = __ldcg(r.hub_v + i);
-      core_list_neighbours<kCoreAhead>(g, r, nxt, to, v, __ldcg(r.core + v), __ldcg(r.hub_old + i), wid, wpb);
+      core_list_neighbours<kCoreAhead>(g, r, nxt, to, v, __ldcg(r.core + v), __ldcg(r.hub_old + i), wid, wpb, beat);
     }
     for (unsigned long long i = gwarp(); i < nl; i += nwarps()) {
       const int32_t v = __ldcg(r.log_v + i);
-      core_list_neighbours<2>(g, r, nxt, to, v, __ldcg(r.core + v), __ldcg(r.log_old + i), 0, 1);
+      core_list_neighbours<2>(g, r, nxt, to, v, __ldcg(r.core + v), __ldcg(r.log_old + i), 0, 1, beat);
     }
     if (!grid_barrier(&st->barrier, goal, &s_ok)) return;
   }

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "grid_barrier.cuh"
+
 namespace lgbc {
 
 constexpr int kWarp = 32;
@@ -62,38 +64,6 @@ struct BatchCtl {
   int hubs;                       // a hub takes part in this level (bottom-up, backward)
   unsigned long long next_union[kMaxWords];  // lanes of Q_{L+1}, accumulated after its appends
 };
-
-// ---------------------------------------------------------------------------
-// Kernels of one cooperative launch
-// ---------------------------------------------------------------------------
-struct GridBarrier {  // zeroed before the launch
-  unsigned long long arrived;
-  int failed;
-};
-
-// Grid barrier: every block adds one to an ever-growing count and waits until
-// all have.  The wait is bounded: a block that gives up, or sees that another
-// has, reports it, and the kernel returns.  All blocks are resident (the
-// launch is cooperative), so that happens only if the GPU is wedged.
-constexpr unsigned kBarrierPolls = 1u << 23;  // some seconds
-
-__device__ __forceinline__ bool grid_barrier(GridBarrier* st, unsigned long long& goal, int* ok) {
-  __syncthreads();
-  goal += gridDim.x;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(&st->arrived, 1ull);
-    unsigned polls = 0;
-    while (*reinterpret_cast<volatile unsigned long long*>(&st->arrived) < goal &&
-           *reinterpret_cast<volatile int*>(&st->failed) == 0) {
-      if (++polls > kBarrierPolls) atomicExch(&st->failed, 1);
-    }
-    __threadfence();
-    *ok = *reinterpret_cast<volatile int*>(&st->failed) == 0;
-  }
-  __syncthreads();
-  return *ok != 0;
-}
 
 // ---------------------------------------------------------------------------
 // Warp helpers

@@ -46,3 +46,21 @@ def test_vertex_counts(n, tuning):
     for kind in (lgbc.SimpleGraph, lgbc.SimpleDiGraph):
         bfs(kind.from_edge_arrays(n, e[0], e[1]), [n - 1], tuning)
         bfs(kind.from_edge_arrays(n, e[0], e[1]), rng.integers(0, n, 9).tolist(), tuning)
+
+
+@pytest.mark.parametrize("tuning", ["bottomup", "auto"])
+@pytest.mark.parametrize("length", [4095, 4096, 4097, 8192, 8193, 20000])
+def test_long_in_lists_without_a_hit(length, tuning):
+    # one thread walks the in-list of a vertex that a bottom-up level does not
+    # reach, in stretches of 4,096 entries; its last entry is reached late or never
+    tail = 6
+    n = length + tail + 2
+    hub = n - 1
+    chain = length + np.arange(tail + 1)  # vertices after the list's own
+    src = np.concatenate([np.arange(length), chain[:-1], [chain[-1]]])
+    dst = np.concatenate([np.full(length, hub), chain[1:], [hub]])
+    g = lgbc.SimpleDiGraph.from_edge_arrays(n, src, dst)
+    bfs(g, [int(chain[0])], tuning)       # the hub's last entry, six levels on
+    bfs(g, [length - 1], tuning)          # the last of the list itself
+    g = lgbc.SimpleDiGraph.from_edge_arrays(n, src[:-1], dst[:-1])
+    bfs(g, [int(chain[0])], tuning)       # never
