@@ -9,7 +9,7 @@
 // is instruction issue: 64 % of the issue slots busy with 32 warps per SM
 // (ALU pipe 52 %), the rest barriers and fixed latencies; DRAM is idle.
 // Measured (exact betweenness, batches -> here): G(10,000, 50,000) 11.7 ->
-// 4.08 ms; 24 Barabasi-Albert graphs of up to 20,000 vertices 448 -> 150 ms;
+// 4.10 ms; 24 Barabasi-Albert graphs of up to 20,000 vertices 448 -> 150 ms;
 // a 50-vertex digraph 289 -> 36 us.
 //
 // Replaces, per source, dijkstra_shortest_paths(g, s; allpaths, trackvertices)
@@ -38,8 +38,8 @@
 //   path count, bits 31 = 0     being counted (the level after the frontier)
 //   path count, bit 31          counted; the forward sweep leaves it alone
 //   psi, bit 30 = level & 1     finished by the backward sweep
-// psi lies in (2^-48, 2^15], so 6 bits of exponent (bits 29..24 of hi) leave
-// 56 for the significand: 3 more than binary64.  A vertex of level L has
+// psi lies in (2^-48, 2^15], so 6 bits of exponent (the low ones of lo) leave
+// 56 for the significand: 3 more than binary64 (psi_pack in xf64.cuh).  A vertex of level L has
 // successors only at level L + 1, and every other neighbour is a path count
 // still or finished with the other parity while level L is swept, so the two
 // top bits of hi decide in both sweeps and no level is stored per vertex.
@@ -198,13 +198,6 @@ __device__ __forceinline__ uint32_t shared_at(const void* p) {
 }
 
 // ---- Brandes: path counts, then psi, in two words per vertex ---------------
-// psi = M 2^(b - 103) with M in [2^55, 2^56), b the 6-bit exponent; a sum is
-// m 2^(e - 103) and takes up to 255 terms before m must be brought below 2^56
-// again.  Each add truncates less than 2^-55 of the largest term so far.
-struct PsiSum {
-  uint64_t m;
-  int32_t e;
-};
 // Reciprocals of the path counts below this come from a table in shared
 // memory (most are a handful; the rest are computed).
 constexpr int kRecipTable = 512;
@@ -314,25 +307,10 @@ struct BrandesState {
           "@p ld.shared.u32 %1, [%3];\n\t}"
           : "+r"(h[k]), "=&r"(l[k]) : "r"(parity), "r"(lo_s + at[k]));
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int b = static_cast<int>(h[k] >> 24);
-      const uint64_t M = (static_cast<uint64_t>(h[k] & 0xFFFFFFu) << 32) | l[k];
-      const int E = a.e > b ? a.e : b;
-      a.m = xf_shr(a.m, static_cast<uint32_t>(E - a.e)) + xf_shr(M, static_cast<uint32_t>(E - b));
-      a.e = E;
-    }
+    for (int k = 0; k < 4; ++k) psi_add(a, l[k], h[k], (k & 1) != 0);
   }
-  static __device__ __forceinline__ void after32(Sum& a) {
-    const int sh = max(0, 8 - xf_clz(a.m));
-    a.m >>= sh;
-    a.e += sh;
-  }
-  static __device__ __forceinline__ Value value(Sum a) {
-    if (a.m == 0) return xf_zero();
-    after32(a);
-    const int lz = xf_clz(a.m);  // at least 8
-    return xf64{a.m << (lz - 1), a.e + 983 - lz};
-  }
+  static __device__ __forceinline__ void after32(Sum& a) { psi_norm(a); }
+  static __device__ __forceinline__ Value value(Sum a) { return psi_value(a); }
   static __device__ __forceinline__ Value none() { return xf_zero(); }
   static __device__ __forceinline__ Value warp_sum(Value x) { return warp_sum_x(x); }
   __device__ __forceinline__ Early early(int v) const { return part[v]; }
@@ -348,12 +326,9 @@ struct BrandesState {
       r = xf_recip_u64(s);
     }
     const xf64 psi = xf_add(acc, r);
-    uint64_t M = (psi.m + 63u + ((psi.m >> 7) & 1u)) >> 7;  // to 56 bits, ties to even
-    const uint32_t up = static_cast<uint32_t>(M >> 56);
-    M >>= up;
-    lo[v] = static_cast<uint32_t>(M);
-    hi[v] = static_cast<uint32_t>(M >> 32) | static_cast<uint32_t>(psi.e - 975 + static_cast<int>(up)) << 24 |
-            static_cast<uint32_t>(L & 1) << 30;
+    const uint64_t word = psi_pack(psi);
+    lo[v] = static_cast<uint32_t>(word);
+    hi[v] = static_cast<uint32_t>(word >> 32) | static_cast<uint32_t>(L & 1) << 30;
     if (acc.m == 0) return;
     xf64 d;
     if (shi == 0u) {  // 63 x 32 bits

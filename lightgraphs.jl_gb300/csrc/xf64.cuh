@@ -279,6 +279,56 @@ __host__ __device__ __forceinline__ xf64 xg_packed_sum(xg64 a) {
 // The extended value of a normalised gather accumulator.
 __host__ __device__ __forceinline__ xf64 xg_to_xf(xg64 a) { return xf64{a.m << 5, a.e}; }
 
+// ---- psi in two words ----------------------------------------------------------
+// The psi of the shared-memory sweeps, which lies in (2^-48, 2^15]:
+//
+//   w = (56-bit significand, bit 61 set) | (6-bit exponent b),   psi = (w & ~63) 2^(b - 109),
+//
+// so that the two top bits are free.  The word nearest to a value is within
+// 2^-56 of it, against binary64's 2^-53.  A sum is m 2^(e - 105): a term enters
+// with m in [2^57, 2^58), as in the gathers above, and 32 of them fit before
+// psi_norm.  Each add drops what lies below the 58 bits, half a unit on average:
+// with `up` (every other term) a whole one is added, so that long rows are not
+// biased, but not for terms of 30 bits or fewer, which lose nothing (many
+// vertices have psi = 1).  Rows of 64 random terms: -2e-16 from the plain sum
+// of 56-bit terms, 6e-18 with both.
+struct PsiSum {
+  uint64_t m;
+  int32_t e;
+};
+
+__host__ __device__ __forceinline__ uint64_t psi_pack(xf64 x) {
+  const uint64_t r = x.m + 63u + ((x.m >> 7) & 1u);  // to 56 bits, ties to even
+  const uint32_t up = static_cast<uint32_t>(r >> 63);
+  return ((r & ~127ull) >> (1u + up)) | static_cast<uint32_t>(x.e - 975 + static_cast<int>(up));
+}
+
+// a += the term of the words lo and hi (the top bits clear; both zero: nothing).
+__host__ __device__ __forceinline__ void psi_add(PsiSum& a, uint32_t lo, uint32_t hi, bool up) {
+  const int b = static_cast<int>(lo & 63u);
+  const uint32_t low = lo & ~63u;
+  const uint64_t w = (static_cast<uint64_t>(hi) << 32) | low;
+  const int E = a.e > b ? a.e : b;
+  a.m = xf_shr(a.m, static_cast<uint32_t>(E - a.e)) + xf_shr(w, static_cast<uint32_t>(E + 4 - b)) +
+        (up ? (low < 1u ? low : 1u) : 0u);
+  a.e = E;
+}
+
+// m below 2^58 again.
+__host__ __device__ __forceinline__ void psi_norm(PsiSum& a) {
+  const int top = 6 - xf_clz(a.m);
+  const int sh = top > 0 ? top : 0;
+  a.m >>= sh;
+  a.e += sh;
+}
+
+__host__ __device__ __forceinline__ xf64 psi_value(PsiSum a) {
+  if (a.m == 0) return xf_zero();
+  psi_norm(a);
+  const int lz = xf_clz(a.m);  // at least 6
+  return xf64{a.m << (lz - 1), a.e + 981 - lz};
+}
+
 #ifdef __CUDACC__
 // Sum over the warp (zeros allowed): every value is aligned to the largest
 // exponent and the 63-bit significands are added exactly as four 16-bit
