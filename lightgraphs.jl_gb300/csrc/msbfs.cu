@@ -303,7 +303,8 @@ template <class T, class A> __device__ __forceinline__ void acc_row(A& acc, T x)
 template <> __device__ __forceinline__ void acc_row(unsigned long long& acc, unsigned long long x) { acc += x; }
 // FP64 dependencies: psi rows hold 64-bit words in the format that the gather
 // accumulator adds at least cost (xg_pack; as binary64 bits, unpacked at each
-// add, R-MAT 20 from 4,096 sources took 155.3 ms instead of 150.0).  In a
+// add, R-MAT 20 from 4,096 sources took 155.3 ms instead of 150.0, 151.2 since
+// terms of few bits are told from the others).  In a
 // two-word batch the first of every four slots (lanes 0 .. 31 of 128) holds
 // binary64 and adds on the FP64 pipe instead (its running sum's bits kept in
 // m) while the others add on the integer pipes: the two units work in
@@ -340,12 +341,12 @@ template <int W, class A> __device__ __forceinline__ void make_room(A (&a)[2 * W
 template <int W> __device__ __forceinline__ xf64 gather_value(XgAcc a, int k) {
   if (k < kFp64Slots<W>) return xf_from_bits(a.m);
   xg_norm(a);
-  return xg_packed_sum(a);
+  return xg_packed_sum(a, kXgPsiBias);
 }
 
 // The word of an extended psi that goes to slot k of a row.
 template <int W> __device__ __forceinline__ unsigned long long psi_word(xf64 x, int k) {
-  return k < kFp64Slots<W> ? xf_to_bits(x) : xg_pack(x);
+  return k < kFp64Slots<W> ? xf_to_bits(x) : xg_pack(x, kXgPsiBias);
 }
 template <> __device__ __forceinline__ void acc_row(double& acc, double x) { acc += x; }
 template <> __device__ __forceinline__ void acc_row(df32& acc, float2 x) { acc_add(acc, x.x, x.y); }

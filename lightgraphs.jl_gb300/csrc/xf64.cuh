@@ -250,30 +250,37 @@ __host__ __device__ __forceinline__ void xg_norm(xg64& a) {
 // The terms of the gathers as 64-bit words that enter the accumulator without
 // unpacking: w 2^(b - 186), where b = the low byte of w and the whole word is
 // the significand (top bit set, or just below it).  The word nearest to a value is
-// within 2^-56 of it, against binary64's 2^-53.  psi = (1 + delta) / sigma lies
-// in [2^-64, 2^32), so b stays in [59, 156].  An accumulator of packed terms
-// holds exponents less kXgPackBias.
+// within 2^-56 of it, against binary64's 2^-53.  `bias` sets where b = 0 lies
+// (186 stands for a bias of 900).  psi = (1 + delta) / sigma lies in
+// (2^-64, 2^31], so with kXgPsiBias b stays in [29, 124]: below 128, so that the
+// word of a value of few bits, psi = 1 of a leaf or a whole number in a tree,
+// lies just above it and the shift drops the rest.  An accumulator of packed
+// terms holds exponents less the bias.
 constexpr int kXgPackBias = 900;
+constexpr int kXgPsiBias = 930;
 
-__host__ __device__ __forceinline__ uint64_t xg_pack(xf64 x) {
-  const uint32_t b = static_cast<uint32_t>(x.e - kXgPackBias);
+__host__ __device__ __forceinline__ uint64_t xg_pack(xf64 x, int bias = kXgPackBias) {
+  const uint32_t b = static_cast<uint32_t>(x.e - bias);
   const uint64_t s = (x.m << 1) - b;
   const uint64_t r = s + 128u;
   return ((r < s ? s : r) & ~255ull) | b;  // no carry out of the top: truncated there
 }
 
 // a += the packed term w.  The shifts drop half a unit on average: with `up`
-// (every other term) a whole one is added, so that long sums are not biased.
+// (every other term) a whole one is added, so that long sums are not biased,
+// but not for terms of 32 bits or fewer, which lose nothing.
 __host__ __device__ __forceinline__ void xg_add_packed(xg64& a, uint64_t w, uint32_t up) {
-  const int ex = static_cast<int>(static_cast<uint32_t>(w) & 255u);
+  const uint32_t lo = static_cast<uint32_t>(w), rest = lo >> 8;
+  const int ex = static_cast<int>(lo & 255u);
   const int E = a.e > ex ? a.e : ex;
-  a.m = xg_shr(a.m, static_cast<uint32_t>(E - a.e)) + xg_shr(w, static_cast<uint32_t>(E + 6 - ex)) + up;
+  a.m = xg_shr(a.m, static_cast<uint32_t>(E - a.e)) + xg_shr(w, static_cast<uint32_t>(E + 6 - ex)) +
+        (up ? (rest < 1u ? rest : 1u) : 0u);
   a.e = E;
 }
 
 // The extended value of a normalised accumulator of packed terms.
-__host__ __device__ __forceinline__ xf64 xg_packed_sum(xg64 a) {
-  return xf64{a.m << 5, a.m ? a.e + kXgPackBias : 0};
+__host__ __device__ __forceinline__ xf64 xg_packed_sum(xg64 a, int bias = kXgPackBias) {
+  return xf64{a.m << 5, a.m ? a.e + bias : 0};
 }
 
 // The extended value of a normalised gather accumulator.
