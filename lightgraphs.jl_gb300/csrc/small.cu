@@ -63,12 +63,85 @@ constexpr uint32_t kCountLimitHi = 1u << 16;
 // ---------------------------------------------------------------------------
 // Plan: one block per graph, then all for the columns.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) k_small_plan(const SmallGraph* graphs) {
+
+// One stable pass of a radix sort of n < 2^16 vertex ids by digit(v) in [0, 256),
+// by a block of 1,024 threads: warp w takes the w-th of 32 equal stretches of
+// `from` (null: the ids in order), counts its digits and then places its ids
+// behind those of the warps before it.
+constexpr int kPlanWarps = 32;
+template <class D>
+__device__ __forceinline__ void sort_pass(int n, const int32_t* from, int32_t* to, D digit,
+                                          uint16_t (*counts)[256]) {
+  __shared__ int digit_base[256];
+  constexpr int kAhead = 4;
+  const int ln = lane_id(), w = threadIdx.x >> 5;
+  const int turns = (n + kPlanWarps * kWarp - 1) / (kPlanWarps * kWarp);
+  const int i0 = w * turns * kWarp, i1 = min(n, i0 + turns * kWarp);
+  auto walk = [&](auto put) {  // put(id, digit, the lanes of that digit), warp-uniformly
+    for (int i = i0; i < i1; i += kAhead * kWarp) {
+      int v[kAhead], d[kAhead];
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        const int at = i + q * kWarp + ln;
+        v[q] = at < i1 ? (from ? from[at] : at) : -1;
+      }
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) d[q] = v[q] >= 0 ? digit(v[q]) : -1;
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        put(v[q], d[q], __match_any_sync(kFull, d[q]));
+        __syncwarp();
+      }
+    }
+  };
+  for (int k = threadIdx.x; k < kPlanWarps * 256; k += blockDim.x) counts[k >> 8][k & 255] = 0;
+  __syncthreads();
+  walk([&](int, int d, unsigned peers) {
+    if (d >= 0 && ln == __ffs(peers) - 1) counts[w][d] = static_cast<uint16_t>(counts[w][d] + __popc(peers));
+  });
+  __syncthreads();
+  int total = 0;
+  if (threadIdx.x < 256)
+    for (int k = 0; k < kPlanWarps; ++k) {
+      const int c = counts[k][threadIdx.x];
+      counts[k][threadIdx.x] = static_cast<uint16_t>(total);
+      total += c;
+    }
+  int incl = total;
+#pragma unroll
+  for (int o = 1; o < kWarp; o <<= 1) {
+    const int y = __shfl_up_sync(kFull, incl, o);
+    if (ln >= o) incl += y;
+  }
+  if (threadIdx.x < 256) digit_base[threadIdx.x] = incl;  // within its 32 digits
+  __syncthreads();
+  int before = 0;
+  if (threadIdx.x < 256)
+    for (int k = 0; k < w; ++k) before += digit_base[32 * k + 31];
+  __syncthreads();
+  if (threadIdx.x < 256) digit_base[threadIdx.x] = before + incl - total;
+  __syncthreads();
+  walk([&](int v, int d, unsigned peers) {
+    const int lead = __ffs(peers) - 1;
+    int at = 0;
+    if (d >= 0 && ln == lead) {
+      at = counts[w][d];
+      counts[w][d] = static_cast<uint16_t>(at + __popc(peers));
+    }
+    at = __shfl_sync(kFull, at, lead);
+    if (d >= 0) to[digit_base[d] + at + __popc(peers & ((1u << ln) - 1u))] = v;
+  });
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(kPlanWarps* kWarp) k_small_plan(const SmallGraph* graphs) {
   extern __shared__ int hist[];  // vertices per row length (in groups), then their first rank
+  __shared__ uint16_t counts[kPlanWarps][256];
+  __shared__ int total_groups, longest;
   const SmallGraph G = graphs[blockIdx.x];
   const int n = G.n;
   const int bins = (n + 3) / 4 + 1;
-  int* first = hist;             // [bins] rank of the next vertex of the bin
+  int* first = hist;             // [bins] vertices of the bin
   int* start = hist + bins;      // [bins] first rank of the bin
   int* base = hist + 2 * bins;   // [bins] first group of the bin
   for (int b = threadIdx.x; b < bins; b += blockDim.x) first[b] = 0;
@@ -79,10 +152,11 @@ __global__ void __launch_bounds__(1024) k_small_plan(const SmallGraph* graphs) {
   // longest rows first: a warp scans the bins downwards
   if (threadIdx.x < kWarp) {
     const int ln = lane_id();
-    int rank = 0, grp = 0;
+    int rank = 0, grp = 0, most = 0;
     for (int top = bins - 1; top >= 0; top -= kWarp) {
       const int b = top - ln;
       const int c = b >= 0 ? first[b] : 0;
+      if (c > 0) most = max(most, b);
       int ic = c, ig = c * b;
 #pragma unroll
       for (int o = 1; o < kWarp; o <<= 1) {
@@ -94,22 +168,32 @@ __global__ void __launch_bounds__(1024) k_small_plan(const SmallGraph* graphs) {
       }
       if (b >= 0) {
         start[b] = rank + ic - c;
-        first[b] = rank + ic - c;
         base[b] = grp + ig - c * b;
       }
       rank += __shfl_sync(kFull, ic, kWarp - 1);
       grp += __shfl_sync(kFull, ig, kWarp - 1);
     }
-    if (ln == 0) G.row[n] = static_cast<uint32_t>(grp);
+    most = static_cast<int>(__reduce_max_sync(kFull, static_cast<unsigned>(most)));
+    if (ln == 0) {
+      total_groups = grp;
+      longest = most;
+    }
   }
   __syncthreads();
-  for (int v = threadIdx.x; v < n; v += blockDim.x) {
-    const int b = groups_of(v);
-    const int r = atomicAdd(&first[b], 1);
+  // Ranks by id within a length: with ranks as atomics come, the same graph had
+  // another plan in every call, and items (ranges of ranks) sums of other sources.
+  const int top = longest;
+  int32_t* by_low = top < 256 ? G.orig : reinterpret_cast<int32_t*>(G.row);  // rows are written below
+  sort_pass(n, nullptr, by_low, [&](int v) { return (top - groups_of(v)) & 255; }, counts);
+  if (top >= 256) sort_pass(n, by_low, G.orig, [&](int v) { return (top - groups_of(v)) >> 8; }, counts);
+  for (int r = threadIdx.x; r < n; r += blockDim.x) {
+    const int v = G.orig[r], b = groups_of(v);
     G.rank[v] = r;
-    G.orig[r] = v;
     G.row[r] = static_cast<uint32_t>(base[b] + (r - start[b]) * b);
-    if (b > kSmallWarpGroups) atomicMax(G.nwarp, r + 1);
+  }
+  if (threadIdx.x == 0) {
+    G.row[n] = static_cast<uint32_t>(total_groups);
+    *G.nwarp = bins > kSmallWarpGroups + 1 ? start[kSmallWarpGroups] : 0;
   }
   __syncthreads();  // also orders this block's global writes before the reads below
   {
@@ -141,7 +225,9 @@ __global__ void __launch_bounds__(1024) k_small_plan(const SmallGraph* graphs) {
 }
 
 // The columns of the planned rows, a warp per vertex: most of the plan's work.
-// One block's plan of 16,384 vertices took 380 us, the two kernels take 45 + 53.
+// One block's plan of 16,384 vertices took 380 us, the two kernels take 72 + 69 on
+// cold caches (52 + 69 with ranks as atomics came, 31 + 12 either way for 10,000
+// vertices of short rows, which one sort pass orders).
 __global__ void __launch_bounds__(256) k_small_columns(const SmallGraph* graphs) {
   const SmallGraph G = graphs[blockIdx.y];
   const int n = G.n;
@@ -995,7 +1081,7 @@ int small_stress_configure(size_t max_dyn_smem) { return sweep_configure<StressS
 
 int small_plan(cudaStream_t s, const SmallGraph* graphs, int count, int64_t max_n) {
   const size_t bins = static_cast<size_t>((max_n + 3) / 4 + 1);
-  k_small_plan<<<count, 1024, 3 * bins * sizeof(int), s>>>(graphs);
+  k_small_plan<<<count, kPlanWarps * kWarp, 3 * bins * sizeof(int), s>>>(graphs);
   // eight vertices a warp, and no more blocks than are resident
   const int64_t x = std::max<int64_t>(1, std::min((max_n + 63) / 64, kSmallColumnBlocks / count));
   k_small_columns<<<dim3(static_cast<unsigned>(x), static_cast<unsigned>(count)), 256, 0, s>>>(graphs);
