@@ -244,8 +244,9 @@ int lgbc_set_tuning(lgbc_graph *g, const lgbc_tuning *t);
  * (hub_degree), the source-batch width (lanes), the direction-switch
  * thresholds (alpha, beta), the gather cuts (dense_edges, segment_degree) and
  * the hub item order (hub_order); the result stays set on the handle (read
- * it with lgbc_get_tuning).  Every setting gives the same results; only the
- * speed differs.  cache_path (may be NULL) is a text file of "signature alpha
+ * it with lgbc_get_tuning).  On a small graph the defaults are measured by the
+ * per-source kernel that they select, and stay unless batches beat it.  Every
+ * setting gives the same results; only the speed differs.  cache_path (may be NULL) is a text file of "signature alpha
  * beta hub_degree lanes dense_edges segment_degree source_order graph_loop
  * stack_vertices hub_order" lines, keyed by n, nnz, directedness and the device's SM
  * count: a matching line is applied without measuring, and a new result is

@@ -1113,8 +1113,6 @@ int ensure_small_counters(lgbc_graph* g) {
   return LGBC_OK;
 }
 
-// Brandes over the k sources at src (device or pinned memory) by the
-// per-source kernel into out (likewise); waits for the stream; 1 when it refuses.
 int run_small(lgbc_graph* g, const int32_t* src, int64_t k, double* out, const double* d_w) {
   SmallWorkspace& w = g->small;
   LGBC_TRY(ensure_plan(g, &w.out, g->d_rowptr, g->d_colidx, g->d_in_rowptr));

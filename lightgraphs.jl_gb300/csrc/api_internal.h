@@ -415,6 +415,12 @@ int finish_handle(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr
 // (run: everything but the graph).
 bool small_bfs_applies(const lgbc_graph* g, int64_t nsrc);
 int run_small_bfs(lgbc_graph* g, SmallBfs run);
+// Whether the per-source kernel takes Brandes calls of this handle, and such a
+// call: the k sources at src (device or pinned memory) into out (likewise); it
+// waits for the stream and returns 1 when it refuses.
+bool same_tuning(const lgbc_tuning& a, const lgbc_tuning& b);
+bool small_applies(const lgbc_graph* g);
+int run_small(lgbc_graph* g, const int32_t* src, int64_t k, double* out, const double* d_w);
 // Stress over g->h_active into d_stress (zeroed by the caller) by the
 // per-source kernel: 1 when it does not take the graph (d_stress zero again).
 int run_small_stress(lgbc_graph* g, unsigned long long* d_stress);

@@ -45,15 +45,23 @@ bool tune_from_cache(const char* path, const std::string& sig, lgbc_tuning* out)
 }
 
 // Milliseconds of one Brandes pass over the k sources already in d_src with
-// tuning t (best of `reps`, after one unmeasured pass).
+// tuning t (best of `reps`, after one unmeasured pass), by the path that a call
+// with t takes: the per-source kernel for the defaults on a small graph.
 int tune_measure(lgbc_graph* g, const lgbc_tuning& t, int64_t k, double* bc_dev, int reps,
                  double* ms_out) {
   g->tune = t;
   LGBC_TRY(ensure_hubs(g));
+  bool small = small_applies(g);
   double best = 1e300;
   for (int r = 0; r <= reps; ++r) {
     LGBC_CUDA(cudaEventRecord(g->ev_start, g->stream));
-    LGBC_TRY(run_betweenness(g, k, 0, bc_dev));
+    int rc = small ? run_small(g, g->d_src, k, bc_dev, nullptr) : run_betweenness(g, k, 0, bc_dev);
+    if (rc == 1) {  // refused: such sources run as batches
+      small = false;
+      r = -1;
+      continue;
+    }
+    LGBC_TRY(rc);
     LGBC_CUDA(cudaEventRecord(g->ev_stop, g->stream));
     LGBC_CUDA(cudaEventSynchronize(g->ev_stop));
     float ms = 0.f;
@@ -99,8 +107,23 @@ extern "C" int lgbc_tune(lgbc_graph* g, const char* cache_path) {
   // direction-switch thresholds and the two gather-strategy cuts
   lgbc_tuning best = g->tune;
   double best_ms = 0.0;
-  LGBC_TRY(tune_measure(g, best, k, g->d_bc, 2, &best_ms));
   const int reps = 2;
+  LGBC_TRY(tune_measure(g, best, k, g->d_bc, reps, &best_ms));
+  // any other setting asks for batches: the defaults come first where they
+  // mean the per-source kernel
+  lgbc_tuning defaults = kDefaultTuning;
+  defaults.dependency_df32 = best.dependency_df32;
+  if (!same_tuning(best, defaults)) {
+    g->tune = defaults;
+    if (small_applies(g)) {
+      double ms = 0.0;
+      LGBC_TRY(tune_measure(g, defaults, k, g->d_bc, reps, &ms));
+      if (ms < best_ms * 0.98) {
+        best = defaults;
+        best_ms = ms;
+      }
+    }
+  }
   for (int pass = 0; pass < 2; ++pass) {
     auto try_field = [&](auto setter, const auto& values) -> int {
       for (const auto& val : values) {

@@ -71,3 +71,24 @@ def test_tuning_validation():
     h.set_tuning(lanes=7, source_order=0, graph_loop=0, stack_vertices=0)
     t = h.tuning()
     assert (t.lanes, t.source_order, t.graph_loop, t.stack_vertices) == (7, 0, 0, 0)
+
+
+@pytest.mark.parametrize("start", [{}, dict(hub_degree=64, alpha=8.0)])
+def test_tune_keeps_the_per_source_kernel_of_small_graphs(tmp_path, start):
+    # the defaults mean one thread block per source there, 2.5 times as fast as
+    # the best batches; a setting that turns it off has to win against it
+    g = gen.erdos_renyi_nm(10000, 50000, seed=4)
+    h = g.device_handle()
+    defaults = {n: getattr(h.tuning(), n) for n, _ in h.tuning()._fields_}
+    h.set_tuning(**start)
+    cache = tmp_path / "tune.txt"
+    h.tune(cache)
+    t = h.tuning()
+    assert {n: getattr(t, n) for n in defaults} == defaults
+    lgbc.betweenness_centrality(g, [1, 2, 3])
+    assert h.stats()["levels"] == 0  # no batch ran
+    h2 = lgbc.DeviceGraph(g)
+    h2.tune(cache)
+    t = h2.tuning()
+    assert {n: getattr(t, n) for n in defaults} == defaults
+    h2.close()
