@@ -1050,7 +1050,7 @@ bool small_graph(const lgbc_graph* g) {
 
 // The vertex state of one source must fit an SM's shared memory.
 bool small_applies(const lgbc_graph* g) {
-  return small_graph(g) && g->n <= g->small_max_n && !g->small.refused;
+  return small_graph(g) && g->n <= g->small_max_n && !g->small.deep.given_up();
 }
 
 // A block walks every unfinished vertex's edges once a level: with 64 sources
@@ -1108,8 +1108,23 @@ int run_small_bfs(lgbc_graph* g, SmallBfs run) {
 int ensure_small_counters(lgbc_graph* g) {
   SmallWorkspace& w = g->small;
   if (w.counters) return LGBC_OK;
-  LGBC_TRY(dev_alloc(&w.counters, 4));
-  LGBC_CUDA(cudaMemsetAsync(w.counters, 0, 4 * sizeof(int), g->stream));
+  const size_t ints = 4 + (2 * static_cast<size_t>(g->n) + 3) / 4;
+  LGBC_TRY(dev_alloc(&w.counters, ints));
+  LGBC_CUDA(cudaMemsetAsync(w.counters, 0, ints * sizeof(int), g->stream));
+  return LGBC_OK;
+}
+
+uint8_t* small_deep(lgbc_graph* g, bool stress) {
+  return reinterpret_cast<uint8_t*>(g->small.counters + 4) + (stress ? g->n : 0);
+}
+
+// The sources that the kernel refused in the call that has just ended.
+int learn_deep(lgbc_graph* g, bool stress) {
+  DeepSources& d = stress ? g->small.stress_deep : g->small.deep;
+  d.known.resize(static_cast<size_t>(g->n));
+  LGBC_CUDA(cudaMemcpyAsync(d.known.data(), small_deep(g, stress), d.known.size(), cudaMemcpyDeviceToHost, g->stream));
+  LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  d.count = std::count_if(d.known.begin(), d.known.end(), [](uint8_t x) { return x != 0; });
   return LGBC_OK;
 }
 
@@ -1137,6 +1152,7 @@ int run_small(lgbc_graph* g, const int32_t* src, int64_t k, double* out, const d
   run.nsrc = static_cast<int>(k);
   run.next = w.counters;
   run.refused = w.counters + 1;
+  run.deep = small_deep(g, false);
   run.src = src;
   run.weight = d_w;
   run.part = w.part;
@@ -1150,9 +1166,10 @@ int run_small(lgbc_graph* g, const int32_t* src, int64_t k, double* out, const d
   }
   LGBC_CUDA(cudaStreamSynchronize(g->stream));
   if (*refused) {
-    w.refused = true;
+    LGBC_TRY(learn_deep(g, false));
     return 1;
   }
+  w.deep.taken += k;
   g->stats.batches += items;
   return LGBC_OK;
 }
@@ -1160,7 +1177,9 @@ int run_small(lgbc_graph* g, const int32_t* src, int64_t k, double* out, const d
 int run_small_stress(lgbc_graph* g, unsigned long long* d_stress) {
   SmallWorkspace& w = g->small;
   const int64_t k = static_cast<int64_t>(g->h_active.size());
-  if (k == 0 || !small_graph(g) || g->n > g->small_stress_max_n || w.stress_refused) return 1;
+  if (k == 0 || !small_graph(g) || g->n > g->small_stress_max_n || w.stress_deep.given_up() ||
+      w.stress_deep.among(g->h_active))
+    return 1;
   LGBC_TRY(upload_sources(g));
   LGBC_TRY(ensure_plan(g, &w.out, g->d_rowptr, g->d_colidx, g->d_in_rowptr));
   LGBC_TRY(ensure_small_counters(g));
@@ -1171,6 +1190,7 @@ int run_small_stress(lgbc_graph* g, unsigned long long* d_stress) {
   run.nsrc = static_cast<int>(k);
   run.next = w.counters + 2;
   run.refused = w.counters + 3;
+  run.deep = small_deep(g, true);
   run.src = g->d_src;
   run.stress = d_stress;
   LGBC_CUDA(cudaMemsetAsync(w.counters + 2, 0, 2 * sizeof(int), g->stream));
@@ -1180,10 +1200,11 @@ int run_small_stress(lgbc_graph* g, unsigned long long* d_stress) {
   LGBC_CUDA(cudaMemcpyAsync(refused, w.counters + 3, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
   LGBC_CUDA(cudaStreamSynchronize(g->stream));
   if (!*refused) {
+    w.stress_deep.taken += k;
     g->stats.batches += run.nitems;
     return LGBC_OK;
   }
-  w.stress_refused = true;
+  LGBC_TRY(learn_deep(g, true));
   LGBC_CUDA(cudaMemsetAsync(d_stress, 0, static_cast<size_t>(g->n) * 8, g->stream));
   return 1;
 }
@@ -1212,7 +1233,7 @@ int accumulate_active(lgbc_graph* g, int endpoints, double* bc_dev, double* host
     LGBC_CUDA(cudaStreamSynchronize(g->stream));
     return LGBC_OK;
   };
-  if (k > 0 && small_applies(g)) {
+  if (k > 0 && small_applies(g) && !g->small.deep.among(g->h_active)) {
     // A call of few sources and a short result moves both through pinned
     // memory that the kernels read and write themselves: two launches and one
     // wait (a 50-vertex graph 56 us with four copies and two waits, 35 us so).

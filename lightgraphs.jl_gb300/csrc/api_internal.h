@@ -212,16 +212,32 @@ struct SmallPlan {
   }
 };
 
+// Sources that a per-source kernel has refused (too deep, or counts too large):
+// a call that has one runs as batches, without another attempt.  Where most
+// sources are refused, all calls do.
+struct DeepSources {
+  std::vector<uint8_t> known;       // empty: none yet
+  int64_t count = 0, taken = 0;     // refused sources; sources of the calls taken
+  bool given_up() const { return count >= 32 && 16 * count > taken; }
+  bool among(const std::vector<int32_t>& src) const {
+    if (count == 0) return false;
+    for (int32_t v : src)
+      if (known[static_cast<size_t>(v)]) return true;
+    return false;
+  }
+};
+
 // Plans and workspace of the shared-memory kernels for small graphs.
 struct SmallWorkspace {
   SmallPlan out, in;                // in: digraphs only
   SmallSum* sum = nullptr;
   int64_t items = 0;                // parts of a call that *sum was written for
-  int* counters = nullptr;          // [0] next item, [1] refused (zero between calls); [2, 3] for stress
+  // [0] next item, [1] refused (zero between calls); [2, 3] for stress; then
+  // the refused sources of both, n bytes each (zero at first)
+  int* counters = nullptr;
   ulonglong2* part = nullptr;       // partial sums, one n-vector per item
   int64_t part_cap = 0;
-  bool refused = false;             // too deep or counts too large: the batches take this graph
-  bool stress_refused = false;      // too deep, in a stress call
+  DeepSources deep, stress_deep;
   void release() {
     out.release();
     in.release();

@@ -214,6 +214,7 @@ struct SmallRun {
   int nsrc;
   int* next;               // zero: the next item
   int* refused;            // per graph, zero: set when a source is too deep or its counts too large
+  uint8_t* deep;           // n, or null: set at such a source (its own id)
   const int32_t* src;      // sources as the graph's own ids, or null
   const double* weight;    // weights of the sources in src, or null
   ulonglong2* part;        // extended-format sums (xf64.cuh): significand, exponent

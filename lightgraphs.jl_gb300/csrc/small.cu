@@ -532,7 +532,8 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
   extern __shared__ uint32_t sm[];
   __shared__ int lvl[2][kSmallMaxLevels + 2];  // level starts: [0] warp-walked vertices, [1] the others
   __shared__ int s_count[kWarp];
-  __shared__ int s_item, s_stop, s_goal;
+  __shared__ int s_item, s_goal, s_own;
+  __shared__ int s_stop;                       // 1: the graph was refused or a count is too large, 2: refused here
   __shared__ int s_next[2];                    // [L & 1]: next entry of level L's second list
   __shared__ int s_wide[2];                    // [L & 1]: a count of level L is 2^16 or more
   const int tid = threadIdx.x, T = blockDim.x, ln = lane_id(), wid = tid >> 5, W = T >> 5;
@@ -620,6 +621,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
         st.seed(s);
         const int k = s < nw ? 0 : 1;
         const int own = G.orig[s];
+        s_own = own;
         s_goal = *G.nlive + (G.in_rowptr[own + 1] == G.in_rowptr[own] ? 1 : 0);
         q[k ? nw : 0] = static_cast<uint16_t>(s);
         lvl[0][0] = lvl[1][0] = 0;
@@ -668,10 +670,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
           ++L;
           __syncthreads();  // L is even across the block; s_count is read
           if (L + 1 > kSmallMaxLevels) {
-            if (tid == 0) {
-              s_stop = 1;
-              run.refused[I.graph] = 1;
-            }
+            if (tid == 0) s_stop = 2;
             L = 0;
             break;
           }
@@ -728,10 +727,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
         if (L + 2 > kSmallMaxLevels || s_stop) {
           // the batches take the graph: leave the item
           __syncthreads();  // every thread has read s_stop
-          if (tid == 0) {
-            s_stop = 1;
-            run.refused[I.graph] = 1;
-          }
+          if (tid == 0) s_stop = 2;
           L = 0;
           break;
         }
@@ -807,6 +803,10 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
         __syncthreads();
       }
       __syncthreads();
+    }
+    if (tid == 0 && s_stop == 2) {  // refused at the last source begun
+      run.refused[I.graph] = 1;
+      if (run.deep) run.deep[s_own] = 1;
     }
   }
 }

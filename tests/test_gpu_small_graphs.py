@@ -192,3 +192,53 @@ def test_results_and_sources_at_the_sizes_of_the_pinned_areas(n, k):
     want = oracle.gdistances(rp, ci, src.astype(np.int32)).astype(np.int64)
     want[want == oracle.UNREACHED32] = np.iinfo(g.eltype).max
     assert np.array_equal(lgbc.gdistances(g, src + 1), want)
+
+
+def deep_and_shallow():
+    """A digraph of a path of 300 and a random part: sources near the path's head
+    are deeper than a per-source search may be, all others are shallow."""
+    e = np.random.default_rng(7).integers(300, 2000, (2, 8000))
+    i = np.arange(299)
+    return lgbc.SimpleDiGraph.from_edge_arrays(2000, np.concatenate([i, e[0]]), np.concatenate([i + 1, e[1]]))
+
+
+@pytest.mark.parametrize("kind", ["betweenness", "stress"])
+def test_deep_sources_leave_the_others_as_they_are(kind):
+    g = deep_and_shallow()
+    rp, ci, kw = csr_args(g)
+    h = g.device_handle()
+    shallow = np.concatenate([np.arange(290, 299), np.arange(300, 2000, 9)])
+    deep = np.asarray([3, 100, 171])
+
+    def call(src):
+        if kind == "stress":
+            got = lgbc.stress_centrality(g, src + 1)
+            assert np.array_equal(got, oracle.stress(rp, ci, src.astype(np.int32), **kw))
+        else:
+            got = lgbc.betweenness_centrality(g, src + 1, normalize=False)
+            assert_bc_close(got, oracle_bc(g, src, normalize=False))
+        return got, h.stats()["levels"], h.stats()["kernel_launches"]
+
+    first, levels, _ = call(shallow)
+    assert levels == 0  # the per-source kernel counts none
+    attempt = call(deep)
+    assert attempt[1] > 127
+    again = call(deep)
+    assert again[2] < attempt[2]  # not tried twice
+    assert np.array_equal(again[0], attempt[0])
+    last, levels, _ = call(shallow)
+    assert levels == 0 and np.array_equal(first, last)
+    assert call(np.concatenate([shallow, deep]))[1] > 127
+
+
+def test_graphs_of_deep_sources_are_left_to_batches():
+    # one attempt, then the launches of a handle that never tries (a hub order
+    # other than the default, which a graph without hubs does not notice)
+    g, never = path(2000), path(2000)
+    never.device_handle().set_tuning(hub_order=1)
+    more = []
+    for s in (0, 5, 9):
+        for x in (g, never):
+            check(x, np.arange(s, 2000, 10))
+        more.append(g.device_handle().stats()["kernel_launches"] - never.device_handle().stats()["kernel_launches"])
+    assert more[0] > 0 and more[1:] == [0, 0]
