@@ -376,10 +376,15 @@ int small_chunk(const SmallMany& dev, const std::vector<ManyGraph>& gs, int endp
     if (flags[k] & 1) return fail(LGBC_EINVAL, "rowptr must be non-decreasing");
     if (flags[k] & 2)
       return fail(LGBC_EINVAL, "graph " + std::to_string(gs[k].idx) + ": column index outside [0, n)");
-    if (flags[k] & 4) {  // repeated entries: the batches walk them as they are
-      for (size_t j = 0; j < gs.size(); ++j) rest.push_back(gs[j]);
-      return LGBC_OK;
-    }
+  }
+  if (std::any_of(flags.begin(), flags.end(), [](int f) { return (f & 4) != 0; })) {
+    // a row longer than n has repeated entries: the batches walk those graphs
+    // as they are, and the others start again without them
+    std::vector<ManyGraph> plain;
+    for (size_t k = 0; k < gs.size(); ++k) ((flags[k] & 4) ? rest : plain).push_back(gs[k]);
+    if (plain.empty()) return LGBC_OK;
+    g1.reset();
+    return small_chunk(dev, plain, endpoints, bc_raw_out, rest);
   }
   small_plan(s, d_graphs, count, max_n);
 

@@ -33,3 +33,15 @@ def test_handles_of_one_graph_agree_bit_for_bit(directed):
         got = lgbc.betweenness_centrality(h, src)
         assert want is None or same([got], [want])
         want = got
+
+
+def test_one_graph_with_repeated_entries_leaves_the_others_where_they_are():
+    # a row longer than n is left to the unions; the others' results are those
+    # of a call without that graph, bit for bit
+    graphs = [G.barabasi_albert(n, 3, seed=n) for n in (5000, 1200, 60)]
+    odd = lgbc.SimpleGraph.from_csr([0, 4, 7, 8], [1, 1, 1, 1, 0, 0, 2, 1])
+    want = lgbc.betweenness_centrality_many(graphs)
+    got = lgbc.betweenness_centrality_many([graphs[0], odd, graphs[1], odd, graphs[2]])
+    assert same([got[0], got[2], got[4]], want)
+    alone = lgbc.betweenness_centrality_many([odd])[0]
+    assert same([got[1], got[3]], [alone, alone])
