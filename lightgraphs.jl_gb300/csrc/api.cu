@@ -1177,7 +1177,7 @@ int run_small(lgbc_graph* g, const int32_t* src, int64_t k, double* out, const d
 int run_small_stress(lgbc_graph* g, unsigned long long* d_stress) {
   SmallWorkspace& w = g->small;
   const int64_t k = static_cast<int64_t>(g->h_active.size());
-  if (k == 0 || !small_graph(g) || g->n > g->small_stress_max_n || w.stress_deep.given_up() ||
+  if (k == 0 || k > INT32_MAX || !small_graph(g) || g->n > g->small_stress_max_n || w.stress_deep.given_up() ||
       w.stress_deep.among(g->h_active))
     return 1;
   LGBC_TRY(upload_sources(g));
@@ -1233,7 +1233,7 @@ int accumulate_active(lgbc_graph* g, int endpoints, double* bc_dev, double* host
     LGBC_CUDA(cudaStreamSynchronize(g->stream));
     return LGBC_OK;
   };
-  if (k > 0 && small_applies(g) && !g->small.deep.among(g->h_active)) {
+  if (k > 0 && k <= INT32_MAX && small_applies(g) && !g->small.deep.among(g->h_active)) {
     // A call of few sources and a short result moves both through pinned
     // memory that the kernels read and write themselves: two launches and one
     // wait (a 50-vertex graph 56 us with four copies and two waits, 35 us so).
@@ -1626,7 +1626,7 @@ int gdistances(lgbc_graph* g, const int32_t* src, int64_t nsrc, void* dist_out, 
   LGBC_TRY(check_sources(g, src, nsrc));
   reset_stats(g);
   if (g->n == 0) return LGBC_OK;
-  const bool small = nsrc > 0 && small_bfs_applies(g, 1) && g->nnz <= kSmallSingleNnz;
+  const bool small = nsrc > 0 && small_bfs_applies(g, nsrc) && g->nnz <= kSmallSingleNnz;
   if (small) {
     SmallBfs run{};
     run.nsrc = static_cast<int>(nsrc);
