@@ -90,6 +90,10 @@ int lgbc_gdistances64(lgbc_graph* g, const int32_t* src, int64_t nsrc,
 int lgbc_gdistances_batch(lgbc_graph *g, const int32_t *src, int64_t nsrc,
                           int32_t *dist_out /* nsrc x n */);
 
+/* The same in 64 bits, INT64_MAX where source i does not reach v. */
+int lgbc_gdistances_batch64(lgbc_graph *g, const int32_t *src, int64_t nsrc,
+                            int64_t *dist_out /* nsrc x n */);
+
 /* Path counts and distances of dijkstra_shortest_paths(g, s) with unit
  * weights (src/shortestpaths/dijkstra.jl:59-141): DijkstraState.pathcounts
  * (:10, summed at :102,118, reset to 1 at the source at :135) and .dists,

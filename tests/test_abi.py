@@ -91,3 +91,17 @@ def test_bench_bytes_model():
     assert bench.bc_algorithmic_bytes(n, nnz, k, 128) == 20 * (8 * nnz + 32 * n + 16) + 32 * n * k
     assert bench.bc_algorithmic_bytes(n, nnz, k, 128) == 91225535488
     assert bench.bc_algorithmic_bytes(n, nnz, k, 64) == 40 * (8 * nnz + 32 * n + 16) + 32 * n * k
+
+
+def test_headers_declare_every_exported_symbol():
+    import shutil
+    import subprocess
+    if shutil.which("nm") is None:
+        pytest.skip("nm not available")
+    _lib.lib()
+    path = os.path.join(ROOT, "lightgraphs.jl_gb300", "lib", "liblgbc.so")
+    out = subprocess.run(["nm", "-D", "--defined-only", path], capture_output=True, text=True, check=True).stdout
+    exported = {ln.split()[-1] for ln in out.splitlines()}
+    names = {n for n in exported if re.fullmatch(r"lgbc_[a-z0-9_]+", n)}
+    assert "lgbc_gdistances_batch64" in names
+    assert not names - set(declared_symbols())
