@@ -174,8 +174,9 @@ int lgbc_graph_stats(const lgbc_graph *g, lgbc_stats *out);
  * shape the bit-lane batches.  With every field at its default, betweenness
  * of a graph whose vertex state fits one SM's shared memory (about 22,300
  * vertices, at most 2^20 stored entries) runs one thread block per source
- * instead, unless a search is deeper than 126 levels or a path count reaches
- * 2^48; lgbc_stats.batches then counts the blocks' shares of the sources.
+ * instead, unless the call has a source that reaches a vertex at a distance of
+ * 128 or more or by 2^48 paths or more; lgbc_stats.batches then counts the
+ * blocks' shares of the sources, and no levels are counted.
  * Distances and distance statistics of such graphs (about 18,900 vertices)
  * run 32 sources per thread block in the same way.
  *   alpha, beta   direction switch: go bottom-up when the frontier's edges

@@ -179,7 +179,7 @@ int ms_reset_all(cudaStream_t s, const DevGraph& g, const MsBuffers& b);
 // ---- Brandes on graphs that fit one SM's shared memory: small.cu ----------
 constexpr int kSmallMaxN = 32000;        // 16-bit ids with one to spare; the shared memory bounds n further
 constexpr int kSmallMaxThreads = 1024;
-constexpr int kSmallMaxLevels = 128;     // a deeper search is left to the batches
+constexpr int kSmallMaxLevels = 128;     // levels 0 to 127; a deeper search is left to the batches
 constexpr int kSmallWarpGroups = 16;    // rows of more than 4 * this entries are walked by a warp
 constexpr int kSmallLenBits = 5;         // holds kSmallWarpGroups
 // One SM walks a source's edges alone: at 1.2M entries (20,000 vertices) a

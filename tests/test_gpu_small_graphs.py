@@ -242,3 +242,20 @@ def test_graphs_of_deep_sources_are_left_to_batches():
             check(x, np.arange(s, 2000, 10))
         more.append(g.device_handle().stats()["kernel_launches"] - never.device_handle().stats()["kernel_launches"])
     assert more[0] > 0 and more[1:] == [0, 0]
+
+
+@pytest.mark.parametrize("n", [127, 128, 129, 130])
+def test_where_the_depth_limit_lies(n):
+    # distances up to 127 (a call counts levels only when batches run)
+    g = path(n)
+    check(g, [0])
+    levels = g.device_handle().stats()["levels"]
+    assert levels == 0 if n <= 128 else levels >= 128
+
+
+@pytest.mark.parametrize("endpoints", [False, True])
+def test_many_in_the_large_size_classes(endpoints):
+    # one call's launches for graphs of 8,193 to 11,000 and of more vertices
+    graphs = [G.barabasi_albert(n, 2, seed=n) for n in (8200, 10900, 11100, 12500)]
+    for g, z in zip(graphs, lgbc.betweenness_centrality_many(graphs, normalize=False, endpoints=endpoints)):
+        assert_bc_close(z, oracle_bc(g, normalize=False, endpoints=endpoints, nthreads=16))
