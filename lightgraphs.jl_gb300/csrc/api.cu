@@ -182,11 +182,13 @@ void make_items(const int64_t* rowptr, const int32_t* colidx, int64_t n, int H, 
   items.swap(sorted);
 }
 
-int upload_items(const std::vector<HubItem>& items, HubItem** out) {
+// (In order with the kernels of g's stream: a plain cudaMemcpy returns when the
+// items are staged, and a non-blocking stream does not wait for the rest.)
+int upload_items(lgbc_graph* g, const std::vector<HubItem>& items, HubItem** out) {
   *out = nullptr;
   if (items.empty()) return LGBC_OK;
   LGBC_TRY(dev_alloc(out, items.size()));
-  LGBC_CUDA(cudaMemcpy(*out, items.data(), items.size() * sizeof(HubItem), cudaMemcpyHostToDevice));
+  LGBC_CUDA(cudaMemcpyAsync(*out, items.data(), items.size() * sizeof(HubItem), cudaMemcpyHostToDevice, g->stream));
   return LGBC_OK;
 }
 
@@ -248,11 +250,11 @@ int build_hubs(lgbc_graph* g, const int64_t* rowptr, const int32_t* colidx, cons
   std::vector<HubItem> items;
   make_items(rowptr, colidx, n, H, order, slot_of, items);
   g->hubs.n_out = static_cast<int64_t>(items.size());
-  LGBC_TRY(upload_items(items, &g->hubs.out_items));
+  LGBC_TRY(upload_items(g, items, &g->hubs.out_items));
   if (g->directed) {
     make_items(in_rowptr, in_colidx, n, H, order, slot_of, items);
     g->hubs.n_in = static_cast<int64_t>(items.size());
-    LGBC_TRY(upload_items(items, &g->hubs.in_items));
+    LGBC_TRY(upload_items(g, items, &g->hubs.in_items));
   } else {
     g->hubs.in_items = g->hubs.out_items;
     g->hubs.n_in = g->hubs.n_out;
@@ -806,7 +808,8 @@ int create_replicated(lgbc_graph* g, int64_t copies, lgbc_graph** out) {
     const int64_t n = g->n, nnz = g->nnz, N = copies * n, NNZ = copies * nnz;
     LGBC_TRY(init_handle(st, N, g->directed));
     st->nnz = NNZ;
-    LGBC_CUDA(cudaStreamSynchronize(g->stream));  // g's CSR is complete
+    LGBC_TRY(ensure_hubs(g));
+    LGBC_CUDA(cudaStreamSynchronize(g->stream));  // g's CSR and hub items are complete
     LGBC_TRY(dev_alloc(&st->d_rowptr, static_cast<size_t>(N + 1)));
     LGBC_TRY(dev_alloc(&st->d_colidx, static_cast<size_t>(std::max<int64_t>(NNZ, 1))));
     st->launches += replicate_csr(st->cfg, st->stream, g->d_rowptr, g->d_colidx, n, nnz, copies,
@@ -827,7 +830,6 @@ int create_replicated(lgbc_graph* g, int64_t copies, lgbc_graph** out) {
     st->max_in = g->max_in;
     st->max_out = g->max_out;
     st->sigma_limit = g->sigma_limit;
-    LGBC_TRY(ensure_hubs(g));
     st->tune = g->tune;
     const HubTable& from = g->hubs;
     HubTable& to = st->hubs;
