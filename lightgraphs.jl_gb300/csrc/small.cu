@@ -6,8 +6,8 @@
 // of lanes set in it.  Here a block keeps one source's path counts, then its
 // dependencies, in shared memory (8 bytes per vertex) and walks every edge
 // once per sweep, so the random accesses never leave the SM.  What bounds it
-// is instruction issue: 64 % of the issue slots busy with 32 warps per SM
-// (ALU pipe 52 %), the rest barriers and fixed latencies; DRAM is idle.
+// is instruction issue: 62 % of the issue slots busy with 32 warps per SM
+// (ALU pipe 50 %), the rest barriers and fixed latencies; DRAM is idle.
 // Measured (exact betweenness, batches -> here): G(10,000, 50,000) 11.7 ->
 // 4.10 ms; 24 Barabasi-Albert graphs of up to 20,000 vertices 448 -> 150 ms;
 // a 50-vertex digraph 289 -> 36 us.
