@@ -69,3 +69,16 @@ def test_wide_distances_take_a_bounded_buffer():
     far = narrow == np.iinfo(np.int32).max
     assert far.any() and np.array_equal(far, wide == np.iinfo(np.int64).max)
     assert np.array_equal(narrow[~far], wide[~far])
+
+
+@pytest.mark.parametrize("n,k", [(20000, 64), (20000, 65), (20000, 150), (200000, 200)])
+def test_wide_tables_of_several_batches(n, k):
+    # 64-bit rows wait on the device until 2^25 of them (or the last) are copied:
+    # one batch, several in one copy, two copies
+    e = np.random.default_rng(n).integers(0, n, (2, 2 * n))
+    src = np.random.default_rng(k).choice(n, k, replace=False) + 1
+    narrow, wide = (lgbc.multi_gdistances(lgbc.SimpleGraph.from_edge_arrays(n, e[0], e[1], eltype=t), src)
+                    for t in (np.int32, np.int64))
+    far = narrow == np.iinfo(np.int32).max
+    assert wide.dtype == np.int64 and np.array_equal(far, wide == np.iinfo(np.int64).max)
+    assert np.array_equal(narrow[~far], wide[~far])
