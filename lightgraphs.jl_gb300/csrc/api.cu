@@ -2,6 +2,8 @@
 // host side of the level loops.  All arithmetic runs in the kernels of
 // msbfs.cu / bfs.cu / util.cu; there is no CPU fallback.  The other entry
 // points live in api_many.cu, api_learned.cu and api_more.cu.
+#include <numeric>
+
 #include "api_internal.h"
 
 using namespace lgbc;
@@ -1058,10 +1060,18 @@ bool small_applies(const lgbc_graph* g) {
 // A block walks every unfinished vertex's edges once a level: with 64 sources
 // or fewer (two blocks at most) the batches' whole grid catches up between
 // 0.43M entries (R-MAT 14: 391 against 399 us) and 0.9M (305 against 269 us);
-// 500 sources took 312 against 1,743 us there.
-bool small_bfs_applies(const lgbc_graph* g, int64_t nsrc) {
+// 500 sources took 312 against 1,743 us there.  A row of more than 64 entries
+// takes a warp and a round trip to L2 whatever its length: with 64 sources or
+// fewer, distance sums of G(4,000, 200,000) took 231 against 172 us, of
+// G(2,500, 87,500) 119 against 167; distances, for which the batches have less
+// to do, 202 against 135 us on G(4,000, 140,000), 122 against 138 on the latter.
+// With 65 sources it is 584 against 362 us on G(8,000, 400,000) and 292 against
+// 360 on G(4,000, 200,000).
+bool small_bfs_applies(const lgbc_graph* g, int64_t nsrc, bool rows) {
+  const int64_t walk = g->long_in + g->nnz / 256;
   return small_graph(g) && g->n <= g->small_bfs_max_n && nsrc <= INT32_MAX &&
-         (nsrc > kMaxLanes || g->nnz <= int64_t(1) << 19);
+         (nsrc > kMaxLanes || g->nnz <= int64_t(1) << 19) &&
+         (nsrc > kMaxLanes * 3 / 2 || walk <= (nsrc > kMaxLanes ? 8000 : rows ? 2800 : 4000));
 }
 
 // The plan of one of g's two CSRs (an undirected graph has one).
@@ -1362,10 +1372,10 @@ void degree_pass(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr)
   const int directed = g->directed;
   g->has_degree.assign(static_cast<size_t>(n), 0);
   uint8_t* has = g->has_degree.data();
-  std::vector<int64_t> max_in(8, 0), max_out(8, 0);
+  std::vector<int64_t> max_in(8, 0), max_out(8, 0), long_in(8, 0);
   std::vector<std::vector<std::pair<int64_t, int32_t>>> tops(8);  // max-heaps of (-degree, id)
   const int parts = parallel_parts(n, [&](int p, int64_t vb, int64_t ve) {
-    int64_t mi = 0, mo = 0;
+    int64_t mi = 0, mo = 0, li = 0;
     auto& top = tops[static_cast<size_t>(p)];
     for (int64_t v = vb; v < ve; ++v) {
       const int64_t dout = rowptr[v + 1] - rowptr[v];
@@ -1374,6 +1384,7 @@ void degree_pass(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr)
       has[v] = d > 0 ? 1 : 0;
       mi = std::max(mi, din);
       mo = std::max(mo, dout);
+      li += din > 4 * kSmallWarpGroups ? 1 : 0;
       if (d <= 0) continue;
       if (top.size() < static_cast<size_t>(kLandmarks)) {
         top.emplace_back(-d, static_cast<int32_t>(v));
@@ -1386,6 +1397,7 @@ void degree_pass(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr)
     }
     max_in[static_cast<size_t>(p)] = mi;
     max_out[static_cast<size_t>(p)] = mo;
+    long_in[static_cast<size_t>(p)] = li;
   });
   int64_t mi = 0;
   g->max_out = *std::max_element(max_out.begin(), max_out.end());
@@ -1395,6 +1407,7 @@ void degree_pass(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr)
     all.insert(all.end(), tops[static_cast<size_t>(p)].begin(), tops[static_cast<size_t>(p)].end());
   }
   g->max_in = mi;
+  g->long_in = std::accumulate(long_in.begin(), long_in.end(), int64_t(0));
   g->sigma_limit = ~0ull / static_cast<unsigned long long>(mi + 1);
   std::sort(all.begin(), all.end());
   g->landmarks.clear();
@@ -1631,7 +1644,7 @@ int gdistances(lgbc_graph* g, const int32_t* src, int64_t nsrc, void* dist_out, 
   LGBC_TRY(check_sources(g, src, nsrc));
   reset_stats(g);
   if (g->n == 0) return LGBC_OK;
-  const bool small = nsrc > 0 && small_bfs_applies(g, nsrc) && g->nnz <= kSmallSingleNnz;
+  const bool small = nsrc > 0 && small_bfs_applies(g, 1, true) && nsrc <= INT32_MAX && g->nnz <= kSmallSingleNnz;
   if (small) {
     SmallBfs run{};
     run.nsrc = static_cast<int>(nsrc);
@@ -1657,7 +1670,7 @@ int gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, void* dist
   if (nsrc > 0 && g->n > 0 && !dist_out) return fail(LGBC_EINVAL, "null output");
   reset_stats(g);
   if (nsrc == 0 || g->n == 0) return LGBC_OK;
-  if (small_bfs_applies(g, nsrc)) {
+  if (small_bfs_applies(g, nsrc, true)) {
     // at most 2^26 distances on the device at a time
     const int64_t rows = std::min<int64_t>(nsrc, std::max<int64_t>(kWarp, (int64_t(1) << 26) / g->n / kWarp * kWarp));
     for (int64_t s0 = 0; s0 < nsrc; s0 += rows) {

@@ -333,6 +333,7 @@ struct lgbc_graph {
   int64_t small_max_n = 0;          // largest graph of the per-source kernel on this device
   int64_t small_stress_max_n = 0, small_bfs_max_n = 0;  // and of the stress and distance kernels
   int64_t max_out = 0, max_in = 0;  // largest out- and in-list
+  int64_t long_in = 0;              // in-lists that the shared-memory kernels walk by warps
   int32_t* d_src = nullptr;         // device copy of a call's source list
   int64_t d_src_cap = 0;
   double* d_bc = nullptr;           // device result buffer for host-buffer calls
@@ -427,9 +428,9 @@ int init_handle(lgbc_graph* g, int64_t n, int directed);
 // from the device when the hub items need them).
 int finish_handle(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr,
                   const int32_t* colidx = nullptr, const int32_t* in_colidx = nullptr);
-// Whether the shared-memory distance kernel takes nsrc searches, and the call
-// (run: everything but the graph).
-bool small_bfs_applies(const lgbc_graph* g, int64_t nsrc);
+// Whether the shared-memory distance kernel takes nsrc searches (rows: whose
+// distances are wanted one by one), and the call (run: everything but the graph).
+bool small_bfs_applies(const lgbc_graph* g, int64_t nsrc, bool rows);
 int run_small_bfs(lgbc_graph* g, SmallBfs run);
 // Whether the per-source kernel takes Brandes calls of this handle, and such a
 // call: the k sources at src (device or pinned memory) into out (likewise); it

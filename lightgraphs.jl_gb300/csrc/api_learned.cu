@@ -85,7 +85,7 @@ int distance_stats(lgbc_graph* g, const int32_t* src, int64_t nsrc,
   dsum->assign(static_cast<size_t>(nsrc), 0ull);
   dmax->assign(static_cast<size_t>(nsrc), 0);
   if (nsrc == 0) return LGBC_OK;
-  const bool small = small_bfs_applies(g, nsrc);
+  const bool small = small_bfs_applies(g, nsrc, false);
   if (!small) LGBC_TRY(ensure_ms(g, false));
   if (nsrc > g->d_stats_cap) {
     dev_free(g->d_stats);

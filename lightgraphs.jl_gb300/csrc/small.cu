@@ -825,6 +825,8 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_sweeps(SmallRun r
 // paths: distance sums from all 3,000 vertices of G(3,000, 18,000) 11.6 ms ->
 // 82 us, one BFS on G(1,001, 5,003) 222 -> 29 us as a call.
 // ---------------------------------------------------------------------------
+// ROWS: distances are written (their code costs the statistics 10 % on long rows).
+template <bool ROWS>
 __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_bfs(SmallBfs run) {
   extern __shared__ uint32_t sm[];
   __shared__ unsigned long long s_cnt[kWarp], s_sum[kWarp];
@@ -843,8 +845,8 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_bfs(SmallBfs run)
   const int64_t row0 = static_cast<int64_t>(first) * n;
   int32_t* dist = run.dist ? run.dist + row0 : nullptr;
   long long* dist64 = run.dist64 ? run.dist64 + row0 : nullptr;
-  const bool put_dist = dist || dist64;
   auto put = [&](int64_t at, int32_t d) {
+    if (!ROWS) return;
     if (dist) dist[at] = d;
     if (dist64) dist64[at] = d == kUnreached ? INT64_MAX : static_cast<long long>(d);
   };
@@ -887,9 +889,12 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_bfs(SmallBfs run)
       if (ln == 0) {
         next[v] = got;
         if (got) vis[v] |= got;
-        if (got && put_dist) put_level(got, v);
       }
       fresh += (got >> ln) & 1u;
+      if (ROWS && got) {  // lane j: source j's row
+        const int own = G.orig[v];
+        if ((got >> ln) & 1u) put(static_cast<int64_t>(ln) * n + own, level);
+      }
     }
     for (int c = nw / kWarp + wid; c < nc; c += W) {
       const int v = c * kWarp + ln;
@@ -911,7 +916,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_bfs(SmallBfs run)
           fresh += __popc(warp_transpose32(got));
           if (got) {
             vis[v] |= got;
-            if (put_dist) put_level(got, v);
+            if (ROWS) put_level(got, v);
           }
         }
       }
@@ -925,7 +930,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads, 1) k_small_bfs(SmallBfs run)
     front = next;
     next = t;
   }
-  if (put_dist)
+  if (ROWS)
     for (int v = tid; v < n; v += T) {
       const int own = G.orig[v];
       for (uint32_t miss = full & ~vis[v]; miss; miss &= miss - 1u)
@@ -1054,9 +1059,10 @@ size_t small_bfs_smem(int64_t n) {
 
 int small_bfs_configure(size_t max_dyn_smem) {
   cudaFuncAttributes fa{};
-  if (cudaFuncGetAttributes(&fa, k_small_bfs) != cudaSuccess) return 0;
+  if (cudaFuncGetAttributes(&fa, k_small_bfs<true>) != cudaSuccess) return 0;
   const size_t room = max_dyn_smem > fa.sharedSizeBytes ? max_dyn_smem - fa.sharedSizeBytes : 0;
-  cudaFuncSetAttribute(k_small_bfs, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(room));
+  cudaFuncSetAttribute(k_small_bfs<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(room));
+  cudaFuncSetAttribute(k_small_bfs<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(room));
   int64_t n = std::min<int64_t>(kSmallMaxN, static_cast<int64_t>(room / 12));
   while (n > 0 && small_bfs_smem(n) > room) --n;
   return static_cast<int>(n);
@@ -1069,7 +1075,7 @@ int small_bfs(const LaunchCfg& c, cudaStream_t s, const SmallBfs& run, int64_t n
   per_sm = std::max<int64_t>(1, std::min<int64_t>(per_sm, (blocks + c.sms - 1) / c.sms));
   int threads = static_cast<int>(kSmallMaxThreads / per_sm);
   threads = std::max(64, std::min(threads, static_cast<int>((n + 31) & ~int64_t(31)))) & ~31;
-  k_small_bfs<<<blocks, threads, smem, s>>>(run);
+  (run.dist || run.dist64 ? k_small_bfs<true> : k_small_bfs<false>)<<<blocks, threads, smem, s>>>(run);
   return 1;
 }
 

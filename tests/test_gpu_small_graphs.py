@@ -259,3 +259,24 @@ def test_many_in_the_large_size_classes(endpoints):
     graphs = [G.barabasi_albert(n, 2, seed=n) for n in (8200, 10900, 11100, 12500)]
     for g, z in zip(graphs, lgbc.betweenness_centrality_many(graphs, normalize=False, endpoints=endpoints)):
         assert_bc_close(z, oracle_bc(g, normalize=False, endpoints=endpoints, nthreads=16))
+
+
+@pytest.mark.parametrize("n,degree,k,rows_small,stats_small", [
+    (1500, 100, 3, True, True), (2400, 40, 64, True, True), (3000, 80, 5, False, True),
+    (4000, 90, 64, False, False), (4000, 90, 65, True, True), (7000, 90, 96, False, False), (7000, 90, 97, True, True)])
+def test_distances_over_long_rows(n, degree, k, rows_small, stats_small):
+    # few searches of a graph of many rows of more than 64 entries run over the
+    # whole grid (and count levels), rows on both sides written by every lane
+    g = random_graph(n, n * degree // 2, n + degree)
+    rp, ci, _ = csr_args(g)
+    h = g.device_handle()
+    src = np.random.default_rng(k).choice(n, k, replace=False).astype(np.int32)
+    want = oracle.gdistances_many(rp, ci, src, nthreads=8).astype(np.int64)
+    far = want == oracle.UNREACHED32
+    assert np.array_equal(lgbc.multi_gdistances(g, src + 1), np.where(far, np.iinfo(g.eltype).max, want))
+    assert (h.stats()["levels"] == 0) == rows_small
+    reached, dsum, dmax = lgbc.distance.distance_stats(g, src)
+    assert (h.stats()["levels"] == 0) == stats_small
+    assert np.array_equal(reached, (~far).sum(1))
+    assert np.array_equal(dsum, np.where(far, 0, want).sum(1))
+    assert np.array_equal(dmax, np.where(far, 0, want).max(1))
