@@ -1689,9 +1689,11 @@ int gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, void* dist
   LGBC_TRY(ensure_ms(g, false));
   const int lanes = kMaxLanes;
   LGBC_TRY(ensure_dist(g, static_cast<int64_t>(lanes) * g->n));
-  // 64-bit rows that wait on the device for one copy
+  // short tables leave through the pinned result buffer, 64-bit rows of larger
+  // ones wait on the device for one copy
+  const bool direct = direct_dist(g, nsrc, wide);
   const int64_t batch = lanes * g->n;
-  const int64_t room = wide && batch <= kWidePiece ? std::min(nsrc * g->n, kWidePiece / batch * batch) : 0;
+  const int64_t room = wide && !direct && batch <= kWidePiece ? std::min(nsrc * g->n, kWidePiece / batch * batch) : 0;
   int64_t held = 0;
   if (room > 0) LGBC_TRY(ensure_wide(g, room));
   for (int64_t s0 = 0; s0 < nsrc; s0 += lanes) {
@@ -1699,8 +1701,10 @@ int gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, void* dist
     const int64_t count = nl * g->n;
     g->launches += fill_i32(g->cfg, g->stream, g->d_dist, count, kUnreached);
     LGBC_TRY(run_ms_batch(g, g->d_src + s0, nl, kSigmaNone, nullptr, g->d_dist, g->n));
-    if (room == 0) {
-      LGBC_TRY(copy_dist(g, dist_out, s0 * g->n, count, wide));
+    if (direct && wide) {
+      g->launches += widen_dist(g->cfg, g->stream, g->d_dist, count, reinterpret_cast<int64_t*>(g->h_out) + s0 * g->n);
+    } else if (room == 0) {
+      LGBC_TRY(copy_dist(g, direct ? g->h_out : dist_out, s0 * g->n, count, wide));
     } else {
       g->launches += widen_dist(g->cfg, g->stream, g->d_dist, count, g->d_wide + held);
       held += count;
@@ -1713,6 +1717,7 @@ int gdistances_batch(lgbc_graph* g, const int32_t* src, int64_t nsrc, void* dist
     g->stats.batches++;
   }
   LGBC_CUDA(cudaStreamSynchronize(g->stream));
+  take_direct(g, nsrc, dist_out, wide);
   finish_stats(g);
   return LGBC_OK;
 }

@@ -119,3 +119,19 @@ def test_unions_of_graphs_that_the_kernel_refuses(endpoints):
               gen.erdos_renyi_nm(24000, 12000, seed=1), gen.erdos_renyi_nm(23000, 9000, seed=2)]
     for g, z in zip(graphs, lgbc.betweenness_centrality_many(graphs, normalize=False, endpoints=endpoints)):
         assert_bc_close(z, oracle_bc(g, normalize=False, endpoints=endpoints, nthreads=16))
+
+
+@pytest.mark.parametrize("dtype", [np.int32, np.int64])
+@pytest.mark.parametrize("n,k", [(1, 1), (33, 70), (1000, 3), (1024, 8), (1025, 8), (2048, 8), (2049, 8), (127, 129)])
+def test_short_distance_tables(n, k, dtype):
+    # tables up to the 64 KB that leave through pinned memory, in both types
+    e = np.random.default_rng(n).integers(0, n, (2, 2 * n))
+    g = lgbc.SimpleGraph.from_edge_arrays(n, e[0], e[1], eltype=dtype)
+    rp, ci, _ = csr_args(g)
+    batches(g)
+    src = np.random.default_rng(k).integers(0, n, k).astype(np.int32)
+    want = oracle.gdistances_many(rp, ci, src).astype(np.int64)
+    want[want == oracle.UNREACHED32] = np.iinfo(dtype).max
+    for _ in range(2):
+        got = lgbc.multi_gdistances(g, src + 1)
+        assert got.dtype == dtype and np.array_equal(got, want)
