@@ -1057,6 +1057,23 @@ bool small_applies(const lgbc_graph* g) {
   return small_graph(g) && g->n <= g->small_max_n && !g->small.deep.given_up();
 }
 
+// Graphs of many sources that the batches still take faster.  Trees: with one
+// block per SM (n > 11,000) nothing hides the barriers of their many thin
+// levels (20,000 vertices by preferential attachment, all sources 29.9 against
+// 18.2 ms, 2,432 of them 3.8 against 4.5; 10,500 vertices 7.1 against 7.1; a star
+// of 17,000 5.4 against 7.5, of 20,000 12.8 against 9.5).  Nearly complete
+// graphs: a source with one missing neighbour walks every edge twice, where a
+// batch looks up the missing ones (1,000 vertices, 99.5 % of the edges, all
+// sources 1.92 against 0.96 ms, 300 of them 0.53 against 0.78; 90 % 1.68 against
+// 1.49; complete ones stop after one level, 0.06 against 0.35 ms at 600 vertices).
+bool batches_win(const lgbc_graph* g, int64_t k) {
+  const int64_t n = g->n, nnz = g->nnz;
+  if (g->directed) return false;
+  const bool tree = nnz <= 2 * n && 100 * g->linked >= 99 * n && (2 * g->max_out < n || n > 18000);
+  if (tree && n > 11000) return k >= 32 * static_cast<int64_t>(g->cfg.sms);
+  return n >= 800 && nnz < n * (n - 1) && 20 * nnz >= 19 * n * (n - 1) && k > 4 * static_cast<int64_t>(g->cfg.sms);
+}
+
 // A block walks every unfinished vertex's edges once a level: with 64 sources
 // or fewer (two blocks at most) the batches' whole grid catches up between
 // 0.43M entries (R-MAT 14: 391 against 399 us) and 0.9M (305 against 269 us);
@@ -1245,7 +1262,7 @@ int accumulate_active(lgbc_graph* g, int endpoints, double* bc_dev, double* host
     LGBC_CUDA(cudaStreamSynchronize(g->stream));
     return LGBC_OK;
   };
-  if (k > 0 && k <= INT32_MAX && small_applies(g) && !g->small.deep.among(g->h_active)) {
+  if (k > 0 && k <= INT32_MAX && small_applies(g) && !batches_win(g, k) && !g->small.deep.among(g->h_active)) {
     // A call of few sources and a short result moves both through pinned
     // memory that the kernels read and write themselves: two launches and one
     // wait (a 50-vertex graph 56 us with four copies and two waits, 35 us so).
@@ -1372,10 +1389,10 @@ void degree_pass(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr)
   const int directed = g->directed;
   g->has_degree.assign(static_cast<size_t>(n), 0);
   uint8_t* has = g->has_degree.data();
-  std::vector<int64_t> max_in(8, 0), max_out(8, 0), long_in(8, 0);
+  std::vector<int64_t> max_in(8, 0), max_out(8, 0), long_in(8, 0), linked(8, 0);
   std::vector<std::vector<std::pair<int64_t, int32_t>>> tops(8);  // max-heaps of (-degree, id)
   const int parts = parallel_parts(n, [&](int p, int64_t vb, int64_t ve) {
-    int64_t mi = 0, mo = 0, li = 0;
+    int64_t mi = 0, mo = 0, li = 0, lk = 0;
     auto& top = tops[static_cast<size_t>(p)];
     for (int64_t v = vb; v < ve; ++v) {
       const int64_t dout = rowptr[v + 1] - rowptr[v];
@@ -1386,6 +1403,7 @@ void degree_pass(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr)
       mo = std::max(mo, dout);
       li += din > 4 * kSmallWarpGroups ? 1 : 0;
       if (d <= 0) continue;
+      ++lk;
       if (top.size() < static_cast<size_t>(kLandmarks)) {
         top.emplace_back(-d, static_cast<int32_t>(v));
         std::push_heap(top.begin(), top.end());
@@ -1398,6 +1416,7 @@ void degree_pass(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr)
     max_in[static_cast<size_t>(p)] = mi;
     max_out[static_cast<size_t>(p)] = mo;
     long_in[static_cast<size_t>(p)] = li;
+    linked[static_cast<size_t>(p)] = lk;
   });
   int64_t mi = 0;
   g->max_out = *std::max_element(max_out.begin(), max_out.end());
@@ -1408,6 +1427,7 @@ void degree_pass(lgbc_graph* g, const int64_t* rowptr, const int64_t* in_rowptr)
   }
   g->max_in = mi;
   g->long_in = std::accumulate(long_in.begin(), long_in.end(), int64_t(0));
+  g->linked = std::accumulate(linked.begin(), linked.end(), int64_t(0));
   g->sigma_limit = ~0ull / static_cast<unsigned long long>(mi + 1);
   std::sort(all.begin(), all.end());
   g->landmarks.clear();

@@ -334,6 +334,7 @@ struct lgbc_graph {
   int64_t small_stress_max_n = 0, small_bfs_max_n = 0;  // and of the stress and distance kernels
   int64_t max_out = 0, max_in = 0;  // largest out- and in-list
   int64_t long_in = 0;              // in-lists that the shared-memory kernels walk by warps
+  int64_t linked = 0;               // vertices of degree > 0
   int32_t* d_src = nullptr;         // device copy of a call's source list
   int64_t d_src_cap = 0;
   double* d_bc = nullptr;           // device result buffer for host-buffer calls

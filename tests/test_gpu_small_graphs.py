@@ -280,3 +280,24 @@ def test_distances_over_long_rows(n, degree, k, rows_small, stats_small):
     assert np.array_equal(reached, (~far).sum(1))
     assert np.array_equal(dsum, np.where(far, 0, want).sum(1))
     assert np.array_equal(dmax, np.where(far, 0, want).max(1))
+
+
+def dense(n, share):
+    a, b = np.triu_indices(n, 1)
+    keep = np.random.default_rng(n).random(len(a)) < share
+    return lgbc.SimpleGraph.from_edge_arrays(n, a[keep], b[keep])
+
+
+@pytest.mark.parametrize("make,k,small", [
+    (lambda: G.barabasi_albert(11500, 1, seed=1), 4800, True), (lambda: G.barabasi_albert(11500, 1, seed=1), 5000, False),
+    (lambda: G.barabasi_albert(10900, 1, seed=2), 5000, True), (lambda: G.barabasi_albert(11500, 2, seed=3), 5000, True),
+    (lambda: lgbc.SimpleGraph.from_edge_arrays(11500, np.zeros(11499, int), np.arange(1, 11500)), 5000, True),
+    (lambda: random_graph(20000, 9000, 4), 5000, True),
+    (lambda: dense(800, 0.98), 600, True), (lambda: dense(800, 0.98), 700, False), (lambda: dense(800, 1.0), 700, True),
+    (lambda: dense(790, 0.98), 700, True), (lambda: dense(800, 0.93), 700, True)])
+def test_graphs_of_many_sources_that_batches_take(make, k, small):
+    # trees past one block per SM, nearly complete graphs, and what lies next to them
+    g = make()
+    src = np.random.default_rng(k).choice(g.nv(), k, replace=False)
+    check(g, src)
+    assert (g.device_handle().stats()["levels"] == 0) == small
