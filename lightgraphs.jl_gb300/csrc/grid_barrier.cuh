@@ -48,6 +48,12 @@ constexpr unsigned kBeatEntries = 4096;
 struct BarrierBeat {
   unsigned count = 0;
   __host__ __device__ __forceinline__ bool turn_due() { return (++count & (kBeatTurns - 1u)) == 0u; }
+  // A turn that counts for `units`.
+  __host__ __device__ __forceinline__ bool work_due(unsigned units) {
+    const unsigned before = count / kBeatTurns;
+    count += units;
+    return count / kBeatTurns != before;
+  }
   __host__ __device__ __forceinline__ bool entry_due() { return (++count & (kBeatEntries - 1u)) == 0u; }
 };
 

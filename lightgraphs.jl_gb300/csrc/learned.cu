@@ -101,6 +101,12 @@ __device__ __forceinline__ int core_entries(const DevGraph& g, int32_t v) {
   return d > kCoreCached ? kCoreCached + 1 : static_cast<int>(d);
 }
 
+// Turns that v's rows count for: a block or a warp walks 2^16 entries in some
+// hundred microseconds.
+__device__ __forceinline__ unsigned core_units(const DevGraph& g, int32_t v) {
+  return 1u + static_cast<unsigned>((g.rowptr[v + 1] - g.rowptr[v] + g.in_rowptr[v + 1] - g.in_rowptr[v]) >> 16);
+}
+
 // Entry j of v's out-list followed by its in-list (a digraph counts every arc
 // at both ends); -1 past the end.
 __device__ __forceinline__ int32_t core_entry(const DevGraph& g, int32_t v, int64_t o0, int64_t n0,
@@ -263,8 +269,8 @@ __device__ __forceinline__ void core_search_hubs(const DevGraph& g, const int32_
   __shared__ int s_h;
   const bool dir = is_digraph(g);
   for (unsigned long long i = blockIdx.x; i < nl; i += gridDim.x) {
-    beat_turn(bar, beat);
     const int32_t v = __ldcg(hubs + i);
+    if (beat.work_due(core_units(g, v)) && lane_id() == 0) beat_now(bar);
     const int32_t c = __ldcg(core + v);
     if (threadIdx.x == 0) atomicAnd(flag + (v >> 5), ~(1u << (v & 31)));
     const int cap = c < kCoreHist ? c : kCoreHist;
@@ -275,7 +281,6 @@ __device__ __forceinline__ void core_search_hubs(const DevGraph& g, const int32_
     // took 80 dependent round trips, 60 us, in every pass that searched it.
     auto bin_list = [&](const int32_t* ci, int64_t e0, int64_t e1) {
       for (int64_t b0 = e0 + (threadIdx.x & ~(kWarp - 1)); b0 < e1; b0 += kCoreAhead * static_cast<int64_t>(blockDim.x)) {
-        beat_turn(bar, beat);
         int bin[kCoreAhead];
 #pragma unroll
         for (int q = 0; q < kCoreAhead; ++q) {
@@ -361,13 +366,12 @@ __device__ __forceinline__ void core_list_neighbours(const DevGraph& g, const Co
                                                      int32_t v, int32_t lo, int32_t old, int first, int step,
                                                      BarrierBeat& beat) {
   const int ln = lane_id();
-  beat_turn(&r.state->barrier, beat);
+  if (beat.work_due(core_units(g, v)) && ln == 0) beat_now(&r.state->barrier);
   for (int side = 0; side < (is_digraph(g) ? 2 : 1); ++side) {
     const int64_t* rp = side ? g.in_rowptr : g.rowptr;
     const int32_t* ci = side ? g.in_colidx : g.colidx;
     const int64_t e1 = rp[v + 1];
     for (int64_t e = rp[v] + first * AHEAD * kWarp; e < e1; e += static_cast<int64_t>(step) * AHEAD * kWarp) {
-      beat_turn(&r.state->barrier, beat);
       int32_t u[AHEAD];
       bool ok[AHEAD];
 #pragma unroll

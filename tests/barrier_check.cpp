@@ -23,6 +23,8 @@ int main() {
   unsigned beats = 0;
   for (unsigned turn = 0; turn < 10 * kBeatTurns; ++turn) beats += turns.turn_due() ? 1u : 0u;
   for (unsigned entry = 0; entry < 10 * kBeatEntries; ++entry) beats += entries.entry_due() ? 1u : 0u;
+  BarrierBeat rows;  // units of 1 and of several beats' worth
+  for (unsigned row = 0; row < 10 * kBeatTurns; ++row) beats += rows.work_due(row % 8 == 0 ? 4 * kBeatTurns : 0u) ? 1u : 0u;
   std::printf("%u\n", beats);
   return 0;
 }
