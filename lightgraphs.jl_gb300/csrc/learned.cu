@@ -94,6 +94,8 @@ static_assert(kCoreCached == kCoreSlots * kWarp, "a warp's registers hold a row"
 constexpr int kCoreThread = 16;
 // Entries of a long row that a thread has in flight.
 constexpr int kCoreAhead = 8;
+// Lowered vertices per warp from which on their lanes list neighbours apart.
+constexpr int kCoreWide = 8;
 
 __device__ __forceinline__ int core_entries(const DevGraph& g, int32_t v) {
   int64_t d = g.rowptr[v + 1] - g.rowptr[v];
@@ -390,6 +392,38 @@ __device__ __forceinline__ void core_list_neighbours(const DevGraph& g, const Co
   }
 }
 
+// The neighbours of nl lowered vertices, for long logs: 32 at a time, those of at
+// most kCoreThread entries by their own lane, so that an append serves 32 of
+// them (one append for each was 1.4 ms of 5 on a random graph of 4M vertices);
+// the others one at a time by the warp.
+__device__ __forceinline__ void core_list_many(const DevGraph& g, const CoreRun& r, CoreSlot* nxt, int parity,
+                                               unsigned long long nl, BarrierBeat& beat) {
+  const int ln = lane_id();
+  for (unsigned long long base = static_cast<unsigned long long>(gwarp()) * kWarp; base < nl;
+       base += static_cast<unsigned long long>(nwarps()) * kWarp) {
+    beat_turn(&r.state->barrier, beat);
+    const bool in = base + ln < nl;
+    const int32_t v = in ? __ldcg(r.log_v + base + ln) : 0;
+    const int32_t old = in ? __ldcg(r.log_old + base + ln) : 0;
+    const int32_t lo = in ? __ldcg(r.core + v) : 0;
+    const int ent = in ? core_entries(g, v) : 0;
+    const int mine = ent <= kCoreThread ? ent : 0;
+    const int64_t o0 = in ? g.rowptr[v] : 0;
+    const int64_t n0 = in ? g.rowptr[v + 1] - o0 : 0;
+    const int most = static_cast<int>(__reduce_max_sync(kFull, static_cast<unsigned>(mine)));
+    for (int k = 0; k < most; ++k) {
+      const int32_t u = k < mine ? core_entry(g, v, o0, n0, k) : -1;
+      const int32_t cu = u >= 0 && u != v ? __ldcg(r.core + u) : lo;
+      core_list(g, r, nxt, parity, cu > lo && cu <= old, u);
+    }
+    for (unsigned rest = __ballot_sync(kFull, ent > kCoreThread); rest; rest &= rest - 1u) {
+      const int j = __ffs(rest) - 1;
+      core_list_neighbours<2>(g, r, nxt, parity, __shfl_sync(kFull, v, j), __shfl_sync(kFull, lo, j),
+                              __shfl_sync(kFull, old, j), 0, 1, beat);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(256) k_core_run(DevGraph g, CoreRun r) {
   __shared__ int s_ok;
   __shared__ unsigned long long s_n[4];  // read and written a grid barrier apart
@@ -442,10 +476,13 @@ __global__ void __launch_bounds__(256) k_core_run(DevGraph g, CoreRun r) {
       const int32_t v = __ldcg(r.hub_v + i);
       core_list_neighbours<kCoreAhead>(g, r, nxt, to, v, __ldcg(r.core + v), __ldcg(r.hub_old + i), wid, wpb, beat);
     }
-    for (unsigned long long i = gwarp(); i < nl; i += nwarps()) {
-      const int32_t v = __ldcg(r.log_v + i);
-      core_list_neighbours<2>(g, r, nxt, to, v, __ldcg(r.core + v), __ldcg(r.log_old + i), 0, 1, beat);
-    }
+    if (nl >= kCoreWide * static_cast<unsigned long long>(nwarps()))
+      core_list_many(g, r, nxt, to, nl, beat);
+    else
+      for (unsigned long long i = gwarp(); i < nl; i += nwarps()) {
+        const int32_t v = __ldcg(r.log_v + i);
+        core_list_neighbours<2>(g, r, nxt, to, v, __ldcg(r.core + v), __ldcg(r.log_old + i), 0, 1, beat);
+      }
     if (!grid_barrier(&st->barrier, goal, &s_ok)) return;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) st->passes = pass;

@@ -345,3 +345,19 @@ def test_core_numbers_and_features_at_row_lengths(degree):
     # a lane adds degree / 32 terms one after the other, then five pairs
     rtol = (degree / 32 + 8) * 2.0**-24 + 4 * 2.0**-24
     np.testing.assert_allclose(lgbc.features(g), oracle.features(rp, ci), rtol=rtol, atol=rtol)
+
+
+@pytest.mark.parametrize("directed", [False, True])
+@pytest.mark.parametrize("n,m", [(60000, 240000), (150000, 300000), (150000, 2400000)])
+def test_core_numbers_of_long_logs(n, m, directed):
+    # so many vertices lowered in a pass that lanes list their neighbours apart:
+    # rows on both sides of the 16 entries that a lane takes, with hubs
+    rng = np.random.default_rng(n + m)
+    e = rng.integers(0, n, (2, m))
+    hub = np.stack([np.repeat(np.arange(3), 2000), rng.integers(3, n, 6000)])
+    e = np.concatenate([e, hub], 1)
+    e = e[:, e[0] != e[1]]
+    g = (lgbc.SimpleDiGraph if directed else lgbc.SimpleGraph).from_edge_arrays(n, e[0], e[1])
+    from conftest import csr_args
+    rp, ci, kw = csr_args(g)
+    np.testing.assert_array_equal(lgbc.core_number(g), oracle.core_number(rp, ci, **kw))

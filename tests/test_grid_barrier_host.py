@@ -57,4 +57,4 @@ def test_loops_between_barriers_beat():
     run = run[:run.index("\n}\n")]
     assert run.count("beat_turn(") >= 2 and "entry_due()) beat_now(" in run
     core = open(os.path.join(CSRC, "learned.cu")).read()
-    assert core.count("beat_turn(") >= 4 and core.count("work_due(core_units(g, v))") == 2
+    assert core.count("beat_turn(") >= 5 and core.count("work_due(core_units(g, v))") == 2
