@@ -73,3 +73,23 @@ def test_known_answers_and_measures():
         lgbc.eccentricity(lgbc.SimpleGraph.from_edges(3, [(1, 2)]))
     with pytest.raises(lgbc.MethodError):
         lgbc.closeness_centrality(g, np.ones((5, 5)))
+
+
+@pytest.mark.parametrize("directed", [False, True])
+def test_statistics_of_large_sparse_graphs(directed):
+    # more vertices than two units of 32 for every warp, odd, with hubs
+    n = 700001
+    rng = np.random.default_rng(8)
+    e = np.concatenate([rng.integers(0, n, (2, 1200000)),
+                        np.stack([np.repeat([5, 6], 3000), rng.integers(0, n, 6000)])], 1)
+    g = (lgbc.SimpleDiGraph if directed else lgbc.SimpleGraph).from_edge_arrays(n, e[0], e[1], eltype=np.int32)
+    rp, ci = g.csr()
+    for k in (1, 3):
+        src = rng.integers(0, n, k).astype(np.int32)
+        want = oracle.gdistances_many(rp, ci, src, nthreads=3).astype(np.int64)
+        far = want == oracle.UNREACHED32
+        reached, dsum, dmax = lgbc.distance.distance_stats(g, src)
+        assert np.array_equal(reached, (~far).sum(1))
+        assert np.array_equal(dsum, np.where(far, 0, want).sum(1))
+        assert np.array_equal(dmax, np.where(far, 0, want).max(1))
+        assert np.array_equal(lgbc.multi_gdistances(g, src + 1), np.where(far, np.iinfo(np.int32).max, want))
