@@ -175,10 +175,12 @@ int lgbc_graph_stats(const lgbc_graph *g, lgbc_stats *out);
  * of a graph whose vertex state fits one SM's shared memory (about 22,300
  * vertices, at most 2^20 stored entries) runs one thread block per source
  * instead, unless the call has a source that reaches a vertex at a distance of
- * 128 or more or by 2^48 paths or more; lgbc_stats.batches then counts the
- * blocks' shares of the sources, and no levels are counted.
+ * 128 or more or by 2^48 paths or more, or batches were measured faster (many
+ * sources of a tree or of a nearly complete graph); lgbc_stats.batches then
+ * counts the blocks' shares of the sources, and no levels are counted.
  * Distances and distance statistics of such graphs (about 18,900 vertices)
- * run 32 sources per thread block in the same way.
+ * run 32 sources per thread block in the same way, unless the call has few
+ * sources and the graph many rows of more than 64 entries.
  *   alpha, beta   direction switch: go bottom-up when the frontier's edges
  *                 exceed (unvisited edges)/alpha; return top-down when the
  *                 frontier has fewer than n/beta vertices.
